@@ -526,30 +526,54 @@ rope_row_norm_kernel(const TI* __restrict__ qkv, int row_stride, int in_splits, 
 // The same for bfloat16 rows and gains whose heads, turned part and pitches come in steps of 8 elements: 16-byte loads and
 // stores, eight neighbouring elements a thread.  An element's partner is read from the row in shared memory, and the two
 // products of a turn are rounded apart as in rotate_pair, so an element gets the bits that the kernel above gives it
-// from the same sums of squares (the sums themselves are added up in another order here; a model always runs one of the two).
-__global__ void __launch_bounds__(256)
-rope_row_norm_vec_kernel(const bf16* __restrict__ qkv, int row_stride, bf16* __restrict__ q_out, int q_stride,
+// from the same sums of squares (the sums themselves are added up in another order here).
+// TI float: the row comes as 32-bit slabs.  Then a token's whole row, values too, is summed into shared memory first, four
+// neighbouring columns a thread with all slabs' loads in flight: a decoded token's 3,072 columns came in twelve rounds of 4-byte loads
+// before.  Measured: 24.6 us a launch of 8 tokens before; see sandwich_norm_vec_kernel for the step.
+template <typename TI>
+__global__ void __launch_bounds__(sizeof(TI) == 4 ? 768 : 256)
+rope_row_norm_vec_kernel(const TI* __restrict__ qkv, int row_stride, int in_splits, size_t in_split_stride, bf16* __restrict__ q_out, int q_stride,
                          const int* __restrict__ positions, const int* __restrict__ slots, const float* __restrict__ inv_freq,
                          bf16* __restrict__ k_pages, bf16* __restrict__ v_pages, int nq, int nkv, int hd, int rot_dim,
                          int page_size, int interleaved, int vd, const bf16* __restrict__ wq, const bf16* __restrict__ wk,
                          int q_count, int k_count, float eps, const float* __restrict__ bias, float* __restrict__ v_first,
                          const float* __restrict__ lam, int mix_mode, float turn_scale) {
-    extern __shared__ float row[];            // [(nq + nkv) * hd] the token's q and k parts, [half] sines, [half] cosines
+    extern __shared__ __align__(16) float row[];      // [(nq + nkv) * hd] the token's q and k parts, (slabs: [nkv * vd] its values,) [half] sines, [half] cosines
     __shared__ float scratch[32];
+    constexpr bool SLABS = sizeof(TI) == 4;
     pdl_launch_dependents();
     const int t = blockIdx.x;
     const int slot = slots ? slots[t] : -1;
     const float pos = (float)positions[t];
-    const int half = rot_dim >> 1, qw = nq * hd, kw = nkv * hd;
-    float* sn = row + qw + kw;
+    const int half = rot_dim >> 1, qw = nq * hd, kw = nkv * hd, vw = nkv * vd;
+    float* sn = row + qw + kw + (SLABS ? vw : 0);
     float* cs = sn + half;
     for (int j = threadIdx.x; j < half; j += blockDim.x) {
         sincosf(pos * inv_freq[j], &sn[j], &cs[j]);
         if (turn_scale != 1.0f) { sn[j] *= turn_scale; cs[j] *= turn_scale; }
     }
     pdl_wait();
-    const bf16* x = qkv + (size_t)t * row_stride;
+    const TI* x = qkv + (size_t)t * row_stride;
     float ssq = 0.f, ssk = 0.f;
+    if constexpr (SLABS) {
+        const int columns = slot < 0 ? qw + kw : qw + kw + vw;
+        for (int c0 = threadIdx.x * 4; c0 < columns; c0 += blockDim.x * 4) {
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int sp = 0; sp < in_splits; sp += 8) {          // part 0 + part 1 + ... in order; eight loads are in flight at a time
+                float4 part[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+                    if (sp + u < in_splits) part[u] = *reinterpret_cast<const float4*>(x + (size_t)(sp + u) * in_split_stride + c0);
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+                    if (sp + u < in_splits) { v.x += part[u].x; v.y += part[u].y; v.z += part[u].z; v.w += part[u].w; }
+            }
+            if (bias) { v.x += bias[c0]; v.y += bias[c0 + 1]; v.z += bias[c0 + 2]; v.w += bias[c0 + 3]; }    // joins the finished sum
+            *reinterpret_cast<float4*>(row + c0) = v;
+            const float ss = v.x * v.x + v.y * v.y + (v.z * v.z + v.w * v.w);
+            if (c0 < qw) ssq += ss; else if (c0 < qw + kw) ssk += ss;          // qw and kw are multiples of 8: a group lies in one part
+        }
+    } else
     for (int c0 = threadIdx.x * 8; c0 < qw + kw; c0 += blockDim.x * 8) {
         const uint4 raw = *reinterpret_cast<const uint4*>(x + c0);
         const __nv_bfloat162* p2 = reinterpret_cast<const __nv_bfloat162*>(&raw);
@@ -604,7 +628,20 @@ rope_row_norm_vec_kernel(const bf16* __restrict__ qkv, int row_stride, bf16* __r
     const float l = mix_mode == 2 ? lam[0] : 0.f;
     for (int item = threadIdx.x; item < nkv * v_per; item += blockDim.x) {
         const int kvh = item / v_per, c0 = (item % v_per) * 8;
-        uint4 raw = *reinterpret_cast<const uint4*>(x + qw + kw + kvh * vd + c0);
+        uint4 raw;
+        if constexpr (SLABS) {
+            __nv_bfloat162* h2 = reinterpret_cast<__nv_bfloat162*>(&raw);
+            const float* src = row + qw + kw + kvh * vd + c0;
+            float* keep = v_first + (size_t)t * vw + kvh * vd + c0;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                float2 v = make_float2(src[2 * e], src[2 * e + 1]);
+                if (mix_mode == 1) { keep[2 * e] = v.x; keep[2 * e + 1] = v.y; }
+                else if (mix_mode == 2) { v.x = fmaf(l, keep[2 * e], (1.0f - l) * v.x); v.y = fmaf(l, keep[2 * e + 1], (1.0f - l) * v.y); }
+                h2[e] = __floats2bfloat162_rn(v.x, v.y);
+            }
+        } else {
+        raw = *reinterpret_cast<const uint4*>(x + qw + kw + kvh * vd + c0);
         if (bias != nullptr || mix_mode != 0) {
             // as in the kernel above: the bias, then the values left for later layers (unrounded) or blended with an earlier layer's
             __nv_bfloat162* h2 = reinterpret_cast<__nv_bfloat162*>(&raw);
@@ -617,6 +654,7 @@ rope_row_norm_vec_kernel(const bf16* __restrict__ qkv, int row_stride, bf16* __r
                 else if (mix_mode == 2) { v.x = fmaf(l, keep[2 * e], (1.0f - l) * v.x); v.y = fmaf(l, keep[2 * e + 1], (1.0f - l) * v.y); }
                 h2[e] = __floats2bfloat162_rn(v.x, v.y);
             }
+        }
         }
         *reinterpret_cast<uint4*>(v_pages + (((size_t)(slot / page_size) * nkv + kvh) * page_size + slot % page_size) * vd + c0) = raw;
     }
@@ -652,18 +690,26 @@ WLLM_API int wllm_rope_row_norm_kv_write(const void* qkv, int in_dtype, int row_
             rot_dim, page_size, interleaved, vd, wq, wk, w_dtype, q_count, k_count, eps, bias, v_first, lam, mix_mode, turn_scale); \
     } while (0)
     const bool aligned = !(((uintptr_t)qkv | (uintptr_t)q_out | (uintptr_t)k_pages | (uintptr_t)v_pages | (uintptr_t)wq | (uintptr_t)wk) & 15);
-    if (in_dtype == WLLM_BF16 && out_dtype == WLLM_BF16 && w_dtype == WLLM_BF16 && in_splits == 1 && aligned && hd % 8 == 0 &&
-        vd % 8 == 0 && rot_dim % 8 == 0 && row_stride % 8 == 0 && q_stride % 8 == 0) {
-        static bool raised = false;
-        if (!raised && smem > 48 * 1024) {
-            const cudaError_t e = cudaFuncSetAttribute(rope_row_norm_vec_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-            if (e != cudaSuccess) return 1000 + (int)e;
-            raised = true;
-        }
-        return wllm_launch(rope_row_norm_vec_kernel, n, 256, smem, stream, (const bf16*)qkv, row_stride, (bf16*)q_out, q_stride,
-                           positions, slots, inv_freq, (bf16*)k_pages, (bf16*)v_pages, nq, nkv, hd, rot_dim, page_size, interleaved,
-                           vd, (const bf16*)wq, (const bf16*)wk, q_count, k_count, eps, bias, v_first, lam, mix_mode, turn_scale);
+    const bool eights = out_dtype == WLLM_BF16 && w_dtype == WLLM_BF16 && aligned && hd % 8 == 0 && vd % 8 == 0 && rot_dim % 8 == 0 && q_stride % 8 == 0;
+#define RV(TI, THREADS, SMEM) do { \
+        static bool raised = false; \
+        if (!raised && SMEM > 48 * 1024) { \
+            const cudaError_t e = cudaFuncSetAttribute(rope_row_norm_vec_kernel<TI>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); \
+            if (e != cudaSuccess) return 1000 + (int)e; \
+            raised = true; \
+        } \
+        return wllm_launch(rope_row_norm_vec_kernel<TI>, n, THREADS, SMEM, stream, (const TI*)qkv, row_stride, in_splits, (size_t)in_split_stride, \
+                           (bf16*)q_out, q_stride, positions, slots, inv_freq, (bf16*)k_pages, (bf16*)v_pages, nq, nkv, hd, rot_dim, page_size, \
+                           interleaved, vd, (const bf16*)wq, (const bf16*)wk, q_count, k_count, eps, bias, v_first, lam, mix_mode, turn_scale); \
+    } while (0)
+    if (eights && in_dtype == WLLM_BF16 && in_splits == 1 && row_stride % 8 == 0) RV(bf16, 256, smem);
+    // slabs, or a row that a 32-bit product left whole: the values lie in shared memory too
+    const size_t smem_v = smem + (size_t)nkv * vd * sizeof(float);
+    if (eights && in_dtype == WLLM_F32 && row_stride % 4 == 0 && in_split_stride % 4 == 0 && smem_v <= 200 * 1024) {
+        const int groups = (nq * hd + nkv * (hd + vd)) / 4, threads = groups >= 768 ? 768 : (groups > 256 ? (groups + 31) / 32 * 32 : 256);
+        RV(float, threads, smem_v);
     }
+#undef RV
     if (in_dtype == WLLM_BF16 && out_dtype == WLLM_BF16) RN(bf16, bf16);
     if (in_dtype == WLLM_F32 && out_dtype == WLLM_BF16) RN(float, bf16);
     if (in_dtype == WLLM_F32 && out_dtype == WLLM_F32) RN(float, float);
