@@ -1,0 +1,64 @@
+"""The delta rule in blocks of tokens, beside the walk token by token and the recurrence in 64 bits."""
+from __future__ import annotations
+
+import pytest
+import torch
+
+DEV = "cuda:0"
+pytestmark = pytest.mark.gpu
+
+
+def _plain(q, k, v, beta, g, S):
+    """q, k [n, H, D], v [n, H, V], beta [n, H], g [n, H, D or 1], S [H, D, V]; 64 bits."""
+    out = []
+    for t in range(q.shape[0]):
+        S = S * g[t][:, :, None]
+        u = beta[t][:, None] * (v[t] - torch.einsum("hdv,hd->hv", S, k[t]))
+        S = S + k[t][:, :, None] * u[:, None, :]
+        out.append(torch.einsum("hdv,hd->hv", S, q[t]))
+    return torch.stack(out), S
+
+
+# lengths around a block and the first length that is walked in blocks, beside requests that are not; a long one
+@pytest.mark.parametrize("lens", [[16], [1, 23, 15, 17, 1], [24, 0, 200]])
+@pytest.mark.parametrize("sizes", [(2, 1, 8, 5), (3, 3, 72, 16), (4, 2, 128, 128), (1, 1, 256, 33)])      # channels a thread; ragged columns
+@pytest.mark.parametrize("memory", ["short", "long", "mixed"])                                           # decays near 0, near 1, both
+@pytest.mark.parametrize("channel", [False, True])
+def test_blocks_of_tokens_give_the_recurrence(lens, sizes, memory, channel):
+    from wllm_b200.kernels import ops
+    H, G, D, V = sizes
+    gen = torch.Generator().manual_seed(sum(lens) * 7 + D + channel)
+    n, R = sum(lens), len(lens)
+    unit = lambda x: x / x.norm(dim=-1, keepdim=True)
+    q, k = unit(torch.randn(n, G, D, generator=gen)) * D ** -0.5, unit(torch.randn(n, G, D, generator=gen) + 0.3)
+    v, beta = torch.randn(n, H, V, generator=gen), torch.rand(n, H, generator=gen)
+    lo, hi = {"short": (0.5, 40.0), "long": (1e-4, 1e-2), "mixed": (1e-4, 40.0)}[memory]
+    x = torch.rand(n, H, D if channel else 1, generator=gen)
+    rate = lo * (hi / lo) ** x.double()
+    decay = (torch.expm1(-rate) if channel else torch.exp(-rate)[..., 0]).float()
+    g = (1 + decay.double()) if channel else decay.double()[..., None]
+    starts = [sum(lens[:i]) for i in range(R)]
+    slots = [(2 * i + 1) % (2 * R) for i in range(R)]
+    state = torch.randn(2 * R, H, D, V, generator=gen)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    rep = H // G
+    want = state.double().clone()
+    want_o = torch.zeros(n, H, V, dtype=torch.float64)
+    for s0, m, slot in zip(starts, lens, slots):
+        if m:
+            part = slice(s0, s0 + m)
+            want_o[part], want[slot] = _plain(q[part].double().repeat_interleave(rep, 1), k[part].double().repeat_interleave(rep, 1), v[part].double(),
+                                              beta[part].double(), g[part], state[slot].double())
+    d = lambda x: x.reshape(x.shape[0], -1).contiguous().to(DEV)
+    errors = {}
+    for way in ("walk", "blocks"):
+        S, o = state.clone().to(DEV), torch.full((n, H * V), float("nan"), device=DEV)
+        scratch = torch.full((ops.delta_block_floats(n, R, H, D),), float("nan"), device=DEV) if way == "blocks" else None
+        ops.delta_scan(d(q), d(k), d(v), d(beta), d(decay), S, o, i32(starts), i32(lens), i32(slots), H, G, D, V, channel, scratch, max(lens))
+        err_o = (o.cpu().double().view(n, H, V) - want_o).norm() / want_o.norm()
+        err_s = (S.cpu().double() - want).norm() / want.norm()
+        errors[way] = float(err_o), float(err_s)
+    # 32-bit sums over D channels and eight tokens: some 2^-24 sqrt(D) of the result, and no further off than token by token by more
+    # than the scatter of such sums
+    for a, b in zip(errors["walk"], errors["blocks"]):
+        assert b < 2e-6 and b < 1.5 * a + 1e-7, errors

@@ -24,6 +24,7 @@
 //                           u = beta (v - g a) and o = g b + u (k . q), which is S^T q of the state that already holds the token's update.
 //                           Decays per key channel come as g - 1 (a channel that forgets slowly has g close to one, and the rounding of g
 //                           itself would grow with its memory): the lane's channels are decayed first, S + (g - 1) S, then summed.
+//   wllm_delta_blocks       the same recurrence for portions of a bfloat16 model, eight tokens at a time (see delta_block_prepare_kernel).
 #include "common.cuh"
 
 __device__ __forceinline__ float dr_any(const void* p, int dtype, size_t i) {
@@ -197,7 +198,7 @@ __global__ void __launch_bounds__(THREADS)
 delta_scan_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
                   const float* __restrict__ beta, const float* __restrict__ decay, float* __restrict__ state,
                   float* __restrict__ out, const int* __restrict__ req_q_start, const int* __restrict__ req_q_len,
-                  const int* __restrict__ req_slot, int H, int G, int D, int V) {
+                  const int* __restrict__ req_slot, int H, int G, int D, int V, int below) {
     constexpr int DP = LPC * NE;                        // channels of a row in shared memory
     constexpr int DR_COLS = THREADS / LPC;              // value columns of the CTA
     // two stages of [TT][DP] q, [TT][DP] k, (CHANNEL: [TT][DP] decay,) [TT][16] v, [TT] beta, [TT] decay; [TT] k.q
@@ -206,7 +207,7 @@ delta_scan_kernel(const float* __restrict__ q, const float* __restrict__ k, cons
     pdl_begin();
     const int r = blockIdx.z, h = blockIdx.y;
     const int len = req_q_len[r], slot = req_slot[r];
-    if (len <= 0 || slot < 0) return;                      // a request that brings no token
+    if (len <= 0 || slot < 0 || len >= below) return;      // a request that brings no token, or one that is walked in blocks
     const int g = h / (H / G), t0 = req_q_start[r];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = lane & (LPC - 1);
     const int col0 = blockIdx.x * DR_COLS, mine = threadIdx.x / LPC, col = col0 + mine;
@@ -358,10 +359,10 @@ WLLM_API int wllm_delta_conv_update(const void* fused, int in_dtype, int row_str
 }
 
 // state [slots, H, D, V]; out [n, H, V].  Requests by start, length and state slot; a length of 0 or a slot of -1 is passed by.
-// decay [n, H], or (channel) [n, H, D] as g - 1.
+// decay [n, H], or (channel) [n, H, D] as g - 1.  Requests of `below` tokens or more are passed by (wllm_delta_blocks takes them).
 WLLM_API int wllm_delta_scan(const float* q, const float* k, const float* v, const float* beta, const float* decay, int channel, float* state,
                              float* out, const int* req_q_start, const int* req_q_len, const int* req_slot, int requests, int H,
-                             int G, int D, int V, cudaStream_t stream) {
+                             int G, int D, int V, int below, cudaStream_t stream) {
     if (requests <= 0) return WLLM_OK;
     if (H <= 0 || H > 65535 || G <= 0 || H % G != 0 || requests > 65535 || D <= 0 || D > 256 || V <= 0) return WLLM_BAD_SIZE;
     // heads of up to 32 channels: eight lanes a column, four channels each; above: sixteen lanes, 4, 8 or 16 channels each
@@ -378,7 +379,7 @@ WLLM_API int wllm_delta_scan(const float* q, const float* k, const float* v, con
         raised = true;
     }
 #define SCAN2(NE, LPC, TH, C) wllm_launch(delta_scan_kernel<NE, LPC, TH, C>, grid, TH, smem, stream, q, k, v, beta, decay, state, out, \
-                                          req_q_start, req_q_len, req_slot, H, G, D, V)
+                                          req_q_start, req_q_len, req_slot, H, G, D, V, below)
 #define SCAN(NE, LPC, TH) (channel ? SCAN2(NE, LPC, TH, true) : SCAN2(NE, LPC, TH, false))
     if (D <= 32) return SCAN(4, 8, DR_THREADS);
     if (D <= 64) return SCAN(4, 16, DR_THREADS);
@@ -386,4 +387,331 @@ WLLM_API int wllm_delta_scan(const float* q, const float* k, const float* v, con
     return SCAN(16, 16, DR_THREADS);
 #undef SCAN
 #undef SCAN2
+}
+
+// ---------------------------------------------------------------------------------------------------
+// The recurrence in blocks of eight tokens.  The walk above is bound by its chain: every token's state waits for two sums over a
+// column's lanes of the state before it, some 600 cycles a token while the arithmetic fills a tenth of them.  Over a block that starts from S
+// everything but S and the values can be worked out beforehand.  With G_i the product of the decays of tokens 0 .. i,
+// A_ij = k_i . (G_i / G_j) k_j for j < i, P_ij = q_i . (G_i / G_j) k_j for j <= i, and T = (1 + diag(beta) A)^-1 diag(beta):
+//
+//     r_i = v_i - (G_i k_i)^T S;    o_i = (G_i q_i)^T S + sum_j N_ij r_j,  N = P T;    S <- G_7 S + sum_j M_j r_j^T,  M_j = sum_l T_lj (G_7 / G_l) k_l
+//
+// so that a block costs one pass over S for sixteen sums, one exchange, and one pass that updates it.  All of it in 32 bits.  The
+// ratios G_i / G_j are running products from token j + 1 on (no quotients, nothing overflows however fast a channel forgets), and
+// decays given as g - 1 stay so: G_7 - 1 is carried and S + (G_7 - 1) S taken.
+//
+//   prepare   a CTA per (block, head, request), a thread a key channel: the 28 + 36 sums over the channels by a transposing tree (a warp's 64
+//             values meet in 62 exchanges instead of 320), T by substitution, and the block's matrices in one contiguous piece.
+//   walk      a CTA of eight warps has 16 columns of one (request, head), a warp two; a lane holds a thirty-second of the key channels of both,
+//             in pairs (two products an instruction).  The 32 sums of a block and warp meet in 31 exchanges.  Shared memory bounds it: a row's
+//             16-byte loads take four wavefronts a warp whether its lanes' addresses differ or not, so all 32 lanes lie along the channels.
+//             (Four warps of four columns each, sixteen lanes a column: one warp a scheduler waits out its loads and exchanges, 354 us where this
+//             form takes 267.)
+//             Blocks arrive through a ring of cp.async stages.  The grid seldom exceeds the device's SMs, and a kernel that is
+//             launched early finds some SMs still full: it asks for more than half an SM's shared memory then, so that its CTAs do
+//             not pile up in pairs (the walk above took 1,490 us for 682 that way in a 2,048-token prompt of 16 heads of 128 x 128).
+// Measured, 16 heads of 128 x 128: 2,048 tokens with a decay per channel 682 us by the walk above when it has the device to itself and 1,490 us in a
+// step, 267 us here (the whole step 2,879 -> 1,704 us); prompts of 340, 680 and 1,021 tokens together 551 -> 264 us (2,026 -> 1,792 us).
+// Portions of fewer than two blocks stay on the walk above, and so do 32-bit models, whose results do not depend on how a prompt is cut.
+// ---------------------------------------------------------------------------------------------------
+constexpr int DB = 8;                 // tokens of a block
+constexpr int DB_COLS = 16, DB_THREADS = 256;
+constexpr int DB_GROUP = 2, DB_STAGES = 3;       // blocks of a stage (the warps meet once a stage and drift apart inside it); stages
+__host__ __device__ constexpr int db_channels(int D) { return D <= 64 ? 64 : (D <= 128 ? 128 : 256); }
+// a block's piece: [8][DP] G k, [8][DP] G q, [8][DP] M, [DP] G_7 - 1 (or G_7), [8][8] N
+__host__ __device__ constexpr int db_floats(int DP) { return (3 * DB + 1) * DP + DB * DB; }
+__host__ __device__ constexpr int db_stage_floats(int DP) { return db_floats(DP) + DB * DB_COLS; }      // with the values of the CTA's columns
+// where a request's blocks begin: t0 / 8 + r grows by at least its number of blocks from one request to the next
+__device__ __forceinline__ size_t db_first(int t0, int r) { return (size_t)(t0 / DB + r); }
+
+template <int DP, bool CHANNEL>
+__global__ void __launch_bounds__(DP)
+delta_block_prepare_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ beta, const float* __restrict__ decay,
+                           float* __restrict__ blocks, const int* __restrict__ req_q_start, const int* __restrict__ req_q_len,
+                           const int* __restrict__ req_slot, int H, int G, int D, int from) {
+    constexpr int WARPS = DP / 32, PAIRS = DB * (DB - 1) / 2;         // sums: 28 of A, then 36 of P
+    __shared__ float sums[WARPS][64], A[DB][DB], P[DB][DB], T[DB][DB], bt[DB];
+    pdl_begin();
+    const int r = blockIdx.z, h = blockIdx.y, len = req_q_len[r];
+    if (len < from || req_slot[r] < 0 || blockIdx.x * DB >= (unsigned)len) return;
+    const int t0 = req_q_start[r], first = t0 + blockIdx.x * DB, count = min(DB, len - (int)blockIdx.x * DB), g = h / (H / G);
+    const int d = threadIdx.x, warp = d >> 5, lane = d & 31;
+    float kk[DB], qq[DB], e[DB];
+#pragma unroll
+    for (int i = 0; i < DB; ++i) {             // tokens past the portion's end: no key, no query, no step, no decay
+        const bool in = i < count && d < D;
+        const size_t at = ((size_t)(first + i) * G + g) * D + d;
+        kk[i] = in ? k[at] : 0.f;
+        qq[i] = in ? q[at] : 0.f;
+        if (CHANNEL) e[i] = in ? decay[((size_t)(first + i) * H + h) * D + d] : 0.f;
+        else e[i] = i < count ? decay[(size_t)(first + i) * H + h] : 1.f;
+    }
+    if (d < DB) bt[d] = d < count ? beta[(size_t)(first + d) * H + h] : 0.f;
+    auto decayed = [&](float x, int i) { return CHANNEL ? fmaf(e[i], x, x) : e[i] * x; };
+    float* piece = blocks + ((db_first(t0, r) + blockIdx.x) * H + h) * db_floats(DP);
+    float x[64], last[DB];                      // last[j] = (G_7 / G_j) k_j
+#pragma unroll
+    for (int j = 0; j < DB; ++j) {
+        float w = kk[j];
+        x[PAIRS + j * (j + 1) / 2 + j] = qq[j] * w;
+#pragma unroll
+        for (int i = j + 1; i < DB; ++i) {
+            w = decayed(w, i);
+            x[i * (i - 1) / 2 + j] = kk[i] * w;
+            x[PAIRS + i * (i + 1) / 2 + j] = qq[i] * w;
+        }
+        last[j] = w;
+    }
+    float E = CHANNEL ? 0.f : 1.f;               // G_i - 1, or G_i
+#pragma unroll
+    for (int i = 0; i < DB; ++i) {
+        E = CHANNEL ? fmaf(e[i], E, E) + e[i] : e[i] * E;
+        piece[i * DP + d] = CHANNEL ? fmaf(E, kk[i], kk[i]) : E * kk[i];
+        piece[(DB + i) * DP + d] = CHANNEL ? fmaf(E, qq[i], qq[i]) : E * qq[i];
+    }
+    piece[3 * DB * DP + d] = E;
+    // 64 values over 32 lanes: each exchange halves the values a lane keeps; lane l ends with values 2 l' and 2 l' + 1, l' = l
+#pragma unroll
+    for (int half = 32, off = 16; off > 0; half >>= 1, off >>= 1) {
+        const bool upper = lane & off;
+#pragma unroll
+        for (int i = 0; i < 32; ++i)
+            if (i < half) {
+                const float keep = upper ? x[i + half] : x[i], send = upper ? x[i] : x[i + half];
+                x[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+            }
+    }
+    sums[warp][2 * lane] = x[0];
+    sums[warp][2 * lane + 1] = x[1];
+    __syncthreads();
+    if (d < 64) {
+        float v = sums[0][d];
+#pragma unroll
+        for (int w = 1; w < WARPS; ++w) v += sums[w][d];
+        int at = d < PAIRS ? d : d - PAIRS, i = d < PAIRS ? 1 : 0;
+        const int width = d < PAIRS ? 0 : 1;       // row i of A holds i sums, of P i + 1
+        while (at >= i + width) { at -= i + width; ++i; }
+        (d < PAIRS ? A : P)[i][at] = v;
+    }
+    __syncthreads();
+    if (d < DB) {                                // column d of T
+        float t[DB];
+#pragma unroll
+        for (int i = 0; i < DB; ++i) {
+            float v = i == d ? 1.f : 0.f;
+#pragma unroll
+            for (int j = 0; j < DB; ++j)
+                if (j < i && j >= d) v = fmaf(-A[i][j], t[j], v);
+            t[i] = i >= d ? bt[i] * v : 0.f;
+            T[i][d] = t[i];
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int l = 0; l < DB; ++l) {
+        float m = 0.f;
+#pragma unroll
+        for (int j = l; j < DB; ++j) m = fmaf(T[j][l], last[j], m);
+        piece[(2 * DB + l) * DP + d] = m;
+    }
+    if (d < 64) {
+        const int i = d >> 3, l = d & 7;
+        float v = 0.f;
+        for (int j = l; j <= i; ++j) v = fmaf(P[i][j], T[j][l], v);
+        piece[(3 * DB + 1) * DP + d] = v;
+    }
+}
+
+__device__ __forceinline__ float2 dr_fma2(float2 a, float2 b, float2 c) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)),
+        "l"(*reinterpret_cast<unsigned long long*>(&c)));
+    return *reinterpret_cast<float2*>(&d);
+}
+__device__ __forceinline__ float2 dr_mul2(float2 a, float2 b) { return make_float2(a.x * b.x, a.y * b.y); }
+
+// channels of a lane: 4 lane + 128 j + 0 .. 3 (two: 2 lane, 2 lane + 1), as pairs
+template <int NP>
+__device__ __forceinline__ void db_row(const float* row, int lane, float2 (&w)[NP]) {
+    if constexpr (NP == 1) w[0] = *reinterpret_cast<const float2*>(row + 2 * lane);
+    else {
+#pragma unroll
+        for (int j = 0; j < NP / 2; ++j) {
+            const float4 t = *reinterpret_cast<const float4*>(row + 4 * lane + 128 * j);
+            w[2 * j] = make_float2(t.x, t.y);
+            w[2 * j + 1] = make_float2(t.z, t.w);
+        }
+    }
+}
+template <int NP>
+__device__ __forceinline__ int db_channel(int lane, int p) { return NP == 1 ? 2 * lane : 4 * lane + 128 * (p >> 1) + 2 * (p & 1); }
+
+template <int DP, bool CHANNEL>
+__global__ void __launch_bounds__(DB_THREADS)
+delta_block_walk_kernel(const float* __restrict__ blocks, const float* __restrict__ v, float* __restrict__ state, float* __restrict__ out,
+                        const int* __restrict__ req_q_start, const int* __restrict__ req_q_len, const int* __restrict__ req_slot, int H,
+                        int D, int V, int from) {
+    constexpr int FLOATS = db_floats(DP), STAGE = db_stage_floats(DP), NP = DP / 64;        // NP pairs of channels a thread and column
+    extern __shared__ __align__(16) float db_smem[];                         // [DB_STAGES][DB_GROUP][STAGE]: a block's piece, [8][16] values
+    __shared__ __align__(16) float rs[DB_THREADS / 32][2 * DB];
+    pdl_begin();
+    const int r = blockIdx.z, h = blockIdx.y;
+    const int len = req_q_len[r], slot = req_slot[r];
+    if (len < from || slot < 0) return;
+    const int t0 = req_q_start[r], count = (len + DB - 1) / DB;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int col0 = blockIdx.x * DB_COLS, col = col0 + 2 * warp;            // this warp's columns: col, col + 1
+    const float* src = blocks + (db_first(t0, r) * H + h) * FLOATS;
+    auto load = [&](int group) {
+#pragma unroll
+        for (int u = 0; u < DB_GROUP; ++u) {
+            const int b = group * DB_GROUP + u;
+            if (b >= count) break;
+            const float* piece = src + (size_t)b * H * FLOATS;
+            float* to = db_smem + ((group % DB_STAGES) * DB_GROUP + u) * STAGE;
+            for (int i = threadIdx.x * 4; i < FLOATS; i += DB_THREADS * 4) dr_cp16(to + i, piece + i);
+            if (threadIdx.x < DB * DB_COLS) {      // (places outside the portion or the head repeat its last token or column, and reach nothing)
+                const int t = min(b * DB + (int)threadIdx.x / DB_COLS, len - 1), c = min(col0 + (int)threadIdx.x % DB_COLS, V - 1);
+                dr_cp4(to + FLOATS + threadIdx.x, v + ((size_t)(t0 + t) * H + h) * V + c);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");                 // (an empty group keeps the count of groups)
+    };
+    for (int a = 0; a < DB_STAGES - 1; ++a) load(a);
+    float2 S[2][NP];
+    float* Sg = state + (((size_t)slot * H + h) * D) * V;
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+        const int c = db_channel<NP>(lane, p);
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+            const bool in = col + m < V;
+            S[m][p].x = in && c < D ? Sg[(size_t)c * V + col + m] : 0.f;
+            S[m][p].y = in && c + 1 < D ? Sg[(size_t)(c + 1) * V + col + m] : 0.f;
+        }
+    }
+    // lane 8 m + i ends with the sum behind r_i of column m, lane 16 + 8 m + i with that behind its output
+    const int tok = lane & 7, mine = (lane >> 3) & 1;
+    for (int b = 0; b < count; ++b) {
+        const int group = b / DB_GROUP;
+        if (b % DB_GROUP == 0) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(DB_STAGES - 2) : "memory");
+            __syncthreads();                    // the stage is here for everyone, and the one before is read to its end
+            load(group + DB_STAGES - 1);        // into the stage before
+        }
+        const float* K = db_smem + ((group % DB_STAGES) * DB_GROUP + b % DB_GROUP) * STAGE;
+        const float* M = K + 2 * DB * DP;
+        const float* E = M + DB * DP;
+        const float* N = E + DP;
+        const float vt = K[FLOATS + tok * DB_COLS + 2 * warp + mine];
+        float x[32];
+#pragma unroll
+        for (int i = 0; i < 2 * DB; ++i) {      // rows of G k, then of G q
+            float2 w[NP], acc[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+            db_row<NP>(K + i * DP, lane, w);
+#pragma unroll
+            for (int p = 0; p < NP; ++p) {
+                acc[0] = dr_fma2(w[p], S[0][p], acc[0]);
+                acc[1] = dr_fma2(w[p], S[1][p], acc[1]);
+            }
+            x[(i & 8) * 2 + (i & 7)] = acc[0].x + acc[0].y;
+            x[(i & 8) * 2 + 8 + (i & 7)] = acc[1].x + acc[1].y;
+        }
+        // 32 sums over 32 lanes in 31 exchanges: lane l ends with sum l
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) {
+            const bool upper = lane & off;
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+                if (i < off) {
+                    const float keep = upper ? x[i + off] : x[i], send = upper ? x[i] : x[i + off];
+                    x[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+                }
+        }
+        if (lane < 16) rs[warp][lane] = vt - x[0];
+        __syncwarp();
+        float rj[2][DB];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) *reinterpret_cast<float4*>(&rj[u >> 1][4 * (u & 1)]) = *reinterpret_cast<const float4*>(&rs[warp][4 * u]);
+        if (lane >= 16 && b * DB + tok < len && col + mine < V) {
+            float nr[DB], o = x[0];
+            *reinterpret_cast<float4*>(nr) = *reinterpret_cast<const float4*>(N + tok * DB);
+            *reinterpret_cast<float4*>(nr + 4) = *reinterpret_cast<const float4*>(N + tok * DB + 4);
+#pragma unroll
+            for (int j = 0; j < DB; ++j) o = fmaf(nr[j], mine ? rj[1][j] : rj[0][j], o);
+            out[((size_t)(t0 + b * DB + tok) * H + h) * V + col + mine] = o;
+        }
+        __syncwarp();                           // r is read to its end before the next block's takes its place
+        float2 e[NP];
+        db_row<NP>(E, lane, e);
+#pragma unroll
+        for (int p = 0; p < NP; ++p)
+#pragma unroll
+            for (int m = 0; m < 2; ++m) S[m][p] = CHANNEL ? dr_fma2(e[p], S[m][p], S[m][p]) : dr_mul2(e[p], S[m][p]);
+#pragma unroll
+        for (int l = 0; l < DB; ++l) {
+            float2 w[NP];
+            db_row<NP>(M + l * DP, lane, w);
+#pragma unroll
+            for (int p = 0; p < NP; ++p)
+#pragma unroll
+                for (int m = 0; m < 2; ++m) S[m][p] = dr_fma2(w[p], make_float2(rj[m][l], rj[m][l]), S[m][p]);
+        }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+        const int c = db_channel<NP>(lane, p);
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+            if (col + m >= V) continue;
+            if (c < D) Sg[(size_t)c * V + col + m] = S[m][p].x;
+            if (c + 1 < D) Sg[(size_t)(c + 1) * V + col + m] = S[m][p].y;
+        }
+    }
+}
+
+// Floats of scratch that wllm_delta_blocks needs for n tokens of `requests` requests.
+WLLM_API long long wllm_delta_block_floats(int n, int requests, int H, int D) {
+    return ((long long)n / DB + requests + 1) * H * db_floats(db_channels(D));
+}
+
+template <int DP, bool CHANNEL>
+static int launch_blocks(const float* q, const float* k, const float* v, const float* beta, const float* decay, float* state, float* out,
+                         float* blocks, const int* req_q_start, const int* req_q_len, const int* req_slot, int requests, int max_len, int H,
+                         int G, int D, int V, int from, int sms, cudaStream_t stream) {
+    const int code = wllm_launch(delta_block_prepare_kernel<DP, CHANNEL>, dim3((max_len + DB - 1) / DB, H, requests), DP, 0, stream, q, k, beta, decay,
+                                 blocks, req_q_start, req_q_len, req_slot, H, G, D, from);
+    if (code != WLLM_OK) return code;
+    const dim3 grid((V + DB_COLS - 1) / DB_COLS, H, requests);
+    constexpr size_t stage = (size_t)db_stage_floats(DP) * sizeof(float);      // 7,168, 13,568 or 26,368 bytes
+    static bool raised = false;
+    if (!raised) {
+        const cudaError_t e = cudaFuncSetAttribute(delta_block_walk_kernel<DP, CHANNEL>, cudaFuncAttributeMaxDynamicSharedMemorySize, 176 * 1024);
+        if (e != cudaSuccess) return 1000 + (int)e;
+        raised = true;
+    }
+    size_t smem = DB_STAGES * DB_GROUP * stage;          // 42, 80 or 155 KB
+    const size_t least = ((long long)grid.x * grid.y * grid.z <= sms ? 120 : 80) * 1024;       // at most one CTA an SM, or two
+    if (smem < least) smem = least;
+    return wllm_launch(delta_block_walk_kernel<DP, CHANNEL>, grid, DB_THREADS, smem, stream, (const float*)blocks, v, state, out, req_q_start,
+                       req_q_len, req_slot, H, D, V, from);
+}
+
+// wllm_delta_scan for the requests of `from` tokens or more (the longest has max_len); blocks: scratch of wllm_delta_block_floats floats,
+// 16-byte aligned; sms: the device's multiprocessors.
+WLLM_API int wllm_delta_blocks(const float* q, const float* k, const float* v, const float* beta, const float* decay, int channel, float* state,
+                               float* out, float* blocks, const int* req_q_start, const int* req_q_len, const int* req_slot, int requests,
+                               int max_len, int H, int G, int D, int V, int from, int sms, cudaStream_t stream) {
+    if (requests <= 0 || max_len < from) return WLLM_OK;
+    if (H <= 0 || H > 65535 || G <= 0 || H % G != 0 || requests > 65535 || D <= 0 || D > 256 || V <= 0 || from < 1) return WLLM_BAD_SIZE;
+    if ((uintptr_t)blocks & 15) return WLLM_BAD_ALIGN;
+#define BLOCKS2(DP, C) launch_blocks<DP, C>(q, k, v, beta, decay, state, out, blocks, req_q_start, req_q_len, req_slot, requests, max_len, H, G, \
+                                            D, V, from, sms, stream)
+#define BLOCKS(DP) (channel ? BLOCKS2(DP, true) : BLOCKS2(DP, false))
+    const int DP = db_channels(D);
+    return DP == 64 ? BLOCKS(64) : (DP == 128 ? BLOCKS(128) : BLOCKS(256));
+#undef BLOCKS
+#undef BLOCKS2
 }

@@ -1254,23 +1254,45 @@ def delta_conv_update(fused, parts: int, offsets: dict, heads: int, kv_heads: in
                                       _ptr(conv_state), _stream()), "delta_conv_update")
 
 
+DELTA_BLOCKS_FROM = 16      # portions of at least two blocks of eight tokens are walked block by block (csrc/delta_rule.cu)
+
+
+def delta_block_floats(n: int, requests: int, heads: int, dim: int) -> int:
+    """Scratch of `delta_scan` for portions walked in blocks, in floats."""
+    fn = load_family("delta_rule").wllm_delta_block_floats
+    fn.restype = ctypes.c_longlong
+    return int(fn(n, requests, heads, dim))
+
+
 def delta_scan(q, k, v, beta, decay, state, out, req_q_start, req_q_len, req_slot, heads: int, kv_heads: int, dim: int, vdim: int,
-               channel: bool = False):
+               channel: bool = False, blocks: torch.Tensor | None = None, max_q_len: int = 0):
     """The gated delta rule over every request's tokens of the step, in order, from and to its state slot:
     S <- decay S; u = beta (v - S^T k); S <- S + k u^T; out = S^T q.  q, k [n, kv_heads * dim], v, out [n, heads * vdim],
     beta, decay [n, heads], state [slots, heads, dim, vdim], all float32 (csrc/delta_rule.cu).  `channel`: decay
-    [n, heads * dim], one per key channel, given as decay - 1 (lowrank_map)."""
-    _need_cuda(q, k, v, beta, decay, state, out, req_q_start, req_q_len, req_slot)
+    [n, heads * dim], one per key channel, given as decay - 1 (lowrank_map).  `blocks` (float32 scratch of delta_block_floats; the
+    longest request has max_q_len tokens): requests of DELTA_BLOCKS_FROM tokens or more are walked in blocks
+    of eight tokens, whose sums run in another order."""
+    _need_cuda(q, k, v, beta, decay, state, out, req_q_start, req_q_len, req_slot, blocks)
     n = q.shape[0]
     assert all(t.dtype == torch.float32 and t.is_contiguous() for t in (q, k, v, beta, decay, state, out))
     assert q.shape == k.shape == (n, kv_heads * dim) and v.shape == out.shape == (n, heads * vdim) and beta.shape == (n, heads)
     assert decay.shape == (n, heads * dim if channel else heads)
     assert state.shape[1:] == (heads, dim, vdim)
     lib = load_family("delta_rule")
+    R, below = req_q_len.shape[0], 2 ** 31 - 1
+    index = (_ptr(_int32(req_q_start, "req_q_start")), _ptr(_int32(req_q_len, "req_q_len")), _ptr(_int32(req_slot, "req_slot")))
+    name = f"delta_scan(heads={heads}/{kv_heads}, dim={dim}/{vdim})"
+    if blocks is not None and max_q_len >= DELTA_BLOCKS_FROM:
+        assert blocks.dtype == torch.float32 and blocks.is_contiguous() and blocks.numel() >= delta_block_floats(n, R, heads, dim)
+        _check(lib.wllm_delta_blocks(_ptr(q), _ptr(k), _ptr(v), _ptr(beta), _ptr(decay), 1 if channel else 0, _ptr(state), _ptr(out),
+                                     _ptr(blocks), *index, R, max_q_len, heads, kv_heads, dim, vdim, DELTA_BLOCKS_FROM, sm_count(), _stream()), name)
+        global launches
+        launches += 1         # the blocks' matrices, then the walk
+        if R == 1:
+            return out
+        below = DELTA_BLOCKS_FROM
     _check(lib.wllm_delta_scan(_ptr(q), _ptr(k), _ptr(v), _ptr(beta), _ptr(decay), 1 if channel else 0, _ptr(state), _ptr(out),
-                               _ptr(_int32(req_q_start, "req_q_start")), _ptr(_int32(req_q_len, "req_q_len")),
-                               _ptr(_int32(req_slot, "req_slot")), req_q_len.shape[0], heads, kv_heads, dim, vdim, _stream()),
-           f"delta_scan(heads={heads}/{kv_heads}, dim={dim}/{vdim})")
+                               *index, R, heads, kv_heads, dim, vdim, below, _stream()), name)
     return out
 
 

@@ -330,8 +330,12 @@ class DeltaRule:
         if channel:
             ops.lowrank_map(fused, parts, off["a_low"], self.decay_up, H, D, decay, self.dt_bias, self.a_log)
         o = ctx.buffer(self.tag + "delta_o", (n, H * V), f32)
+        # portions of a bfloat16 model in blocks of tokens; a 32-bit model's walk gives the same bits however a prompt is cut
+        blocks = None
+        if self.model_dtype == torch.bfloat16 and ctx.max_q_len >= ops.DELTA_BLOCKS_FROM:
+            blocks = ctx.buffer(self.tag + "delta_blocks", (ops.delta_block_floats(n, ctx.n_requests, H, D),), f32)
         ops.delta_scan(q, k, v, beta, decay, ctx.state(cache.state_names["state"]), o, ctx.req_q_start, ctx.req_q_len, ctx.req_slot,
-                       H, G, D, V, channel)
+                       H, G, D, V, channel, blocks, ctx.max_q_len)
         gated = ctx.buffer(self.tag + "delta_gated", (n, H * V), self.model_dtype)
         if self.gate_maps is None:
             ops.head_gate_norm(o, fused, parts, off["g"], self.norm_weight, self.eps, gated, H, V)
