@@ -62,3 +62,40 @@ def test_blocks_of_tokens_give_the_recurrence(lens, sizes, memory, channel):
     # than the scatter of such sums
     for a, b in zip(errors["walk"], errors["blocks"]):
         assert b < 2e-6 and b < 1.5 * a + 1e-7, errors
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("sizes", [(2, 1, 8, 5), (4, 2, 128, 128), (1, 1, 200, 256)])       # a part of a warp's lanes; all of them; two rounds
+@pytest.mark.parametrize("lens", [[64], [3, 61, 1], [130, 7]])                             # runs that end in the middle and hold several requests
+def test_runs_of_tokens_are_prepared_as_one_by_one(lens, sizes, dtype):
+    """A step of 64 tokens or more takes the kernel that walks runs; the same requests in portions of at most 31 tokens do not: the same bits."""
+    from wllm_b200.kernels import ops
+    H, G, D, V = sizes
+    gen = torch.Generator().manual_seed(sum(lens) + D)
+    n, R, C, T = sum(lens), len(lens), 2 * G * D + H * V, 4
+    off = {"q": 0, "k": G * D, "v": 2 * G * D, "b": C, "a": C + H}
+    fused = torch.randn(n, C + 2 * H + 3, generator=gen).to(dtype).to(DEV)
+    taps = [torch.randn(c, T, generator=gen).to(dtype).to(DEV) for c in (G * D, G * D, H * V)]
+    a_log, dt_bias = (torch.randn(H, generator=gen).to(dtype).to(DEV) for _ in range(2))
+    starts = [sum(lens[:i]) for i in range(R)]
+    conv0 = torch.randn(R, T - 1, C, generator=gen)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+
+    def run(pieces):
+        """pieces: [(request, from, to)] lists, one a step; the outputs of all tokens."""
+        conv, res = conv0.clone().to(DEV), [torch.empty(n, w, device=DEV) for w in (G * D, G * D, H * V, H, H)]
+        for step in pieces:
+            rows = torch.cat([torch.arange(starts[r] + a, starts[r] + b) for r, a, b in step]).to(DEV)
+            x, m = fused[rows].contiguous(), [b - a for _, a, b in step]
+            at = [sum(m[:i]) for i in range(len(m))]
+            req = torch.cat([torch.full((c,), i, dtype=torch.int32) for i, c in enumerate(m)]).to(DEV)
+            part = [torch.empty(sum(m), t.shape[1], device=DEV) for t in res]
+            slots = i32([r for r, _, _ in step])
+            ops.delta_prepare(x, 0, off, H, G, D, V, T, *taps, a_log, dt_bias, req, i32(at), slots, conv, 1e-6, D ** -0.5, *part)
+            ops.delta_conv_update(x, 0, off, H, G, D, V, T, i32(at), i32(m), slots, conv)
+            for t, p in zip(res, part):
+                t[rows] = p
+        return res + [conv]
+    whole = run([[(r, 0, m) for r, m in enumerate(lens)]])
+    cut = run([[(r, a, min(a + 31, m))] for r, m in enumerate(lens) for a in range(0, m, 31)])
+    assert all(torch.equal(a, b) for a, b in zip(whole, cut))

@@ -112,6 +112,99 @@ delta_prepare_kernel(const void* __restrict__ fused, int in_dtype, int row_strid
     }
 }
 
+// The same for many tokens, inputs in one tensor, convolutions of four taps: a warp takes a head of DR_RUN neighbouring tokens, so that a channel's
+// taps and every input are read once a run instead of once a token and tap (a request that begins inside the run reads its first inputs'
+// predecessors from the state as above).  Lanes, sums and their order are those of the kernel above: the bits are the same.
+// Measured: 2,048 tokens, 48 heads of 128 channels, 166 us alone before; the whole step 1,704 -> 1,620 us (2,041 tokens, 24 heads: 1,792 -> 1,735).
+constexpr int DR_RUN = 8, DR_RUN_TAPS = 4;
+template <typename TI, int PER>
+__global__ void __launch_bounds__(128)
+delta_prepare_run_kernel(const TI* __restrict__ fused, int row_stride, int q_off, int k_off, int v_off, int b_off, int a_off, int n, int H, int G,
+                         int D, int V, const void* __restrict__ conv_q, const void* __restrict__ conv_k, const void* __restrict__ conv_v,
+                         const void* __restrict__ a_log, const void* __restrict__ dt_bias, int w_dtype, const int* __restrict__ token_req,
+                         const int* __restrict__ req_q_start, const int* __restrict__ req_slot, const float* __restrict__ conv_state,
+                         float unit_eps, float q_scale, float* __restrict__ q, float* __restrict__ k, float* __restrict__ v,
+                         float* __restrict__ beta, float* __restrict__ decay) {
+    constexpr int TAPS = DR_RUN_TAPS;
+    pdl_launch_dependents();
+    const int first = blockIdx.x * DR_RUN, count = min(DR_RUN, n - first), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int unit = blockIdx.y * 4 + warp;
+    if (unit > 2 * G + H) return;
+    if (unit == 2 * G + H) {
+        pdl_wait();
+        for (int i = lane; i < count * H; i += 32) {
+            const int t = first + i / H, h = i % H;
+            beta[(size_t)t * H + h] = 1.0f / (1.0f + expf(-to_f32(fused[(size_t)t * row_stride + b_off + h])));
+            if (a_off < 0) continue;
+            const float az = to_f32(fused[(size_t)t * row_stride + a_off + h]);
+            decay[(size_t)t * H + h] = expf(-expf(dr_any(a_log, w_dtype, h)) * dr_softplus(az + dr_any(dt_bias, w_dtype, h)));
+        }
+        return;
+    }
+    const int C = 2 * G * D + H * V;
+    int col0, chan0, size, head;
+    const void* w;
+    if (unit < G) { head = unit; size = D; col0 = q_off + head * D; chan0 = head * D; w = conv_q; }
+    else if (unit < 2 * G) { head = unit - G; size = D; col0 = k_off + head * D; chan0 = G * D + head * D; w = conv_k; }
+    else { head = unit - 2 * G; size = V; col0 = v_off + head * V; chan0 = 2 * G * D + head * V; w = conv_v; }
+    float taps[PER][TAPS];                       // written by no kernel: read while the predecessor still runs
+#pragma unroll
+    for (int e = 0; e < PER; ++e)
+#pragma unroll
+        for (int j = 0; j < TAPS; ++j)
+            taps[e][j] = lane + 32 * e < size ? dr_any(w, w_dtype, (size_t)(head * size + lane + 32 * e) * TAPS + j) : 0.f;
+    pdl_wait();
+    float x[DR_RUN][PER];
+#pragma unroll
+    for (int i = 0; i < DR_RUN; ++i)
+#pragma unroll
+        for (int e = 0; e < PER; ++e)
+            x[i][e] = i < count && lane + 32 * e < size ? to_f32(fused[(size_t)(first + i) * row_stride + col0 + lane + 32 * e]) : 0.f;
+    float* dst = unit < G ? q + (size_t)head * D : (unit < 2 * G ? k + (size_t)head * D : v + (size_t)head * V);
+    const size_t pitch = unit < 2 * G ? (size_t)G * D : (size_t)H * V;
+    float back[TAPS - 1][PER];                   // the inputs of the TAPS - 1 tokens in front, the oldest first
+    int r_before = -1;
+#pragma unroll
+    for (int i = 0; i < DR_RUN; ++i) {
+        if (i >= count) break;
+        const int t = first + i, r = token_req[t];
+        if (r != r_before) {                     // the run's first token, or a request's
+            const int at = t - req_q_start[r], slot = req_slot[r];
+#pragma unroll
+            for (int j = 1; j < TAPS; ++j)
+#pragma unroll
+                for (int e = 0; e < PER; ++e) {
+                    const int c = lane + 32 * e;
+                    float y = 0.f;
+                    if (c < size) {
+                        if (at - j >= 0) y = to_f32(fused[(size_t)(t - j) * row_stride + col0 + c]);
+                        else if (slot >= 0) y = conv_state[((size_t)slot * (TAPS - 1) + (TAPS - 1 + at - j)) * C + chan0 + c];
+                    }
+                    back[TAPS - 1 - j][e] = y;
+                }
+            r_before = r;
+        }
+        float y[PER], ss = 0.f;
+#pragma unroll
+        for (int e = 0; e < PER; ++e) {
+            float acc = 0.f;
+#pragma unroll
+            for (int j = 0; j < TAPS - 1; ++j) acc = fmaf(taps[e][j], back[j][e], acc);
+            acc = fmaf(taps[e][TAPS - 1], x[i][e], acc);
+            y[e] = lane + 32 * e < size ? dr_silu(acc) : 0.f;
+            ss = fmaf(y[e], y[e], ss);
+#pragma unroll
+            for (int j = 0; j + 1 < TAPS - 1; ++j) back[j][e] = back[j + 1][e];
+            back[TAPS - 2][e] = x[i][e];
+        }
+        float inv = 1.f;
+        if (unit < 2 * G) inv = (1.0f / sqrtf(warp_sum(ss) + unit_eps)) * (unit < G ? q_scale : 1.0f);
+#pragma unroll
+        for (int e = 0; e < PER; ++e)
+            if (lane + 32 * e < size) dst[(size_t)t * pitch + lane + 32 * e] = unit < 2 * G ? y[e] * inv : y[e];
+    }
+}
+
 // grid (requests, ceil(C / 256)): a thread a channel; the taps - 1 inputs that end at the request's last token of this step
 __global__ void __launch_bounds__(256)
 delta_conv_update_kernel(const void* __restrict__ fused, int in_dtype, int row_stride, int parts, size_t part_stride, int q_off,
@@ -341,6 +434,17 @@ WLLM_API int wllm_delta_prepare(const void* fused, int in_dtype, int row_stride,
     if ((in_dtype != WLLM_BF16 && in_dtype != WLLM_F32) || (w_dtype != WLLM_BF16 && w_dtype != WLLM_F32)) return WLLM_BAD_DTYPE;
     const int units = 2 * G + H + 1;
     if ((units + 3) / 4 > 65535) return WLLM_BAD_SIZE;
+    // runs from 64 tokens on: fewer are latency-bound either way, and single tokens also bring the slots' inputs up to date
+    if (n >= 64 && parts == 1 && taps == DR_RUN_TAPS && !shift) {
+        const dim3 rgrid((n + DR_RUN - 1) / DR_RUN, (units + 3) / 4);
+#define RUN(TI, PER) wllm_launch(delta_prepare_run_kernel<TI, PER>, rgrid, 128, 0, stream, (const TI*)fused, row_stride, q_off, k_off, v_off, b_off, \
+                                 a_off, n, H, G, D, V, conv_q, conv_k, conv_v, a_log, dt_bias, w_dtype, token_req, req_q_start, req_slot, \
+                                 (const float*)conv_state, unit_eps, q_scale, q, k, v, beta, decay)
+        const bool few = D <= 128 && V <= 128;
+        if (in_dtype == WLLM_BF16) return few ? RUN(bf16, 4) : RUN(bf16, 8);
+        return few ? RUN(float, 4) : RUN(float, 8);
+#undef RUN
+    }
     return wllm_launch(delta_prepare_kernel, dim3(n, (units + 3) / 4), 128, 0, stream, fused, in_dtype, row_stride, parts,
                        (size_t)part_stride, q_off, k_off, v_off, b_off, a_off, n, H, G, D, V, taps, conv_q, conv_k, conv_v, a_log,
                        dt_bias, w_dtype, token_req, req_q_start, req_q_len, req_slot, conv_state, unit_eps, q_scale, q, k, v, beta, decay, shift);
