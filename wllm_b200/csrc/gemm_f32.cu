@@ -8,8 +8,10 @@
 // A row of C therefore depends on its own row of A only, bit for bit, which makes the 32-bit path of the
 // engine independent of batching.  (Zero padding past K adds fma(0, 0, acc) = acc.)
 //
-// Two kernels with that same arithmetic:
-//   tile kernel    steps of many rows, bound by the FMA pipes: BM x 128 x 16 tiles (BM = 64 or 128), 256
+// Three kernels with that same arithmetic:
+//   wide kernel    steps of more than 64 rows (K and the pitches in steps of 4 floats, 16-byte aligned operands), bound by the FMA pipes:
+//                  see gemm_f32_wide_kernel.
+//   tile kernel    steps of 33 to 64 rows, and operands that the others do not take: BM x 128 x 16 tiles (BM = 64 or 128), 256
 //                  threads with 4 x 8 or 8 x 8 outputs each, operands transposed in shared memory and read
 //                  as float4, the next tile fetched into registers while the current one is multiplied; the
 //                  sums of finished segments wait in shared memory.
@@ -251,6 +253,132 @@ gemm_f32_skinny_kernel(const float* __restrict__ A, int lda, const float* __rest
     }
 }
 
+// ------------------------------------------------------------------------------------------------
+// wide kernel: 128 x 128 tiles, 128 threads with 8 x 16 outputs each, two CTAs an SM.
+//
+// The tile kernel's scheme with two changes.  Neighbouring columns are multiplied two an instruction (fma.rn.f32x2: each half is the fused
+// multiply-add of its own chain, so the bits are the same): the pipes' peak is no higher for it (73.4 against 71.9 TFLOP/s in a loop), but half the
+// instructions compete for the schedulers and the register ports.  And a thread has twice the columns, 24 floats read from shared memory
+// for 128 products instead of 16 for 64.  A launch's last round
+// finds its SMs half empty and runs faster, so the tiles need not divide evenly.  A launch whose tiles would not fill the device twice is
+// cut by segments, a CTA each: the sums go to slabs that the fold kernel adds in the same ascending order.  (A tile that walks several segments
+// keeps their running total in C.)
+// 512 x 32,768 x 2,048 without the guards: 8 x 8 outputs 1,640 us, in pairs 1,501; 8 x 16 1,714, in pairs 1,334 (51.5 TFLOP/s).  Rows left as they lie in
+// memory, brought by cp.async and read four k at a time, cannot be paired: 39 TFLOP/s; A that way and W transposed: 51.
+// A Gemma-2B prompt of 509 tokens, 72 such products of 509 rows, K 2,048 and 16,384: 78.6 -> 54.5 ms, the down products 1,758 -> 758 us each.
+// ------------------------------------------------------------------------------------------------
+constexpr int WT = 128, WTHREADS = 128;
+
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)),
+        "l"(*reinterpret_cast<unsigned long long*>(&c)));
+    return *reinterpret_cast<float2*>(&d);
+}
+
+// grid (row tiles, column tiles, segments with CTAs of their own, or 1); dst: C, or slabs [segment][M][N]
+__global__ void __launch_bounds__(WTHREADS, 2)
+gemm_f32_wide_kernel(const float* __restrict__ A, int lda, const float* __restrict__ W, int ldw, float* __restrict__ dst, int ld_dst,
+                     long long seg_stride, int M, int N, int K) {
+    __shared__ __align__(16) float As[2][TBK][WT + 4];
+    __shared__ __align__(16) float Ws[2][TBK][WT + 4];
+    constexpr int CHUNKS = WT * TBK / 4 / WTHREADS;         // groups of four k a thread and operand: rows crow + 32 i, k ck .. ck + 3
+    pdl_launch_dependents();
+    const int tid = threadIdx.x, m0 = blockIdx.x * WT, n0 = blockIdx.y * WT;       // neighbours in the grid share a tile of W
+    const int k_begin = gridDim.z > 1 ? blockIdx.z * SEG : 0, k_end = gridDim.z > 1 ? min(K, k_begin + SEG) : K;
+    const int tiles = (k_end - k_begin + TBK - 1) / TBK;
+    float* out = dst + (gridDim.z > 1 ? (size_t)blockIdx.z * seg_stride : 0);
+    const int crow = tid >> 2, ck = (tid & 3) * 4;
+    auto fetch = [&](const float* __restrict__ src, int ld, int rows, int r0, int t, float4 (&reg)[CHUNKS]) {
+        const int gk = k_begin + t * TBK + ck;
+#pragma unroll
+        for (int i = 0; i < CHUNKS; ++i) {
+            const int row = r0 + crow + 32 * i;
+            reg[i] = row < rows && gk < k_end ? *reinterpret_cast<const float4*>(src + (size_t)row * ld + gk) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    };
+    auto stash = [&](float (*to)[WT + 4], const float4 (&reg)[CHUNKS]) {
+#pragma unroll
+        for (int i = 0; i < CHUNKS; ++i) {
+            const int row = crow + 32 * i;
+            to[ck][row] = reg[i].x; to[ck + 1][row] = reg[i].y; to[ck + 2][row] = reg[i].z; to[ck + 3][row] = reg[i].w;
+        }
+    };
+    const int tx = tid & 7, ty = tid >> 3;      // outputs: rows 4 ty .. and 64 + 4 ty .., columns 4 tx .. + 32 h (h < 4), four each
+    float2 acc[8][8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[i][j] = make_float2(0.f, 0.f);
+    // what the accumulators hold joins the running total (add) or becomes it
+    const bool vec_out = (ld_dst & 3) == 0 && (seg_stride & 3) == 0 && ((uintptr_t)dst & 15) == 0;
+    auto leave = [&](bool add) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int gm = m0 + (i < 4 ? 4 * ty + i : WT / 2 + 4 * ty + i - 4);
+            if (gm >= M) continue;
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {
+                const int gn = n0 + 32 * h + 4 * tx;
+                float* to = out + (size_t)gm * ld_dst + gn;
+                float4 v = make_float4(acc[i][2 * h].x, acc[i][2 * h].y, acc[i][2 * h + 1].x, acc[i][2 * h + 1].y);
+                if (vec_out && gn + 3 < N) {
+                    if (add) {
+                        const float4 b = *reinterpret_cast<const float4*>(to);
+                        v = make_float4(b.x + v.x, b.y + v.y, b.z + v.z, b.w + v.w);
+                    }
+                    *reinterpret_cast<float4*>(to) = v;
+                } else {
+                    if (gn < N) to[0] = add ? to[0] + v.x : v.x;
+                    if (gn + 1 < N) to[1] = add ? to[1] + v.y : v.y;
+                    if (gn + 2 < N) to[2] = add ? to[2] + v.z : v.z;
+                    if (gn + 3 < N) to[3] = add ? to[3] + v.w : v.w;
+                }
+            }
+        }
+    };
+    float4 ra[CHUNKS], rw[CHUNKS];
+    fetch(W, ldw, N, n0, 0, rw);                // the weights are no kernel's output
+    pdl_wait();
+    fetch(A, lda, M, m0, 0, ra);
+    stash(As[0], ra);
+    stash(Ws[0], rw);
+    __syncthreads();
+    for (int t = 0; t < tiles; ++t) {
+        const int cur = t & 1;
+        if (t + 1 < tiles) {
+            fetch(A, lda, M, m0, t + 1, ra);
+            fetch(W, ldw, N, n0, t + 1, rw);
+        }
+#pragma unroll
+        for (int k = 0; k < TBK; ++k) {
+            float a[8];
+            float2 b[8];
+            *reinterpret_cast<float4*>(a) = *reinterpret_cast<const float4*>(&As[cur][k][4 * ty]);
+            *reinterpret_cast<float4*>(a + 4) = *reinterpret_cast<const float4*>(&As[cur][k][WT / 2 + 4 * ty]);
+#pragma unroll
+            for (int h = 0; h < 4; ++h) *reinterpret_cast<float4*>(&b[2 * h]) = *reinterpret_cast<const float4*>(&Ws[cur][k][32 * h + 4 * tx]);
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int j = 0; j < 8; ++j) acc[i][j] = fma2(make_float2(a[i], a[i]), b[j], acc[i][j]);
+        }
+        if (t + 1 < tiles) {
+            stash(As[cur ^ 1], ra);
+            stash(Ws[cur ^ 1], rw);
+            if (((t + 1) & (SEG / TBK - 1)) == 0) {        // a segment ends here and another follows
+                leave(t + 1 > SEG / TBK);
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) acc[i][j] = make_float2(0.f, 0.f);
+            }
+        }
+        __syncthreads();
+    }
+    leave(tiles > SEG / TBK);
+}
+
 // C[m][n] = the segments' sums added in ascending order.
 __global__ void __launch_bounds__(256)
 gemm_f32_fold_kernel(const float* __restrict__ parts, float* __restrict__ C, int ldc, int M, int N, int segs) {
@@ -316,10 +444,35 @@ static int launch_tile(const float* A, int lda, const float* W, int ldw, float* 
     return wllm_launch(gemm_f32_tile_kernel<BM, VEC>, grid, 256, totals, stream, A, lda, W, ldw, C, ldc, M, N, K);
 }
 
-// Floats of scratch that a product of these sizes needs (0: none): the skinny kernel's partial sums.
-WLLM_API long long wllm_gemm_f32_scratch_floats(int M, int N, int K) {
+// Whether a product of the wide kernel is cut by segments: its tiles fill fewer than two rounds of two CTAs an SM.  The slabs cost some five per cent
+// (a segment of an output is 1,024 products and 8 bytes there and back), an uneven last round of more than two costs less.
+static int wide_splits(int M, int N, int K) {
+    static int sms = 0;
+    if (!sms) {
+        int dev = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 148;
+    }
     const int segs = (K + SEG - 1) / SEG;
-    return (M <= 32 && segs > 1) ? (long long)segs * M * N : 0;
+    const long long tiles = (long long)((M + WT - 1) / WT) * ((N + WT - 1) / WT);
+    return segs > 1 && segs <= 65535 && tiles < 4ll * sms ? segs : 1;
+}
+
+static int launch_wide(const float* A, int lda, const float* W, int ldw, float* C, int ldc, int M, int N, int K, float* scratch,
+                       long long scratch_floats, cudaStream_t stream) {
+    // without room for the slabs the tiles walk their segments one after the other: the same bits
+    int segs = wide_splits(M, N, K);
+    if (segs > 1 && (scratch == nullptr || scratch_floats < (long long)segs * M * N)) segs = 1;
+    const dim3 grid((M + WT - 1) / WT, (N + WT - 1) / WT, segs);
+    const int st = wllm_launch(gemm_f32_wide_kernel, grid, WTHREADS, 0, stream, A, lda, W, ldw, segs > 1 ? scratch : C, segs > 1 ? N : ldc,
+                               (long long)M * N, M, N, K);
+    if (st != WLLM_OK || segs == 1) return st;
+    return wllm_launch(gemm_f32_fold_kernel, dim3((unsigned)(((size_t)M * N + 255) / 256)), 256, 0, stream, (const float*)scratch, C, ldc, M, N, segs);
+}
+
+// Floats of scratch that a product of these sizes wants (0: none): partial sums of the skinny kernel, or of the wide one.
+WLLM_API long long wllm_gemm_f32_scratch_floats(int M, int N, int K) {
+    const int segs = M <= 32 ? (K + SEG - 1) / SEG : (M > 64 && K % 4 == 0 ? wide_splits(M, N, K) : 1);
+    return segs > 1 ? (long long)segs * M * N : 0;
 }
 
 WLLM_API int wllm_gemm_f32(const float* A, int lda, const float* W, int ldw, float* C, int ldc, int M, int N, int K,
@@ -334,6 +487,7 @@ WLLM_API int wllm_gemm_f32(const float* A, int lda, const float* W, int ldw, flo
         if (vec) return launch_tile<64, true>(A, lda, W, ldw, C, ldc, M, N, K, stream);
         return launch_tile<64, false>(A, lda, W, ldw, C, ldc, M, N, K, stream);
     }
+    if (vec && (N + WT - 1) / WT <= 65535) return launch_wide(A, lda, W, ldw, C, ldc, M, N, K, scratch, scratch_floats, stream);
     if (vec) return launch_tile<128, true>(A, lda, W, ldw, C, ldc, M, N, K, stream);
     return launch_tile<128, false>(A, lda, W, ldw, C, ldc, M, N, K, stream);
 }
