@@ -1066,13 +1066,16 @@ WLLM_API long long wllm_attention_mma_prefill_halves_floats(int requests, int ma
 // Tokens of requests with q_len > 1 (and of those with q_len == 1 too unless skip_single).
 // `cap`, `keep`: as for decode; either sends the launch to the kernel that walks a list of tiles (prefill_kernel).
 // `slopes`: as for decode; the tensor-memory kernels take them as they take the cap (no tile is shared by two CTAs then).
+// `multi` (with skip_single; 0: not known): how many of the requests bring several tokens.
 WLLM_API int wllm_attention_mma_prefill_biased(const void* q, int q_stride, void* out, int out_stride, const void* k_pages,
                                                const void* v_pages, long long pool_pages, const int* req_q_start,
                                                const int* req_q_len, const int* req_ctx_len, const int* block_table,
                                                int max_pages, int requests, int max_q_len, int nq, int nkv, int page_size,
-                                               int window, float scale, int skip_single, int split_above, float* halves,
+                                               int window, float scale, int skip_single, int multi, int split_above, float* halves,
                                                int* status, const float* sinks, float cap, int keep, const float* slopes,
                                                cudaStream_t stream) {
+    if (!skip_single || multi < 0) multi = 0;
+    if (multi > requests) return WLLM_BAD_SIZE;
     if (cap < 0.f || keep < 0 || (keep > 0 && window <= 0)) return WLLM_BAD_SIZE;
     const bool listed = cap > 0.f || keep > 0 || slopes != nullptr;
     // split_above > 0 (tensor-memory kernel only): a tile of 128 rows that walks more than split_above tiles of
@@ -1118,9 +1121,9 @@ WLLM_API int wllm_attention_mma_prefill_biased(const void* q, int q_stride, void
     // (the tensor-memory kernels walk a list of key tiles too and take the cap; a launch with kept keys shares no tile)
     if (use_tc && use_pair && max_q_len * (nq / nkv) > TC_BM && (out_stride % 8 == 0) && (((uintptr_t)out & 15) == 0)) {
         const int pair_tiles = (max_q_len * (nq / nkv) + 2 * TC_BM - 1) / (2 * TC_BM);
-        return wllm_launch(prefill_pair_kernel, dim3(2 * nkv, requests, pair_tiles), TC_THREADS, PR_SMEM, stream,
+        return wllm_launch(prefill_pair_kernel, dim3(2 * nkv, multi > 0 ? multi : requests, pair_tiles), TC_THREADS, PR_SMEM, stream,
                            (const bf16*)q, q_stride, (bf16*)out, out_stride, km, vm, req_q_start, req_q_len, req_ctx_len,
-                           block_table, max_pages, nq, nkv, page_size, window, scale * LOG2E, skip_single, status, sinks,
+                           block_table, max_pages, nq, nkv, page_size, window, scale * LOG2E, skip_single, requests, multi, status, sinks,
                            cap * LOG2E, keep, slopes);
     }
 #endif
@@ -1152,7 +1155,7 @@ WLLM_API int wllm_attention_mma_prefill_capped(const void* q, int q_stride, void
                                                int* status, const float* sinks, float cap, int keep, cudaStream_t stream) {
     return wllm_attention_mma_prefill_biased(q, q_stride, out, out_stride, k_pages, v_pages, pool_pages, req_q_start, req_q_len,
                                              req_ctx_len, block_table, max_pages, requests, max_q_len, nq, nkv, page_size, window,
-                                             scale, skip_single, split_above, halves, status, sinks, cap, keep, nullptr, stream);
+                                             scale, skip_single, 0, split_above, halves, status, sinks, cap, keep, nullptr, stream);
 }
 
 WLLM_API int wllm_attention_mma_prefill_sinks(const void* q, int q_stride, void* out, int out_stride, const void* k_pages,

@@ -212,7 +212,7 @@ prefill_tc_kernel(const bf16* __restrict__ q, int q_stride, bf16* __restrict__ o
             if (lane == 0) mbar_arrive(q_full);
         }
 
-        const int pos_row = m_row < rows ? pos0 + m_row / rep : -1;            // a row past the end sees no key
+        const int pos_row = m_row < rows ? pos0 + m_row / rep : pos_hi;        // past the end: see prefill_pair_kernel
         int first_row = first_visible_key(pos_row, window), kept_row = 0;
         if (keep > 0) { if (first_row <= keep) first_row = 0; else kept_row = keep; }
         // `slopes` (null: none): the score of a key loses slope_h * (p - key), after the scale and the cap; such scores are
@@ -431,6 +431,9 @@ prefill_tc_kernel(const bf16* __restrict__ q, int q_stride, bf16* __restrict__ o
 // Barriers as in the two-CTA GEMM: `full` barriers (and q_full, p_full) live in the first CTA and are
 // arrived on by both; `empty`, s_full and pv_done exist in both and are arrived on by commit multicast.
 // Both CTAs allocate and free tensor memory together and pass a cluster barrier before they leave.
+// Beside decoded tokens the grid counts the requests of several tokens alone (`multi`), and a CTA looks its request up: a CTA that leaves at once still
+// takes its turn for an SM's whole shared memory (a prompt of 1,531 tokens, 8 heads of 256, beside 24 requests of one
+// token: 32.4 us, counted alone 31.3; beside 47: 47.3 and 31.2).
 constexpr int PR_BN = 128, PR_STAGES = 2;
 constexpr int PR_Q_BYTES = TC_BM * ROWB;                   // this CTA's 128 query rows
 constexpr int PR_K_BYTES = (PR_BN / 2) * ROWB;             // 64 keys x head size
@@ -439,18 +442,31 @@ constexpr int PR_SMEM = 1024 + PR_Q_BYTES + PR_STAGES * (PR_K_BYTES + PR_V_BYTES
 constexpr uint32_t IDESC_PR_S = umma_idesc(2 * TC_BM, PR_BN, false, false);
 constexpr uint32_t IDESC_PR_PV = umma_idesc(2 * TC_BM, HD, false, true);
 
+// The nth request (from 0) that brings several tokens, -1 past the last; a warp together.
+__device__ __forceinline__ int nth_of_several(const int* __restrict__ req_q_len, int requests, int nth) {
+    const int lane = threadIdx.x & 31;
+    for (int r0 = 0; r0 < requests; r0 += 32) {
+        const unsigned found = __ballot_sync(0xffffffffu, r0 + lane < requests && req_q_len[r0 + lane] > 1);
+        const int count = __popc(found);
+        if (nth < count) return r0 + (int)__fns(found, 0, nth + 1);
+        nth -= count;
+    }
+    return -1;
+}
+
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
 prefill_pair_kernel(const bf16* __restrict__ q, int q_stride, bf16* __restrict__ out, int out_stride,
                     const __grid_constant__ CUtensorMap k_map, const __grid_constant__ CUtensorMap v_map,
                     const int* __restrict__ req_q_start, const int* __restrict__ req_q_len, const int* __restrict__ req_ctx_len,
                     const int* __restrict__ block_table, int max_pages, int nq, int nkv, int page_size, int window, float scale2,
-                    int skip_single, int* __restrict__ status, const float* __restrict__ sinks, float capl, int keep,
+                    int skip_single, int requests, int multi, int* __restrict__ status, const float* __restrict__ sinks, float capl, int keep,
                   const float* __restrict__ slopes) {
     extern __shared__ unsigned char smem_raw[];
     pdl_begin();
     // grid (2 x key/value heads, requests, tiles): the pairs start in the order x, y, z, the tiles that walk the most
     // keys (the last rows of every head and request) first, so that the short ones fill the SMs behind them
-    const int g = blockIdx.x >> 1, r = blockIdx.y;
+    const int g = blockIdx.x >> 1, r = multi > 0 ? nth_of_several(req_q_len, requests, blockIdx.y) : (int)blockIdx.y;
+    if (r < 0) return;
     const int q_len = req_q_len[r];
     if (q_len <= 0 || (skip_single && q_len == 1)) return;             // the same for both CTAs of a pair
     const int rep = nq / nkv, rows = q_len * rep;
@@ -507,7 +523,8 @@ prefill_pair_kernel(const bf16* __restrict__ q, int q_stride, bf16* __restrict__
 
     if (warp == 0 || warp == 6) {
         // ---------------- TMA producers: warp 0 this CTA's half of the key tiles, warp 6 of the value tiles ----------------
-        if (lane == 0) {
+        // (one lane issues the copies; the value tiles' warp stays together to clear stray rows)
+        {
             const int kv = warp == 6;
             const uint32_t full0 = kv ? lead_v_full : lead_k_full, empty0 = kv ? v_empty : k_empty;
             const uint32_t ring = kv ? v_s : k_s, stage_bytes = kv ? PR_V_BYTES : PR_K_BYTES;
@@ -520,7 +537,7 @@ prefill_pair_kernel(const bf16* __restrict__ q, int q_stride, bf16* __restrict__
             int n = 0, edges = 0;
             for (; n < T && ok; ++n) {
                 const int s = n % PR_STAGES, ph = (n / PR_STAGES) & 1, tile_start = tile_of(n) * PR_BN + row_lo;
-                if (!mbar_wait(empty0 + 8 * s, ph ^ 1)) { ok = false; break; }
+                if (!__all_sync(0xffffffffu, mbar_wait(empty0 + 8 * s, ph ^ 1))) { ok = false; break; }
                 const uint32_t bar = full0 + 8 * s, dst = ring + s * stage_bytes;
                 // A value tile that reaches past the request's last key (or in front of the window's first) holds, in
                 // those rows, whatever the page holds; their weight is zero, but zero times something that is no
@@ -529,8 +546,8 @@ prefill_pair_kernel(const bf16* __restrict__ q, int q_stride, bf16* __restrict__
                 // arrival in place of the byte count.
                 const int key0 = tile_of(n) * PR_BN;
                 const bool edge = kv && (key0 + PR_BN > ctx || key0 < key_lo);      // (a tile of kept keys lies before key_lo)
-                if (edge) mbar_expect_tx(v_edge, stage_bytes); else mbar_expect_tx_cluster(bar, stage_bytes);
-                for (int r0 = 0; r0 < row_n; r0 += box_rows) {
+                if (lane == 0) { if (edge) mbar_expect_tx(v_edge, stage_bytes); else mbar_expect_tx_cluster(bar, stage_bytes); }
+                for (int r0 = 0; r0 < row_n && lane == 0; r0 += box_rows) {
                     const int key = tile_start + r0, index = key >> page_shift;
                     int page = index < max_pages ? table[index] : 0;
                     if (page < 0) page = 0;
@@ -541,20 +558,22 @@ prefill_pair_kernel(const bf16* __restrict__ q, int q_stride, bf16* __restrict__
                     }
                 }
                 if (edge) {
-                    if (!mbar_wait(v_edge, edges & 1)) { ok = false; break; }
+                    if (!__all_sync(0xffffffffu, mbar_wait(v_edge, edges & 1))) { ok = false; break; }
                     ++edges;
-                    if (key0 + PR_BN > ctx) zero_value_rows<PR_BN>(dst, HD / 128, max(0, ctx - key0), PR_BN, 0, 1);
+                    if (key0 + PR_BN > ctx) zero_value_rows<PR_BN>(dst, HD / 128, max(0, ctx - key0), PR_BN, lane, 32);
                     // in front of the window's first key, but behind the kept keys
-                    if (key0 < key_lo) zero_value_rows<PR_BN>(dst, HD / 128, min(PR_BN, max(0, kept_cta - key0)), min(PR_BN, key_lo - key0), 0, 1);
-                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                    mbar_arrive_cluster_release(bar);
+                    if (key0 < key_lo) zero_value_rows<PR_BN>(dst, HD / 128, min(PR_BN, max(0, kept_cta - key0)), min(PR_BN, key_lo - key0), lane, 32);
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // every lane's own stores
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_cluster_release(bar);
                 }
             }
             for (int k = 0; k < PR_STAGES && ok; ++k, ++n) {          // nothing in flight at the exit
                 const int s = n % PR_STAGES, ph = (n / PR_STAGES) & 1;
-                if (!mbar_wait(empty0 + 8 * s, ph ^ 1)) ok = false;
+                if (!__all_sync(0xffffffffu, mbar_wait(empty0 + 8 * s, ph ^ 1))) ok = false;
             }
-            if (!ok) atomicExch(status, GAVE_UP_TC_LOAD);
+            if (!ok && lane == 0) atomicExch(status, GAVE_UP_TC_LOAD);
+            __syncwarp();
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer: the first CTA's, for both ----------------
@@ -608,7 +627,9 @@ prefill_pair_kernel(const bf16* __restrict__ q, int q_stride, bf16* __restrict__
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(lead_q_full);
 
-        const int pos_row = m_row < rows ? pos0 + m_row / rep : -1;            // a row past the end sees no key
+        // A row past the end (zeros, stored nowhere) keeps the last row company: a row that sees no key would take its warp's every tile off the
+        // path without masks (1,531 tokens, 8 heads of 256: 49.2 us so, 31.1 now, as 1,536 take).
+        const int pos_row = m_row < rows ? pos0 + m_row / rep : pos_hi;
         int first_row = first_visible_key(pos_row, window), kept_row = 0;
         if (keep > 0) { if (first_row <= keep) first_row = 0; else kept_row = keep; }
         // `slopes` (null: none): the score of a key loses slope_h * (p - key), after the scale and the cap; such scores are

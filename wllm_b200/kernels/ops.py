@@ -695,8 +695,9 @@ def attention_mma_prefill(q, out, k_pages, v_pages, req_q_start, req_q_len, req_
                           nq: int, nkv: int, hd: int, page_size: int, window: int, scale: float,
                           skip_single: bool, split_above: int = 0, halves: torch.Tensor | None = None,
                           sinks: torch.Tensor | None = None, cap: float = 0.0, keep: int = 0,
-                          slopes: torch.Tensor | None = None) -> None:
+                          slopes: torch.Tensor | None = None, multi: int = 0) -> None:
     """bfloat16 attention of the requests that bring several tokens (csrc/attention_mma.cu, prefill).
+    `multi` (with skip_single): exactly how many do, so that the launch counts them alone; 0: not known.
     split_above > 0 (head sizes in steps of 64): a tile of 128 rows that walks more than that many tiles of 64
     keys is computed by two CTAs, half of the keys each; `halves` (float32) holds their partial results.
     `cap`, `keep`, `slopes`: as for attention_mma_decode; with any of them the mma.sync kernel that walks a list of key tiles runs."""
@@ -715,7 +716,7 @@ def attention_mma_prefill(q, out, k_pages, v_pages, req_q_start, req_q_len, req_
                                                 _ptr(_int32(req_ctx_len, "req_ctx_len")),
                                                 _ptr(_int32(block_table, "block_table")), block_table.shape[1],
                                                 req_q_len.shape[0], max_q_len, nq, nkv, page_size, window, c_float(scale),
-                                                1 if skip_single else 0, split_above, _ptr(halves) if split_above > 0 else None,
+                                                1 if skip_single else 0, multi, split_above, _ptr(halves) if split_above > 0 else None,
                                                 _ptr(_status_word(q.device)), _ptr(sinks), c_float(cap), keep, _ptr(slopes), _stream()),
            f"attention_mma_prefill(head_dim={hd}, heads={nq}/{nkv})")
 

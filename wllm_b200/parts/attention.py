@@ -325,7 +325,7 @@ class PagedAttention:
             split_above, halves = (0, None) if listed or self.blocks else self._shared_tiles(ctx, skip_single=decode)
             ops.attention_mma_prefill(q, out, k_pages, v_pages, ctx.req_q_start, ctx.req_q_len, ctx.req_ctx_len, table,
                                       ctx.max_q_len, nq, nkv, hd, ps, window, scale, skip_single=decode,
-                                      split_above=split_above, halves=halves, **extra)
+                                      split_above=split_above, halves=halves, multi=ctx.num_multi if decode else 0, **extra)
 
     def _shared_tiles(self, ctx, skip_single: bool):
         """Whether this step's prefill attention shares its heavy tiles between two CTAs (ops.prefill_share_plan),
