@@ -99,3 +99,26 @@ def test_runs_of_tokens_are_prepared_as_one_by_one(lens, sizes, dtype):
     whole = run([[(r, 0, m) for r, m in enumerate(lens)]])
     cut = run([[(r, a, min(a + 31, m))] for r, m in enumerate(lens) for a in range(0, m, 31)])
     assert all(torch.equal(a, b) for a, b in zip(whole, cut))
+
+
+@pytest.mark.parametrize("sizes", [(2, 1, 33, 5), (3, 3, 64, 64), (4, 2, 128, 128), (2, 2, 100, 65), (1, 1, 256, 200)])     # channels a thread; ragged columns
+@pytest.mark.parametrize("channel", [False, True])
+def test_single_tokens_have_the_walks_bits(sizes, channel):
+    from wllm_b200.kernels import ops
+    H, G, D, V = sizes
+    R = 5
+    gen = torch.Generator().manual_seed(D + V + channel)
+    rand = lambda *shape: torch.randn(*shape, generator=gen).to(DEV)
+    q, k, v, beta = rand(R, G * D), rand(R, G * D), rand(R, H * V), torch.sigmoid(rand(R, H))
+    rate = torch.exp(3 * rand(R, H * D if channel else H) - 3)
+    decay = torch.expm1(-rate) if channel else torch.exp(-rate)
+    state = rand(2 * R, H, D, V)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    index = i32([0, 1, 2, 3, 4]), i32([1, 1, 0, 1, 1]), i32([3, 0, 5, -1, 9])          # one brings no token, one has no slot
+    res = []
+    for single in (False, True):
+        S, o = state.clone(), torch.full((R, H * V), float("nan"), device=DEV)
+        ops.delta_scan(q, k, v, beta, decay, S, o, *index, H, G, D, V, channel, single=single)
+        res.append((S, torch.nan_to_num(o, nan=-1.0)))
+    assert torch.equal(res[0][0], res[1][0]) and torch.equal(res[0][1], res[1][1])
+    assert not torch.equal(res[1][0], state)

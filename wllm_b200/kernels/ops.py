@@ -1266,13 +1266,13 @@ def delta_block_floats(n: int, requests: int, heads: int, dim: int) -> int:
 
 
 def delta_scan(q, k, v, beta, decay, state, out, req_q_start, req_q_len, req_slot, heads: int, kv_heads: int, dim: int, vdim: int,
-               channel: bool = False, blocks: torch.Tensor | None = None, max_q_len: int = 0):
+               channel: bool = False, blocks: torch.Tensor | None = None, max_q_len: int = 0, single: bool = False):
     """The gated delta rule over every request's tokens of the step, in order, from and to its state slot:
     S <- decay S; u = beta (v - S^T k); S <- S + k u^T; out = S^T q.  q, k [n, kv_heads * dim], v, out [n, heads * vdim],
     beta, decay [n, heads], state [slots, heads, dim, vdim], all float32 (csrc/delta_rule.cu).  `channel`: decay
     [n, heads * dim], one per key channel, given as decay - 1 (lowrank_map).  `blocks` (float32 scratch of delta_block_floats; the
     longest request has max_q_len tokens): requests of DELTA_BLOCKS_FROM tokens or more are walked in blocks
-    of eight tokens, whose sums run in another order."""
+    of eight tokens, whose sums run in another order.  `single`: no request brings more than one token (the same bits, another kernel)."""
     _need_cuda(q, k, v, beta, decay, state, out, req_q_start, req_q_len, req_slot, blocks)
     n = q.shape[0]
     assert all(t.dtype == torch.float32 and t.is_contiguous() for t in (q, k, v, beta, decay, state, out))
@@ -1293,7 +1293,7 @@ def delta_scan(q, k, v, beta, decay, state, out, req_q_start, req_q_len, req_slo
             return out
         below = DELTA_BLOCKS_FROM
     _check(lib.wllm_delta_scan(_ptr(q), _ptr(k), _ptr(v), _ptr(beta), _ptr(decay), 1 if channel else 0, _ptr(state), _ptr(out),
-                               *index, R, heads, kv_heads, dim, vdim, below, _stream()), name)
+                               *index, R, heads, kv_heads, dim, vdim, below, 1 if single else 0, _stream()), name)
     return out
 
 

@@ -335,7 +335,7 @@ class DeltaRule:
         if self.model_dtype == torch.bfloat16 and ctx.max_q_len >= ops.DELTA_BLOCKS_FROM:
             blocks = ctx.buffer(self.tag + "delta_blocks", (ops.delta_block_floats(n, ctx.n_requests, H, D),), f32)
         ops.delta_scan(q, k, v, beta, decay, ctx.state(cache.state_names["state"]), o, ctx.req_q_start, ctx.req_q_len, ctx.req_slot,
-                       H, G, D, V, channel, blocks, ctx.max_q_len)
+                       H, G, D, V, channel, blocks, ctx.max_q_len, single)
         gated = ctx.buffer(self.tag + "delta_gated", (n, H * V), self.model_dtype)
         if self.gate_maps is None:
             ops.head_gate_norm(o, fused, parts, off["g"], self.norm_weight, self.eps, gated, H, V)
