@@ -122,3 +122,28 @@ def test_single_tokens_have_the_walks_bits(sizes, channel):
         res.append((S, torch.nan_to_num(o, nan=-1.0)))
     assert torch.equal(res[0][0], res[1][0]) and torch.equal(res[0][1], res[1][1])
     assert not torch.equal(res[1][0], state)
+
+
+@pytest.mark.parametrize("parts", [0, 1, 17])                         # a tensor; a slab; more than are asked for at once
+@pytest.mark.parametrize("sizes", [(2, 1, 8, 5), (4, 2, 128, 128), (1, 1, 200, 256)])
+def test_single_tokens_are_prepared_as_portions_of_one(parts, sizes):
+    """With the slots' inputs brought up to date in the same kernel, beside the two kernels of steps with portions: the same bits."""
+    from wllm_b200.kernels import ops
+    H, G, D, V = sizes
+    gen = torch.Generator().manual_seed(parts + D)
+    R, C, T = 5, 2 * G * D + H * V, 4
+    off = {"q": 0, "k": G * D, "v": 2 * G * D, "b": C, "a": C + H}
+    fused = torch.randn(*([parts] if parts else []), R, C + 2 * H, generator=gen).to(DEV)
+    taps = [torch.randn(c, T, generator=gen).to(DEV) for c in (G * D, G * D, H * V)]
+    a_log, dt_bias = (torch.randn(H, generator=gen).to(DEV) for _ in range(2))
+    conv0 = torch.randn(2 * R, T - 1, C, generator=gen).to(DEV)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    starts, lens, slots = i32([0, 1, 2, 3, 4]), i32([1, 1, 0, 1, 1]), i32([3, 0, 5, -1, 9])      # one brings no token, one has no slot
+    res = []
+    for shift in (None, lens):
+        conv, out = conv0.clone(), [torch.empty(R, w, device=DEV) for w in (G * D, G * D, H * V, H, H)]
+        ops.delta_prepare(fused, parts, off, H, G, D, V, T, *taps, a_log, dt_bias, starts, starts, slots, conv, 1e-6, D ** -0.5, *out, shift=shift)
+        if shift is None:
+            ops.delta_conv_update(fused, parts, off, H, G, D, V, T, starts, lens, slots, conv)
+        res.append(out + [conv])
+    assert all(torch.equal(a, b) for a, b in zip(*res))

@@ -59,6 +59,7 @@ __device__ __forceinline__ float la_in(const void* p, int dtype, int parts, size
 // prepare: grid (tiles of TT tokens, heads), 128 threads
 // ---------------------------------------------------------------------------------------------------
 constexpr int PREP_RK = 32;      // columns of the low-rank map taken at a time
+constexpr int PREP_ALL = 256;
 
 // What a row z of the low-rank map becomes, by form (see the head of this file); rate = exp(A_log_h) of form 2
 __device__ __forceinline__ float lowrank_out(int form, float z, float inv_tau, float rate) {
@@ -80,7 +81,9 @@ linattn_prepare_kernel(const void* __restrict__ fused, int in_dtype, int row_str
                        float q_scale, float k_scale, const void* __restrict__ w2, const void* __restrict__ b2,
                        int w_dtype, float inv_tau, float* __restrict__ q, float* __restrict__ k,
                        float* __restrict__ v, float* __restrict__ decay, int form, const void* __restrict__ a_log) {
-    __shared__ __align__(16) float low_s[PREP_RK][TT];      // the tokens' low-rank vectors, a run of PREP_RK columns at a time
+    // the tokens' low-rank vectors, a run of PREP_RK columns at a time; a lone token's first PREP_ALL columns at once (its slabs' loads would
+    // otherwise be waited for run by run)
+    __shared__ __align__(16) float low_s[TT == 1 ? PREP_ALL : PREP_RK][TT];
     pdl_begin();
     const int t_lo = blockIdx.x * TT, h = blockIdx.y;
     const int count = min(TT, n - t_lo);
@@ -117,6 +120,14 @@ linattn_prepare_kernel(const void* __restrict__ fused, int in_dtype, int row_str
     // tokens' low-rank vectors come from shared memory.  The sum over r runs in ascending order whatever the tiling.
     const bool vec = ((uintptr_t)w2 & 15) == 0 && rank % 8 == 0;
     const float rate = form == 2 ? expf(la_any(a_log, w_dtype, h)) : 0.f;
+    const bool at_once = TT == 1 && rank <= PREP_ALL;
+    if (at_once) {
+        for (int r = threadIdx.x; r < (rank + PREP_RK - 1) / PREP_RK * PREP_RK; r += blockDim.x) {
+            const float low = r < rank ? la_in<MULTI>(fused, in_dtype, parts, part_stride, (size_t)t_lo * row_stride + a_off + r) : 0.f;
+            low_s[r][0] = form == 1 ? tanhf(low) : low;
+        }
+        __syncthreads();
+    }
     for (int c0 = 0; c0 < D; c0 += 128) {
         const int c = c0 + threadIdx.x;
         const size_t ch = (size_t)h * D + min(c, D - 1);
@@ -125,9 +136,9 @@ linattn_prepare_kernel(const void* __restrict__ fused, int in_dtype, int row_str
 #pragma unroll
         for (int tt = 0; tt < TT; ++tt) z[tt] = bias;
         for (int r0 = 0; r0 < rank; r0 += PREP_RK) {
-            const int rk = min(PREP_RK, rank - r0);
-            __syncthreads();
-            for (int idx = threadIdx.x; idx < TT * PREP_RK; idx += blockDim.x) {
+            const int rk = min(PREP_RK, rank - r0), low0 = at_once ? r0 : 0;
+            if (!at_once) __syncthreads();
+            for (int idx = at_once ? TT * PREP_RK : threadIdx.x; idx < TT * PREP_RK; idx += blockDim.x) {
                 const int r = idx / TT, tt = idx % TT;
                 float low = (tt < count && r < rk)
                     ? la_in<MULTI>(fused, in_dtype, parts, part_stride, (size_t)(t_lo + tt) * row_stride + a_off + r0 + r) : 0.f;
@@ -163,11 +174,11 @@ linattn_prepare_kernel(const void* __restrict__ fused, int in_dtype, int row_str
 #pragma unroll
                 for (int r = 0; r < PREP_RK; ++r) wr[r] = r < rk ? la_any(w2, w_dtype, ch * rank + r0 + r) : 0.f;
             }
-            __syncthreads();
+            if (!at_once) __syncthreads();
 #pragma unroll
             for (int r = 0; r < PREP_RK; ++r) {
 #pragma unroll
-                for (int tt = 0; tt < TT; ++tt) z[tt] = fmaf(low_s[r][tt], wr[r], z[tt]);
+                for (int tt = 0; tt < TT; ++tt) z[tt] = fmaf(low_s[low0 + r][tt], wr[r], z[tt]);
             }
         }
         if (c < D) {
