@@ -9,7 +9,7 @@
 // inputs in front of the sequence count as zero) and pass SiLU; q and k are then scaled to unit length head by head.  Query and key heads may be
 // fewer than value heads (head h reads q/k head h / (H / G)).  The state and the convolutions' last taps - 1 inputs live in
 // the cache manager's state slots and are carried from step to step, so a whole prompt, a portion and a single decoded token
-// are one case and give the same bits.
+// are one case and, token by token, give the same bits (wllm_delta_blocks adds in another order).
 //
 //   wllm_delta_prepare      from a fused projection row (q | k | v | ... | b | a in one matrix product, possibly still in split-K
 //                           slabs): convolution and SiLU of q, k and v, the unit norms x / sqrt(sum(x^2) + eps) (q also times

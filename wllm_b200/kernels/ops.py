@@ -817,7 +817,7 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None) 
     assert out.stride(1) == 1 and out.shape == (M, N) and out.dtype == torch.float32
     lib = load_family("gemm_f32")
     lib.wllm_gemm_f32_scratch_floats.restype = ctypes.c_longlong
-    need = lib.wllm_gemm_f32_scratch_floats(M, N, K)       # partial sums of the few-rows kernel when K has several segments
+    need = lib.wllm_gemm_f32_scratch_floats(M, N, K)       # partial sums, when segments of K have CTAs of their own
     scratch = torch.empty(need, dtype=torch.float32, device=a.device) if need else None
     _check(lib.wllm_gemm_f32(_ptr(a), a.stride(0), _ptr(w), w.stride(0), _ptr(out), out.stride(0), M, N, K, _ptr(scratch),
                              ctypes.c_longlong(need), _stream()), "gemm_f32")

@@ -306,7 +306,7 @@ class PagedAttention:
             return
         decode = ctx.num_single > 0 and nq // nkv <= 16
         extra = {"sinks": self.sinks} if self.sinks is not None else {}
-        # the kernels that walk a list of key tiles (mma.sync) take a cap, kept first keys and a bias by distance
+        # prefill: no tile is shared by two CTAs; decode: a cap or kept first keys take the kernel that walks a list of key tiles
         listed = self.softcap > 0 or self.keep_first > 0 or self.slopes is not None
         if listed:
             extra.update(cap=self.softcap, keep=self.keep_first, slopes=self.slopes)
