@@ -38,14 +38,17 @@ def test_joined_norms_of_every_row_size(H, parts, center):
     assert torch.equal(before, resid) and (some.cpu().double() - r2).abs().max() <= 2.0 ** -8 * r2.abs().max() + 2e-5
 
 
-@pytest.mark.parametrize("heads", [(1, 1, 8, 8, 8), (16, 4, 128, 128, 64), (16, 4, 128, 256, 128)])    # one group a part; all threads once; a second round
-@pytest.mark.parametrize("parts", [1, 8, 9])
-def test_turned_rows_from_slabs(heads, parts):
+@pytest.mark.parametrize("heads", [(1, 1, 8, 8, 8), (16, 4, 128, 128, 64), (16, 4, 128, 256, 128), (2, 1, 64, 64, 24)])    # one group a part; all threads once; a second round; partners that are no whole groups
+@pytest.mark.parametrize("parts", [0, 1, 8, 9])                       # a bfloat16 tensor; slabs in one round of loads, in two
+@pytest.mark.parametrize("biased", [False, True])
+def test_turned_rows_from_tensors_and_slabs(heads, parts, biased):
     from wllm_b200.kernels import ops
     nq, nkv, hd, vd, rot = heads
     g = torch.Generator().manual_seed(hd + parts)
     n, ps, eps, qw, kw = 5, 16, 1e-5, nq * hd, nkv * hd
-    x = torch.randn(parts, n, qw + kw + nkv * vd, generator=g)
+    x = torch.randn(*([parts] if parts else []), n, qw + kw + nkv * vd, generator=g)
+    x = x if parts else x.bfloat16()
+    bias = torch.randn(qw + kw + nkv * vd, generator=g) if biased else None
     q_gain, k_gain = (torch.randn(m, generator=g).bfloat16() for m in (qw, kw))
     freq = torch.tensor([100.0 ** (-2.0 * i / rot) for i in range(rot // 2)])
     positions, slots = torch.arange(40, 40 + n, dtype=torch.int32), torch.randperm(3 * ps, generator=g)[:n].to(torch.int32)
@@ -53,8 +56,9 @@ def test_turned_rows_from_slabs(heads, parts):
     kp, vp = torch.zeros(3, nkv, ps, hd, dtype=torch.bfloat16, device=DEV), torch.zeros(3, nkv, ps, vd, dtype=torch.bfloat16, device=DEV)
     q_out = torch.empty(n, qw, dtype=torch.bfloat16, device=DEV)
     ops.rope_row_norm_kv_write(x.to(DEV), q_out, positions.to(DEV), slots.to(DEV), freq.to(DEV), kp, vp, nq, nkv, hd, rot, ps, q_gain.to(DEV),
-                               k_gain.to(DEV), eps, qw, kw, in_splits=parts, vd=vd)
-    W = x.double().sum(0)
+                               k_gain.to(DEV), eps, qw, kw, in_splits=parts, vd=vd, bias=bias.to(DEV) if biased else None)
+    W = x.double().sum(0) if parts else x.double()
+    W = W + bias.double() if biased else W
 
     def turned(y, gain, m):
         y = (_norm(y, False, eps) * gain.double()).view(n, m, hd)
