@@ -147,3 +147,38 @@ def test_single_tokens_are_prepared_as_portions_of_one(parts, sizes):
             ops.delta_conv_update(fused, parts, off, H, G, D, V, T, starts, lens, slots, conv)
         res.append(out + [conv])
     assert all(torch.equal(a, b) for a, b in zip(*res))
+
+
+@pytest.mark.parametrize("bad", ["v", "k", "q", "beta", "decay"])
+@pytest.mark.parametrize("what", [float("inf"), float("nan")])
+@pytest.mark.parametrize("n,at", [(24, 13), (24, 8), (17, 16)])                # inside a block; its first token; a portion's last, beside places past its end
+@pytest.mark.parametrize("channel", [False, True])
+def test_what_is_no_number_reaches_no_earlier_token(n, at, what, bad, channel):
+    """One input that overflowed: the tokens in front of it, the other head and (for a value) the other columns keep their bits, and what the walk
+    token by token leaves finite is finite."""
+    from wllm_b200.kernels import ops
+    H, D, V = 2, 72, 20
+    gen = torch.Generator().manual_seed(n + at)
+    rand = lambda *shape: torch.randn(*shape, generator=gen).to(DEV)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    unit = lambda x: (x / x.norm(dim=-1, keepdim=True)).reshape(n, -1).contiguous()
+    arg = {"q": unit(rand(n, H, D)), "k": unit(rand(n, H, D)), "v": rand(n, H * V), "beta": torch.sigmoid(rand(n, H))}
+    rate = torch.exp(rand(n, H * D if channel else H) - 3)
+    arg["decay"], state = torch.expm1(-rate) if channel else torch.exp(-rate), rand(1, H, D, V)
+    place = {"v": 5, "k": 7, "q": 7, "beta": 0, "decay": 7 if channel else 0}[bad]         # head 0
+
+    def run(arg, blocks):
+        S, o = state.clone(), torch.empty(n, H * V, device=DEV)
+        scratch = torch.full((ops.delta_block_floats(n, 1, H, D),), float("nan"), device=DEV) if blocks else None
+        ops.delta_scan(*arg.values(), S, o, i32([0]), i32([n]), i32([0]), H, H, D, V, channel, scratch, n)
+        return o.view(n, H, V), S[0]
+    clean_o, clean_S = run(arg, True)
+    arg[bad] = arg[bad].clone()
+    arg[bad][at, place] = what
+    (o, S), (walk_o, walk_S) = run(arg, True), run(arg, False)
+    assert torch.equal(o[:at], clean_o[:at]) and torch.equal(o[:, 1], clean_o[:, 1]) and torch.equal(S[1], clean_S[1])
+    if bad == "v":
+        others = [c for c in range(V) if c != 5]
+        assert torch.equal(o[:, 0, others], clean_o[:, 0, others]) and torch.equal(S[0][:, others], clean_S[0][:, others])
+    assert bool(o.isfinite()[walk_o.isfinite()].all()) and bool(S.isfinite()[walk_S.isfinite()].all())
+    assert not bool(o[at, 0].isfinite().all())

@@ -918,7 +918,7 @@ delta_block_walk_kernel(const float* __restrict__ blocks, const float* __restric
                     x[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
                 }
         }
-        if (lane < 16) rs[warp][lane] = vt - x[0];
+        if (lane < 16) rs[warp][lane] = b * DB + tok < len ? vt - x[0] : 0.f;        // (past the end a value that is no number must not reach the state)
         __syncwarp();
         float rj[2][DB];
 #pragma unroll
@@ -928,7 +928,8 @@ delta_block_walk_kernel(const float* __restrict__ blocks, const float* __restric
             *reinterpret_cast<float4*>(nr) = *reinterpret_cast<const float4*>(N + tok * DB);
             *reinterpret_cast<float4*>(nr + 4) = *reinterpret_cast<const float4*>(N + tok * DB + 4);
 #pragma unroll
-            for (int j = 0; j < DB; ++j) o = fmaf(nr[j], mine ? rj[1][j] : rj[0][j], o);
+            for (int j = 0; j < DB; ++j)        // a select, not N's zeros: a later token's r may be no number
+                if (j <= tok) o = fmaf(nr[j], mine ? rj[1][j] : rj[0][j], o);
             out[((size_t)(t0 + b * DB + tok) * H + h) * V + col + mine] = o;
         }
         __syncwarp();                           // r is read to its end before the next block's takes its place
