@@ -182,3 +182,36 @@ def test_what_is_no_number_reaches_no_earlier_token(n, at, what, bad, channel):
         assert torch.equal(o[:, 0, others], clean_o[:, 0, others]) and torch.equal(S[0][:, others], clean_S[0][:, others])
     assert bool(o.isfinite()[walk_o.isfinite()].all()) and bool(S.isfinite()[walk_S.isfinite()].all())
     assert not bool(o[at, 0].isfinite().all())
+
+
+@pytest.mark.parametrize("several", [{40: 50, 71: 16, 72: 200}, {0: 31, 31: 17, 32: 24, 63: 90}, {69: 70}])      # among more than a warp's lanes; at its borders
+@pytest.mark.parametrize("order", ["ascending", "descending"])                                                       # of the requests' tokens in the step
+@pytest.mark.parametrize("channel", [False, True])
+def test_requests_in_blocks_are_found_beside_single_tokens(several, order, channel):
+    """A launch that counts the requests in blocks alone, one over all requests, and the walk token by token, beside 70 requests of one token."""
+    from wllm_b200.kernels import ops
+    H, G, D, V = 2, 1, 40, 20
+    R = max(70, max(several) + 1)
+    lens = [several.get(r, 1) for r in range(R)]
+    n, gen = sum(lens), torch.Generator().manual_seed(len(several))
+    by_place = range(R) if order == "ascending" else range(R - 1, -1, -1)
+    starts, at = [0] * R, 0
+    for r in by_place:
+        starts[r], at = at, at + lens[r]
+    rand = lambda *shape: torch.randn(*shape, generator=gen).to(DEV)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    unit = lambda x: (x / x.norm(dim=-1, keepdim=True)).reshape(n, -1).contiguous()
+    rate = torch.exp(rand(n, H * D if channel else H) - 3)
+    args = unit(rand(n, G, D)), unit(rand(n, G, D)), rand(n, H * V), torch.sigmoid(rand(n, H)), torch.expm1(-rate) if channel else torch.exp(-rate)
+    state, res = rand(R, H, D, V), []
+    for walked in (len(several), 0, None):
+        S, o = state.clone(), torch.full((n, H * V), float("nan"), device=DEV)
+        scratch = None if walked is None else torch.full((ops.delta_block_floats(n, R, H, D),), float("nan"), device=DEV)
+        ops.delta_scan(*args, S, o, i32(starts), i32(lens), i32(range(R)), H, G, D, V, channel, scratch, max(lens), walked=walked or 0)
+        res.append((o, S))
+    (o, S), (all_o, all_S), (walk_o, walk_S) = res
+    assert torch.equal(o, all_o) and torch.equal(S, all_S)
+    # two orders of 32-bit sums over 40 channels and 200 tokens
+    assert float((o - walk_o).norm() / walk_o.norm()) < 2e-6 and float((S - walk_S).norm() / walk_S.norm()) < 2e-6
+    ones = [starts[r] for r in range(R) if lens[r] == 1]
+    assert torch.equal(o[ones], walk_o[ones])

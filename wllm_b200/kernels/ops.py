@@ -1266,12 +1266,12 @@ def delta_block_floats(n: int, requests: int, heads: int, dim: int) -> int:
 
 
 def delta_scan(q, k, v, beta, decay, state, out, req_q_start, req_q_len, req_slot, heads: int, kv_heads: int, dim: int, vdim: int,
-               channel: bool = False, blocks: torch.Tensor | None = None, max_q_len: int = 0, single: bool = False):
+               channel: bool = False, blocks: torch.Tensor | None = None, max_q_len: int = 0, single: bool = False, walked: int = 0):
     """The gated delta rule over every request's tokens of the step, in order, from and to its state slot:
     S <- decay S; u = beta (v - S^T k); S <- S + k u^T; out = S^T q.  q, k [n, kv_heads * dim], v, out [n, heads * vdim],
     beta, decay [n, heads], state [slots, heads, dim, vdim], all float32 (csrc/delta_rule.cu).  `channel`: decay
     [n, heads * dim], one per key channel, given as decay - 1 (lowrank_map).  `blocks` (float32 scratch of delta_block_floats; the
-    longest request has max_q_len tokens): requests of DELTA_BLOCKS_FROM tokens or more are walked in blocks
+    longest request has max_q_len tokens): requests of DELTA_BLOCKS_FROM tokens or more (exactly `walked`; 0: not known) are walked in blocks
     of eight tokens, whose sums run in another order.  `single`: no request brings more than one token (the same bits, another kernel)."""
     _need_cuda(q, k, v, beta, decay, state, out, req_q_start, req_q_len, req_slot, blocks)
     n = q.shape[0]
@@ -1286,10 +1286,10 @@ def delta_scan(q, k, v, beta, decay, state, out, req_q_start, req_q_len, req_slo
     if blocks is not None and max_q_len >= DELTA_BLOCKS_FROM:
         assert blocks.dtype == torch.float32 and blocks.is_contiguous() and blocks.numel() >= delta_block_floats(n, R, heads, dim)
         _check(lib.wllm_delta_blocks(_ptr(q), _ptr(k), _ptr(v), _ptr(beta), _ptr(decay), 1 if channel else 0, _ptr(state), _ptr(out),
-                                     _ptr(blocks), *index, R, max_q_len, heads, kv_heads, dim, vdim, DELTA_BLOCKS_FROM, sm_count(), _stream()), name)
+                                     _ptr(blocks), *index, R, walked, max_q_len, heads, kv_heads, dim, vdim, DELTA_BLOCKS_FROM, sm_count(), _stream()), name)
         global launches
         launches += 1         # the blocks' matrices, then the walk
-        if R == 1:
+        if walked == R:
             return out
         below = DELTA_BLOCKS_FROM
     _check(lib.wllm_delta_scan(_ptr(q), _ptr(k), _ptr(v), _ptr(beta), _ptr(decay), 1 if channel else 0, _ptr(state), _ptr(out),

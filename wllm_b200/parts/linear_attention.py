@@ -309,6 +309,15 @@ class DeltaRule:
         fused, parts = ops.project(x, self.w_in, lambda name, shape, dt: ctx.buffer(self.tag + "delta_in_" + name, shape, dt))
         return self.mix(fused, parts, 0, ctx, cache)
 
+    @staticmethod
+    def _walked(ctx) -> int:
+        """How many of the step's requests are walked in blocks (0: their lengths are not on the host); counted once a step."""
+        if getattr(ctx, "host", None) is None:
+            return 0
+        if "delta_walked" not in ctx.memo:
+            ctx.memo["delta_walked"] = int((ctx.host["req_q_len"] >= ops.DELTA_BLOCKS_FROM).sum())
+        return ctx.memo["delta_walked"]
+
     def mix(self, fused: torch.Tensor, parts: int, col0: int, ctx, cache: CacheRef):
         """The mixer on the columns from col0 of a fused product [n, W] (or partial sums [parts, n, W])."""
         n, H, G, D, V, f32 = fused.shape[-2], self.heads, self.kv_heads, self.dim, self.vdim, torch.float32
@@ -331,11 +340,12 @@ class DeltaRule:
             ops.lowrank_map(fused, parts, off["a_low"], self.decay_up, H, D, decay, self.dt_bias, self.a_log)
         o = ctx.buffer(self.tag + "delta_o", (n, H * V), f32)
         # portions of a bfloat16 model in blocks of tokens; a 32-bit model's walk gives the same bits however a prompt is cut
-        blocks = None
+        blocks, walked = None, 0
         if self.model_dtype == torch.bfloat16 and ctx.max_q_len >= ops.DELTA_BLOCKS_FROM:
+            walked = self._walked(ctx)
             blocks = ctx.buffer(self.tag + "delta_blocks", (ops.delta_block_floats(n, ctx.n_requests, H, D),), f32)
         ops.delta_scan(q, k, v, beta, decay, ctx.state(cache.state_names["state"]), o, ctx.req_q_start, ctx.req_q_len, ctx.req_slot,
-                       H, G, D, V, channel, blocks, ctx.max_q_len, single)
+                       H, G, D, V, channel, blocks, ctx.max_q_len, single, walked)
         gated = ctx.buffer(self.tag + "delta_gated", (n, H * V), self.model_dtype)
         if self.gate_maps is None:
             ops.head_gate_norm(o, fused, parts, off["g"], self.norm_weight, self.eps, gated, H, V)
