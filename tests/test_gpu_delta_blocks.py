@@ -215,3 +215,33 @@ def test_requests_in_blocks_are_found_beside_single_tokens(several, order, chann
     assert float((o - walk_o).norm() / walk_o.norm()) < 2e-6 and float((S - walk_S).norm() / walk_S.norm()) < 2e-6
     ones = [starts[r] for r in range(R) if lens[r] == 1]
     assert torch.equal(o[ones], walk_o[ones])
+
+
+@pytest.mark.parametrize("channel", [False, True])
+def test_portions_in_turns_have_the_bits_of_one(channel):
+    """Scratch for every block, for some blocks of each request down to one, and for less."""
+    from wllm_b200.kernels import ops
+    H, G, D, V, lens = 2, 1, 72, 20, [24, 1, 0, 203, 16, 9]
+    R, n, gen = len(lens), sum(lens), torch.Generator().manual_seed(3)
+    rand = lambda *shape: torch.randn(*shape, generator=gen).to(DEV)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    unit = lambda x: (x / x.norm(dim=-1, keepdim=True)).reshape(n, -1).contiguous()
+    rate = torch.exp(rand(n, H * D if channel else H) - 3)
+    args = unit(rand(n, G, D)), unit(rand(n, G, D)), rand(n, H * V), torch.sigmoid(rand(n, H)), torch.expm1(-rate) if channel else torch.exp(-rate)
+    state, res = rand(R, H, D, V), []
+    floats = ops.delta_block_floats(8, 0, H, D)                       # of a block
+    starts = [sum(lens[:r]) for r in range(R)]
+    for blocks, walked in ((n // 8 + R, 3), (15, 3), (3 * 13, 3), (6, 3), (3, 3), (6, 0)):
+        S, o = state.clone(), torch.full((n, H * V), float("nan"), device=DEV)
+        scratch = torch.full((blocks * floats,), float("nan"), device=DEV)
+        ops.delta_scan(*args, S, o, i32(starts), i32(lens), i32(range(R)), H, G, D, V, channel, scratch, max(lens), walked=walked)
+        res.append((o, S))
+    assert all(torch.equal(o, res[0][0]) and torch.equal(S, res[0][1]) for o, S in res) and bool(res[0][0].isfinite().all())
+    with pytest.raises(ops.KernelError):
+        ops.delta_scan(*args, state.clone(), o, i32(starts), i32(lens), i32(range(R)), H, G, D, V, channel, scratch[:2 * floats], max(lens), walked=3)
+
+
+def test_scratch_of_long_portions_is_bounded():
+    from wllm_b200.kernels import ops
+    assert ops.delta_block_floats(2048, 1, 16, 128) == 257 * 16 * (25 * 128 + 64)
+    assert ops.delta_block_floats(16384, 1, 64, 128) <= 32 << 20 and ops.delta_block_floats(1 << 20, 4, 32, 256) <= 32 << 20

@@ -711,37 +711,41 @@ __host__ __device__ constexpr int db_channels(int D) { return D <= 64 ? 64 : (D 
 // a block's piece: [8][DP] G k, [8][DP] G q, [8][DP] M, [DP] G_7 - 1 (or G_7), [8][8] N
 __host__ __device__ constexpr int db_floats(int DP) { return (3 * DB + 1) * DP + DB * DB; }
 __host__ __device__ constexpr int db_stage_floats(int DP) { return db_floats(DP) + DB * DB_COLS; }      // with the values of the CTA's columns
-// The nth request (from 0) of `from` tokens or more: its index (-1 past the last) and, in `before`, the blocks of such requests in front of it: where
-// its pieces begin.  The grids count these requests alone: beside decoded tokens a CTA of a request that has none would still take its turn for
+// A turn takes `turn` blocks of every request from its block b0 on.  The nth request (from 0) of `from` tokens or more that has any: its index (-1 past
+// the last) and, in `before`, the turn's blocks of such requests in front of it: where its pieces begin.  The grids count these requests alone: beside decoded tokens a CTA of a request that has none would still take its turn for
 // the walk's shared memory.  A warp together.
-__device__ __forceinline__ int db_request(const int* __restrict__ req_q_len, int requests, int from, int nth, size_t& before) {
+__device__ __forceinline__ int db_request(const int* __restrict__ req_q_len, int requests, int from, int b0, int turn, int nth, size_t& before) {
     const int lane = threadIdx.x & 31;
     before = 0;
+    if (requests == 1) return req_q_len[0] >= from ? 0 : -1;
     for (int r0 = 0; r0 < requests; r0 += 32) {
-        const int len = r0 + lane < requests ? req_q_len[r0 + lane] : 0, blocks = len >= from ? (len + DB - 1) / DB : 0;
+        const int len = r0 + lane < requests ? req_q_len[r0 + lane] : 0, blocks = len >= from ? min((len + DB - 1) / DB - b0, turn) : 0;
         const unsigned found = __ballot_sync(0xffffffffu, blocks > 0);
-        const int count = __popc(found), at = nth < count ? (int)__fns(found, 0, nth + 1) : 32;
-        before += __reduce_add_sync(0xffffffffu, lane < at ? blocks : 0);
-        if (nth < count) return r0 + at;
-        nth -= count;
+        const unsigned here = __ballot_sync(0xffffffffu, blocks > 0 && __popc(found & ((1u << lane) - 1)) == nth);
+        const int at = here ? __ffs(here) - 1 : 32;
+        before += __reduce_add_sync(0xffffffffu, lane < at ? max(blocks, 0) : 0);
+        if (here) return r0 + at;
+        nth -= __popc(found);
     }
     return -1;
 }
 
+// (the bounds of both kernels keep the compiler from fitting one more CTA an SM with fewer registers: the walk of 2,041 tokens, a decay per channel,
+// takes 289 us instead of 276 then)
 template <int DP, bool CHANNEL>
-__global__ void __launch_bounds__(DP)
+__global__ void __launch_bounds__(DP, 896 / DP)
 delta_block_prepare_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ beta, const float* __restrict__ decay,
                            float* __restrict__ blocks, const int* __restrict__ req_q_start, const int* __restrict__ req_q_len,
-                           const int* __restrict__ req_slot, int requests, int H, int G, int D, int from) {
+                           const int* __restrict__ req_slot, int requests, int H, int G, int D, int from, int b0, int turn) {
     constexpr int WARPS = DP / 32, PAIRS = DB * (DB - 1) / 2;         // sums: 28 of A, then 36 of P
     __shared__ float sums[WARPS][64], A[DB][DB], P[DB][DB], T[DB][DB], bt[DB];
     pdl_begin();
     size_t before;
-    const int r = db_request(req_q_len, requests, from, blockIdx.z, before), h = blockIdx.y;
+    const int r = db_request(req_q_len, requests, from, b0, turn, blockIdx.z, before), h = blockIdx.y;
     if (r < 0 || req_slot[r] < 0) return;
-    const int len = req_q_len[r];
-    if (blockIdx.x * DB >= (unsigned)len) return;
-    const int t0 = req_q_start[r], first = t0 + blockIdx.x * DB, count = min(DB, len - (int)blockIdx.x * DB), g = h / (H / G);
+    const int at0 = (b0 + (int)blockIdx.x) * DB, len = req_q_len[r];
+    if (at0 >= len) return;
+    const int first = req_q_start[r] + at0, count = min(DB, len - at0), g = h / (H / G);
     const int d = threadIdx.x, warp = d >> 5, lane = d & 31;
     float kk[DB], qq[DB], e[DB];
 #pragma unroll
@@ -854,20 +858,20 @@ template <int NP>
 __device__ __forceinline__ int db_channel(int lane, int p) { return NP == 1 ? 2 * lane : 4 * lane + 128 * (p >> 1) + 2 * (p & 1); }
 
 template <int DP, bool CHANNEL>
-__global__ void __launch_bounds__(DB_THREADS)
+__global__ void __launch_bounds__(DB_THREADS, 2)
 delta_block_walk_kernel(const float* __restrict__ blocks, const float* __restrict__ v, float* __restrict__ state, float* __restrict__ out,
                         const int* __restrict__ req_q_start, const int* __restrict__ req_q_len, const int* __restrict__ req_slot, int requests,
-                        int H, int D, int V, int from) {
+                        int H, int D, int V, int from, int b0, int turn) {
     constexpr int FLOATS = db_floats(DP), STAGE = db_stage_floats(DP), NP = DP / 64;        // NP pairs of channels a thread and column
     extern __shared__ __align__(16) float db_smem[];                         // [DB_STAGES][DB_GROUP][STAGE]: a block's piece, [8][16] values
     __shared__ __align__(16) float rs[DB_THREADS / 32][2 * DB];
     pdl_begin();
     size_t before;
-    const int r = db_request(req_q_len, requests, from, blockIdx.z, before), h = blockIdx.y;
+    const int r = db_request(req_q_len, requests, from, b0, turn, blockIdx.z, before), h = blockIdx.y;
     if (r < 0) return;
-    const int len = req_q_len[r], slot = req_slot[r];
+    const int len = min(req_q_len[r] - b0 * DB, turn * DB), slot = req_slot[r];
     if (slot < 0) return;
-    const int t0 = req_q_start[r], count = (len + DB - 1) / DB;
+    const int t0 = req_q_start[r] + b0 * DB, count = (len + DB - 1) / DB;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int col0 = blockIdx.x * DB_COLS, col = col0 + 2 * warp;            // this warp's columns: col, col + 1
     const float* src = blocks + (before * H + h) * FLOATS;
@@ -981,18 +985,20 @@ delta_block_walk_kernel(const float* __restrict__ blocks, const float* __restric
     }
 }
 
-// Floats of scratch that wllm_delta_blocks needs for n tokens of `requests` requests.
+// Floats of scratch that wllm_delta_blocks wants for n tokens of `requests` requests: every block's piece, or DB_SCRATCH floats (128 MB; 5,100 tokens of 16 heads
+// of 128), whichever is less, but eight blocks a request.  Longer portions are walked in turns, the state handed on through its slot: the same bits.
+constexpr long long DB_SCRATCH = 32ll << 20;
 WLLM_API long long wllm_delta_block_floats(int n, int requests, int H, int D) {
-    return ((long long)n / DB + requests + 1) * H * db_floats(db_channels(D));
+    const long long block = (long long)H * db_floats(db_channels(D)), all = (long long)n / DB + requests;
+    long long most = DB_SCRATCH / block;
+    if (most < 8ll * requests) most = 8ll * requests;
+    return (all < most ? all : most) * block;
 }
 
 template <int DP, bool CHANNEL>
 static int launch_blocks(const float* q, const float* k, const float* v, const float* beta, const float* decay, float* state, float* out,
-                         float* blocks, const int* req_q_start, const int* req_q_len, const int* req_slot, int requests, int walked, int max_len,
-                         int H, int G, int D, int V, int from, int sms, cudaStream_t stream) {
-    const int code = wllm_launch(delta_block_prepare_kernel<DP, CHANNEL>, dim3((max_len + DB - 1) / DB, H, walked), DP, 0, stream, q, k, beta, decay,
-                                 blocks, req_q_start, req_q_len, req_slot, requests, H, G, D, from);
-    if (code != WLLM_OK) return code;
+                         float* blocks, const int* req_q_start, const int* req_q_len, const int* req_slot, int requests, int walked, int most,
+                         int H, int G, int D, int V, int from, int turn, int sms, cudaStream_t stream) {
     const dim3 grid((V + DB_COLS - 1) / DB_COLS, H, walked);
     constexpr size_t stage = (size_t)db_stage_floats(DP) * sizeof(float);      // 7,168, 13,568 or 26,368 bytes
     static bool raised = false;
@@ -1004,24 +1010,37 @@ static int launch_blocks(const float* q, const float* k, const float* v, const f
     size_t smem = DB_STAGES * DB_GROUP * stage;          // 42, 80 or 155 KB
     const size_t least = ((long long)grid.x * grid.y * grid.z <= sms ? 120 : 80) * 1024;       // at most one CTA an SM, or two
     if (smem < least) smem = least;
-    return wllm_launch(delta_block_walk_kernel<DP, CHANNEL>, grid, DB_THREADS, smem, stream, (const float*)blocks, v, state, out, req_q_start,
-                       req_q_len, req_slot, requests, H, D, V, from);
+    for (int b0 = 0; b0 < most; b0 += turn) {
+        const int mine = most - b0 < turn ? most - b0 : turn;
+        int code = wllm_launch(delta_block_prepare_kernel<DP, CHANNEL>, dim3(mine, H, walked), DP, 0, stream, q, k, beta, decay, blocks, req_q_start,
+                               req_q_len, req_slot, requests, H, G, D, from, b0, mine);
+        if (code == WLLM_OK)
+            code = wllm_launch(delta_block_walk_kernel<DP, CHANNEL>, grid, DB_THREADS, smem, stream, (const float*)blocks, v, state, out, req_q_start,
+                               req_q_len, req_slot, requests, H, D, V, from, b0, mine);
+        if (code != WLLM_OK) return code;
+    }
+    return WLLM_OK;
 }
 
-// wllm_delta_scan for the requests of `from` tokens or more (the longest has max_len; `walked`: how many there are, 0: not known); blocks: scratch of
-// wllm_delta_block_floats floats, 16-byte aligned; sms: the device's multiprocessors.
+// wllm_delta_scan for the requests of `from` tokens or more among the step's n (the longest has max_len; `walked`: how many there are, 0: not known).
+// blocks: scratch, 16-byte aligned, of the floats that wllm_delta_block_floats names or of any less that hold a block of each (more turns, the
+// same bits); sms: the device's multiprocessors.
 WLLM_API int wllm_delta_blocks(const float* q, const float* k, const float* v, const float* beta, const float* decay, int channel, float* state,
-                               float* out, float* blocks, const int* req_q_start, const int* req_q_len, const int* req_slot, int requests,
-                               int walked, int max_len, int H, int G, int D, int V, int from, int sms, cudaStream_t stream) {
+                               float* out, float* blocks, long long blocks_floats, const int* req_q_start, const int* req_q_len, const int* req_slot,
+                               int n, int requests, int walked, int max_len, int H, int G, int D, int V, int from, int sms, cudaStream_t stream) {
     if (requests <= 0 || max_len < from) return WLLM_OK;
     if (walked <= 0) walked = requests;
     if (walked > requests) return WLLM_BAD_SIZE;
     if (H <= 0 || H > 65535 || G <= 0 || H % G != 0 || requests > 65535 || D <= 0 || D > 256 || V <= 0 || from < 1) return WLLM_BAD_SIZE;
     if ((uintptr_t)blocks & 15) return WLLM_BAD_ALIGN;
-#define BLOCKS2(DP, C) launch_blocks<DP, C>(q, k, v, beta, decay, state, out, blocks, req_q_start, req_q_len, req_slot, requests, walked, max_len, H, \
-                                            G, D, V, from, sms, stream)
+    const int DP = db_channels(D), most = (max_len + DB - 1) / DB;
+    const long long room = blocks_floats / ((long long)H * db_floats(DP));             // blocks of all heads
+    const long long each = room >= (long long)n / DB + walked ? most : room / walked;  // (all of them, wherever they lie)
+    if (each < 1) return WLLM_BAD_SIZE;
+    const int turn = each < most ? (int)each : most;
+#define BLOCKS2(DP, C) launch_blocks<DP, C>(q, k, v, beta, decay, state, out, blocks, req_q_start, req_q_len, req_slot, requests, walked, most, H, \
+                                            G, D, V, from, turn, sms, stream)
 #define BLOCKS(DP) (channel ? BLOCKS2(DP, true) : BLOCKS2(DP, false))
-    const int DP = db_channels(D);
     return DP == 64 ? BLOCKS(64) : (DP == 128 ? BLOCKS(128) : BLOCKS(256));
 #undef BLOCKS
 #undef BLOCKS2

@@ -1259,7 +1259,7 @@ DELTA_BLOCKS_FROM = 16      # portions of at least two blocks of eight tokens ar
 
 
 def delta_block_floats(n: int, requests: int, heads: int, dim: int) -> int:
-    """Scratch of `delta_scan` for portions walked in blocks, in floats."""
+    """Scratch that `delta_scan` wants for portions walked in blocks, in floats (with less it takes them in more turns)."""
     fn = load_family("delta_rule").wllm_delta_block_floats
     fn.restype = ctypes.c_longlong
     return int(fn(n, requests, heads, dim))
@@ -1270,7 +1270,7 @@ def delta_scan(q, k, v, beta, decay, state, out, req_q_start, req_q_len, req_slo
     """The gated delta rule over every request's tokens of the step, in order, from and to its state slot:
     S <- decay S; u = beta (v - S^T k); S <- S + k u^T; out = S^T q.  q, k [n, kv_heads * dim], v, out [n, heads * vdim],
     beta, decay [n, heads], state [slots, heads, dim, vdim], all float32 (csrc/delta_rule.cu).  `channel`: decay
-    [n, heads * dim], one per key channel, given as decay - 1 (lowrank_map).  `blocks` (float32 scratch of delta_block_floats; the
+    [n, heads * dim], one per key channel, given as decay - 1 (lowrank_map).  `blocks` (float32 scratch, see delta_block_floats; the
     longest request has max_q_len tokens): requests of DELTA_BLOCKS_FROM tokens or more (exactly `walked`; 0: not known) are walked in blocks
     of eight tokens, whose sums run in another order.  `single`: no request brings more than one token (the same bits, another kernel)."""
     _need_cuda(q, k, v, beta, decay, state, out, req_q_start, req_q_len, req_slot, blocks)
@@ -1284,9 +1284,9 @@ def delta_scan(q, k, v, beta, decay, state, out, req_q_start, req_q_len, req_slo
     index = (_ptr(_int32(req_q_start, "req_q_start")), _ptr(_int32(req_q_len, "req_q_len")), _ptr(_int32(req_slot, "req_slot")))
     name = f"delta_scan(heads={heads}/{kv_heads}, dim={dim}/{vdim})"
     if blocks is not None and max_q_len >= DELTA_BLOCKS_FROM:
-        assert blocks.dtype == torch.float32 and blocks.is_contiguous() and blocks.numel() >= delta_block_floats(n, R, heads, dim)
+        assert blocks.dtype == torch.float32 and blocks.is_contiguous()
         _check(lib.wllm_delta_blocks(_ptr(q), _ptr(k), _ptr(v), _ptr(beta), _ptr(decay), 1 if channel else 0, _ptr(state), _ptr(out),
-                                     _ptr(blocks), *index, R, walked, max_q_len, heads, kv_heads, dim, vdim, DELTA_BLOCKS_FROM, sm_count(), _stream()), name)
+                                     _ptr(blocks), ctypes.c_longlong(blocks.numel()), *index, n, R, walked, max_q_len, heads, kv_heads, dim, vdim, DELTA_BLOCKS_FROM, sm_count(), _stream()), name)
         global launches
         launches += 1         # the blocks' matrices, then the walk
         if walked == R:
