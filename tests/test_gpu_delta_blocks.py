@@ -245,3 +245,56 @@ def test_scratch_of_long_portions_is_bounded():
     from wllm_b200.kernels import ops
     assert ops.delta_block_floats(2048, 1, 16, 128) == 257 * 16 * (25 * 128 + 64)
     assert ops.delta_block_floats(16384, 1, 64, 128) <= 32 << 20 and ops.delta_block_floats(1 << 20, 4, 32, 256) <= 32 << 20
+
+
+@pytest.mark.parametrize("design", ["Vifirax", "Gudarax"])                  # a decay per key channel, per head
+def test_a_long_portion_beside_many_single_tokens(design, monkeypatch):
+    """A whole bfloat16 step: a prompt that is walked in blocks, a short one and forty decoded tokens that are not; then a step of single tokens from the
+    states it left.  Beside the same steps by the walk alone."""
+    from wllm_b200.config import EngineConfig, resolve_architecture
+    from wllm_b200.engine import ComposedModel, StepEntry, build_runner
+    from wllm_b200.kernels import ops
+    from wllm_b200.parts.linear_attention import DeltaRule
+    dense, mixer = {"kind": "dense", "ff": 96}, {"heads": 4, "kv_heads": 2, "dim": 40, "vdim": 24, "conv": 4}
+    raw = {"architecture": design, "vocab": 211, "width": 64, "norm": {"eps": 1e-6}, "layers": [
+        {"type": "delta", "mlp": dense, "mixer": mixer} if design == "Gudarax" else
+        {"type": "channel_delta", "mlp": dense, "mixer": {**mixer, "kv_heads": 4, "decay_rank": 8, "gate_rank": 8}}] * 2}
+    if design == "Gudarax":
+        raw.update(max_positions=4096, embedding={"scale": 1.0}, token_side={"dim": 16})
+    arch = resolve_architecture(design)
+    cfg = arch.config_class.from_dict(raw, where=design)
+    gen = torch.Generator().manual_seed(5)
+    weights = {}
+    model = ComposedModel(arch.make_plan(cfg), torch.bfloat16)
+    for ps in model.param_specs():
+        shape = tuple(ps.shape)
+        t = torch.randn(shape, generator=gen) * (1.0 if ps.name.endswith("embed") else 0.3 if len(shape) > 1 else 0.1)
+        weights[ps.name] = (t + (1.0 if len(shape) == 1 and design == "Gudarax" else 0.0)).bfloat16().to(DEV)
+    draw = lambda n: torch.randint(0, 211, (n,), generator=gen).tolist()
+    prompt, short, firsts, seconds, thirds = draw(620), draw(30), [draw(3) for _ in range(40)], draw(40), draw(42)
+    asked = []
+    plain_scan = ops.delta_scan
+
+    def spy(*args, **kw):
+        asked.append((args[15] is not None, args[18]))
+        return plain_scan(*args, **kw)
+    monkeypatch.setattr(ops, "delta_scan", spy)
+
+    def steps(blocks):
+        if not blocks:
+            monkeypatch.setattr(DeltaRule, "BLOCKS_FROM", 1 << 30)
+            monkeypatch.setattr(DeltaRule, "CHANNEL_BLOCKS_FROM", 1 << 30)
+        model = ComposedModel(arch.make_plan(cfg), torch.bfloat16)
+        model.load(weights.__getitem__)
+        model.config = cfg
+        runner = build_runner(model, EngineConfig(dtype="bfloat16", block_size=64, max_num_seqs=42, device=DEV), num_pages=64)
+        rcs = [runner.cache.open(i) for i in range(42)]
+        runner.step([StepEntry(rc, t, []) for rc, t in zip(rcs, firsts)])
+        asked.clear()
+        out = [runner.step([StepEntry(rc, [t], [0]) for rc, t in zip(rcs[:20], seconds)] + [StepEntry(rcs[40], prompt, [0, 299, 619])] +
+                           [StepEntry(rc, [t], [0]) for rc, t in zip(rcs[20:40], seconds[20:])] + [StepEntry(rcs[41], short, [29])])]
+        assert asked == [(blocks, 1 if blocks else 0)] * 2, asked
+        return out + [runner.step([StepEntry(rc, [t], [0]) for rc, t in zip(rcs, thirds)])]
+    for got, want in zip(steps(True), steps(False)):
+        # two programs whose 32-bit sums fall differently, rounded to bfloat16 in two layers
+        assert bool(got.isfinite().all()) and float((got - want).norm() / want.norm()) < 2.5e-2

@@ -700,9 +700,9 @@ WLLM_API int wllm_delta_scan(const float* q, const float* k, const float* v, con
 //             Blocks arrive through a ring of cp.async stages.  The grid seldom exceeds the device's SMs, and a kernel that is
 //             launched early finds some SMs still full: it asks for more than half an SM's shared memory then, so that its CTAs do
 //             not pile up in pairs (the walk above took 1,490 us for 682 that way in a 2,048-token prompt of 16 heads of 128 x 128).
-// Measured, 16 heads of 128 x 128: 2,048 tokens with a decay per channel 682 us by the walk above when it has the device to itself and 1,490 us in a
-// step, 267 us here (the whole step 2,879 -> 1,704 us); prompts of 340, 680 and 1,021 tokens together 551 -> 264 us (2,026 -> 1,792 us).
-// Portions of fewer than two blocks stay on the walk above, and so do 32-bit models, whose results do not depend on how a prompt is cut.
+// Measured, 16 heads of 128 x 128, launches back to back: 2,048 tokens with a decay per channel 1,005 us by the walk above, 276 us here, a decay per head
+// 800 and 273 us; 64 tokens 38 and 16, 30 and 16 us.  (The step of a 2,048-token prompt that it first replaced the walk in: 2,879 -> 1,704 us.)
+// Which portions come here the caller says (`from`); 32-bit models stay on the walk, whose results do not depend on how a prompt is cut.
 // ---------------------------------------------------------------------------------------------------
 constexpr int DB = 8;                 // tokens of a block
 constexpr int DB_COLS = 16, DB_THREADS = 256;
@@ -1022,13 +1022,21 @@ static int launch_blocks(const float* q, const float* k, const float* v, const f
     return WLLM_OK;
 }
 
-// wllm_delta_scan for the requests of `from` tokens or more among the step's n (the longest has max_len; `walked`: how many there are, 0: not known).
-// blocks: scratch, 16-byte aligned, of the floats that wllm_delta_block_floats names or of any less that hold a block of each (more turns, the
+// wllm_delta_scan with the requests of `from` tokens or more among the step's n in blocks (the longest has max_len; `walked`: how many there are, 0: not
+// known), the others, if there are any, token by token behind them.  One call, since a step of short portions is bound by the host; launched: how many
+// kernels it was.  blocks: scratch, 16-byte aligned, of the floats that wllm_delta_block_floats names or of any less that hold a block of each (more turns, the
 // same bits); sms: the device's multiprocessors.
 WLLM_API int wllm_delta_blocks(const float* q, const float* k, const float* v, const float* beta, const float* decay, int channel, float* state,
                                float* out, float* blocks, long long blocks_floats, const int* req_q_start, const int* req_q_len, const int* req_slot,
-                               int n, int requests, int walked, int max_len, int H, int G, int D, int V, int from, int sms, cudaStream_t stream) {
-    if (requests <= 0 || max_len < from) return WLLM_OK;
+                               int n, int requests, int walked, int max_len, int H, int G, int D, int V, int from, int sms, int* launched,
+                               cudaStream_t stream) {
+    *launched = 0;
+    if (requests <= 0) return WLLM_OK;
+    if (max_len < from) {
+        *launched = 1;
+        return wllm_delta_scan(q, k, v, beta, decay, channel, state, out, req_q_start, req_q_len, req_slot, requests, H, G, D, V, from, 0, stream);
+    }
+    const bool rest = walked != requests;
     if (walked <= 0) walked = requests;
     if (walked > requests) return WLLM_BAD_SIZE;
     if (H <= 0 || H > 65535 || G <= 0 || H % G != 0 || requests > 65535 || D <= 0 || D > 256 || V <= 0 || from < 1) return WLLM_BAD_SIZE;
@@ -1038,10 +1046,13 @@ WLLM_API int wllm_delta_blocks(const float* q, const float* k, const float* v, c
     const long long each = room >= (long long)n / DB + walked ? most : room / walked;  // (all of them, wherever they lie)
     if (each < 1) return WLLM_BAD_SIZE;
     const int turn = each < most ? (int)each : most;
+    *launched = 2 * ((most + turn - 1) / turn) + (rest ? 1 : 0);
 #define BLOCKS2(DP, C) launch_blocks<DP, C>(q, k, v, beta, decay, state, out, blocks, req_q_start, req_q_len, req_slot, requests, walked, most, H, \
                                             G, D, V, from, turn, sms, stream)
 #define BLOCKS(DP) (channel ? BLOCKS2(DP, true) : BLOCKS2(DP, false))
-    return DP == 64 ? BLOCKS(64) : (DP == 128 ? BLOCKS(128) : BLOCKS(256));
+    const int code = DP == 64 ? BLOCKS(64) : (DP == 128 ? BLOCKS(128) : BLOCKS(256));
 #undef BLOCKS
 #undef BLOCKS2
+    if (code != WLLM_OK || !rest) return code;
+    return wllm_delta_scan(q, k, v, beta, decay, channel, state, out, req_q_start, req_q_len, req_slot, requests, H, G, D, V, from, 0, stream);
 }

@@ -26,6 +26,11 @@ class ComposedModel:
         # captured decode steps replay the launches their parts chose at capture (see parts/base.py); the run that
         # warms a capture up is undone for per-request state by the runner
         self.graph_safe = all(getattr(p, "graph_safe", False) for p in self.parts() + self.blocks)
+        # a part that weighs its launches against the device's time asks how much of a step it is
+        kinds = [{type(p) for p in self.blocks[run.block].parts()} for run in plan.runs]
+        for p in self.parts():
+            if hasattr(p, "share"):
+                p.share = sum(type(p) in k for k in kinds) / len(kinds)
         self.loaded = False
 
     def _assign_caches(self):

@@ -1255,7 +1255,7 @@ def delta_conv_update(fused, parts: int, offsets: dict, heads: int, kv_heads: in
                                       _ptr(conv_state), _stream()), "delta_conv_update")
 
 
-DELTA_BLOCKS_FROM = 16      # portions of at least two blocks of eight tokens are walked block by block (csrc/delta_rule.cu)
+DELTA_BLOCKS_FROM = 16      # the shortest requests that are walked in blocks of eight tokens: two blocks (csrc/delta_rule.cu)
 
 
 def delta_block_floats(n: int, requests: int, heads: int, dim: int) -> int:
@@ -1266,12 +1266,13 @@ def delta_block_floats(n: int, requests: int, heads: int, dim: int) -> int:
 
 
 def delta_scan(q, k, v, beta, decay, state, out, req_q_start, req_q_len, req_slot, heads: int, kv_heads: int, dim: int, vdim: int,
-               channel: bool = False, blocks: torch.Tensor | None = None, max_q_len: int = 0, single: bool = False, walked: int = 0):
+               channel: bool = False, blocks: torch.Tensor | None = None, max_q_len: int = 0, single: bool = False, walked: int = 0,
+               blocks_from: int = DELTA_BLOCKS_FROM):
     """The gated delta rule over every request's tokens of the step, in order, from and to its state slot:
     S <- decay S; u = beta (v - S^T k); S <- S + k u^T; out = S^T q.  q, k [n, kv_heads * dim], v, out [n, heads * vdim],
     beta, decay [n, heads], state [slots, heads, dim, vdim], all float32 (csrc/delta_rule.cu).  `channel`: decay
     [n, heads * dim], one per key channel, given as decay - 1 (lowrank_map).  `blocks` (float32 scratch, see delta_block_floats; the
-    longest request has max_q_len tokens): requests of DELTA_BLOCKS_FROM tokens or more (exactly `walked`; 0: not known) are walked in blocks
+    longest request has max_q_len tokens): requests of `blocks_from` tokens or more (exactly `walked`; 0: not known) are walked in blocks
     of eight tokens, whose sums run in another order.  `single`: no request brings more than one token (the same bits, another kernel)."""
     _need_cuda(q, k, v, beta, decay, state, out, req_q_start, req_q_len, req_slot, blocks)
     n = q.shape[0]
@@ -1280,20 +1281,20 @@ def delta_scan(q, k, v, beta, decay, state, out, req_q_start, req_q_len, req_slo
     assert decay.shape == (n, heads * dim if channel else heads)
     assert state.shape[1:] == (heads, dim, vdim)
     lib = load_family("delta_rule")
-    R, below = req_q_len.shape[0], 2 ** 31 - 1
+    R = req_q_len.shape[0]
     index = (_ptr(_int32(req_q_start, "req_q_start")), _ptr(_int32(req_q_len, "req_q_len")), _ptr(_int32(req_slot, "req_slot")))
     name = f"delta_scan(heads={heads}/{kv_heads}, dim={dim}/{vdim})"
-    if blocks is not None and max_q_len >= DELTA_BLOCKS_FROM:
+    if blocks is not None and max_q_len >= blocks_from:
         assert blocks.dtype == torch.float32 and blocks.is_contiguous()
+        launched = ctypes.c_int()
         _check(lib.wllm_delta_blocks(_ptr(q), _ptr(k), _ptr(v), _ptr(beta), _ptr(decay), 1 if channel else 0, _ptr(state), _ptr(out),
-                                     _ptr(blocks), ctypes.c_longlong(blocks.numel()), *index, n, R, walked, max_q_len, heads, kv_heads, dim, vdim, DELTA_BLOCKS_FROM, sm_count(), _stream()), name)
+                                     _ptr(blocks), ctypes.c_longlong(blocks.numel()), *index, n, R, walked, max_q_len, heads, kv_heads, dim, vdim,
+                                     blocks_from, sm_count(), ctypes.byref(launched), _stream()), name)
         global launches
-        launches += 1         # the blocks' matrices, then the walk
-        if walked == R:
-            return out
-        below = DELTA_BLOCKS_FROM
+        launches += launched.value - 1
+        return out
     _check(lib.wllm_delta_scan(_ptr(q), _ptr(k), _ptr(v), _ptr(beta), _ptr(decay), 1 if channel else 0, _ptr(state), _ptr(out),
-                               *index, R, heads, kv_heads, dim, vdim, below, 1 if single else 0, _stream()), name)
+                               *index, R, heads, kv_heads, dim, vdim, 2 ** 31 - 1, 1 if single else 0, _stream()), name)
     return out
 
 

@@ -224,6 +224,17 @@ class ParallelMean:
 @MIXERS.register("delta_rule")
 class DeltaRule:
     graph_safe = True
+    share = 1.0              # of the model's layers that hold such a mixer (the model says)
+    # From where on a bfloat16 model's portions are walked in blocks of tokens: the mean of the longest portion and of the step's tokens, times `share`.
+    # On the device blocks are faster from the first (16 tokens of 16 heads of 128 alone: 13.5 us by the walk, 9.1 in blocks; beside 32 single tokens
+    # from 128 on), but they are one launch more, two where other requests are walked beside them, of some ten microseconds on a host that a step
+    # of few tokens waits for.  Where a step becomes bound by the device (us, walk and blocks): one such layer of four, a decay per head, 512
+    # tokens 1,117 and 1,145, 768 1,247 and 1,176; a decay per channel 384 852 and 870, 512 946 and 889; five layers of six, 192 1,405 and 1,448, 256 1,452
+    # and 1,423; per channel 64 1,196 and 1,239, 128 1,456 and 1,259.
+    BLOCKS_FROM, CHANNEL_BLOCKS_FROM = 192, 128
+    # The shortest request that takes part: many short ones fill the device either way (64 of 20 tokens 230 us by the walk, 292 in blocks; 32 of 40 194
+    # and 195, per channel 233 and 200; 16 of 64 144 and 136, 176 and 137).
+    REQUEST_FROM = 40
 
     def __init__(self, spec, hidden_size: int, model_dtype: torch.dtype):
         self.heads, self.kv_heads = int(spec.num_heads), int(spec.num_kv_heads)
@@ -309,14 +320,14 @@ class DeltaRule:
         fused, parts = ops.project(x, self.w_in, lambda name, shape, dt: ctx.buffer(self.tag + "delta_in_" + name, shape, dt))
         return self.mix(fused, parts, 0, ctx, cache)
 
-    @staticmethod
-    def _walked(ctx) -> int:
-        """How many of the step's requests are walked in blocks (0: their lengths are not on the host); counted once a step."""
-        if getattr(ctx, "host", None) is None:
-            return 0
-        if "delta_walked" not in ctx.memo:
-            ctx.memo["delta_walked"] = int((ctx.host["req_q_len"] >= ops.DELTA_BLOCKS_FROM).sum())
-        return ctx.memo["delta_walked"]
+    def _in_blocks(self, ctx, n: int) -> tuple:
+        """(floats of scratch, requests walked in blocks (0: their lengths are not on the host)), worked out once a step."""
+        key = ("delta_blocks", self.heads, self.dim)
+        if key not in ctx.memo:
+            host = getattr(ctx, "host", None)
+            ctx.memo[key] = (ops.delta_block_floats(n, ctx.n_requests, self.heads, self.dim),
+                             0 if host is None else int((host["req_q_len"] >= self.REQUEST_FROM).sum()))
+        return ctx.memo[key]
 
     def mix(self, fused: torch.Tensor, parts: int, col0: int, ctx, cache: CacheRef):
         """The mixer on the columns from col0 of a fused product [n, W] (or partial sums [parts, n, W])."""
@@ -339,13 +350,14 @@ class DeltaRule:
         if channel:
             ops.lowrank_map(fused, parts, off["a_low"], self.decay_up, H, D, decay, self.dt_bias, self.a_log)
         o = ctx.buffer(self.tag + "delta_o", (n, H * V), f32)
-        # portions of a bfloat16 model in blocks of tokens; a 32-bit model's walk gives the same bits however a prompt is cut
+        # (a 32-bit model's walk gives the same bits however a prompt is cut)
         blocks, walked = None, 0
-        if self.model_dtype == torch.bfloat16 and ctx.max_q_len >= ops.DELTA_BLOCKS_FROM:
-            walked = self._walked(ctx)
-            blocks = ctx.buffer(self.tag + "delta_blocks", (ops.delta_block_floats(n, ctx.n_requests, H, D),), f32)
+        if self.model_dtype == torch.bfloat16 and ctx.max_q_len >= self.REQUEST_FROM and \
+                (ctx.max_q_len + n) * self.share >= 2 * (self.CHANNEL_BLOCKS_FROM if channel else self.BLOCKS_FROM):
+            floats, walked = self._in_blocks(ctx, n)
+            blocks = ctx.buffer(self.tag + "delta_blocks", (floats,), f32)
         ops.delta_scan(q, k, v, beta, decay, ctx.state(cache.state_names["state"]), o, ctx.req_q_start, ctx.req_q_len, ctx.req_slot,
-                       H, G, D, V, channel, blocks, ctx.max_q_len, single, walked)
+                       H, G, D, V, channel, blocks, ctx.max_q_len, single, walked, self.REQUEST_FROM)
         gated = ctx.buffer(self.tag + "delta_gated", (n, H * V), self.model_dtype)
         if self.gate_maps is None:
             ops.head_gate_norm(o, fused, parts, off["g"], self.norm_weight, self.eps, gated, H, V)
