@@ -66,9 +66,9 @@ def test_blocks_of_tokens_give_the_recurrence(lens, sizes, memory, channel):
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("sizes", [(2, 1, 8, 5), (4, 2, 128, 128), (1, 1, 200, 256)])       # a part of a warp's lanes; all of them; two rounds
-@pytest.mark.parametrize("lens", [[64], [3, 61, 1], [130, 7]])                             # runs that end in the middle and hold several requests
+@pytest.mark.parametrize("lens", [[2800], [3, 2797, 1], [1030, 7, 1766]])                  # runs that end in the middle and hold several requests
 def test_runs_of_tokens_are_prepared_as_one_by_one(lens, sizes, dtype):
-    """A step of 64 tokens or more takes the kernel that walks runs; the same requests in portions of at most 31 tokens do not: the same bits."""
+    """A step of so many tokens takes the kernel that walks runs; the same requests in portions of at most 31 tokens do not: the same bits."""
     from wllm_b200.kernels import ops
     H, G, D, V = sizes
     gen = torch.Generator().manual_seed(sum(lens) + D)

@@ -53,7 +53,10 @@ constexpr int DR_MAX_PER_LANE = 8;       // key or value channels a lane holds o
 
 // grid (tokens, ceil(units / 4)), 128 threads; unit < G: a query head, < 2G: a key head, < 2G + H: a value head, 2G + H: the
 // token's beta and decay of every head.
-__global__ void __launch_bounds__(128)
+// MULTI: the inputs may be slabs.  A tensor's tokens do without the registers of sixteen loads in flight, so that nine CTAs share an SM, not five
+// (48 heads of 128, 64 tokens: 12.7 us with them, 8.0 without; 24 heads, 128 tokens 12.6 and 7.9).
+template <bool MULTI>
+__global__ void __launch_bounds__(128, MULTI ? 5 : 9)
 delta_prepare_kernel(const void* __restrict__ fused, int in_dtype, int row_stride, int parts, size_t part_stride, int q_off,
                      int k_off, int v_off, int b_off, int a_off, int n, int H, int G, int D, int V, int taps,
                      const void* __restrict__ conv_q, const void* __restrict__ conv_k, const void* __restrict__ conv_v,
@@ -62,15 +65,16 @@ delta_prepare_kernel(const void* __restrict__ fused, int in_dtype, int row_strid
                      const int* __restrict__ req_slot, float* __restrict__ conv_state, float unit_eps, float q_scale, float* __restrict__ q,
                      float* __restrict__ k, float* __restrict__ v, float* __restrict__ beta, float* __restrict__ decay, int shift) {
     pdl_begin();
+    auto in = [&](size_t at) { return MULTI ? dr_in(fused, in_dtype, parts, part_stride, at) : dr_any(fused, in_dtype, at); };
     const int t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int unit = blockIdx.y * 4 + warp;
     if (unit > 2 * G + H) return;
     if (unit == 2 * G + H) {
         for (int h = lane; h < H; h += 32) {
-            const float bz = dr_in(fused, in_dtype, parts, part_stride, (size_t)t * row_stride + b_off + h);
+            const float bz = in((size_t)t * row_stride + b_off + h);
             beta[(size_t)t * H + h] = 1.0f / (1.0f + expf(-bz));
             if (a_off < 0) continue;                        // decays per key channel: worked out elsewhere
-            const float az = dr_in(fused, in_dtype, parts, part_stride, (size_t)t * row_stride + a_off + h);
+            const float az = in((size_t)t * row_stride + a_off + h);
             decay[(size_t)t * H + h] = expf(-expf(dr_any(a_log, w_dtype, h)) * dr_softplus(az + dr_any(dt_bias, w_dtype, h)));
         }
         return;
@@ -94,7 +98,7 @@ delta_prepare_kernel(const void* __restrict__ fused, int in_dtype, int row_strid
             float acc = 0.f;
             for (int j = taps - 1; j >= 0; --j) {            // the oldest input first: one order for every way of cutting
                 float x;
-                if (i - j >= 0) x = dr_in(fused, in_dtype, parts, part_stride, (size_t)(t - j) * row_stride + col0 + c);
+                if (i - j >= 0) x = in((size_t)(t - j) * row_stride + col0 + c);
                 else x = slot >= 0 ? conv_state[((size_t)slot * (taps - 1) + (taps - 1 + i - j)) * C + chan0 + c] : 0.f;
                 acc = fmaf(dr_any(w, w_dtype, (size_t)(head * size + c) * taps + (taps - 1 - j)), x, acc);
                 // every request brings one token: input j tokens back becomes input j + 1 back of the next one
@@ -602,13 +606,16 @@ WLLM_API int wllm_delta_prepare(const void* fused, int in_dtype, int row_stride,
     if ((in_dtype != WLLM_BF16 && in_dtype != WLLM_F32) || (w_dtype != WLLM_BF16 && w_dtype != WLLM_F32)) return WLLM_BAD_DTYPE;
     const int units = 2 * G + H + 1;
     if ((units + 3) / 4 > 65535) return WLLM_BAD_SIZE;
-    // runs from 64 tokens on: fewer are latency-bound either way, and single tokens also bring the slots' inputs up to date
-    if (n >= 64 && parts == 1 && taps == DR_RUN_TAPS && !shift) {
+    // Runs where the CTAs of a token (and four heads) each would not be on the SMs at once, nine an SM: until then a run's eight tokens one after the
+    // other are the longer chain.  48 heads of 128, 104 tokens (1,352 CTAs) 8.1 us a token each and 9.9 in runs, 128 (1,664) 12.6 and 9.9, 512 31 and 19;
+    // 24 heads, 192 tokens 8.0 and 9.9, 224 (1,568) 12.1 and 9.9; heads of 64, 1,568 CTAs 7.7 and 8.3, 2,400 8.7 and 8.4.  Runs of heads over
+    // 128 hold twice the registers and take twice the time: from a third round on (256, 2,048 CTAs 22.4 and 24.1).
+    const bool few = D <= 128 && V <= 128;
+    if ((long long)n * ((units + 3) / 4) > (few ? 1400 : 2700) && parts == 1 && taps == DR_RUN_TAPS && !shift) {
         const dim3 rgrid((n + DR_RUN - 1) / DR_RUN, (units + 3) / 4);
 #define RUN(TI, PER) wllm_launch(delta_prepare_run_kernel<TI, PER>, rgrid, 128, 0, stream, (const TI*)fused, row_stride, q_off, k_off, v_off, b_off, \
                                  a_off, n, H, G, D, V, conv_q, conv_k, conv_v, a_log, dt_bias, w_dtype, token_req, req_q_start, req_slot, \
                                  (const float*)conv_state, unit_eps, q_scale, q, k, v, beta, decay)
-        const bool few = D <= 128 && V <= 128;
         if (in_dtype == WLLM_BF16) return few ? RUN(bf16, 4) : RUN(bf16, 8);
         return few ? RUN(float, 4) : RUN(float, 8);
 #undef RUN
@@ -617,11 +624,11 @@ WLLM_API int wllm_delta_prepare(const void* fused, int in_dtype, int row_stride,
 #define ONE(PER) wllm_launch(delta_prepare_single_kernel<PER>, dim3(n, (units + 3) / 4), 128, 0, stream, fused, in_dtype, row_stride, parts, \
                              (size_t)part_stride, q_off, k_off, v_off, b_off, a_off, H, G, D, V, conv_q, conv_k, conv_v, a_log, dt_bias, w_dtype, \
                              token_req, req_q_len, req_slot, conv_state, unit_eps, q_scale, q, k, v, beta, decay)
-        return D <= 128 && V <= 128 ? ONE(4) : ONE(8);
+        return few ? ONE(4) : ONE(8);
 #undef ONE
     }
-    return wllm_launch(delta_prepare_kernel, dim3(n, (units + 3) / 4), 128, 0, stream, fused, in_dtype, row_stride, parts,
-                       (size_t)part_stride, q_off, k_off, v_off, b_off, a_off, n, H, G, D, V, taps, conv_q, conv_k, conv_v, a_log,
+    return wllm_launch(parts > 1 ? delta_prepare_kernel<true> : delta_prepare_kernel<false>, dim3(n, (units + 3) / 4), 128, 0, stream, fused, in_dtype,
+                       row_stride, parts, (size_t)part_stride, q_off, k_off, v_off, b_off, a_off, n, H, G, D, V, taps, conv_q, conv_k, conv_v, a_log,
                        dt_bias, w_dtype, token_req, req_q_start, req_q_len, req_slot, conv_state, unit_eps, q_scale, q, k, v, beta, decay, shift);
 }
 
