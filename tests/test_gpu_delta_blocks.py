@@ -298,3 +298,31 @@ def test_a_long_portion_beside_many_single_tokens(design, monkeypatch):
     for got, want in zip(steps(True), steps(False)):
         # two programs whose 32-bit sums fall differently, rounded to bfloat16 in two layers
         assert bool(got.isfinite().all()) and float((got - want).norm() / want.norm()) < 2.5e-2
+
+
+@pytest.mark.parametrize("parts", [0, 1, 2, 9, 17])                    # a tensor; a slab; fewer than are asked for at once; more
+@pytest.mark.parametrize("lens", [[5, 1, 9], [120, 1, 40], [3] * 40])    # CTAs that lie on the device at once; more of them; more requests
+def test_inputs_in_slabs_are_their_sums(parts, lens):
+    """The convolutions' inputs and kept inputs from slabs, however many loads are in flight, beside the same from their sum, added up in order."""
+    from wllm_b200.kernels import ops
+    H, G, D, V, T = 32, 16, 40, 24, 4
+    gen = torch.Generator().manual_seed(parts + len(lens))
+    n, R, C = sum(lens), len(lens), 2 * G * D + H * V
+    off = {"q": 0, "k": G * D, "v": 2 * G * D, "b": C, "a": C + H}
+    fused = torch.randn(*([parts] if parts else []), n, C + 2 * H, generator=gen).to(DEV)
+    whole = fused if not parts else fused[0].clone()
+    for part in fused[1:] if parts else ():
+        whole += part
+    taps = [torch.randn(c, T, generator=gen).to(DEV) for c in (G * D, G * D, H * V)]
+    a_log, dt_bias = (torch.randn(H, generator=gen).to(DEV) for _ in range(2))
+    conv0 = torch.randn(R, T - 1, C, generator=gen).to(DEV)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    starts, slots = i32([sum(lens[:r]) for r in range(R)]), i32(range(R))
+    req = torch.cat([torch.full((m,), r, dtype=torch.int32) for r, m in enumerate(lens)]).to(DEV)
+    res = []
+    for x, p in ((fused, parts), (whole, 0)):
+        conv, out = conv0.clone(), [torch.empty(n, w, device=DEV) for w in (G * D, G * D, H * V, H, H)]
+        ops.delta_prepare(x, p, off, H, G, D, V, T, *taps, a_log, dt_bias, req, starts, slots, conv, 1e-6, D ** -0.5, *out)
+        ops.delta_conv_update(x, p, off, H, G, D, V, T, starts, i32(lens), slots, conv)
+        res.append(out + [conv])
+    assert all(torch.equal(a, b) for a, b in zip(*res))

@@ -31,16 +31,23 @@ __device__ __forceinline__ float dr_any(const void* p, int dtype, size_t i) {
     return dtype == WLLM_BF16 ? __bfloat162float(reinterpret_cast<const bf16*>(p)[i]) : reinterpret_cast<const float*>(p)[i];
 }
 // element i of a row that may come as `parts` 32-bit slabs `stride` elements apart, added in slab order
+// An input from a tensor (AT_ONCE 0) or, where parts > 1, from slabs: part 0 + part 1 + ..., AT_ONCE loads in flight, the additions a chain.
+template <int AT_ONCE>
 __device__ __forceinline__ float dr_in(const void* p, int dtype, int parts, size_t stride, size_t i) {
-    if (parts == 1) return dr_any(p, dtype, i);
+    if (AT_ONCE == 0 || parts == 1) return dr_any(p, dtype, i);
     const float* f = reinterpret_cast<const float*>(p) + i;
+    if (AT_ONCE == 1) {
+        float v = f[0];
+        for (int s = 1; s < parts; ++s) v += f[(size_t)s * stride];
+        return v;
+    }
     float v = 0.f;
-    for (int s0 = 0; s0 < parts; s0 += 16) {          // sixteen loads in flight, the additions a chain
-        float part[16];
+    for (int s0 = 0; s0 < parts; s0 += AT_ONCE) {
+        float part[AT_ONCE ? AT_ONCE : 1];
 #pragma unroll
-        for (int u = 0; u < 16; ++u) part[u] = s0 + u < parts ? f[(size_t)(s0 + u) * stride] : 0.f;
+        for (int u = 0; u < AT_ONCE; ++u) part[u] = s0 + u < parts ? f[(size_t)(s0 + u) * stride] : 0.f;
 #pragma unroll
-        for (int u = 0; u < 16; ++u)
+        for (int u = 0; u < AT_ONCE; ++u)
             if (s0 + u < parts) v = s0 + u == 0 ? part[u] : v + part[u];
     }
     return v;
@@ -53,10 +60,12 @@ constexpr int DR_MAX_PER_LANE = 8;       // key or value channels a lane holds o
 
 // grid (tokens, ceil(units / 4)), 128 threads; unit < G: a query head, < 2G: a key head, < 2G + H: a value head, 2G + H: the
 // token's beta and decay of every head.
-// MULTI: the inputs may be slabs.  A tensor's tokens do without the registers of sixteen loads in flight, so that nine CTAs share an SM, not five
-// (48 heads of 128, 64 tokens: 12.7 us with them, 8.0 without; 24 heads, 128 tokens 12.6 and 7.9).
-template <bool MULTI>
-__global__ void __launch_bounds__(128, MULTI ? 5 : 9)
+// AT_ONCE: slabs with eight loads in flight take registers that leave five CTAs an SM, one after the other nine, as a tensor's tokens.  48 heads of
+// 128 in five slabs, us with sixteen, eight and one at once: 24 tokens (312 CTAs) 14.9, 10.7, 11.3; 64 (832) 20.8, 16.9, 13.5.  A tensor, 64 tokens:
+// 12.7 with the registers, 8.0 without.
+constexpr int DR_PREPARE_CTAS = 5 * 148;
+template <int AT_ONCE>
+__global__ void __launch_bounds__(128, AT_ONCE > 1 ? 5 : 9)
 delta_prepare_kernel(const void* __restrict__ fused, int in_dtype, int row_stride, int parts, size_t part_stride, int q_off,
                      int k_off, int v_off, int b_off, int a_off, int n, int H, int G, int D, int V, int taps,
                      const void* __restrict__ conv_q, const void* __restrict__ conv_k, const void* __restrict__ conv_v,
@@ -65,7 +74,7 @@ delta_prepare_kernel(const void* __restrict__ fused, int in_dtype, int row_strid
                      const int* __restrict__ req_slot, float* __restrict__ conv_state, float unit_eps, float q_scale, float* __restrict__ q,
                      float* __restrict__ k, float* __restrict__ v, float* __restrict__ beta, float* __restrict__ decay, int shift) {
     pdl_begin();
-    auto in = [&](size_t at) { return MULTI ? dr_in(fused, in_dtype, parts, part_stride, at) : dr_any(fused, in_dtype, at); };
+    auto in = [&](size_t at) { return dr_in<AT_ONCE>(fused, in_dtype, parts, part_stride, at); };
     const int t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int unit = blockIdx.y * 4 + warp;
     if (unit > 2 * G + H) return;
@@ -235,10 +244,10 @@ delta_prepare_single_kernel(const void* __restrict__ fused, int in_dtype, int ro
     if (unit == 2 * G + H) {
         pdl_wait();
         for (int h = lane; h < H; h += 32) {
-            const float bz = dr_in(fused, in_dtype, parts, part_stride, (size_t)t * row_stride + b_off + h);
+            const float bz = dr_in<16>(fused, in_dtype, parts, part_stride, (size_t)t * row_stride + b_off + h);
             beta[(size_t)t * H + h] = 1.0f / (1.0f + expf(-bz));
             if (a_off < 0) continue;
-            const float az = dr_in(fused, in_dtype, parts, part_stride, (size_t)t * row_stride + a_off + h);
+            const float az = dr_in<16>(fused, in_dtype, parts, part_stride, (size_t)t * row_stride + a_off + h);
             decay[(size_t)t * H + h] = expf(-expf(dr_any(a_log, w_dtype, h)) * dr_softplus(az + dr_any(dt_bias, w_dtype, h)));
         }
         return;
@@ -265,7 +274,7 @@ delta_prepare_single_kernel(const void* __restrict__ fused, int in_dtype, int ro
         const int c = lane + 32 * e;
 #pragma unroll
         for (int j = 0; j < TAPS - 1; ++j) x[e][j] = c < size && slot >= 0 ? st[(size_t)j * C + c] : 0.f;
-        x[e][TAPS - 1] = c < size ? dr_in(fused, in_dtype, parts, part_stride, (size_t)t * row_stride + col0 + c) : 0.f;
+        x[e][TAPS - 1] = c < size ? dr_in<16>(fused, in_dtype, parts, part_stride, (size_t)t * row_stride + col0 + c) : 0.f;
     }
     float y[PER], ss = 0.f;
 #pragma unroll
@@ -289,7 +298,10 @@ delta_prepare_single_kernel(const void* __restrict__ fused, int in_dtype, int ro
         if (lane + 32 * e < size) dst[lane + 32 * e] = unit < 2 * G ? y[e] * inv : y[e];
 }
 
-// grid (requests, ceil(C / 256)): a thread a channel; the taps - 1 inputs that end at the request's last token of this step
+// grid (requests, ceil(C / 256)): a thread a channel; the taps - 1 inputs that end at the request's last token of this step.  AT_ONCE: as above (6,144
+// channels, us with sixteen, eight and one at once: a tensor, 48 requests 5.8 with the registers, 3.9 without; eight slabs, 1 request 3.6, 3.1, 4.6, 64 9.5,
+// 7.7, 6.5)
+template <int AT_ONCE>
 __global__ void __launch_bounds__(256)
 delta_conv_update_kernel(const void* __restrict__ fused, int in_dtype, int row_stride, int parts, size_t part_stride, int q_off,
                          int k_off, int v_off, int H, int G, int D, int V, int taps, const int* __restrict__ req_q_start,
@@ -307,7 +319,7 @@ delta_conv_update_kernel(const void* __restrict__ fused, int in_dtype, int row_s
     for (int s = 0; s < DR_MAX_TAPS; ++s) {
         if (s < keep) {
             const int src = len - keep + s;               // place among this step's tokens; negative: an input kept from before
-            vals[s] = src >= 0 ? dr_in(fused, in_dtype, parts, part_stride, (size_t)(t0 + src) * row_stride + col)
+            vals[s] = src >= 0 ? dr_in<AT_ONCE>(fused, in_dtype, parts, part_stride, (size_t)(t0 + src) * row_stride + col)
                                : st[(size_t)(s + len) * C];
         }
     }
@@ -627,7 +639,8 @@ WLLM_API int wllm_delta_prepare(const void* fused, int in_dtype, int row_stride,
         return few ? ONE(4) : ONE(8);
 #undef ONE
     }
-    return wllm_launch(parts > 1 ? delta_prepare_kernel<true> : delta_prepare_kernel<false>, dim3(n, (units + 3) / 4), 128, 0, stream, fused, in_dtype,
+    const bool many = (long long)n * ((units + 3) / 4) > DR_PREPARE_CTAS;
+    return wllm_launch(parts == 1 ? delta_prepare_kernel<0> : many ? delta_prepare_kernel<1> : delta_prepare_kernel<8>, dim3(n, (units + 3) / 4), 128, 0, stream, fused, in_dtype,
                        row_stride, parts, (size_t)part_stride, q_off, k_off, v_off, b_off, a_off, n, H, G, D, V, taps, conv_q, conv_k, conv_v, a_log,
                        dt_bias, w_dtype, token_req, req_q_start, req_q_len, req_slot, conv_state, unit_eps, q_scale, q, k, v, beta, decay, shift);
 }
@@ -640,8 +653,9 @@ WLLM_API int wllm_delta_conv_update(const void* fused, int in_dtype, int row_str
     if (in_dtype != WLLM_BF16 && in_dtype != WLLM_F32) return WLLM_BAD_DTYPE;
     const int C = 2 * G * D + H * V;
     if ((C + 255) / 256 > 65535) return WLLM_BAD_SIZE;
-    return wllm_launch(delta_conv_update_kernel, dim3(requests, (C + 255) / 256), 256, 0, stream, fused, in_dtype, row_stride, parts,
-                       (size_t)part_stride, q_off, k_off, v_off, H, G, D, V, taps, req_q_start, req_q_len, req_slot, conv_state);
+    const bool many = (long long)requests * ((C + 255) / 256) > 4 * 148;
+    return wllm_launch(parts == 1 ? delta_conv_update_kernel<0> : many ? delta_conv_update_kernel<1> : delta_conv_update_kernel<8>,
+                       dim3(requests, (C + 255) / 256), 256, 0, stream, fused, in_dtype, row_stride, parts, (size_t)part_stride, q_off, k_off, v_off, H, G, D, V, taps, req_q_start, req_q_len, req_slot, conv_state);
 }
 
 // state [slots, H, D, V]; out [n, H, V].  Requests by start, length and state slot; a length of 0 or a slot of -1 is passed by.
