@@ -9,12 +9,12 @@
 // engine independent of batching.  (Zero padding past K adds fma(0, 0, acc) = acc.)
 //
 // Three kernels with that same arithmetic:
-//   wide kernel    steps of more than 64 rows (K and the pitches in steps of 4 floats, 16-byte aligned operands), bound by the FMA pipes:
-//                  see gemm_f32_wide_kernel.
-//   tile kernel    steps of 33 to 64 rows, and operands that the others do not take: BM x 128 x 16 tiles (BM = 64 or 128), 256
+//   tile kernel    steps of more than 32 rows, bound by the FMA pipes: BM x 128 x 16 tiles (BM = 64 or 128), 256
 //                  threads with 4 x 8 or 8 x 8 outputs each, operands transposed in shared memory and read
 //                  as float4, the next tile fetched into registers while the current one is multiplied; the
 //                  sums of finished segments wait in shared memory.
+//   wide kernel    steps of more than 64 rows (K and the pitches in steps of 4 floats, 16-byte aligned operands) where it is faster: tiles cut by
+//                  segments, a CTA each, and very many tiles; see gemm_f32_wide_kernel and wide_segments.
 //   skinny kernel  steps of at most 32 rows, bound by streaming W once: a warp owns 32 rows of W and one
 //                  segment (so a matrix of few rows and long K still gives every SM many warps), streams it
 //                  through its own ring of cp.async stages and keeps one chain per row of A in each lane;
@@ -260,12 +260,11 @@ gemm_f32_skinny_kernel(const float* __restrict__ A, int lda, const float* __rest
 // multiply-add of its own chain, so the bits are the same): the pipes' peak is no higher for it (73.4 against 71.9 TFLOP/s in a loop), but half the
 // instructions compete for the schedulers and the register ports.  And a thread has twice the columns, 24 floats read from shared memory
 // for 128 products instead of 16 for 64.  A launch's last round
-// finds its SMs half empty and runs faster, so the tiles need not divide evenly.  A launch whose tiles would not fill the device twice is
-// cut by segments, a CTA each: the sums go to slabs that the fold kernel adds in the same ascending order.  (A tile that walks several segments
-// keeps their running total in C.)
-// 512 x 32,768 x 2,048 without the guards: 8 x 8 outputs 1,640 us, in pairs 1,501; 8 x 16 1,714, in pairs 1,334 (51.5 TFLOP/s).  Rows left as they lie in
-// memory, brought by cp.async and read four k at a time, cannot be paired: 39 TFLOP/s; A that way and W transposed: 51.
-// A Gemma-2B prompt of 509 tokens, 72 such products of 509 rows, K 2,048 and 16,384: 78.6 -> 54.5 ms, the down products 1,758 -> 758 us each.
+// finds its SMs half empty and runs faster, so the tiles need not divide evenly.  Tiles cut by segments leave their
+// sums in slabs that the fold kernel adds in the same ascending order, in turns of as many segments as WIDE_SLABS floats hold; a tile that walks several
+// segments keeps their running total in C.  (Rows left as they lie in memory, brought by cp.async and read four k at a time, cannot be paired: 39 TFLOP/s;
+// A that way and W transposed: 51.)  Which products come here: wide_segments.  Measured in turn with the tile kernel, us: 509 x 2,048 x 16,384 cut 1,766 ->
+// 766, 509 x 2,048 x 2,048 cut 261 -> 212, 4,096 x 32,768 x 2,048 whole 11,347 -> 11,084 (49.6 TFLOP/s).
 // ------------------------------------------------------------------------------------------------
 constexpr int WT = 128, WTHREADS = 128;
 
@@ -379,15 +378,16 @@ gemm_f32_wide_kernel(const float* __restrict__ A, int lda, const float* __restri
     leave(tiles > SEG / TBK);
 }
 
-// C[m][n] = the segments' sums added in ascending order.
+// C[m][n] = the segments' sums added in ascending order, behind (add) those that it holds.
 __global__ void __launch_bounds__(256)
-gemm_f32_fold_kernel(const float* __restrict__ parts, float* __restrict__ C, int ldc, int M, int N, int segs) {
+gemm_f32_fold_kernel(const float* __restrict__ parts, float* __restrict__ C, int ldc, int M, int N, int segs, bool add) {
     pdl_begin();
     const size_t idx = (size_t)blockIdx.x * 256 + threadIdx.x;
     if (idx >= (size_t)M * N) return;
-    float total = parts[idx];
+    float* to = C + (idx / N) * ldc + idx % N;
+    float total = add ? *to + parts[idx] : parts[idx];
     for (int s = 1; s < segs; ++s) total = total + parts[(size_t)s * M * N + idx];
-    C[(idx / N) * ldc + idx % N] = total;
+    *to = total;
 }
 
 template <int BM, int STAGES>
@@ -408,7 +408,7 @@ static int launch_skinny_as(const float* A, int lda, const float* W, int ldw, fl
                                A, lda, W, ldw, dst, segs > 1 ? N : ldc, (long long)M * N, M, N, K, segs, tasks);
     if (st != WLLM_OK || segs == 1) return st;
     return wllm_launch(gemm_f32_fold_kernel, dim3((unsigned)(((size_t)M * N + 255) / 256)), 256, 0, stream,
-                       (const float*)scratch, C, ldc, M, N, segs);
+                       (const float*)scratch, C, ldc, M, N, segs, false);
 }
 
 template <int BM>
@@ -444,9 +444,28 @@ static int launch_tile(const float* A, int lda, const float* W, int ldw, float* 
     return wllm_launch(gemm_f32_tile_kernel<BM, VEC>, grid, 256, totals, stream, A, lda, W, ldw, C, ldc, M, N, K);
 }
 
-// Whether a product of the wide kernel is cut by segments: its tiles fill fewer than two rounds of two CTAs an SM.  The slabs cost some five per cent
-// (a segment of an output is 1,024 products and 8 bytes there and back), an uneven last round of more than two costs less.
-static int wide_splits(int M, int N, int K) {
+// The most slabs' floats that a product asks for (256 MB).  A product that is cut has at most 592 tiles, so that a turn has some 4,000 CTAs and more,
+// fourteen rounds of two an SM; slabs without a bound were 600 MB for 4,608 x 2,048 x 16,384.  (4,096 x 2,048 x 16,384: 5,672 us at once, 6,071 in turns of four.)
+constexpr long long WIDE_SLABS = 64ll << 20;
+
+// Segments of a turn for `floats` of scratch.
+static int turn_of(int M, int N, int segs, long long floats) {
+    const long long room = floats / ((long long)M * N);
+    return (int)(room < segs ? (room < 65535 ? room : 65535) : (segs < 65535 ? segs : 65535));
+}
+
+// Half rounds of two CTAs an SM: a last round that leaves every SM one CTA or none takes half a round's time.
+static long long half_rounds(long long ctas, int sms) {
+    const long long rest = ctas % (2 * sms);
+    return 2 * (ctas / (2 * sms)) + (rest == 0 ? 0 : (rest <= sms ? 1 : 2));
+}
+
+// How a product of more than 64 rows runs: its segments (more than one), each with CTAs of its own; 1: the wide kernel's tiles walk them; 0: the tile
+// kernel's do.  Cut, where the tiles leave SMs idle, or where that takes fewer half rounds of a segment each by more than the slabs' five per cent.
+// Whole, the tile kernel is the faster one until some fourteen tiles an SM.  us by the tile kernel, cut, whole, K 2,048: 64 tiles 261, 212, 257;
+// 192 416, 335, 432; 256 414, 442, 432; 320 636, 552, 646; 384 635, 658, 666; 512 826, 767, 843; 576 828, 875, 851; 1,024 1,445 and 1,482
+// whole, 1,536 2,246 and 2,227 to 2,270, 2,048 2,851 and 2,859, 3,072 4,268 and 4,222, 8,192 11,347 and 11,084.  K 508: 32 tiles 58 and 67.
+static int wide_segments(int M, int N, int K) {
     static int sms = 0;
     if (!sms) {
         int dev = 0;
@@ -454,32 +473,51 @@ static int wide_splits(int M, int N, int K) {
     }
     const int segs = (K + SEG - 1) / SEG;
     const long long tiles = (long long)((M + WT - 1) / WT) * ((N + WT - 1) / WT);
-    return segs > 1 && segs <= 65535 && tiles < 4ll * sms ? segs : 1;
+    if (segs > 1 && tiles < 4ll * sms) {
+        const int turn = turn_of(M, N, segs, WIDE_SLABS);
+        if (tiles <= sms && turn > 1) return segs;
+        if (turn > 1 && 21 * (segs / turn * half_rounds(tiles * turn, sms) + half_rounds(tiles * (segs % turn), sms)) < 20 * segs * half_rounds(tiles, sms))
+            return segs;
+    }
+    return tiles >= 14ll * sms ? 1 : 0;
 }
 
-static int launch_wide(const float* A, int lda, const float* W, int ldw, float* C, int ldc, int M, int N, int K, float* scratch,
-                       long long scratch_floats, cudaStream_t stream) {
-    // without room for the slabs the tiles walk their segments one after the other: the same bits
-    int segs = wide_splits(M, N, K);
-    if (segs > 1 && (scratch == nullptr || scratch_floats < (long long)segs * M * N)) segs = 1;
-    const dim3 grid((M + WT - 1) / WT, (N + WT - 1) / WT, segs);
-    const int st = wllm_launch(gemm_f32_wide_kernel, grid, WTHREADS, 0, stream, A, lda, W, ldw, segs > 1 ? scratch : C, segs > 1 ? N : ldc,
-                               (long long)M * N, M, N, K);
-    if (st != WLLM_OK || segs == 1) return st;
-    return wllm_launch(gemm_f32_fold_kernel, dim3((unsigned)(((size_t)M * N + 255) / 256)), 256, 0, stream, (const float*)scratch, C, ldc, M, N, segs);
+// turn: segments with CTAs of their own at a time; 1: a tile's CTA walks them all
+static int launch_wide(const float* A, int lda, const float* W, int ldw, float* C, int ldc, int M, int N, int K, float* scratch, int turn,
+                       cudaStream_t stream) {
+    const int segs = (K + SEG - 1) / SEG;
+    dim3 grid((M + WT - 1) / WT, (N + WT - 1) / WT);
+    if (turn < 2) return wllm_launch(gemm_f32_wide_kernel, grid, WTHREADS, 0, stream, A, lda, W, ldw, C, ldc, (long long)M * N, M, N, K);
+    for (int s0 = 0; s0 < segs; s0 += turn) {
+        grid.z = segs - s0 < turn ? segs - s0 : turn;
+        int st = wllm_launch(gemm_f32_wide_kernel, grid, WTHREADS, 0, stream, A + (size_t)s0 * SEG, lda, W + (size_t)s0 * SEG, ldw, scratch, N,
+                             (long long)M * N, M, N, K - s0 * SEG);
+        if (st == WLLM_OK)
+            st = wllm_launch(gemm_f32_fold_kernel, dim3((unsigned)(((size_t)M * N + 255) / 256)), 256, 0, stream, (const float*)scratch, C, ldc, M, N,
+                             (int)grid.z, s0 > 0);
+        if (st != WLLM_OK) return st;
+    }
+    return WLLM_OK;
 }
 
-// Floats of scratch that a product of these sizes wants (0: none): partial sums of the skinny kernel, or of the wide one.
-WLLM_API long long wllm_gemm_f32_scratch_floats(int M, int N, int K) {
-    const int segs = M <= 32 ? (K + SEG - 1) / SEG : (M > 64 && K % 4 == 0 ? wide_splits(M, N, K) : 1);
-    return segs > 1 ? (long long)segs * M * N : 0;
+static bool vec_operands(const void* A, int lda, const void* W, int ldw, int K) {
+    return K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && (uintptr_t)A % 16 == 0 && (uintptr_t)W % 16 == 0;
+}
+
+// Floats of scratch that a product of these operands and sizes wants (0: none): partial sums of the skinny kernel, which needs them, or of the wide one,
+// which does with any less.
+WLLM_API long long wllm_gemm_f32_scratch_floats(const float* A, int lda, const float* W, int ldw, int M, int N, int K) {
+    if (M <= 0 || N <= 0 || K <= 0 || !vec_operands(A, lda, W, ldw, K)) return 0;
+    if (M <= 32) return K > SEG ? (long long)((K + SEG - 1) / SEG) * M * N : 0;
+    const int segs = M > 64 ? wide_segments(M, N, K) : 0, turn = segs > 1 ? turn_of(M, N, segs, WIDE_SLABS) : 0;
+    return turn > 1 ? (long long)turn * M * N : 0;
 }
 
 WLLM_API int wllm_gemm_f32(const float* A, int lda, const float* W, int ldw, float* C, int ldc, int M, int N, int K,
                            float* scratch, long long scratch_floats, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return WLLM_OK;
-    if (K <= 0 || lda < K || ldw < K || ldc < N) return WLLM_BAD_SIZE;
-    const bool vec = (K % 4 == 0) && (lda % 4 == 0) && (ldw % 4 == 0) && ((uintptr_t)A % 16 == 0) && ((uintptr_t)W % 16 == 0);
+    if (K <= 0 || lda < K || ldw < K || ldc < N || (M > 32 && (N + TBN - 1) / TBN > 65535)) return WLLM_BAD_SIZE;
+    const bool vec = vec_operands(A, lda, W, ldw, K);
     if (vec && M <= 8) return launch_skinny<8>(A, lda, W, ldw, C, ldc, M, N, K, scratch, scratch_floats, stream);
     if (vec && M <= 16) return launch_skinny<16>(A, lda, W, ldw, C, ldc, M, N, K, scratch, scratch_floats, stream);
     if (vec && M <= 32) return launch_skinny<32>(A, lda, W, ldw, C, ldc, M, N, K, scratch, scratch_floats, stream);
@@ -487,7 +525,10 @@ WLLM_API int wllm_gemm_f32(const float* A, int lda, const float* W, int ldw, flo
         if (vec) return launch_tile<64, true>(A, lda, W, ldw, C, ldc, M, N, K, stream);
         return launch_tile<64, false>(A, lda, W, ldw, C, ldc, M, N, K, stream);
     }
-    if (vec && (N + WT - 1) / WT <= 65535) return launch_wide(A, lda, W, ldw, C, ldc, M, N, K, scratch, scratch_floats, stream);
+    const int segs = vec ? wide_segments(M, N, K) : 0;
+    // without room for two slabs the tile kernel's tiles walk their segments: the same bits
+    const int turn = segs > 1 ? turn_of(M, N, segs, scratch == nullptr ? 0 : scratch_floats) : segs;
+    if (turn > 1 || segs == 1) return launch_wide(A, lda, W, ldw, C, ldc, M, N, K, scratch, turn, stream);
     if (vec) return launch_tile<128, true>(A, lda, W, ldw, C, ldc, M, N, K, stream);
     return launch_tile<128, false>(A, lda, W, ldw, C, ldc, M, N, K, stream);
 }

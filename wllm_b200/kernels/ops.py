@@ -817,13 +817,21 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None) 
     assert out.stride(1) == 1 and out.shape == (M, N) and out.dtype == torch.float32
     lib = load_family("gemm_f32")
     lib.wllm_gemm_f32_scratch_floats.restype = ctypes.c_longlong
-    need = lib.wllm_gemm_f32_scratch_floats(M, N, K)       # partial sums, when segments of K have CTAs of their own
-    scratch = torch.empty(need, dtype=torch.float32, device=a.device) if need else None
+    # partial sums, when segments of K have CTAs of their own
+    need = lib.wllm_gemm_f32_scratch_floats(_ptr(a), a.stride(0), _ptr(w), w.stride(0), M, N, K)
+    scratch = None
+    if need:
+        try:
+            scratch = torch.empty(need, dtype=torch.float32, device=a.device)
+        except torch.OutOfMemoryError:
+            if M <= 32:
+                raise
+            need = 0             # the tiles of many rows can walk their segments: the same bits
     _check(lib.wllm_gemm_f32(_ptr(a), a.stride(0), _ptr(w), w.stride(0), _ptr(out), out.stride(0), M, N, K, _ptr(scratch),
                              ctypes.c_longlong(need), _stream()), "gemm_f32")
     if need:
         global launches
-        launches += 1        # the kernel that adds the partial sums
+        launches += 2 * -(-K // (1024 * (need // (M * N)))) - 1      # a turn of segments, the kernel that adds its sums; the next turn
     return out
 
 
