@@ -339,8 +339,8 @@ def test_attention_with_a_bias_by_distance_at_every_edge_of_its_window(window, d
 @pytest.mark.parametrize("hd,n0", [(32, 236), (64, 236), (64, 100), (128, 150)])
 @pytest.mark.parametrize("window", [40, 17, 130, 0])
 def test_tensor_core_attention_with_a_bias_by_distance(window, hd, n0):
-    """The bfloat16 kernels on mma.sync with slopes: a prompt's portion over several tiles of rows and decoded rows of three
-    requests whose keys are cut into splits, one key standing out at every edge of the window, pages of 16 and 64 in
+    """The bfloat16 kernels with slopes (heads of 32 on the kernels that walk a list of tiles, others on tensor memory and the warp-specialised
+    decode kernel): a prompt's portion over several tiles of rows and decoded rows of three requests whose keys are cut into splits, one key standing out at every edge of the window, pages of 16 and 64 in
     scrambled order; grouped heads, so that a tile's rows carry different slopes."""
     from wllm_b200.kernels import ops
     g = torch.Generator().manual_seed(window * 7 + hd)
@@ -378,6 +378,43 @@ def test_tensor_core_attention_with_a_bias_by_distance(window, hd, n0):
                                          split_keys, max_splits, scratch, slopes=sl)
                 err = (od.cpu().double() - want[-3:]).abs().max()
                 assert err < 0.03, ("decode", ps, edge, split_keys, float(err))
+    assert ops.tc_gemm_status(DEV) == 0
+
+
+@pytest.mark.parametrize("hd", [128, 256])
+@pytest.mark.parametrize("rep,G", [(2, 2), (9, 1), (16, 2)])                # heads of a group in the first eight rows; past them; all sixteen
+@pytest.mark.parametrize("window", [0, 70])
+@pytest.mark.parametrize("sinks", [False, True])
+def test_decoded_tokens_with_a_bias_by_distance_in_every_row_of_a_group(hd, rep, G, window, sinks):
+    """The warp-specialised decode kernel: pages smaller than a tile of 32 keys, of one and of two; splits that end inside and between tiles; a slope
+    for each of a group's heads, steep and flat, beside a term of the softmax's denominator of its own."""
+    from wllm_b200.kernels import ops
+    g = torch.Generator().manual_seed(hd + rep + window)
+    H, L, R, dtype = rep * G, 260, 4, torch.bfloat16
+    ctx, scale = [L, 1, 33, 200], hd ** -0.5
+    slopes = [2.0 ** (-8.0 * (h + 1) / H) for h in range(H)]
+    sink = torch.randn(H, generator=g) * 2 if sinks else None
+    k, v = torch.randn(L, G, hd, generator=g).to(dtype), torch.randn(L, G, hd, generator=g).to(dtype)
+    q = torch.randn(R, H, hd, generator=g).to(dtype)
+    want = torch.zeros(R, H, hd, dtype=torch.float64)
+    for r, n in enumerate(ctx):
+        first = max(0, n - window) if window else 0
+        for h in range(H):
+            s = k[first:n, h // rep].double() @ q[r, h].double() * scale - slopes[h] * torch.arange(n - 1 - first, -1, -1).double()
+            e = torch.exp(s - s.max())
+            z = e.sum() + (torch.exp(sink[h].double() - s.max()) if sinks else 0.0)
+            want[r, h] = (e / z) @ v[first:n, h // rep].double()
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    for ps in (16, 32, 64):
+        kp, vp, table = paged(k, v, ps, 3 + ps)
+        for split_keys, max_splits in ((512, 1), (64, 5), (96, 3)):
+            scratch, out = torch.empty(ops.attention_mma_scratch_floats(R, H, hd, max_splits), device=DEV), torch.empty(R, H * hd, dtype=dtype, device=DEV)
+            ops.attention_mma_decode(q.reshape(R, -1).to(DEV), out, kp, vp, i32(range(R)), i32([1] * R), i32(ctx), table.expand(R, -1).contiguous(), H, G, hd,
+                                     ps, window, scale, split_keys, max_splits, scratch, sinks=sink.to(DEV) if sinks else None,
+                                     slopes=torch.tensor(slopes, device=DEV))
+            # weights and results rounded to bfloat16: half a unit of 2^-8 each of values up to |v|
+            err = float((out.cpu().double().view(R, H, hd) - want).abs().max())
+            assert err < 2.0 ** -8 * float(v.abs().max()), (ps, split_keys, err)
     assert ops.tc_gemm_status(DEV) == 0
 
 

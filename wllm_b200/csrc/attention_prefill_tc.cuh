@@ -473,7 +473,7 @@ prefill_pair_kernel(const bf16* __restrict__ q, int q_stride, bf16* __restrict__
     const uint32_t rank = cluster_ctarank();
     const int tile = (int)gridDim.z - 1 - (int)blockIdx.z;
     if (tile * 2 * TC_BM >= rows) return;
-    const int row0 = tile * 2 * TC_BM + (int)rank * TC_BM;             // may lie past the end: then all rows are masked
+    const int row0 = tile * 2 * TC_BM + (int)rank * TC_BM;             // may lie past the end: its rows are zeros that keep the last row company
     const int ctx = req_ctx_len[r], q_start = req_q_start[r], pos0 = ctx - q_len;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;

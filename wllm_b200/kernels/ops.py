@@ -700,7 +700,7 @@ def attention_mma_prefill(q, out, k_pages, v_pages, req_q_start, req_q_len, req_
     `multi` (with skip_single): exactly how many do, so that the launch counts them alone; 0: not known.
     split_above > 0 (head sizes in steps of 64): a tile of 128 rows that walks more than that many tiles of 64
     keys is computed by two CTAs, half of the keys each; `halves` (float32) holds their partial results.
-    `cap`, `keep`, `slopes`: as for attention_mma_decode; with any of them the mma.sync kernel that walks a list of key tiles runs."""
+    `cap`, `keep`, `slopes`: as for attention_mma_decode; with any of them no tile is shared by two CTAs."""
     _need_cuda(q, out, k_pages, v_pages, req_q_start, req_q_len, req_ctx_len, block_table, halves, sinks, slopes)
     assert slopes is None or (slopes.dtype == torch.float32 and slopes.shape == (nq,) and slopes.is_contiguous())
     assert sinks is None or (sinks.dtype == torch.float32 and sinks.shape == (nq,) and sinks.is_contiguous())
