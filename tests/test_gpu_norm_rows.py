@@ -72,3 +72,28 @@ def test_turned_rows_from_tensors_and_slabs(heads, parts, biased):
     for got, want in ((q_out.cpu().double().view(n, nq, hd), want_q), (got_k, want_k[keep]), (got_v, want_v[keep])):
         assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + 2e-5 * want.abs().max()).all()       # one rounding to bfloat16, 32-bit before
     assert int((kp.float().abs().sum(-1) > 0).sum()) == int(keep.sum()) * nkv
+
+
+@pytest.mark.parametrize("H", [4, 508, 2048, 2052, 4096, 4100])       # as above
+@pytest.mark.parametrize("parts", [(0, 0), (2, 0), (17, 9)])           # of the two branches
+@pytest.mark.parametrize("center", [False, True])
+def test_joined_norms_of_two_branches(H, parts, center):
+    from wllm_b200.kernels import ops
+    g = torch.Generator().manual_seed(H + sum(parts))
+    n, eps, factor = 5, 1e-5, 0.7
+    x = torch.randn(n, H, generator=g) * 2
+    a, b = (torch.randn(*([p] if p else []), n, H, generator=g) for p in parts)
+    a, b = a if parts[0] else a.bfloat16(), b if parts[1] else b.bfloat16()
+    wp, w, ga, gb = (torch.randn(H, generator=g).bfloat16() for _ in range(4))
+    whole = lambda t, p: t.double().sum(0) if p else t.double()
+    u = factor * (_norm(whole(a, parts[0]), False, eps) * ga.double() + _norm(whole(b, parts[1]), False, eps) * gb.double())
+    r = x.double() + _norm(u, center, eps) * wp.double()
+    want = _norm(r, center, eps) * (1 + w.double())
+    resid, out = x.to(DEV), torch.empty(n, H, device=DEV)
+    ops.sandwich_norm(resid, (a.to(DEV), parts[0]), out, wp.to(DEV), center, eps, w.to(DEV), 1.0, center, eps, gain_a=ga.to(DEV), b=(b.to(DEV), parts[1]),
+                      gain_b=gb.to(DEV), inner_eps=eps, factor=factor)
+    # 32-bit sums of some twenty parts and of a row's squares: a few 2^-24 of values up to ten.  (H = 4 with the mean off: u may nearly cancel, and its norm
+    # divides by what is left, so the bound grows by the ratio.)
+    c = u - u.mean(-1, keepdim=True) if center else u
+    grown = max(1.0, float((u.abs().amax(-1) / c.pow(2).mean(-1).sqrt()).max()))
+    assert (resid.cpu().double() - r).abs().max() < 2e-5 * grown and (out.cpu().double() - want).abs().max() < 2e-5 * grown * max(1.0, float(want.abs().max()))
