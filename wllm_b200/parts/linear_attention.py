@@ -37,7 +37,8 @@ ranks are the checkpoint's unless the maps say `rank`.
 spec options: num_heads, num_kv_heads, key_dim, value_dim, conv_taps, eps, unit_norm_eps, q_scale, q_proj/k_proj/v_proj/g_proj/
 o_proj, q_conv/k_conv/v_conv [channels, taps], beta_proj, decay_proj [heads, hidden], decay_log, decay_bias [heads],
 head_norm_weight [value_dim] (checkpoint names).  One product makes q | k | v | g | beta | decay; what enters the
-recurrence is 32-bit (csrc/delta_rule.cu).
+recurrence is 32-bit (csrc/delta_rule.cu).  A 32-bit model's recurrence walks token by token and gives the same bits however a prompt
+is cut; a bfloat16 model's long portions are walked in blocks of eight tokens, whose sums run in another order.
 """
 from __future__ import annotations
 
