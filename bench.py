@@ -961,6 +961,20 @@ GUDARAX_SIZES = {
 }
 
 
+def _delta_rule_options(n: int, lens, heads: int, dim: int, dev) -> tuple:
+    """The options of delta_prepare and delta_scan with which a bfloat16 model's step of one prompt of n tokens, or of n single tokens, runs the delta rule."""
+    import torch
+
+    from wllm_b200.kernels import ops
+    from wllm_b200.parts.linear_attention import DeltaRule
+    if lens.shape[0] == n:
+        return {"shift": lens}, {"single": True}
+    if n < DeltaRule.REQUEST_FROM:
+        return {"shift": None}, {}
+    scratch = torch.empty(ops.delta_block_floats(n, 1, heads, dim), device=dev)
+    return {"shift": None}, {"blocks": scratch, "max_q_len": n, "walked": 1, "blocks_from": DeltaRule.REQUEST_FROM}
+
+
 def gudarax_config(size: dict) -> dict:
     """Four layers: attention in a window (the first of the two that blend values), latent attention, the delta rule, attention again;
     dense feed-forwards behind the first two, routed experts behind the others; a token input in every layer."""
@@ -1108,14 +1122,16 @@ def gudarax_kernel_table(size: dict, pk: dict, T: int, batch: int, context: int)
         dq, dk, dvv = torch.empty(n, GD, device=dev), torch.empty(n, GD, device=dev), torch.empty(n, HV, device=dev)
         beta, decay = torch.empty(n, dh, device=dev), torch.empty(n, dh, device=dev)
         conv_state = torch.zeros(batch + 1, taps - 1, 2 * GD + HV, device=dev)
+        as_run, walk = _delta_rule_options(n, rl, dh, dd, dev)
         row(f"{tag}/delta rule: inputs (convolutions, SiLU, unit norms, step sizes, decays)",
             lambda: ops.delta_prepare(fused, 0, off, dh, dg, dd, dv, taps, *conv, a_log, dt_bias, token_req, rs, rslot, conv_state, 1e-6, dd ** -0.5,
-                                      dq, dk, dvv, beta, decay), n * ((2 * GD + HV + 2 * dh) * 2 * min(taps, 2) + (2 * GD + HV + 2 * dh) * 4))
-        row(f"{tag}/delta rule: the convolutions' kept inputs",
-            lambda: ops.delta_conv_update(fused, 0, off, dh, dg, dd, dv, taps, rs, rl, rslot, conv_state), R * (taps - 1) * (2 * GD + HV) * (2 + 4))
+                                      dq, dk, dvv, beta, decay, **as_run), n * ((2 * GD + HV + 2 * dh) * 2 * min(taps, 2) + (2 * GD + HV + 2 * dh) * 4))
+        if as_run["shift"] is None:
+            row(f"{tag}/delta rule: the convolutions' kept inputs",
+                lambda: ops.delta_conv_update(fused, 0, off, dh, dg, dd, dv, taps, rs, rl, rslot, conv_state), R * (taps - 1) * (2 * GD + HV) * (2 + 4))
         dstate = torch.zeros(batch + 1, dh, dd, dv, device=dev)
         do = torch.empty(n, HV, device=dev)
-        row(f"{tag}/delta rule: recurrence", lambda: ops.delta_scan(dq, dk, dvv, beta, decay, dstate, do, rs, rl, rslot, dh, dg, dd, dv),
+        row(f"{tag}/delta rule: recurrence", lambda: ops.delta_scan(dq, dk, dvv, beta, decay, dstate, do, rs, rl, rslot, dh, dg, dd, dv, **walk),
             n * (2 * GD + 2 * HV + 2 * dh) * 4 + R * 2 * dh * dd * dv * 4, 6.0 * n * dh * dd * dv)
         gated = torch.empty(n, HV, dtype=bf, device=dev)
         row(f"{tag}/head norm and gate", lambda: ops.head_gate_norm(do, fused, 0, off["g"], nw, 1e-6, gated, dh, dv), n * HV * (4 + 2 + 2))
@@ -1313,11 +1329,13 @@ def fusanex_kernel_table(size: dict, pk: dict, T: int, batch: int, context: int)
         dq, dk, dv = (torch.empty(n, HD, device=dev) for _ in range(3))
         beta, ddecay = torch.empty(n, G, device=dev), torch.empty(n, G, device=dev)
         conv_state = torch.zeros(batch + 1, taps - 1, 3 * HD, device=dev)
+        as_run, walk = _delta_rule_options(n, ctx.req_q_len, G, md, dev)
         row(f"{tag}/delta rule: inputs (convolutions, SiLU, unit norms, step sizes, decays)",
             lambda: ops.delta_prepare(dfused, 0, off, G, G, md, md, taps, *conv, a_log, dt_bias, ctx.token_req, ctx.req_q_start, ctx.req_slot, conv_state,
-                                      1e-6, md ** -0.5, dq, dk, dv, beta, ddecay), n * (3 * HD + 2 * G) * (2 + 4))
+                                      1e-6, md ** -0.5, dq, dk, dv, beta, ddecay, **as_run), n * (3 * HD + 2 * G) * (2 + 4))
         dstate, do = torch.zeros(batch + 1, G, md, md, device=dev), torch.empty(n, HD, device=dev)
-        row(f"{tag}/delta rule: recurrence", lambda: ops.delta_scan(dq, dk, dv, beta, ddecay, dstate, do, ctx.req_q_start, ctx.req_q_len, ctx.req_slot, G, G, md, md),
+        row(f"{tag}/delta rule: recurrence", lambda: ops.delta_scan(dq, dk, dv, beta, ddecay, dstate, do, ctx.req_q_start, ctx.req_q_len, ctx.req_slot, G, G, md, md,
+                                                                                   **walk),
             n * (4 * HD + 2 * G) * 4 + R * 2 * G * md * md * 4, 6.0 * n * G * md * md)
         s = W // blocks
         fused = rnd(n, 2 * W, dtype=bf)
@@ -1567,12 +1585,12 @@ def vifirax_kernel_table(size: dict, pk: dict, T: int, batch: int, context: int)
         dq, dk, dvv, beta = torch.empty(n, GD, device=dev), torch.empty(n, GD, device=dev), torch.empty(n, HV, device=dev), torch.empty(n, dh, device=dev)
         decay = torch.empty(n, dh, device=dev)
         cstate = torch.zeros(batch + 1, dtaps - 1, 2 * GD + HV, device=dev)
-        shift = None if one else ctx.req_q_len
-        prep = lambda o_, a_, b_, d_, s_: ops.delta_prepare(fused, 0, o_, dh, dg, dd, dv, dtaps, *conv, a_, b_, ctx.token_req, ctx.req_q_start, ctx.req_slot, cstate, 1e-6,
-                                                            dd ** -0.5, dq, dk, dvv, beta, d_, shift=s_)
+        as_run, walk = _delta_rule_options(n, ctx.req_q_len, dh, dd, dev)
+        prep = lambda o_, a_, b_, d_: ops.delta_prepare(fused, 0, o_, dh, dg, dd, dv, dtaps, *conv, a_, b_, ctx.token_req, ctx.req_q_start, ctx.req_slot, cstate, 1e-6,
+                                                            dd ** -0.5, dq, dk, dvv, beta, d_, **as_run)
         moved = n * (2 * GD + HV) * (2 + 4)
-        row(f"{tag}/delta rule: inputs (convolutions, SiLU, unit norms, step sizes, decays)", lambda: prep(off, a_log, dt_bias, decay, None), moved)
-        row(f"{tag}/delta rule: inputs without decays", lambda: prep({k: v for k, v in off.items() if k != "a"}, None, None, None, shift), moved,
+        row(f"{tag}/delta rule: inputs (convolutions, SiLU, unit norms, step sizes, decays)", lambda: prep(off, a_log, dt_bias, decay), moved)
+        row(f"{tag}/delta rule: inputs without decays", lambda: prep({k: v for k, v in off.items() if k != "a"}, None, None, None), moved,
             like=f"{tag}/delta rule: inputs (convolutions, SiLU, unit norms, step sizes, decays)")
         low, up, ub, ulog = rnd(n, 2 * rank, dtype=bf), rnd(dh * dd, rank, dtype=bf, scale=0.1), rnd(dh * dd, dtype=bf), rnd(dh, dtype=bf)
         chan = torch.empty(n, dh * dd, device=dev)
@@ -1586,8 +1604,8 @@ def vifirax_kernel_table(size: dict, pk: dict, T: int, batch: int, context: int)
         decay.uniform_(0.9, 1.0)
         chan.uniform_(-0.1, 0.0)
         sb, sf = R * 2 * dh * dd * dv * 4, 6.0 * n * dh * dd * dv
-        row(f"{tag}/delta rule: recurrence", lambda: ops.delta_scan(dq, dk, dvv, beta, decay, state, do, *reqs, dh, dg, dd, dv), n * (2 * GD + 2 * HV + 2 * dh) * 4 + sb, sf)
-        row(f"{tag}/delta rule: recurrence, decays per key channel", lambda: ops.delta_scan(dq, dk, dvv, beta, chan, state, do, *reqs, dh, dg, dd, dv, True),
+        row(f"{tag}/delta rule: recurrence", lambda: ops.delta_scan(dq, dk, dvv, beta, decay, state, do, *reqs, dh, dg, dd, dv, **walk), n * (2 * GD + 2 * HV + 2 * dh) * 4 + sb, sf)
+        row(f"{tag}/delta rule: recurrence, decays per key channel", lambda: ops.delta_scan(dq, dk, dvv, beta, chan, state, do, *reqs, dh, dg, dd, dv, True, **walk),
             n * (2 * GD + 2 * HV + dh + dh * dd) * 4 + sb, sf, like=f"{tag}/delta rule: recurrence")
         hw, gated = rnd(dv, dtype=bf), torch.empty(n, HV, dtype=bf, device=dev)
         row(f"{tag}/head norm and SiLU gate", lambda: ops.head_gate_norm(do, gate, 0, 0, hw, 1e-6, gated, dh, dv), n * HV * (4 + 4 + 2))
