@@ -858,12 +858,6 @@ delta_block_prepare_kernel(const float* __restrict__ q, const float* __restrict_
     }
 }
 
-__device__ __forceinline__ float2 dr_fma2(float2 a, float2 b, float2 c) {
-    unsigned long long d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)),
-        "l"(*reinterpret_cast<unsigned long long*>(&c)));
-    return *reinterpret_cast<float2*>(&d);
-}
 __device__ __forceinline__ float2 dr_mul2(float2 a, float2 b) { return make_float2(a.x * b.x, a.y * b.y); }
 
 // channels of a lane: 4 lane + 128 j + 0 .. 3 (two: 2 lane, 2 lane + 1), as pairs
@@ -949,8 +943,8 @@ delta_block_walk_kernel(const float* __restrict__ blocks, const float* __restric
             db_row<NP>(K + i * DP, lane, w);
 #pragma unroll
             for (int p = 0; p < NP; ++p) {
-                acc[0] = dr_fma2(w[p], S[0][p], acc[0]);
-                acc[1] = dr_fma2(w[p], S[1][p], acc[1]);
+                acc[0] = fma2(w[p], S[0][p], acc[0]);
+                acc[1] = fma2(w[p], S[1][p], acc[1]);
             }
             x[(i & 8) * 2 + (i & 7)] = acc[0].x + acc[0].y;
             x[(i & 8) * 2 + 8 + (i & 7)] = acc[1].x + acc[1].y;
@@ -986,7 +980,7 @@ delta_block_walk_kernel(const float* __restrict__ blocks, const float* __restric
 #pragma unroll
         for (int p = 0; p < NP; ++p)
 #pragma unroll
-            for (int m = 0; m < 2; ++m) S[m][p] = CHANNEL ? dr_fma2(e[p], S[m][p], S[m][p]) : dr_mul2(e[p], S[m][p]);
+            for (int m = 0; m < 2; ++m) S[m][p] = CHANNEL ? fma2(e[p], S[m][p], S[m][p]) : dr_mul2(e[p], S[m][p]);
 #pragma unroll
         for (int l = 0; l < DB; ++l) {
             float2 w[NP];
@@ -994,7 +988,7 @@ delta_block_walk_kernel(const float* __restrict__ blocks, const float* __restric
 #pragma unroll
             for (int p = 0; p < NP; ++p)
 #pragma unroll
-                for (int m = 0; m < 2; ++m) S[m][p] = dr_fma2(w[p], make_float2(rj[m][l], rj[m][l]), S[m][p]);
+                for (int m = 0; m < 2; ++m) S[m][p] = fma2(w[p], make_float2(rj[m][l], rj[m][l]), S[m][p]);
         }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");

@@ -268,13 +268,6 @@ gemm_f32_skinny_kernel(const float* __restrict__ A, int lda, const float* __rest
 // ------------------------------------------------------------------------------------------------
 constexpr int WT = 128, WTHREADS = 128;
 
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-    unsigned long long d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)),
-        "l"(*reinterpret_cast<unsigned long long*>(&c)));
-    return *reinterpret_cast<float2*>(&d);
-}
-
 // grid (row tiles, column tiles, segments with CTAs of their own, or 1); dst: C, or slabs [segment][M][N]
 __global__ void __launch_bounds__(WTHREADS, 2)
 gemm_f32_wide_kernel(const float* __restrict__ A, int lda, const float* __restrict__ W, int ldw, float* __restrict__ dst, int ld_dst,
