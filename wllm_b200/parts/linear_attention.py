@@ -232,7 +232,7 @@ class DeltaRule:
     # of few tokens waits for.  Where a step becomes bound by the device (us, walk and blocks): one such layer of four, a decay per head, 512
     # tokens 1,117 and 1,145, 768 1,247 and 1,176; a decay per channel 384 852 and 870, 512 946 and 889; five layers of six, 192 1,405 and 1,448, 256 1,452
     # and 1,423; per channel 64 1,196 and 1,239, 128 1,456 and 1,259.
-    BLOCKS_FROM, CHANNEL_BLOCKS_FROM = 192, 128
+    BLOCKS_FROM, CHANNEL_BLOCKS_FROM = 192, 104
     # The shortest request that takes part: many short ones fill the device either way (64 of 20 tokens 230 us by the walk, 292 in blocks; 32 of 40 194
     # and 195, per channel 233 and 200; 16 of 64 144 and 136, 176 and 137).
     REQUEST_FROM = 40
