@@ -191,8 +191,8 @@ linattn_prepare_kernel(const void* __restrict__ fused, int in_dtype, int row_str
     }
 }
 
-// The low-rank maps of forms 1 to 3 for many tokens, bfloat16 maps, on the tensor cores (mma.sync): a CTA takes 64 tokens, whose low-rank
-// rows (form 1: through tanh) it holds in shared memory as a high and a low bfloat16 piece each (together some sixteen bits), and walks tiles of 128
+// The low-rank maps for many tokens, bfloat16 maps, on the tensor cores (mma.sync); form 0 of bfloat16 rows alone, whose high pieces are all there is (2,048
+// tokens of rank 64, 1,024 channels: 14 us, 23 on the FMA pipes).  A CTA takes 64 tokens, whose low-rank rows (form 1: through tanh) it holds in shared memory as a high and a low bfloat16 piece each (together some sixteen bits), and walks tiles of 128
 // channels; 2 x 4 warps, 32 tokens by 32 channels each.  grid (CTAs that share the channels' tiles, tiles of tokens), 256 threads.
 constexpr int DEC_TM = 64, DEC_TN = 128, DEC_MAX_RANK = 256;
 
@@ -210,7 +210,7 @@ template <bool MULTI, int FORM>
 __global__ void __launch_bounds__(256)
 linattn_decay_mma_kernel(const void* __restrict__ low, int in_dtype, int row_stride, int parts, size_t part_stride, int a_off, int n, int HD,
                          int rank, const bf16* __restrict__ w2, const bf16* __restrict__ b2, float* __restrict__ decay,
-                         const bf16* __restrict__ a_log, int D) {
+                         const bf16* __restrict__ a_log, int D, float inv_tau) {
     extern __shared__ __align__(16) unsigned char dec_smem[];
     const int kp = (rank + 15) & ~15, pitch = kp + 8;
     bf16* hi = reinterpret_cast<bf16*>(dec_smem);        // [64][pitch]
@@ -281,8 +281,8 @@ linattn_decay_mma_kernel(const void* __restrict__ low, int in_dtype, int row_str
                 for (int j = 0; j < 4; ++j) {
                     const int ch = tile * DEC_TN + wn * 32 + j * 8 + (lane & 3) * 2;
                     float* dst = decay + (size_t)t * HD + ch;
-                    const float y0 = lowrank_out(FORM, acc[mi][j][half * 2] + bias[j][0], 0.f, rate[j][0]);
-                    const float y1 = lowrank_out(FORM, acc[mi][j][half * 2 + 1] + bias[j][1], 0.f, rate[j][1]);
+                    const float y0 = lowrank_out(FORM, acc[mi][j][half * 2] + bias[j][0], inv_tau, rate[j][0]);
+                    const float y1 = lowrank_out(FORM, acc[mi][j][half * 2 + 1] + bias[j][1], inv_tau, rate[j][1]);
                     if (ch + 1 < HD && (HD & 1) == 0) *reinterpret_cast<float2*>(dst) = make_float2(y0, y1);
                     else {
                         if (ch < HD) dst[0] = y0;
@@ -305,7 +305,7 @@ WLLM_API int wllm_linattn_prepare_form(const void* fused, int in_dtype, int row_
     if (a_off >= 0 && (rank <= 0 || !(tau > 0.f) || !w2 || !decay || (form == 2 && !a_log))) return WLLM_BAD_SIZE;
     if ((in_dtype != WLLM_BF16 && in_dtype != WLLM_F32) || (a_off >= 0 && w_dtype != WLLM_BF16 && w_dtype != WLLM_F32))
         return WLLM_BAD_DTYPE;
-    if (q == nullptr && form >= 1 && a_off >= 0 && n >= 64 && w_dtype == WLLM_BF16 && rank % 8 == 0 && rank <= DEC_MAX_RANK && ((uintptr_t)w2 & 15) == 0) {
+    if (q == nullptr && (form >= 1 || (in_dtype == WLLM_BF16 && parts == 1)) && a_off >= 0 && n >= 64 && w_dtype == WLLM_BF16 && rank % 8 == 0 && rank <= DEC_MAX_RANK && ((uintptr_t)w2 & 15) == 0) {
         const int HD = H * D, row_tiles = (n + DEC_TM - 1) / DEC_TM, col_tiles = (HD + DEC_TN - 1) / DEC_TN;
         int share = (2 * 148 + row_tiles - 1) / row_tiles;           // CTAs that share a tile of tokens: some two CTAs an SM in all
         if (share > col_tiles) share = col_tiles;
@@ -314,14 +314,15 @@ WLLM_API int wllm_linattn_prepare_form(const void* fused, int in_dtype, int row_
         if (!raised) {
             cudaError_t e = cudaSuccess;
 #define RAISE(M, F) if (e == cudaSuccess) e = cudaFuncSetAttribute(linattn_decay_mma_kernel<M, F>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024)
-            RAISE(true, 1); RAISE(false, 1); RAISE(true, 2); RAISE(false, 2); RAISE(true, 3); RAISE(false, 3);
+            RAISE(false, 0); RAISE(true, 1); RAISE(false, 1); RAISE(true, 2); RAISE(false, 2); RAISE(true, 3); RAISE(false, 3);
 #undef RAISE
             if (e != cudaSuccess) return 1000 + (int)e;
             raised = true;
         }
 #define DEC2(M, F) wllm_launch(linattn_decay_mma_kernel<M, F>, dim3(share, row_tiles), 256, smem, stream, fused, in_dtype, row_stride, parts, \
-        (size_t)part_stride, a_off, n, HD, rank, (const bf16*)w2, (const bf16*)b2, decay, (const bf16*)a_log, D)
+        (size_t)part_stride, a_off, n, HD, rank, (const bf16*)w2, (const bf16*)b2, decay, (const bf16*)a_log, D, form == 0 ? 1.0f / tau : 0.f)
 #define DEC(M) (form == 1 ? DEC2(M, 1) : form == 2 ? DEC2(M, 2) : DEC2(M, 3))
+        if (form == 0) return DEC2(false, 0);
         return parts > 1 ? DEC(true) : DEC(false);
 #undef DEC
 #undef DEC2

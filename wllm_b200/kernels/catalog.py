@@ -13,6 +13,7 @@ FAMILIES = {
     "attention_simt": [{}],
     "activation": [{}],
     "linear_attention": [{}],
+    "linear_attention_chunks": [{}],
     "delta_rule": [{}],
     "state_space": [{}],
     "rg_lru": [{}],

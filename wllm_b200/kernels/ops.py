@@ -1112,9 +1112,10 @@ def lowrank_map(low: torch.Tensor, parts: int, low_off: int, w2: torch.Tensor, h
 
 
 def linattn_decay(low: torch.Tensor, parts: int, low_off: int, w2: torch.Tensor, b2: torch.Tensor, heads: int, dim: int,
-                  decay: torch.Tensor) -> torch.Tensor:
+                  decay: torch.Tensor, tau: float | None = None) -> torch.Tensor:
     """The decay per key channel of time mixing, minus one: decay [n, heads*dim] = expm1(-exp(w2 @ tanh(low) + b2)), where `low` are the
-    rank = w2.shape[1] columns of the projection `low` [n, W] (or partial sums [parts, n, W]) from `low_off`; 32-bit."""
+    rank = w2.shape[1] columns of the projection `low` [n, W] (or partial sums [parts, n, W]) from `low_off`; 32-bit.  With `tau` that of gated
+    linear attention instead, as linattn_prepare makes it: sigmoid(w2 @ low + b2)^(1/tau)."""
     _need_cuda(low, w2, b2, decay)
     ptr, dt, row_stride, nparts, part_stride, n = _fused_args(low, parts)
     assert w2.shape[0] == heads * dim and w2.is_contiguous() and b2.shape == (heads * dim,) and b2.dtype == w2.dtype and b2.is_contiguous()
@@ -1123,9 +1124,58 @@ def linattn_decay(low: torch.Tensor, parts: int, low_off: int, w2: torch.Tensor,
     lib = load_family("linear_attention")
     null = _ptr(None)
     _check(lib.wllm_linattn_prepare_form(ptr, dt, row_stride, nparts, part_stride, 0, 0, 0, low_off, n, heads, dim, dim, w2.shape[1], null,
-                                         null, 0, c_float(1.0), c_float(1.0), _ptr(w2), _ptr(b2), _dt(w2), c_float(1.0), null, null, null,
-                                         _ptr(decay), 1, null, _stream()), "linattn_decay")
+                                         null, 0, c_float(1.0), c_float(1.0), _ptr(w2), _ptr(b2), _dt(w2), c_float(1.0 if tau is None else tau), null, null, null,
+                                         _ptr(decay), 1 if tau is None else 0, null, _stream()), "linattn_decay")
     return decay
+
+
+LINATTN_CHUNKS_FROM = 128      # portions of at least this many tokens
+
+
+def linattn_chunks_ok(fused, parts: int, offsets, dim: int, vdim: int, rot_dim: int, pairing: str = "half") -> bool:
+    """Whether the recurrence's chunked form reads these columns of a fused product: bfloat16 rows (no partial sums) in steps of 16 bytes, heads of
+    64 or 128 key channels and values in steps of 64, turns of pairs half a turn apart over steps of 16 channels."""
+    return (fused.dtype == torch.bfloat16 and parts == 0 and dim in (64, 128) and vdim % 64 == 0 and rot_dim % 16 == 0 and pairing == "half"
+            and fused.stride(1) == 1 and fused.stride(0) % 8 == 0 and fused.data_ptr() % 16 == 0 and all(o % 8 == 0 for o in offsets))
+
+
+def linattn_chunks_bytes(lens, heads: int, dim: int, vdim: int) -> int:
+    """Bytes of scratch that linattn_chunks asks for; `lens`: the requests' tokens (int32 array on the host)."""
+    lib = load_family("linear_attention_chunks")
+    lib.wllm_linattn_chunks_bytes.restype = ctypes.c_longlong
+    return int(lib.wllm_linattn_chunks_bytes(c_void_p(lens.ctypes.data), len(lens), heads, dim, vdim))
+
+
+def linattn_chunks(fused, q_off: int, k_off: int, v_off: int, heads: int, dim: int, vdim: int, positions: torch.Tensor, decay, head_decay,
+                   state: torch.Tensor, out: torch.Tensor, req_q_start: torch.Tensor, req_q_len: torch.Tensor, req_slot: torch.Tensor, lens,
+                   scratch: torch.Tensor, q_scale: float = 1.0, k_scale: float = 1.0, inv_freq: torch.Tensor | None = None, rot_dim: int = 0) -> torch.Tensor:
+    """linattn_prepare's q, k and v and linattn_scan over them in chunks of 64 tokens on the tensor cores (csrc/linear_attention_chunks.cu), from
+    bfloat16 columns of a fused product [n, W] that linattn_chunks_ok accepts.  `decay` [n, heads*dim] per key channel (linattn_decay), or None with
+    `head_decay` [heads]; `lens`: req_q_len on the host (int32); `scratch` (uint8): linattn_chunks_bytes, or less that holds a chunk of every request."""
+    _need_cuda(fused, positions, decay, head_decay, state, out, req_q_start, req_q_len, req_slot, scratch, inv_freq)
+    n, R = fused.shape[0], req_q_len.shape[0]
+    if not linattn_chunks_ok(fused, 0, (q_off, k_off, v_off), dim, vdim, rot_dim):
+        raise KernelError(f"linattn_chunks: {fused.dtype} rows, heads of {dim} by {vdim}, turns over {rot_dim}: see linattn_chunks_ok")
+    assert q_off + heads * dim <= fused.shape[1] and k_off + heads * dim <= fused.shape[1] and v_off + heads * vdim <= fused.shape[1]
+    assert positions.shape == (n,) and lens.dtype.name == "int32" and len(lens) == R and lens.flags["C_CONTIGUOUS"]
+    assert state.dtype == torch.float32 == out.dtype and state.is_contiguous() and out.is_contiguous()
+    assert state.shape[1:] == (heads, dim, vdim) and out.shape == (n, heads * vdim) and scratch.dtype == torch.uint8 and scratch.is_contiguous()
+    if decay is not None:
+        assert decay.dtype == torch.float32 and decay.is_contiguous() and decay.shape == (n, heads * dim)
+    else:
+        assert head_decay.dtype == torch.float32 and head_decay.shape == (heads,) and head_decay.is_contiguous()
+    if rot_dim:
+        assert inv_freq.dtype == torch.float32 and inv_freq.numel() == rot_dim // 2 and inv_freq.is_contiguous()
+    lib = load_family("linear_attention_chunks")
+    launched = ctypes.c_int(0)
+    _check(lib.wllm_linattn_chunks(_ptr(fused), fused.stride(0), q_off, k_off, v_off, _ptr(_int32(positions, "positions")), _ptr(inv_freq), rot_dim,
+                                   c_float(q_scale), c_float(k_scale), _ptr(decay), _ptr(head_decay), _ptr(state), _ptr(out),
+                                   _ptr(_int32(req_q_start, "req_q_start")), _ptr(_int32(req_q_len, "req_q_len")), _ptr(_int32(req_slot, "req_slot")),
+                                   c_void_p(lens.ctypes.data), R, heads, dim, vdim, _ptr(scratch), ctypes.c_longlong(scratch.numel()),
+                                   ctypes.byref(launched), _stream()), f"linattn_chunks(heads={heads}, dim={dim}, vdim={vdim})")
+    global launches
+    launches += launched.value - 1
+    return out
 
 
 LINATTN_SEGMENT_FROM = 128     # portions of at least this many tokens may be cut into segments that run side by side

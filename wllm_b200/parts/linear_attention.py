@@ -14,7 +14,8 @@ spec options: num_heads, key_dim, value_dim, eps, q_scale, k_scale (applied afte
 spec, or None), decay, head_norm_weight (checkpoint name or None), q_proj/k_proj/v_proj/g_proj/o_proj (names).
 All projections that read the mixer's input are one matrix, rows in the order q, k, v, g, down: one product.
 What enters the recurrence is 32-bit (csrc/linear_attention.cu): the rotation, the scales, the decay and the state;
-the projections run in the model's element type.
+the projections run in the model's element type.  Long portions of bfloat16 models run in chunks on the tensor cores
+(csrc/linear_attention_chunks.cu), their 32-bit numbers as three bfloat16 pieces each.
 
 'parallel_mean': two mixers read the same input; each output is root-mean-square normed over the model width with a
 gain of its own, and the result is half their sum.  One product serves both (`input_weights` / `mix`).
@@ -130,18 +131,36 @@ class LinearAttention:
     def mix(self, fused: torch.Tensor, parts: int, col0: int, ctx, cache: CacheRef):
         """The mixer on the columns from col0 of a fused product [n, W] (or partial sums [parts, n, W])."""
         n, H, D, V, f32 = fused.shape[-2], self.heads, self.dim, self.vdim, torch.float32
+        low = self.decay_kind == "low_rank"
+        decay = ctx.buffer(self.tag + "la_decay", (n, H * D), f32) if low else None
+        rot = self.position.rotary_dim if self.position is not None else 0
+        offsets = (col0, col0 + self.off_k, col0 + self.off_v)
+        turn = dict(q_scale=self.q_scale, k_scale=self.k_scale, inv_freq=self.position.inv_freq if rot else None, rot_dim=rot)
+        o = ctx.buffer(self.tag + "la_o", (n, H * V), f32)
+        state = ctx.state(cache.state_names["state"])
+        if ctx.max_q_len >= ops.LINATTN_CHUNKS_FROM and ops.linattn_chunks_ok(fused, parts, offsets, D, V, rot, getattr(self.position, "pairing", "half")):
+            # long portions of bfloat16 models: chunks on the tensor cores, from the product's rows as they are
+            if low:
+                ops.linattn_decay(fused, parts, col0 + self.off_low, self.w_up, self.b_up, H, D, decay, tau=self.tau)
+            lens = ctx.host["req_q_len"]
+            scratch = ctx.buffer(self.tag + "la_chunks", (ops.linattn_chunks_bytes(lens, H, D, V),), torch.uint8)
+            ops.linattn_chunks(fused, *offsets, H, D, V, ctx.positions, decay, self.head_decay, state, o, ctx.req_q_start, ctx.req_q_len,
+                               ctx.req_slot, lens, scratch, **turn)
+        else:
+            self._walk(fused, parts, offsets, turn, decay, state, o, ctx, col0)
+        gated = ctx.buffer(self.tag + "la_gated", (n, H * V), self.model_dtype)
+        ops.head_gate_norm(o, fused, parts, col0 + self.off_g, self.norm_weight, self.eps, gated, H, V)
+        return as_branch(ops.project(gated, self.wo, lambda name, shape, dt: ctx.buffer(self.tag + "la_out_" + name, shape, dt)))
+
+    def _walk(self, fused, parts: int, offsets, turn: dict, decay, state, o, ctx, col0: int) -> None:
+        """The recurrence token by token, from 32-bit inputs."""
+        n, H, D, V, f32 = fused.shape[-2], self.heads, self.dim, self.vdim, torch.float32
         q = ctx.buffer(self.tag + "la_q", (n, H * D), f32)
         k = ctx.buffer(self.tag + "la_k", (n, H * D), f32)
         v = ctx.buffer(self.tag + "la_v", (n, H * V), f32)
         low = self.decay_kind == "low_rank"
-        decay = ctx.buffer(self.tag + "la_decay", (n, H * D), f32) if low else None
-        rot = self.position.rotary_dim if self.position is not None else 0
-        ops.linattn_prepare(fused, parts, col0, col0 + self.off_k, col0 + self.off_v, H, D, V, ctx.positions, q, k, v,
-                            q_scale=self.q_scale, k_scale=self.k_scale,
-                            inv_freq=self.position.inv_freq if rot else None, rot_dim=rot,
-                            low_off=col0 + self.off_low if low else -1, w2=self.w_up, b2=self.b_up,
-                            tau=self.tau if low else 1.0, decay=decay)
-        o = ctx.buffer(self.tag + "la_o", (n, H * V), f32)
+        ops.linattn_prepare(fused, parts, *offsets, H, D, V, ctx.positions, q, k, v, low_off=col0 + self.off_low if low else -1, w2=self.w_up,
+                            b2=self.b_up, tau=self.tau if low else 1.0, decay=decay, **turn)
         # long portions are cut into segments that run side by side; the plan is a function of the step's shape alone
         seg_len, max_seg = ops.linattn_segment_plan(ctx.max_q_len, ctx.num_multi, H, V)
         seg_state = seg_decay = None
@@ -149,11 +168,8 @@ class LinearAttention:
             R = ctx.n_requests
             seg_state = ctx.buffer(self.tag + "la_seg_state", (R * max_seg * H * D * V,), f32)
             seg_decay = ctx.buffer(self.tag + "la_seg_decay", (R * max_seg * H * D,), f32)
-        ops.linattn_scan(q, k, v, decay, self.head_decay, ctx.state(cache.state_names["state"]), o, ctx.req_q_start,
-                         ctx.req_q_len, ctx.req_slot, H, D, V, seg_len, max_seg, seg_state, seg_decay)
-        gated = ctx.buffer(self.tag + "la_gated", (n, H * V), self.model_dtype)
-        ops.head_gate_norm(o, fused, parts, col0 + self.off_g, self.norm_weight, self.eps, gated, H, V)
-        return as_branch(ops.project(gated, self.wo, lambda name, shape, dt: ctx.buffer(self.tag + "la_out_" + name, shape, dt)))
+        ops.linattn_scan(q, k, v, decay, self.head_decay, state, o, ctx.req_q_start, ctx.req_q_len, ctx.req_slot, H, D, V, seg_len, max_seg,
+                         seg_state, seg_decay)
 
 
 @MIXERS.register("parallel_mean")
