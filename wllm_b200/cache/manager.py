@@ -98,6 +98,9 @@ class CacheGroup:
             else:
                 self.key_pages = pool(spec.layers, num_pages, spec.kv_heads, page_size, spec.head_dim)
                 self.value_pages = pool(spec.layers, num_pages, spec.kv_heads, page_size, self.v_head_dim)
+        # a layer's keys and values as views, made once (the pools stay where they are)
+        self._views = [(self.pages[i, 0], self.pages[i, 1]) if self.pages is not None else (self.key_pages[i], self.value_pages[i])
+                       for i in range(spec.layers)] if device is not None else []
 
     def give(self, pages: list) -> None:
         """Pages go back to the pool; with `poison` their contents become NaN first (in stream order, so a step
@@ -110,10 +113,10 @@ class CacheGroup:
             self.pool.give(page)
 
     def keys(self, layer: int) -> torch.Tensor:
-        return self.pages[layer, 0] if self.pages is not None else self.key_pages[layer]
+        return self._views[layer][0]
 
     def values(self, layer: int) -> torch.Tensor:
-        return self.pages[layer, 1] if self.pages is not None else self.value_pages[layer]
+        return self._views[layer][1]
 
     def bytes_per_token(self) -> int:
         per_head = self.spec.head_dim if self.spec.values_in_keys else self.spec.head_dim + self.v_head_dim

@@ -1,4 +1,4 @@
-"""Compiles the CUDA sources under `wllm_b200/csrc` into shared objects and loads them.
+"""Compiles the sources under `wllm_b200/csrc` into shared objects and loads them.
 
 Every kernel family is one `.cu` file with plain C entry points (`extern "C"`,
 raw pointers and a stream), compiled by `nvcc` for sm_100a on first use and
@@ -9,7 +9,8 @@ the flags, so an edited kernel is rebuilt and an unchanged one is found again.
 
 Objects go to `wllm_b200/csrc/_build/` inside the checkout; if that folder cannot
 be written they go to a per-user folder under the system's temporary directory.
-There is no fallback of any other kind: without `nvcc`, or when the compile
+One source holds no kernel: `host_calls.cpp`, a Python module against torch's C++ interface that checks and launches
+what a step calls most.  There is no fallback of any other kind: without `nvcc`, or when the compile
 fails, `KernelBuildError` is raised with the compiler's output.
 """
 from __future__ import annotations
@@ -86,10 +87,29 @@ def _key(source: str, flags: list[str]) -> str:
     return h.hexdigest()[:16]
 
 
+HOST_CALLS = "host_calls"      # the one source without kernels: a Python module (csrc/host_calls.cpp)
+
+
+def _host_flags() -> list[str]:
+    """What a module against torch's C++ interface and this interpreter is compiled with (the versions are part of the object's name)."""
+    import sysconfig
+
+    import torch
+    base = os.path.dirname(torch.__file__)
+    flags = [f"-DWLLM_TORCH=\"{torch.__version__}\"", f"-DWLLM_PYTHON=\"{sys.version.split()[0]}\"",
+             f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-DUSE_CUDA"]
+    for path in (os.path.join(base, "include"), os.path.join(base, "include", "torch", "csrc", "api", "include"), sysconfig.get_paths()["include"]):
+        flags += ["-isystem", path]
+    return flags + ["-L", os.path.join(base, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
+
+
 def library_path(family: str, defines: dict | None = None) -> tuple[str, list[str], str]:
-    source = os.path.join(CSRC, family + ".cu")
+    source = os.path.join(CSRC, family + (".cpp" if family == HOST_CALLS else ".cu"))
     if not os.path.isfile(source):
         raise KernelBuildError(f"no kernel source {source}")
+    if family == HOST_CALLS:
+        flags = _host_flags()
+        return source, flags, f"wllm_{family}-{_key(source, flags)}.so"
     flags = [f"-D{k}={v}" for k, v in sorted((defines or {}).items())]
     tag = "".join(f"_{k.lower()}{v}" for k, v in sorted((defines or {}).items()))
     name = f"wllm_{family}{tag}-{_key(source, flags)}.so"
@@ -167,5 +187,32 @@ def load_family(family: str, defines: dict | None = None) -> ctypes.CDLL:
         return lib
 
 
+_host = None
+
+
+def load_host_calls(kernel_error: type):
+    """The module of native checks and launches (compiled on first use); `kernel_error`: the class of the errors that it raises."""
+    global _host
+    if _host is None:
+        with _lock:
+            if _host is None:
+                import importlib.machinery
+                import importlib.util
+                path = compile_family(HOST_CALLS)
+                try:
+                    loader = importlib.machinery.ExtensionFileLoader("wllm_host_calls", path)
+                    host = importlib.util.module_from_spec(importlib.util.spec_from_file_location("wllm_host_calls", path, loader=loader))
+                    loader.exec_module(host)
+                except ImportError as e:
+                    raise KernelBuildError(f"cannot load {path}: {e}") from e
+                host.errors(kernel_error)
+                _host = host
+    return _host
+
+
+def entry_address(lib: ctypes.CDLL, name: str) -> int:
+    return ctypes.cast(getattr(lib, name), ctypes.c_void_p).value
+
+
 def loaded_libraries() -> list[str]:
-    return sorted(getattr(lib, "_name", "?") for lib in _loaded.values())
+    return sorted(getattr(lib, "_name", "?") for lib in _loaded.values()) + ([_host.__file__] if _host is not None else [])

@@ -7,6 +7,7 @@ from .build import compile_family
 
 # family -> list of define sets to build ahead of time ({} = the family has no variants)
 FAMILIES = {
+    "host_calls": [{}],
     "embedding": [{}],
     "norm": [{}],
     "rope_cache": [{}],

@@ -19,7 +19,7 @@ from ctypes import c_float, c_void_p
 
 import torch
 
-from .build import KernelBuildError, load_family
+from .build import KernelBuildError, entry_address, load_family, load_host_calls
 
 launches = 0
 
@@ -82,6 +82,33 @@ def _check(status: int, what: str) -> None:
     raise KernelError(f"{what}: {_STATUS.get(status, 'status ' + str(status))}")
 
 
+# The functions that a step calls most hand their arguments to csrc/host_calls.cpp, which checks them, calls the entry point and returns its status.
+_host = None
+_bound: set = set()
+
+
+def _host_call(family: str, entry: str):
+    """The module of native calls, with that entry point of that family bound."""
+    global _host
+    if _host is None:
+        _host = load_host_calls(KernelError)
+    if entry not in _bound:
+        _host.bind(entry, entry_address(load_family(family), entry))
+        _bound.add(entry)
+    return _host
+
+
+def _host_attention(hd: int):
+    global _host
+    if _host is None:
+        _host = load_host_calls(KernelError)
+    if hd not in _bound:
+        lib = load_family("attention_mma", {"HEAD_DIM": hd})
+        _host.bind_attention(hd, entry_address(lib, "wllm_attention_mma_decode_biased"), entry_address(lib, "wllm_attention_mma_prefill_biased"))
+        _bound.add(hd)
+    return _host
+
+
 def _int32(t: torch.Tensor, name: str) -> torch.Tensor:
     if t.dtype != torch.int32 or not t.is_contiguous():
         raise KernelError(f"{name} must be a contiguous int32 tensor")
@@ -125,24 +152,11 @@ def rmsnorm(resid: torch.Tensor, delta, weight, eps: float, offset: float, out: 
     `delta` is [S, n, H] float32 partial sums that are added in order.  `center`: the row's mean is taken off
     first (a layer norm without a bias).  `weight` None: nothing is normed, `out` is the residual's rows rounded to
     its element type."""
-    _need_cuda(resid, delta, weight, out, rows)
-    H = resid.shape[1]
-    n = rows.shape[0] if rows is not None else resid.shape[0]
-    assert resid.dtype == torch.float32 and resid.is_contiguous() and out.is_contiguous() and out.shape == (n, H)
-    assert weight is None or (weight.shape == (H,) and weight.is_contiguous())
-    split_stride = 0
-    if delta is not None:
-        assert delta.is_contiguous()
-        if delta_splits:
-            assert delta.shape == (delta_splits,) + tuple(resid.shape) and delta.dtype == torch.float32
-            split_stride = resid.numel()
-        else:
-            assert delta.shape == resid.shape
-    lib = load_family("norm")
-    _check(lib.wllm_norm(_ptr(resid), _ptr(delta), _dt(delta) if delta is not None else _F32, max(1, delta_splits),
-                         ctypes.c_longlong(split_stride), _ptr(weight), _dt(weight) if weight is not None else _F32, c_float(eps), c_float(offset),
-                         1 if center else 0, _ptr(out), _dt(out), _ptr(_int32(rows, "rows") if rows is not None else None),
-                         n, H, _stream()), "norm")
+    status = _host_call("norm", "wllm_norm").norm(resid, delta, weight, eps, offset, out, rows, delta_splits, center)
+    if status:
+        _check(status, "norm")
+    global launches
+    launches += 1
     return out
 
 
@@ -184,21 +198,13 @@ def sandwich_norm(resid: torch.Tensor, a, out: torch.Tensor, post_weight: torch.
         out = norm(resid) * (offset + weight), or, with `weight` None, resid as it is (rounded to out's type).
     `a`, `b`: (tensor [n, H] or float32 partial sums [S, n, H], S or 0).  With `rows` the residual is read at those rows
     and left as it is."""
-    N, H = resid.shape
-    n = rows.shape[0] if rows is not None else N
-    _need_cuda(resid, a[0], out, post_weight, weight, rows, gain_a, gain_b, b[0] if b is not None else None)
-    assert resid.dtype == torch.float32 and resid.is_contiguous() and out.is_contiguous() and out.shape == (n, H)
-    gains = [g for g in (post_weight, weight, gain_a, gain_b) if g is not None]
-    assert all(g.shape == (H,) and g.is_contiguous() and g.dtype == post_weight.dtype for g in gains)
-    assert bias is None or (bias.dtype == torch.float32 and bias.shape == (H,) and bias.is_contiguous())
-    pa = _branch_args(a, N, H)
-    pb = _branch_args(b, N, H) if b is not None else (_ptr(None), _F32, 1, ctypes.c_longlong(0))
-    lib = load_family("norm")
-    _check(lib.wllm_sandwich_norm_offset(_ptr(resid), *pa, _ptr(gain_a), *pb, _ptr(gain_b), c_float(inner_eps), c_float(factor),
-                                         _ptr(post_weight), c_float(post_offset), 1 if post_center else 0, c_float(post_eps),
-                                         _ptr(weight), c_float(offset), 1 if center else 0, c_float(eps), _dt(post_weight),
-                                         _ptr(out), _dt(out), _ptr(_int32(rows, "rows") if rows is not None else None), n, H,
-                                         _ptr(bias), _stream()), "sandwich_norm")
+    status = _host_call("norm", "wllm_sandwich_norm_offset").sandwich(
+        resid, *a, out, post_weight, post_center, post_eps, weight, offset, center, eps, rows, gain_a, *(b if b is not None else (None, 0)), gain_b,
+        inner_eps, factor, post_offset, bias)
+    if status:
+        _check(status, "sandwich_norm")
+    global launches
+    launches += 1
     return out
 
 
@@ -276,28 +282,17 @@ def rope_kv_write(qkv: torch.Tensor, q_out: torch.Tensor, positions: torch.Tenso
     square, y / sqrt(mean(y^2) + eps).  `turn_scale` multiplies the sines and cosines (not with unit_norm_eps)."""
     if pairing not in ("half", "interleaved"):
         raise KernelError(f"rotary pairing {pairing!r} not supported (half, interleaved)")
-    _need_cuda(qkv, q_out, positions, slots, inv_freq, k_pages, v_pages)
-    vd = hd if vd is None else vd
-    width = (nq + nkv) * hd + nkv * vd          # nkv = 0: a row of query heads alone (nothing goes to the pages)
-    assert nkv > 0 or slots is None
-    if in_splits:
-        assert qkv.dim() == 3 and qkv.shape[0] == in_splits and qkv.stride(2) == 1 and qkv.dtype == torch.float32
-        n, row_stride, split_stride = qkv.shape[1], qkv.stride(1), qkv.stride(0)
-    else:
-        assert qkv.dim() == 2 and qkv.stride(1) == 1
-        n, row_stride, split_stride = qkv.shape[0], qkv.stride(0), 0
-    assert qkv.shape[-1] == width and q_out.shape == (n, nq * hd) and q_out.stride(1) == 1
-    assert inv_freq.dtype == torch.float32 and inv_freq.numel() == rot_dim // 2 and inv_freq.is_contiguous()
-    if slots is not None:
-        assert k_pages.is_contiguous() and v_pages.is_contiguous() and k_pages.dtype == q_out.dtype == v_pages.dtype
-    lib = load_family("rope_cache")
-    _check(lib.wllm_rope_kv_write_general(_ptr(qkv), _dt(qkv), row_stride, max(1, in_splits), ctypes.c_longlong(split_stride),
-                                          _ptr(q_out), _dt(q_out), q_out.stride(0), _ptr(_int32(positions, "positions")),
-                                          _ptr(_int32(slots, "slots") if slots is not None else None), _ptr(inv_freq),
-                                          _ptr(k_pages), _ptr(v_pages), n, nq, nkv, hd, rot_dim, page_size,
-                                          1 if pairing == "interleaved" else 0, vd, 0 if unit_norm_eps is None else 1,
-                                          c_float(unit_norm_eps or 0.0), c_float(turn_scale), _stream()),
-           "rope_kv_write")
+    # (nkv = 0: a row of query heads alone, nothing goes to the pages)
+    status = _host_call("rope_cache", "wllm_rope_kv_write_general").rope(
+        qkv, q_out, positions, slots, inv_freq, k_pages, v_pages, nq, nkv, hd, rot_dim, page_size, in_splits, pairing == "interleaved", vd, unit_norm_eps,
+        turn_scale)
+    if status:
+        _check(status, "rope_kv_write")
+    global launches
+    launches += 1
+
+
+_MIX = {None: 0, "first": 1, "later": 2}
 
 
 def rope_row_norm_kv_write(qkv: torch.Tensor, q_out: torch.Tensor, positions: torch.Tensor, slots, inv_freq: torch.Tensor,
@@ -315,32 +310,15 @@ def rope_row_norm_kv_write(qkv: torch.Tensor, q_out: torch.Tensor, positions: to
     alone.  `turn_scale` multiplies the sines and cosines."""
     if pairing not in ("half", "interleaved"):
         raise KernelError(f"rotary pairing {pairing!r} not supported (half, interleaved)")
-    _need_cuda(qkv, q_out, positions, slots, inv_freq, k_pages, v_pages, q_gain, k_gain)
-    vd = hd if vd is None else vd
-    width = (nq + nkv) * hd + nkv * vd
-    ptr, dt, row_stride, nparts, part_stride, n = _fused_args(qkv, in_splits)
-    assert qkv.shape[-1] >= width and q_out.shape == (n, nq * hd) and q_out.stride(1) == 1
-    assert inv_freq.dtype == torch.float32 and inv_freq.numel() == rot_dim // 2 and inv_freq.is_contiguous()
-    assert q_gain.shape == (nq * hd,) and q_gain.is_contiguous() and (nkv > 0 or slots is None)
-    assert (nkv == 0 and k_gain is None) or (k_gain.shape == (nkv * hd,) and k_gain.dtype == q_gain.dtype and k_gain.is_contiguous())
-    if slots is not None:
-        assert k_pages.is_contiguous() and v_pages.is_contiguous() and k_pages.dtype == q_out.dtype == v_pages.dtype
     if mix not in (None, "first", "later"):
         raise KernelError(f"value mixing {mix!r}: 'first' or 'later'")
-    _need_cuda(bias, v_first, blend)
-    assert bias is None or (bias.dtype == torch.float32 and bias.shape == (width,) and bias.is_contiguous())
-    if mix is not None:
-        assert v_first.dtype == torch.float32 and v_first.shape == (n, nkv * vd) and v_first.is_contiguous()
-        assert mix == "first" or (blend.dtype == torch.float32 and blend.numel() == 1)
-    lib = load_family("rope_cache")
-    _check(lib.wllm_rope_row_norm_kv_write(ptr, dt, row_stride, nparts, part_stride, _ptr(q_out), _dt(q_out), q_out.stride(0),
-                                           _ptr(_int32(positions, "positions")),
-                                           _ptr(_int32(slots, "slots") if slots is not None else None), _ptr(inv_freq),
-                                           _ptr(k_pages), _ptr(v_pages), n, nq, nkv, hd, rot_dim, page_size,
-                                           1 if pairing == "interleaved" else 0, vd, _ptr(q_gain), _ptr(k_gain), _dt(q_gain),
-                                           q_count, k_count, c_float(eps), _ptr(bias), _ptr(v_first if mix is not None else None),
-                                           _ptr(blend if mix == "later" else None), {None: 0, "first": 1, "later": 2}[mix],
-                                           c_float(turn_scale), _stream()), "rope_row_norm_kv_write")
+    status = _host_call("rope_cache", "wllm_rope_row_norm_kv_write").rope_row(
+        qkv, q_out, positions, slots, inv_freq, k_pages, v_pages, nq, nkv, hd, rot_dim, page_size, q_gain, k_gain, eps, q_count, k_count, in_splits,
+        pairing == "interleaved", vd, bias, v_first, blend, _MIX[mix], turn_scale)
+    if status:
+        _check(status, "rope_row_norm_kv_write")
+    global launches
+    launches += 1
 
 
 def rope_head_norm_kv_write(qkv: torch.Tensor, q_out: torch.Tensor, positions: torch.Tensor, slots, inv_freq: torch.Tensor,
@@ -597,6 +575,12 @@ def _status_word(device) -> torch.Tensor:
     return status
 
 
+def _device_status(device: torch.device) -> torch.Tensor:
+    """_status_word of a tensor's device, whose index is known."""
+    status = _tc_status.get(device)
+    return _status_word(device) if status is None else status
+
+
 def mma_head_dim_ok(hd: int) -> bool:
     """Head sizes the tensor-core attention kernels are built for (one build per size)."""
     return hd % 16 == 0 and 16 <= hd <= 256
@@ -641,24 +625,13 @@ def attention_mma_decode(q, out, k_pages, v_pages, req_q_start, req_q_len, req_c
     `sinks`: float32 [nq], one more term e^sink of every row's softmax denominator.  `cap` > 0: scores become
     cap * tanh(score / cap); `keep` > 0 (with a window): the sequence's first `keep` keys stay visible behind the window.
     `slopes`: float32 [nq]; the score of key j from position p loses slopes[head] * (p - j), after the scale and the cap."""
-    _need_cuda(q, out, k_pages, v_pages, req_q_start, req_q_len, req_ctx_len, block_table, scratch, sinks, slopes)
-    assert slopes is None or (slopes.dtype == torch.float32 and slopes.shape == (nq,) and slopes.is_contiguous())
-    assert sinks is None or (sinks.dtype == torch.float32 and sinks.shape == (nq,) and sinks.is_contiguous())
-    assert q.dtype == torch.bfloat16 == out.dtype == k_pages.dtype and q.stride(1) == 1 and out.stride(1) == 1
-    assert k_pages.is_contiguous() and v_pages.is_contiguous() and scratch.dtype == torch.float32
-    R = req_q_len.shape[0]
-    assert scratch.numel() >= attention_mma_scratch_floats(R, nq, hd, max_splits)
-    lib = load_family("attention_mma", {"HEAD_DIM": hd})
-    _check(lib.wllm_attention_mma_decode_biased(_ptr(q), q.stride(0), _ptr(out), out.stride(0), _ptr(k_pages), _ptr(v_pages),
-                                               ctypes.c_longlong(k_pages.shape[0]),
-                                               _ptr(_int32(req_q_start, "req_q_start")), _ptr(_int32(req_q_len, "req_q_len")),
-                                               _ptr(_int32(req_ctx_len, "req_ctx_len")),
-                                               _ptr(_int32(block_table, "block_table")), block_table.shape[1], R, nq, nkv,
-                                               page_size, window, c_float(scale), split_keys, max_splits, _ptr(scratch),
-                                               _ptr(_status_word(q.device)), _ptr(sinks), c_float(cap), keep, _ptr(slopes), _stream()),
-           f"attention_mma_decode(head_dim={hd}, heads={nq}/{nkv})")
+    status = _host_attention(hd).attention_decode(
+        q, out, k_pages, v_pages, req_q_start, req_q_len, req_ctx_len, block_table, nq, nkv, hd, page_size, window, scale, split_keys, max_splits, scratch,
+        _device_status(q.device), sinks, cap, keep, slopes)
+    if status:
+        _check(status, f"attention_mma_decode(head_dim={hd}, heads={nq}/{nkv})")
     global launches
-    launches += 1 if max_splits > 1 else 0    # the merge kernel
+    launches += 2 if max_splits > 1 else 1    # (with the merge kernel)
 
 
 def attention_prefill_halves_floats(requests: int, max_q_len: int, nq: int, nkv: int, hd: int) -> int:
@@ -701,24 +674,14 @@ def attention_mma_prefill(q, out, k_pages, v_pages, req_q_start, req_q_len, req_
     split_above > 0 (head sizes in steps of 64): a tile of 128 rows that walks more than that many tiles of 64
     keys is computed by two CTAs, half of the keys each; `halves` (float32) holds their partial results.
     `cap`, `keep`, `slopes`: as for attention_mma_decode; with any of them no tile is shared by two CTAs."""
-    _need_cuda(q, out, k_pages, v_pages, req_q_start, req_q_len, req_ctx_len, block_table, halves, sinks, slopes)
-    assert slopes is None or (slopes.dtype == torch.float32 and slopes.shape == (nq,) and slopes.is_contiguous())
-    assert sinks is None or (sinks.dtype == torch.float32 and sinks.shape == (nq,) and sinks.is_contiguous())
-    if split_above > 0:
-        assert hd % 64 == 0 and halves is not None and halves.dtype == torch.float32 and halves.is_contiguous()
-        assert halves.numel() >= attention_prefill_halves_floats(req_q_len.shape[0], max_q_len, nq, nkv, hd)
-    assert q.dtype == torch.bfloat16 == out.dtype == k_pages.dtype and q.stride(1) == 1 and out.stride(1) == 1
-    assert k_pages.is_contiguous() and v_pages.is_contiguous()
-    lib = load_family("attention_mma", {"HEAD_DIM": hd})
-    _check(lib.wllm_attention_mma_prefill_biased(_ptr(q), q.stride(0), _ptr(out), out.stride(0), _ptr(k_pages), _ptr(v_pages),
-                                                ctypes.c_longlong(k_pages.shape[0]),
-                                                _ptr(_int32(req_q_start, "req_q_start")), _ptr(_int32(req_q_len, "req_q_len")),
-                                                _ptr(_int32(req_ctx_len, "req_ctx_len")),
-                                                _ptr(_int32(block_table, "block_table")), block_table.shape[1],
-                                                req_q_len.shape[0], max_q_len, nq, nkv, page_size, window, c_float(scale),
-                                                1 if skip_single else 0, multi, split_above, _ptr(halves) if split_above > 0 else None,
-                                                _ptr(_status_word(q.device)), _ptr(sinks), c_float(cap), keep, _ptr(slopes), _stream()),
-           f"attention_mma_prefill(head_dim={hd}, heads={nq}/{nkv})")
+    floats = attention_prefill_halves_floats(req_q_len.shape[0], max_q_len, nq, nkv, hd) if split_above > 0 else 0
+    status = _host_attention(hd).attention_prefill(
+        q, out, k_pages, v_pages, req_q_start, req_q_len, req_ctx_len, block_table, max_q_len, nq, nkv, hd, page_size, window, scale, skip_single, multi,
+        split_above, halves, floats, _device_status(q.device), sinks, cap, keep, slopes)
+    if status:
+        _check(status, f"attention_mma_prefill(head_dim={hd}, heads={nq}/{nkv})")
+    global launches
+    launches += 1
 
 
 ACTIVATIONS = {"gelu_tanh": 0, "silu": 1, "relu": 2, "capped_swish": 3}
@@ -861,9 +824,7 @@ _tc_status: dict = {}
 
 def tc_gemm_ok(a: torch.Tensor, w: torch.Tensor) -> bool:
     """Shapes the tensor-memory GEMM takes: bfloat16, unit inner strides, K and pitches in steps of 8."""
-    return (a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and a.dim() == 2 and w.dim() == 2
-            and a.stride(1) == 1 and w.stride(1) == 1 and a.shape[1] % 8 == 0 and a.stride(0) % 8 == 0
-            and w.stride(0) % 8 == 0 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+    return _host_call("gemm_bf16_tc", "wllm_gemm_bf16_tc_params").tc_gemm_ok(a, w)
 
 
 @functools.lru_cache(maxsize=4096)
@@ -949,29 +910,26 @@ def gemm_bf16_tc(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = No
     clamped gated unit of gated_act, with its `limit` and `slope`) | 'relu_squared' (no gate: out[M, N] = max(a w^T, 0)^2).
     k_splits > 1 ('f32' only) cuts K into parts; `out` is then [k_splits, M, N] partial sums.
     half_rows: the tile of products of at most 128 rows (see tile_plan, which chooses it when None)."""
-    _need_cuda(a, w, out)
-    if not checked and not tc_gemm_ok(a, w):        # `checked`: the caller has asked tc_gemm_ok already
-        raise KernelError("gemm_bf16_tc: bfloat16 operands with K and row pitches in steps of 8 elements, 16-byte "
-                          f"aligned; got a{tuple(a.shape)} stride {a.stride()} w{tuple(w.shape)} stride {w.stride()}")
-    M, K = a.shape
-    N = w.shape[0]
-    assert w.shape[1] == K
     code = _TC_EPILOGUES[epilogue]
-    cols = N // 2 if code in _TC_GATED else N
-    shape = (M, cols) if k_splits == 1 else (k_splits, M, cols)
-    if out is None:
-        out = torch.empty(shape, dtype=torch.float32 if code == 1 else torch.bfloat16, device=a.device)
-    assert out.shape == shape and out.stride(-1) == 1 and out.dtype == (torch.float32 if code == 1 else torch.bfloat16)
-    assert k_splits == 1 or (code == 1 and out.is_contiguous())
-    status = _status_word(a.device)
-    if max_ctas is None:
-        max_ctas = sm_count()
-    lib = load_family("gemm_bf16_tc")
-    if half_rows is None:
-        half_rows = tile_plan(M, N, K, code in _TC_GATED, k_splits > 1)[0]
-    _check(lib.wllm_gemm_bf16_tc_params(_ptr(a), a.stride(0), _ptr(w), w.stride(0), _ptr(out), out.stride(-2), M, N, K, code,
-                                        k_splits, half_rows, _ptr(status), max_ctas, c_float(limit), c_float(slope), _stream()),
-           f"gemm_bf16_tc({M}x{N}x{K}, {epilogue}, {k_splits} parts)")
+    gated = code in _TC_GATED
+    host = _host_call("gemm_bf16_tc", "wllm_gemm_bf16_tc_params")
+    if out is None or half_rows is None:
+        _need_cuda(a, w, out)
+        if not checked and not host.tc_gemm_ok(a, w):        # `checked`: the caller has asked tc_gemm_ok already
+            raise KernelError("gemm_bf16_tc: bfloat16 operands with K and row pitches in steps of 8 elements, 16-byte "
+                              f"aligned; got a{tuple(a.shape)} stride {a.stride()} w{tuple(w.shape)} stride {w.stride()}")
+        M, K = a.shape
+        N = w.shape[0]
+        if out is None:
+            cols = N // 2 if gated else N
+            out = torch.empty((M, cols) if k_splits == 1 else (k_splits, M, cols), dtype=torch.float32 if code == 1 else torch.bfloat16, device=a.device)
+        if half_rows is None:
+            half_rows = tile_plan(M, N, K, gated, k_splits > 1)[0]
+    status = host.gemm(a, w, out, code, gated, k_splits, half_rows, sm_count() if max_ctas is None else max_ctas, limit, slope, _device_status(a.device), checked)
+    if status:
+        _check(status, f"gemm_bf16_tc({a.shape[0]}x{w.shape[0]}x{a.shape[1]}, {epilogue}, {k_splits} parts)")
+    global launches
+    launches += 1
     return out
 
 
