@@ -90,14 +90,19 @@ def _key(source: str, flags: list[str]) -> str:
 HOST_CALLS = "host_calls"      # the one source without kernels: a Python module (csrc/host_calls.cpp)
 
 
-def _host_flags() -> list[str]:
-    """What a module against torch's C++ interface and this interpreter is compiled with (the versions are part of the object's name)."""
+def _host_versions() -> list[str]:
+    """What a module against torch's C++ interface and this interpreter depends on (part of the object's name)."""
+    import torch
+    return [f"-DWLLM_TORCH=\"{torch.__version__}\"", f"-DWLLM_PYTHON=\"{sys.version.split()[0]}\"",
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-DUSE_CUDA"]
+
+
+def _host_paths() -> list[str]:
+    """Where such a module's headers and libraries are (asked when it is compiled: the interpreter takes 17 ms to say)."""
     import sysconfig
 
     import torch
-    base = os.path.dirname(torch.__file__)
-    flags = [f"-DWLLM_TORCH=\"{torch.__version__}\"", f"-DWLLM_PYTHON=\"{sys.version.split()[0]}\"",
-             f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-DUSE_CUDA"]
+    base, flags = os.path.dirname(torch.__file__), []
     for path in (os.path.join(base, "include"), os.path.join(base, "include", "torch", "csrc", "api", "include"), sysconfig.get_paths()["include"]):
         flags += ["-isystem", path]
     return flags + ["-L", os.path.join(base, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
@@ -108,7 +113,7 @@ def library_path(family: str, defines: dict | None = None) -> tuple[str, list[st
     if not os.path.isfile(source):
         raise KernelBuildError(f"no kernel source {source}")
     if family == HOST_CALLS:
-        flags = _host_flags()
+        flags = _host_versions()
         return source, flags, f"wllm_{family}-{_key(source, flags)}.so"
     flags = [f"-D{k}={v}" for k, v in sorted((defines or {}).items())]
     tag = "".join(f"_{k.lower()}{v}" for k, v in sorted((defines or {}).items()))
@@ -130,7 +135,8 @@ def compile_family(family: str, defines: dict | None = None, verbose: bool = Tru
             if os.path.isfile(out):
                 return out
             tmp = out + f".tmp{os.getpid()}"
-            cmd = [_nvcc()] + ARCH_FLAGS + BASE_FLAGS + flags + ["-I", CSRC, "-o", tmp, source, "-lcuda"]
+            cmd = [_nvcc()] + ARCH_FLAGS + BASE_FLAGS + flags + (_host_paths() if family == HOST_CALLS else []) + \
+                ["-I", CSRC, "-o", tmp, source, "-lcuda"]
             if verbose:
                 print(f"[wllm_b200] compiling {family}{' ' + ' '.join(flags) if flags else ''} for sm_100a ...",
                       file=sys.stderr, flush=True)
