@@ -841,8 +841,9 @@ static int launch_chunks(const bf16* fused, int row_stride, int q_off, int k_off
 // turn apart) and scaled.  decay [n, H, D] per key channel, or null with head_decay [H].  D 64 or 128, V in steps of 64.  lens: req_q_len on the host.  Requests
 // of LC_FROM tokens go in chunks, shorter ones token by token.
 // scratch (16-byte aligned): wllm_linattn_chunks_bytes, or less (more turns, the same bits) but a chunk of every request that goes in chunks.  launched: kernels.
-// 2,048 tokens of 8 heads of 128 x 256, launches back to back: 117 us, 223 for linattn_prepare and the walk in segments; 512 37 and 79, 128 32 and 50; 1,531
-// beside 24 single tokens 109 and 211.
+// 8 heads of 128 x 256, launches back to back, us; behind, linattn_prepare and the walk in segments: 2,048 tokens 78 (19 + 29 + 30 kernel by kernel) and 223;
+// 512 33 and 80; 128 32 and 52; 1,531 beside 24 single tokens 87 and 212; 256 beside 47 56 and 145; 16 requests of 130 138 and 151.  Below 128 tokens the host
+// bounds either.
 WLLM_API int wllm_linattn_chunks(const void* fused, int row_stride, int q_off, int k_off, int v_off, const int* positions, const float* inv_freq,
                                  int rot_dim, float q_scale, float k_scale, const float* decay, const float* head_decay, float* state, float* out,
                                  const int* req_q_start, const int* req_q_len, const int* req_slot, const int* lens, int requests, int H, int D, int V,
