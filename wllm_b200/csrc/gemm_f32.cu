@@ -11,10 +11,9 @@
 // Three kernels with that same arithmetic:
 //   tile kernel    steps of more than 32 rows, bound by the FMA pipes: BM x 128 x 16 tiles (BM = 64 or 128), 256
 //                  threads with 4 x 8 or 8 x 8 outputs each, operands transposed in shared memory and read
-//                  as float4, the next tile fetched into registers while the current one is multiplied; the
-//                  sums of finished segments wait in shared memory.
-//   wide kernel    steps of more than 64 rows (K and the pitches in steps of 4 floats, 16-byte aligned operands) where it is faster: tiles cut by
-//                  segments, a CTA each, and very many tiles; see gemm_f32_wide_kernel and wide_segments.
+//                  as float4, the next tile fetched into registers while the current one is multiplied.  A tile's CTA walks its segments (the
+//                  sums of finished ones wait in shared memory), or every segment has a CTA of its own and a second kernel adds the sums: see tile_plan.
+//   wide kernel    very many tiles (K and the pitches in steps of 4 floats, 16-byte aligned operands), where it is faster: see gemm_f32_wide_kernel.
 //   skinny kernel  steps of at most 32 rows, bound by streaming W once: a warp owns 32 rows of W and one
 //                  segment (so a matrix of few rows and long K still gives every SM many warps), streams it
 //                  through its own ring of cp.async stages and keeps one chain per row of A in each lane;
@@ -65,10 +64,18 @@ __device__ __forceinline__ void tile_stash(float (*dst)[ROWS + 4], int tid, cons
     }
 }
 
+// grid (row tiles, column tiles, segments with CTAs of their own, or 1); C: the result, or slabs [segment][M][N] seg_stride apart
 template <int BM, bool VEC>
 __global__ void __launch_bounds__(256, 2)
 gemm_f32_tile_kernel(const float* __restrict__ A, int lda, const float* __restrict__ W, int ldw, float* __restrict__ C,
-                     int ldc, int M, int N, int K) {
+                     int ldc, long long seg_stride, int M, int N, int K) {
+    if (gridDim.z > 1) {
+        const int k0 = blockIdx.z * SEG;
+        A += k0;
+        W += k0;
+        C += (size_t)blockIdx.z * seg_stride;
+        K = min(K - k0, SEG);
+    }
     constexpr int TM = BM / 16;            // 4 or 8 rows a thread: ty*4 + 0..3, and BM/2 + ty*4 + 0..3 when TM = 8
     __shared__ __align__(16) float As[2][TBK][BM + 4];
     __shared__ __align__(16) float Ws[2][TBK][TBN + 4];
@@ -257,36 +264,29 @@ gemm_f32_skinny_kernel(const float* __restrict__ A, int lda, const float* __rest
 // wide kernel: 128 x 128 tiles, 128 threads with 8 x 16 outputs each, two CTAs an SM.
 //
 // The tile kernel's scheme with two changes.  Neighbouring columns are multiplied two an instruction (fma.rn.f32x2: each half is the fused
-// multiply-add of its own chain, so the bits are the same): the pipes' peak is no higher for it (73.4 against 71.9 TFLOP/s in a loop), but half the
-// instructions compete for the schedulers and the register ports.  And a thread has twice the columns, 24 floats read from shared memory
-// for 128 products instead of 16 for 64.  A launch's last round
-// finds its SMs half empty and runs faster, so the tiles need not divide evenly.  Tiles cut by segments leave their
-// sums in slabs that the fold kernel adds in the same ascending order, in turns of as many segments as WIDE_SLABS floats hold; a tile that walks several
-// segments keeps their running total in C.  (Rows left as they lie in memory, brought by cp.async and read four k at a time, cannot be paired: 39 TFLOP/s;
-// A that way and W transposed: 51.)  Which products come here: wide_segments.  Measured in turn with the tile kernel, us: 509 x 2,048 x 16,384 cut 1,766 ->
-// 766, 509 x 2,048 x 2,048 cut 261 -> 212, 4,096 x 32,768 x 2,048 whole 11,347 -> 11,084 (49.6 TFLOP/s).
+// multiply-add of its own chain, so the bits are the same), so that half the instructions compete for the schedulers, and a thread has twice the columns, 24
+// floats read from shared memory for 128 products instead of 16 for 64.  A tile keeps the running total of its segments in C.  From some fourteen tiles an SM on
+// it is the faster one: 4,096 x 32,768 x 2,048 11,347 -> 11,084 us (49.6 TFLOP/s).  Cut by segments it loses to the tile kernel cut that way: 509 x 2,048 x 16,384
+// 759 and 704 us.  (Rows left as they lie in memory, brought by cp.async and read four k at a time, cannot be paired: 39 TFLOP/s; A that way and W transposed: 51.)
 // ------------------------------------------------------------------------------------------------
 constexpr int WT = 128, WTHREADS = 128;
 
-// grid (row tiles, column tiles, segments with CTAs of their own, or 1); dst: C, or slabs [segment][M][N]
+// grid (row tiles, column tiles)
 __global__ void __launch_bounds__(WTHREADS, 2)
-gemm_f32_wide_kernel(const float* __restrict__ A, int lda, const float* __restrict__ W, int ldw, float* __restrict__ dst, int ld_dst,
-                     long long seg_stride, int M, int N, int K) {
+gemm_f32_wide_kernel(const float* __restrict__ A, int lda, const float* __restrict__ W, int ldw, float* __restrict__ out, int ld_out, int M, int N, int K) {
     __shared__ __align__(16) float As[2][TBK][WT + 4];
     __shared__ __align__(16) float Ws[2][TBK][WT + 4];
     constexpr int CHUNKS = WT * TBK / 4 / WTHREADS;         // groups of four k a thread and operand: rows crow + 32 i, k ck .. ck + 3
     pdl_launch_dependents();
     const int tid = threadIdx.x, m0 = blockIdx.x * WT, n0 = blockIdx.y * WT;       // neighbours in the grid share a tile of W
-    const int k_begin = gridDim.z > 1 ? blockIdx.z * SEG : 0, k_end = gridDim.z > 1 ? min(K, k_begin + SEG) : K;
-    const int tiles = (k_end - k_begin + TBK - 1) / TBK;
-    float* out = dst + (gridDim.z > 1 ? (size_t)blockIdx.z * seg_stride : 0);
+    const int tiles = (K + TBK - 1) / TBK;
     const int crow = tid >> 2, ck = (tid & 3) * 4;
     auto fetch = [&](const float* __restrict__ src, int ld, int rows, int r0, int t, float4 (&reg)[CHUNKS]) {
-        const int gk = k_begin + t * TBK + ck;
+        const int gk = t * TBK + ck;
 #pragma unroll
         for (int i = 0; i < CHUNKS; ++i) {
             const int row = r0 + crow + 32 * i;
-            reg[i] = row < rows && gk < k_end ? *reinterpret_cast<const float4*>(src + (size_t)row * ld + gk) : make_float4(0.f, 0.f, 0.f, 0.f);
+            reg[i] = row < rows && gk < K ? *reinterpret_cast<const float4*>(src + (size_t)row * ld + gk) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
     };
     auto stash = [&](float (*to)[WT + 4], const float4 (&reg)[CHUNKS]) {
@@ -303,7 +303,7 @@ gemm_f32_wide_kernel(const float* __restrict__ A, int lda, const float* __restri
 #pragma unroll
         for (int j = 0; j < 8; ++j) acc[i][j] = make_float2(0.f, 0.f);
     // what the accumulators hold joins the running total (add) or becomes it
-    const bool vec_out = (ld_dst & 3) == 0 && (seg_stride & 3) == 0 && ((uintptr_t)dst & 15) == 0;
+    const bool vec_out = (ld_out & 3) == 0 && ((uintptr_t)out & 15) == 0;
     auto leave = [&](bool add) {
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
@@ -312,7 +312,7 @@ gemm_f32_wide_kernel(const float* __restrict__ A, int lda, const float* __restri
 #pragma unroll
             for (int h = 0; h < 4; ++h) {
                 const int gn = n0 + 32 * h + 4 * tx;
-                float* to = out + (size_t)gm * ld_dst + gn;
+                float* to = out + (size_t)gm * ld_out + gn;
                 float4 v = make_float4(acc[i][2 * h].x, acc[i][2 * h].y, acc[i][2 * h + 1].x, acc[i][2 * h + 1].y);
                 if (vec_out && gn + 3 < N) {
                     if (add) {
@@ -383,6 +383,15 @@ gemm_f32_fold_kernel(const float* __restrict__ parts, float* __restrict__ C, int
     *to = total;
 }
 
+static int sm_count() {
+    static int sms = 0;
+    if (!sms) {
+        int dev = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 148;
+    }
+    return sms;
+}
+
 template <int BM, int STAGES>
 static int launch_skinny_as(const float* A, int lda, const float* W, int ldw, float* C, int ldc, int M, int N, int K,
                             float* scratch, cudaStream_t stream) {
@@ -409,37 +418,32 @@ static int launch_skinny(const float* A, int lda, const float* W, int ldw, float
                          float* scratch, long long scratch_floats, cudaStream_t stream) {
     const int segs = (K + SEG - 1) / SEG;
     if (segs > 1 && (scratch == nullptr || scratch_floats < (long long)segs * M * N)) return WLLM_BAD_SIZE;
-    static int sms = 0;
-    if (!sms) {
-        int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-            sms = 148;
-    }
-    const int tasks = ((N + SBN - 1) / SBN) * segs;
+    const int sms = sm_count(), tasks = ((N + SBN - 1) / SBN) * segs;
     constexpr int DEEP = skinny_deep_stages<BM>();
     if (DEEP != SSTAGES_FULL && tasks <= sms * SWARPS)      // at most one CTA's worth of warps an SM: few tasks
         return launch_skinny_as<BM, DEEP>(A, lda, W, ldw, C, ldc, M, N, K, scratch, stream);
     return launch_skinny_as<BM, SSTAGES_FULL>(A, lda, W, ldw, C, ldc, M, N, K, scratch, stream);
 }
 
+// segs > 1: that many segments from A and W on, each with CTAs of its own, into slabs [segment][M][N]
 template <int BM, bool VEC>
-static int launch_tile(const float* A, int lda, const float* W, int ldw, float* C, int ldc, int M, int N, int K,
-                       cudaStream_t stream) {
-    const size_t totals = K > SEG ? (size_t)(BM / 16) * 8 * 256 * sizeof(float) : 0;
+static int launch_tile(const float* A, int lda, const float* W, int ldw, float* C, int ldc, int M, int N, int K, int segs, cudaStream_t stream) {
+    constexpr size_t most = (size_t)(BM / 16) * 8 * 256 * sizeof(float), alone = 96 * 1024;
     static bool raised = false;
-    if (totals > 0 && !raised) {
-        const cudaError_t e = cudaFuncSetAttribute(gemm_f32_tile_kernel<BM, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   (int)((size_t)(BM / 16) * 8 * 256 * sizeof(float)));
+    if (!raised) {
+        const cudaError_t e = cudaFuncSetAttribute(gemm_f32_tile_kernel<BM, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(most > alone ? most : alone));
         if (e != cudaSuccess) return 1000 + (int)e;
         raised = true;
     }
-    const dim3 grid((M + BM - 1) / BM, (N + TBN - 1) / TBN);
-    return wllm_launch(gemm_f32_tile_kernel<BM, VEC>, grid, 256, totals, stream, A, lda, W, ldw, C, ldc, M, N, K);
+    const dim3 grid((M + BM - 1) / BM, (N + TBN - 1) / TBN, segs);
+    size_t smem = segs == 1 && K > SEG ? most : 0;
+    // CTAs that are launched while the kernel before still fills some SMs would pile up in pairs on the others (509 x 2,048 x 2,048 in 128 CTAs: 196 us)
+    if ((long long)grid.x * grid.y * grid.z <= sm_count() && smem < alone) smem = alone;
+    return wllm_launch(gemm_f32_tile_kernel<BM, VEC>, grid, 256, smem, stream, A, lda, W, ldw, C, ldc, (long long)M * N, M, N, K);
 }
 
-// The most slabs' floats that a product asks for (256 MB).  A product that is cut has at most 592 tiles, so that a turn has some 4,000 CTAs and more,
-// fourteen rounds of two an SM; slabs without a bound were 600 MB for 4,608 x 2,048 x 16,384.  (4,096 x 2,048 x 16,384: 5,672 us at once, 6,071 in turns of four.)
-constexpr long long WIDE_SLABS = 64ll << 20;
+// The most slabs' floats that a product asks for (256 MB): slabs without a bound were 600 MB for 4,608 x 2,048 x 16,384.
+constexpr long long SLABS = 64ll << 20;
 
 // Segments of a turn for `floats` of scratch.
 static int turn_of(int M, int N, int segs, long long floats) {
@@ -447,47 +451,44 @@ static int turn_of(int M, int N, int segs, long long floats) {
     return (int)(room < segs ? (room < 65535 ? room : 65535) : (segs < 65535 ? segs : 65535));
 }
 
-// Half rounds of two CTAs an SM: a last round that leaves every SM one CTA or none takes half a round's time.
-static long long half_rounds(long long ctas, int sms) {
-    const long long rest = ctas % (2 * sms);
-    return 2 * (ctas / (2 * sms)) + (rest == 0 ? 0 : (rest <= sms ? 1 : 2));
+// How a product of more than 32 rows runs: tiles of `rows` (64, 128; 0: the wide kernel) rows, segments with CTAs of their own `turn` at a time (1: a tile's CTA
+// walks them all).
+struct TilePlan { int rows, turn; };
+
+// A round gives every SM one tile's segment of 1,024 k: 98 us with 128 rows, 60 with 64 (two CTAs an SM take as long as one behind the other).  Cut by segments
+// there are more of them to deal out, for the slabs' way through memory at some 5 TB/s and another launch.  us as measured, whole with 128 rows, whole 64, cut
+// 128, cut 64 (the model): 509 x 2,048 x 2,048 259, 224, 117 (103), 131 (125); 509 x 2,560 x 2,048 331, 245, 206 (203), 200 (187);
+// 509 x 2,048 x 16,384 2,063, 1,898, 704 (706), 907 (860); 509 x 32,768 x 2,048 1,387 (1,372), 1,759, 1,448 (1,447), 1,849; 256 x 32,768 x 2,048 792 (784), 999,
+// 729 (723), 939; 128 x 2,048 x 2,048 222, 149, 112 (102), 77 (64); 64 x 2,048 x 16,384 cut 64 145, 1,578 whole.
+static TilePlan tile_plan(int M, int N, int K, long long floats) {
+    const int segs = (K + SEG - 1) / SEG, sms = sm_count();
+    const long long cols = (N + TBN - 1) / TBN;
+    TilePlan best = {128, 1};
+    double least = 0;
+    for (int rows = 128; rows >= 64; rows -= 64) {
+        const double round = rows == 128 ? 98 : 60;
+        const long long tiles = (M + rows - 1) / rows * cols;
+        const double whole = round * segs * ((tiles + sms - 1) / sms);
+        if (rows == 128 || whole < least) { least = whole; best = {rows, 1}; }
+        const int turn = turn_of(M, N, segs, floats < SLABS ? floats : SLABS);
+        if (turn < 2) continue;
+        const long long rounds = segs / turn * ((tiles * turn + sms - 1) / sms) + (tiles * (segs % turn) + sms - 1) / sms;
+        const double cut = round * rounds + 4.0 * M * N * (2 * segs + 1) / 5e6 + 3.0 * ((segs + turn - 1) / turn);
+        if (cut < least) { least = cut; best = {rows, turn}; }
+    }
+    if (best.rows == 128 && best.turn == 1 && (M + 127) / 128 * cols >= 14ll * sms) best.rows = 0;
+    return best;
 }
 
-// How a product of more than 64 rows runs: its segments (more than one), each with CTAs of its own; 1: the wide kernel's tiles walk them; 0: the tile
-// kernel's do.  Cut, where the tiles leave SMs idle, or where that takes fewer half rounds of a segment each by more than the slabs' five per cent.
-// Whole, the tile kernel is the faster one until some fourteen tiles an SM.  us by the tile kernel, cut, whole, K 2,048: 64 tiles 261, 212, 257;
-// 192 416, 335, 432; 256 414, 442, 432; 320 636, 552, 646; 384 635, 658, 666; 512 826, 767, 843; 576 828, 875, 851; 1,024 1,445 and 1,482
-// whole, 1,536 2,246 and 2,227 to 2,270, 2,048 2,851 and 2,859, 3,072 4,268 and 4,222, 8,192 11,347 and 11,084.  K 508: 32 tiles 58 and 67.
-static int wide_segments(int M, int N, int K) {
-    static int sms = 0;
-    if (!sms) {
-        int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 148;
-    }
+template <int BM>
+static int launch_cut(const float* A, int lda, const float* W, int ldw, float* C, int ldc, int M, int N, int K, float* scratch, int turn, cudaStream_t stream) {
     const int segs = (K + SEG - 1) / SEG;
-    const long long tiles = (long long)((M + WT - 1) / WT) * ((N + WT - 1) / WT);
-    if (segs > 1 && tiles < 4ll * sms) {
-        const int turn = turn_of(M, N, segs, WIDE_SLABS);
-        if (tiles <= sms && turn > 1) return segs;
-        if (turn > 1 && 21 * (segs / turn * half_rounds(tiles * turn, sms) + half_rounds(tiles * (segs % turn), sms)) < 20 * segs * half_rounds(tiles, sms))
-            return segs;
-    }
-    return tiles >= 14ll * sms ? 1 : 0;
-}
-
-// turn: segments with CTAs of their own at a time; 1: a tile's CTA walks them all
-static int launch_wide(const float* A, int lda, const float* W, int ldw, float* C, int ldc, int M, int N, int K, float* scratch, int turn,
-                       cudaStream_t stream) {
-    const int segs = (K + SEG - 1) / SEG;
-    dim3 grid((M + WT - 1) / WT, (N + WT - 1) / WT);
-    if (turn < 2) return wllm_launch(gemm_f32_wide_kernel, grid, WTHREADS, 0, stream, A, lda, W, ldw, C, ldc, (long long)M * N, M, N, K);
     for (int s0 = 0; s0 < segs; s0 += turn) {
-        grid.z = segs - s0 < turn ? segs - s0 : turn;
-        int st = wllm_launch(gemm_f32_wide_kernel, grid, WTHREADS, 0, stream, A + (size_t)s0 * SEG, lda, W + (size_t)s0 * SEG, ldw, scratch, N,
-                             (long long)M * N, M, N, K - s0 * SEG);
+        const int mine = segs - s0 < turn ? segs - s0 : turn;
+        // (a lone segment at the end, which the kernel walks as a whole product, goes to a slab too)
+        int st = launch_tile<BM, true>(A + (size_t)s0 * SEG, lda, W + (size_t)s0 * SEG, ldw, scratch, N, M, N, K - s0 * SEG, mine, stream);
         if (st == WLLM_OK)
-            st = wllm_launch(gemm_f32_fold_kernel, dim3((unsigned)(((size_t)M * N + 255) / 256)), 256, 0, stream, (const float*)scratch, C, ldc, M, N,
-                             (int)grid.z, s0 > 0);
+            st = wllm_launch(gemm_f32_fold_kernel, dim3((unsigned)(((size_t)M * N + 255) / 256)), 256, 0, stream, (const float*)scratch, C, ldc, M, N, mine, s0 > 0);
         if (st != WLLM_OK) return st;
     }
     return WLLM_OK;
@@ -497,13 +498,13 @@ static bool vec_operands(const void* A, int lda, const void* W, int ldw, int K) 
     return K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && (uintptr_t)A % 16 == 0 && (uintptr_t)W % 16 == 0;
 }
 
-// Floats of scratch that a product of these operands and sizes wants (0: none): partial sums of the skinny kernel, which needs them, or of the wide one,
+// Floats of scratch that a product of these operands and sizes wants (0: none): partial sums of the skinny kernel, which needs them, or of the tile one,
 // which does with any less.
 WLLM_API long long wllm_gemm_f32_scratch_floats(const float* A, int lda, const float* W, int ldw, int M, int N, int K) {
     if (M <= 0 || N <= 0 || K <= 0 || !vec_operands(A, lda, W, ldw, K)) return 0;
     if (M <= 32) return K > SEG ? (long long)((K + SEG - 1) / SEG) * M * N : 0;
-    const int segs = M > 64 ? wide_segments(M, N, K) : 0, turn = segs > 1 ? turn_of(M, N, segs, WIDE_SLABS) : 0;
-    return turn > 1 ? (long long)turn * M * N : 0;
+    const TilePlan plan = tile_plan(M, N, K, SLABS);
+    return plan.turn > 1 ? (long long)plan.turn * M * N : 0;
 }
 
 WLLM_API int wllm_gemm_f32(const float* A, int lda, const float* W, int ldw, float* C, int ldc, int M, int N, int K,
@@ -514,16 +515,18 @@ WLLM_API int wllm_gemm_f32(const float* A, int lda, const float* W, int ldw, flo
     if (vec && M <= 8) return launch_skinny<8>(A, lda, W, ldw, C, ldc, M, N, K, scratch, scratch_floats, stream);
     if (vec && M <= 16) return launch_skinny<16>(A, lda, W, ldw, C, ldc, M, N, K, scratch, scratch_floats, stream);
     if (vec && M <= 32) return launch_skinny<32>(A, lda, W, ldw, C, ldc, M, N, K, scratch, scratch_floats, stream);
-    if (M <= 64) {
-        if (vec) return launch_tile<64, true>(A, lda, W, ldw, C, ldc, M, N, K, stream);
-        return launch_tile<64, false>(A, lda, W, ldw, C, ldc, M, N, K, stream);
+    if (!vec) {
+        if (M <= 64) return launch_tile<64, false>(A, lda, W, ldw, C, ldc, M, N, K, 1, stream);
+        return launch_tile<128, false>(A, lda, W, ldw, C, ldc, M, N, K, 1, stream);
     }
-    const int segs = vec ? wide_segments(M, N, K) : 0;
-    // without room for two slabs the tile kernel's tiles walk their segments: the same bits
-    const int turn = segs > 1 ? turn_of(M, N, segs, scratch == nullptr ? 0 : scratch_floats) : segs;
-    if (turn > 1 || segs == 1) return launch_wide(A, lda, W, ldw, C, ldc, M, N, K, scratch, turn, stream);
-    if (vec) return launch_tile<128, true>(A, lda, W, ldw, C, ldc, M, N, K, stream);
-    return launch_tile<128, false>(A, lda, W, ldw, C, ldc, M, N, K, stream);
+    // without room for two slabs a tile's CTA walks its segments: the same bits
+    const TilePlan plan = tile_plan(M, N, K, scratch == nullptr ? 0 : scratch_floats);
+    if (plan.rows == 0)
+        return wllm_launch(gemm_f32_wide_kernel, dim3((M + WT - 1) / WT, (N + WT - 1) / WT), WTHREADS, 0, stream, A, lda, W, ldw, C, ldc, M, N, K);
+    if (plan.turn > 1)
+        return plan.rows == 64 ? launch_cut<64>(A, lda, W, ldw, C, ldc, M, N, K, scratch, plan.turn, stream)
+                               : launch_cut<128>(A, lda, W, ldw, C, ldc, M, N, K, scratch, plan.turn, stream);
+    return plan.rows == 64 ? launch_tile<64, true>(A, lda, W, ldw, C, ldc, M, N, K, 1, stream) : launch_tile<128, true>(A, lda, W, ldw, C, ldc, M, N, K, 1, stream);
 }
 
 // ------------------------------------------------------------------------------------------------
