@@ -1,0 +1,41 @@
+"""32-bit attention of portions of prompts, dealt out by chunks of keys, beside the tiled kernel: the same bits."""
+from __future__ import annotations
+
+import pytest
+import torch
+
+DEV = "cuda:0"
+pytestmark = pytest.mark.gpu
+
+
+# portions that end in a tile of rows, of keys, of a chunk, one past and one short of them; on cached keys; single tokens beside them
+@pytest.mark.parametrize("lens,before", [([64], [0]), ([1, 33, 65], [0, 5, 63]), ([31, 1, 127, 128], [200, 300, 1, 0]), ([190], [131])])
+@pytest.mark.parametrize("nq,nkv,hd,vd,ps", [(8, 1, 256, 256, 64), (4, 4, 16, 16, 16), (6, 2, 72, 40, 16), (4, 2, 128, 256, 32)])
+@pytest.mark.parametrize("extra", ["plain", "all"])
+def test_chunks_give_the_tiled_kernels_bits(lens, before, nq, nkv, hd, vd, ps, extra):
+    from wllm_b200.kernels import ops
+    g = torch.Generator().manual_seed(sum(lens) + hd)
+    R, n, ctx = len(lens), sum(lens), [m + b for m, b in zip(lens, before)]
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    pages = [-(-c // ps) for c in ctx]
+    table, at = torch.zeros(R, max(pages) + 1, dtype=torch.int32), 1
+    order = torch.randperm(sum(pages), generator=g) + 1
+    for r, p in enumerate(pages):
+        table[r, :p] = order[at - 1:at - 1 + p]
+        at += p
+    # what lies behind a request's last key in its page is no number
+    k, v = (torch.full((sum(pages) + 1, nkv, ps, d), float("nan")) for d in (hd, vd))
+    for r, c in enumerate(ctx):
+        for key in range(c):
+            page = int(table[r, key // ps])
+            k[page, :, key % ps], v[page, :, key % ps] = torch.randn(nkv, hd, generator=g), torch.randn(nkv, vd, generator=g)
+    q = torch.randn(n, nq * hd + 8, generator=g).to(DEV)[:, :nq * hd]
+    meta = (i32([sum(lens[:r]) for r in range(R)]), i32(lens), i32(ctx), table.to(DEV))
+    positions = i32([b + j for m, b in zip(lens, before) for j in range(m)])
+    more = dict(sinks=torch.randn(nq, generator=g).to(DEV), cap=3.0, slopes=torch.rand(nq, generator=g).to(DEV)) if extra == "all" else {}
+    want, got = (torch.full((n, nq * vd), float("nan"), device=DEV) for _ in range(2))
+    ops.paged_attention_simt_tiled(q, want, k.to(DEV), v.to(DEV), *meta, max(lens), nq, nkv, hd, ps, 0, hd ** -0.5, vd=vd, **more)
+    chunks = -(-max(ctx) // 64)
+    scratch = torch.full((n * nq * chunks * (vd + 2),), float("nan"), device=DEV)
+    ops.paged_attention_simt_chunks(q, got, k.to(DEV), v.to(DEV), positions, *meta, max(lens), nq, nkv, hd, ps, hd ** -0.5, scratch, chunks, vd=vd, **more)
+    assert bool(want.isfinite().all()) and torch.equal(want, got)

@@ -553,6 +553,160 @@ paged_attention_simt_tiled_kernel(const T* __restrict__ q, int q_stride, T* __re
     }
 }
 
+// --------------------------------------------------------------------------------------
+// tiled, chunk by chunk: grid (tiles of 32 rows x chunks of 64 keys, kv heads, requests), for steps whose tiles are too few to fill the device one behind the
+// other.  A CTA works out its rows' result over one chunk as the tiled kernel does and leaves m, l, o[vd] in scratch[(row * max_chunks + chunk) * (vd + 2)],
+// where the walk's merge kernel takes them up in order: the same bits.  Without a running total and with one tile of keys and values in shared memory (a tile's
+// values land while its scores are worked out, the next tile's keys during the weighted sum) two CTAs fit on an SM.  Every key is seen from its position on (no window).
+// --------------------------------------------------------------------------------------
+template <typename T, int NE>
+__global__ void __launch_bounds__(TL_WARPS * 32, 2)
+paged_attention_simt_chunk_kernel(const T* __restrict__ q, int q_stride, const T* __restrict__ k_pages, const T* __restrict__ v_pages,
+                                  const int* __restrict__ req_q_start, const int* __restrict__ req_q_len, const int* __restrict__ req_ctx_len,
+                                  const int* __restrict__ block_table, int max_pages, int nq, int nkv, int hd, int page_size, float scale, int vd, float cap,
+                                  const float* __restrict__ slopes, float* __restrict__ scratch, int max_chunks) {
+    constexpr int VN = Vec<T>::N;
+    extern __shared__ __align__(16) unsigned char tl_smem[];
+    __shared__ size_t row_of[CHUNK];               // the chunk's keys in the pools
+    pdl_begin();
+    const int g = blockIdx.y, r = blockIdx.z, c = blockIdx.x % max_chunks, m0 = blockIdx.x / max_chunks * TL_ROWS;
+    const int q_len = req_q_len[r], rep = nq / nkv, rows = q_len * rep;
+    if (m0 >= rows) return;
+    const int ctx = req_ctx_len[r], q_start = req_q_start[r], pos0 = ctx - q_len;
+    const int key_hi = pos0 + (min(rows, m0 + TL_ROWS) - 1) / rep + 1;         // one past the last row's position
+    if (c * CHUNK >= key_hi) return;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int kld = hd + VN;
+    float* qs = reinterpret_cast<float*>(tl_smem);                          // [32 rows][hd] float
+    T* ks = reinterpret_cast<T*>(qs + TL_ROWS * hd);                        // [32 keys][kld]
+    T* vs = ks + 32 * kld;                                                  // [32 keys][vd]
+    if (threadIdx.x < CHUNK) {
+        const int key = min(c * CHUNK + (int)threadIdx.x, key_hi - 1);
+        row_of[threadIdx.x] = ((size_t)block_table[(size_t)r * max_pages + key / page_size] * nkv + g) * page_size + key % page_size;
+    }
+    int pos_r[TL_RPW];
+    float slope_r[TL_RPW];
+#pragma unroll
+    for (int i = 0; i < TL_RPW; ++i) {
+        const int m = m0 + warp * TL_RPW + i;
+        slope_r[i] = slopes ? slopes[g * rep + m % rep] : 0.f;
+        pos_r[i] = m < rows ? pos0 + m / rep : -1;                          // a row past the end takes no key
+    }
+    __syncthreads();
+    // 32 rows of `pieces` 16-byte pieces; keys past the last row's are zeros
+    auto load = [&](int t, T* to, const T* from, int ld, int width, int to_ld) {
+        const int pieces = width / VN, rows_on = (int)blockDim.x / pieces, pieces_on = (int)blockDim.x % pieces;
+        int kl = threadIdx.x / pieces, piece = threadIdx.x % pieces;
+        while (kl < 32) {
+            cp_async_16(to + kl * to_ld + piece * VN, from + row_of[(t & 1) * 32 + kl] * ld + piece * VN, t * 32 + kl < key_hi);
+            kl += rows_on;
+            piece += pieces_on;
+            if (piece >= pieces) { piece -= pieces; ++kl; }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    const int t0 = 2 * c, t1 = min(t0 + 2, (key_hi + 31) >> 5);
+    load(t0, ks, k_pages, hd, hd, kld);
+    load(t0, vs, v_pages, vd, vd, vd);
+    for (int idx = threadIdx.x; idx < TL_ROWS * hd; idx += blockDim.x) {
+        const int m = m0 + idx / hd, d = idx % hd;
+        qs[idx] = m < rows ? to_f32(q[(size_t)(q_start + m / rep) * q_stride + (size_t)(g * rep + m % rep) * hd + d]) : 0.f;
+    }
+    float m_c[TL_RPW], l_c[TL_RPW], o_c[TL_RPW][NE];
+#pragma unroll
+    for (int i = 0; i < TL_RPW; ++i) {
+        m_c[i] = -INFINITY; l_c[i] = 0.f;
+#pragma unroll
+        for (int e = 0; e < NE; ++e) o_c[i][e] = 0.f;
+    }
+    for (int t = t0; t < t1; ++t) {
+        const int tile = t * 32, key = tile + lane;
+        bool act[TL_RPW], any = false;
+#pragma unroll
+        for (int i = 0; i < TL_RPW; ++i) { act[i] = tile <= pos_r[i]; any = any || act[i]; }
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();                          // the tile's keys are here for everyone (and the queries, the first time)
+        float p[TL_RPW] = {0.f, 0.f, 0.f, 0.f};
+        if (any) {
+            const T* kr = ks + (size_t)lane * kld;
+            const float* qw = qs + (size_t)(warp * TL_RPW) * hd;
+            float acc[TL_RPW][4];
+#pragma unroll
+            for (int i = 0; i < TL_RPW; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+#pragma unroll 2
+            for (int d = 0; d < hd; d += VN) {
+                float kv[VN];
+                Vec<T>::load(kr + d, kv);
+#pragma unroll
+                for (int i = 0; i < TL_RPW; ++i) {
+                    float qv[VN];
+#pragma unroll
+                    for (int u = 0; u < VN; u += 4) {
+                        const float4 t4 = *reinterpret_cast<const float4*>(qw + (size_t)i * hd + d + u);
+                        qv[u] = t4.x; qv[u + 1] = t4.y; qv[u + 2] = t4.z; qv[u + 3] = t4.w;
+                    }
+#pragma unroll
+                    for (int u = 0; u < VN; ++u) acc[i][u & 3] = fmaf(qv[u], kv[u], acc[i][u & 3]);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < TL_RPW; ++i) {
+                if (!act[i]) continue;
+                const bool valid = key <= pos_r[i];
+                float s = valid ? ((acc[i][0] + acc[i][1]) + (acc[i][2] + acc[i][3])) * scale : -INFINITY;
+                if (valid && cap > 0.f) s = cap * tanhf(s / cap);
+                if (valid && slope_r[i] != 0.f) s = __fsub_rn(s, __fmul_rn(slope_r[i], (float)(pos_r[i] - key)));
+                const float m_new = fmaxf(m_c[i], warp_max(s));
+                p[i] = valid ? expf(s - m_new) : 0.f;
+                const float corr = expf(m_c[i] - m_new);
+                l_c[i] = fmaf(l_c[i], corr, warp_sum(p[i]));
+#pragma unroll
+                for (int e = 0; e < NE; ++e) o_c[i][e] *= corr;
+                m_c[i] = m_new;
+            }
+        }
+        __syncthreads();                          // everyone is done with the keys
+        if (t + 1 < t1) load(t + 1, ks, k_pages, hd, hd, kld);
+        else asm volatile("cp.async.commit_group;" ::: "memory");
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();                          // the tile's values are here
+        if (any) {
+#pragma unroll 2
+            for (int j = 0; j < 32; ++j) {
+                float v[NE];
+#pragma unroll
+                for (int e = 0; e < NE; ++e) {
+                    const int d = e * 32 + lane;
+                    v[e] = d < vd ? to_f32(vs[(size_t)j * vd + d]) : 0.f;
+                }
+#pragma unroll
+                for (int i = 0; i < TL_RPW; ++i) {
+                    const float pj = __shfl_sync(0xffffffffu, p[i], j);
+#pragma unroll
+                    for (int e = 0; e < NE; ++e) o_c[i][e] = fmaf(pj, v[e], o_c[i][e]);
+                }
+            }
+        }
+        if (t + 1 < t1) {
+            __syncthreads();                      // everyone is done with the values
+            load(t + 1, vs, v_pages, vd, vd, vd);
+        }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < TL_RPW; ++i) {
+        const int m = m0 + warp * TL_RPW + i;
+        if (pos_r[i] < c * CHUNK) continue;
+        float* dst = scratch + (((size_t)(q_start + m / rep) * nq + g * rep + m % rep) * max_chunks + c) * (vd + 2);
+        if (lane == 0) { dst[0] = m_c[i]; dst[1] = l_c[i]; }
+#pragma unroll
+        for (int e = 0; e < NE; ++e) {
+            const int d = e * 32 + lane;
+            if (d < vd) dst[2 + d] = o_c[i][e];
+        }
+    }
+}
+
 template <typename T>
 static int launch_tiled(const void* q, int q_stride, void* out, int out_stride, const void* k_pages, const void* v_pages,
                         const int* req_q_start, const int* req_q_len, const int* req_ctx_len, const int* block_table,
@@ -628,4 +782,42 @@ WLLM_API int wllm_paged_attention_simt_tiled(const void* q, int q_stride, void* 
     return wllm_paged_attention_simt_tiled_general(q, q_stride, out, out_stride, k_pages, v_pages, dtype, req_q_start, req_q_len,
                                                    req_ctx_len, block_table, max_pages, requests, max_q_len, nq, nkv, hd,
                                                    page_size, window, scale, hd, nullptr, 0.f, 0, stream);
+}
+
+// The tiled kernel's result over steps without a window, chunk by chunk, bit for bit.  scratch: n_tokens * nq * max_chunks * (vd + 2) floats; max_chunks: chunks of
+// 64 keys of the longest context; positions [n_tokens].  32-bit rows of up to 256 elements (the bfloat16 form is not built).
+WLLM_API int wllm_paged_attention_simt_chunks(const void* q, int q_stride, void* out, int out_stride, const void* k_pages, const void* v_pages,
+                                              const int* positions, const int* req_q_start, const int* req_q_len, const int* req_ctx_len,
+                                              const int* block_table, int max_pages, int n_tokens, int requests, int max_q_len, int nq, int nkv, int hd,
+                                              int page_size, float scale, int vd, const float* sinks, float cap, const float* slopes, float* scratch,
+                                              int max_chunks, cudaStream_t stream) {
+    if (n_tokens <= 0 || requests <= 0 || max_q_len <= 0) return WLLM_OK;
+    if (hd <= 0 || hd > 256 || hd % 8 != 0 || vd <= 0 || vd > 256 || vd % 8 != 0 || nq <= 0 || nkv <= 0 || nq % nkv != 0 || page_size <= 0 || max_pages <= 0 ||
+        max_chunks < 1 || scratch == nullptr || cap < 0.f || requests > 65535 || nkv > 65535)
+        return WLLM_BAD_SIZE;
+    if (((uintptr_t)k_pages | (uintptr_t)v_pages) & 15) return WLLM_BAD_ALIGN;
+    const long long tiles = ((long long)max_q_len * (nq / nkv) + TL_ROWS - 1) / TL_ROWS;
+    if (tiles * max_chunks > 0x7fffffff) return WLLM_BAD_SIZE;
+    const dim3 grid((unsigned)(tiles * max_chunks), nkv, requests);
+    constexpr int VN = Vec<float>::N, most = (TL_ROWS * 256 + 32 * (256 + VN) + 32 * 256) * (int)sizeof(float);
+    const size_t smem = ((size_t)TL_ROWS * hd + 32 * (hd + VN) + 32 * vd) * sizeof(float);
+    const int blocks = (n_tokens * nq + WARPS - 1) / WARPS;
+#define GO(NE) do { \
+        static bool raised = false; \
+        if (!raised) { \
+            const cudaError_t e = cudaFuncSetAttribute(paged_attention_simt_chunk_kernel<float, NE>, cudaFuncAttributeMaxDynamicSharedMemorySize, most); \
+            if (e != cudaSuccess) return 1000 + (int)e; \
+            raised = true; \
+        } \
+        const int st = wllm_launch(paged_attention_simt_chunk_kernel<float, NE>, grid, TL_WARPS * 32, smem, stream, (const float*)q, q_stride, \
+                                   (const float*)k_pages, (const float*)v_pages, req_q_start, req_q_len, req_ctx_len, block_table, max_pages, nq, nkv, hd, \
+                                   page_size, scale, vd, cap, slopes, scratch, max_chunks); \
+        if (st != WLLM_OK) return st; \
+        return wllm_launch(paged_attention_simt_merge_kernel<float, NE>, blocks, WARPS * 32, 0, stream, (float*)out, out_stride, positions, n_tokens, nq, vd, 0, \
+                           (const float*)scratch, max_chunks, sinks, 0); \
+    } while (0)
+    if (vd <= 64) GO(2);
+    if (vd <= 128) GO(4);
+    GO(8);
+#undef GO
 }

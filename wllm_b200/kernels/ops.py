@@ -527,6 +527,42 @@ def paged_attention_simt(q: torch.Tensor, out: torch.Tensor, k_pages: torch.Tens
     return out
 
 
+SIMT_CHUNK_SCRATCH = 32 << 20      # floats
+
+
+def simt_by_chunks(tokens: int, max_ctx: int, nq: int, nkv: int, vd: int) -> int:
+    """Chunks for paged_attention_simt_chunks, or 0: the tiled kernel, whose tiles of 32 rows walk all their keys, a CTA an SM at a time.  A step of few tiles
+    ends with the longest of them, so its chunks are dealt out one by one as long as the tiles are less than two rounds and their results fit in 128 MB
+    (us, tiled and by chunks, 8 heads of 256 on one: 509 tokens 231 and 92; 100 67 and 45; 1,000, 250 tiles, 629 and 337; four prompts of 500 to 60, 234 tiles,
+    229 and 136; 16 tokens behind 4,000 1,705 and 57)."""
+    chunks, tiles = -(-max_ctx // SIMT_CHUNK), -(-tokens * (nq // nkv) // 32) * nkv
+    return chunks if chunks > 1 and tiles < 2 * sm_count() and tokens * nq * chunks * (vd + 2) <= SIMT_CHUNK_SCRATCH else 0
+
+
+def paged_attention_simt_chunks(q: torch.Tensor, out: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, positions: torch.Tensor,
+                                req_q_start: torch.Tensor, req_q_len: torch.Tensor, req_ctx_len: torch.Tensor, block_table: torch.Tensor, max_q_len: int,
+                                nq: int, nkv: int, hd: int, page_size: int, scale: float, scratch: torch.Tensor, max_chunks: int, vd: int | None = None,
+                                sinks: torch.Tensor | None = None, cap: float = 0.0, slopes: torch.Tensor | None = None) -> None:
+    """paged_attention_simt_tiled for float32 steps without a window, chunk by chunk (csrc/attention_simt.cu): the same bits.  `scratch` float32,
+    tokens * nq * max_chunks * (vd + 2); `max_chunks`: chunks of 64 keys of the longest context."""
+    _need_cuda(q, out, k_pages, v_pages, positions, req_q_start, req_q_len, req_ctx_len, block_table, scratch, sinks, slopes)
+    n, vd = q.shape[0], hd if vd is None else vd
+    assert q.dtype == k_pages.dtype == v_pages.dtype == out.dtype == scratch.dtype == torch.float32
+    assert q.shape == (n, nq * hd) and q.stride(1) == 1 and out.shape == (n, nq * vd) and out.stride(1) == 1 and positions.shape == (n,)
+    assert k_pages.is_contiguous() and v_pages.is_contiguous() and scratch.is_contiguous() and scratch.numel() >= n * nq * max_chunks * (vd + 2)
+    assert sinks is None or (sinks.dtype == torch.float32 and sinks.shape == (nq,) and sinks.is_contiguous())
+    assert slopes is None or (slopes.dtype == torch.float32 and slopes.shape == (nq,) and slopes.is_contiguous())
+    lib = load_family("attention_simt")
+    _check(lib.wllm_paged_attention_simt_chunks(_ptr(q), q.stride(0), _ptr(out), out.stride(0), _ptr(k_pages), _ptr(v_pages),
+                                                _ptr(_int32(positions, "positions")), _ptr(_int32(req_q_start, "req_q_start")),
+                                                _ptr(_int32(req_q_len, "req_q_len")), _ptr(_int32(req_ctx_len, "req_ctx_len")),
+                                                _ptr(_int32(block_table, "block_table")), block_table.shape[1], n, req_q_len.shape[0], max_q_len, nq, nkv, hd,
+                                                page_size, c_float(scale), vd, _ptr(sinks), c_float(cap), _ptr(slopes), _ptr(scratch), max_chunks, _stream()),
+           f"paged_attention_simt_chunks(head_dim={hd}, heads={nq}/{nkv})")
+    global launches
+    launches += 1                # the merge kernel
+
+
 def paged_attention_simt_tiled(q: torch.Tensor, out: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor,
                                req_q_start: torch.Tensor, req_q_len: torch.Tensor, req_ctx_len: torch.Tensor,
                                block_table: torch.Tensor, max_q_len: int, nq: int, nkv: int, hd: int, page_size: int,

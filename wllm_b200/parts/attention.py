@@ -285,8 +285,8 @@ class PagedAttention:
         window = -self.window if self.blocks else (self.window or 0)     # the kernels take a block size as a negative window
         ps, table = ctx.cache.page_size, ctx.group_tables[group]
         if q.dtype != torch.bfloat16 or not ops.mma_head_dim_ok(hd) or self.general:
-            # Three kernels with one result, bit for bit, so the choice is one of speed alone.  Portions of prompts:
-            # 32 rows of a request share every tile of keys.  Few rows over long contexts (decoding): a warp per
+            # Kernels with one result, bit for bit, so the choice is one of speed alone.  Portions of prompts:
+            # 32 rows of a request share every tile of keys (few tiles without a window: chunk of keys by chunk).  Few rows over long contexts (decoding): a warp per
             # (row, chunk of 64 keys).  Otherwise a warp per row.
             extra = {"vd": self.vd, "sinks": self.sinks} if (self.general or self.sinks is not None) else {}
             if self.slopes is not None:
@@ -294,6 +294,15 @@ class PagedAttention:
             if self.softcap > 0 or self.keep_first > 0:
                 extra.update(cap=self.softcap, keep=self.keep_first)
             if ctx.num_multi > 0 and hd <= 256 and self.vd <= 256:
+                by_chunks = 0
+                if q.is_cuda and q.dtype == torch.float32 and not window and self.keep_first == 0:
+                    by_chunks = ops.simt_by_chunks(q.shape[0], ctx.max_ctx, nq, nkv, self.vd)
+                if by_chunks:
+                    scratch = ctx.buffer(self.tag + "attention_chunks", (q.shape[0] * nq * by_chunks * (self.vd + 2),), torch.float32)
+                    extra.pop("keep", None)
+                    ops.paged_attention_simt_chunks(q, out, k_pages, v_pages, ctx.positions, ctx.req_q_start, ctx.req_q_len, ctx.req_ctx_len, table,
+                                                    ctx.max_q_len, nq, nkv, hd, ps, scale, scratch, by_chunks, **extra)
+                    return
                 ops.paged_attention_simt_tiled(q, out, k_pages, v_pages, ctx.req_q_start, ctx.req_q_len, ctx.req_ctx_len,
                                                table, ctx.max_q_len, nq, nkv, hd, ps, window, scale, **extra)
                 return
