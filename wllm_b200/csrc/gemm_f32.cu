@@ -103,18 +103,29 @@ gemm_f32_tile_kernel(const float* __restrict__ A, int lda, const float* __restri
             tile_fetch<BM, VEC>(A, lda, M, K, m0, (t + 1) * TBK, tid, ra);
             tile_fetch<TBN, VEC>(W, ldw, N, K, n0, (t + 1) * TBK, tid, rw);
         }
+        // a k's operands are read while the one before is multiplied, and every other row goes back over the columns: the operand it shares with the row
+        // before stays at the multiplier (512 x 28,416 x 2,048: 50.0 -> 52.6 TFLOP/s; either alone 49.9 and 50.8)
+        float4 fa[2][2], fb[2][2];
+        auto read = [&](int k) {
+            fa[k & 1][0] = *reinterpret_cast<const float4*>(&As[cur][k][ty * 4]);
+            if (TM == 8) fa[k & 1][1] = *reinterpret_cast<const float4*>(&As[cur][k][BM / 2 + ty * 4]);
+            fb[k & 1][0] = *reinterpret_cast<const float4*>(&Ws[cur][k][tx * 4]);
+            fb[k & 1][1] = *reinterpret_cast<const float4*>(&Ws[cur][k][TBN / 2 + tx * 4]);
+        };
+        read(0);
 #pragma unroll
         for (int k = 0; k < TBK; ++k) {
-            const float4 a0 = *reinterpret_cast<const float4*>(&As[cur][k][ty * 4]);
-            const float4 a1 = TM == 8 ? *reinterpret_cast<const float4*>(&As[cur][k][BM / 2 + ty * 4]) : a0;
-            const float4 b0 = *reinterpret_cast<const float4*>(&Ws[cur][k][tx * 4]);
-            const float4 b1 = *reinterpret_cast<const float4*>(&Ws[cur][k][TBN / 2 + tx * 4]);
+            if (k + 1 < TBK) read(k + 1);
+            const float4 a0 = fa[k & 1][0], a1 = TM == 8 ? fa[k & 1][1] : a0, b0 = fb[k & 1][0], b1 = fb[k & 1][1];
             const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
             const float b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
 #pragma unroll
             for (int i = 0; i < TM; ++i)
 #pragma unroll
-                for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+                for (int jj = 0; jj < 8; ++jj) {
+                    const int j = (i & 1) ? 7 - jj : jj;
+                    acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+                }
         }
         if (t + 1 < tiles) {
             tile_stash<BM>(As[cur ^ 1], tid, ra);
@@ -456,8 +467,8 @@ static int turn_of(int M, int N, int segs, long long floats) {
 struct TilePlan { int rows, turn; };
 
 // A round gives every SM one tile's segment of 1,024 k: 98 us with 128 rows, 60 with 64 (two CTAs an SM take as long as one behind the other).  Cut by segments
-// there are more of them to deal out, for the slabs' way through memory at some 5 TB/s and another launch.  us as measured, whole with 128 rows, whole 64, cut
-// 128, cut 64 (the model): 509 x 2,048 x 2,048 259, 224, 117 (103), 131 (125); 509 x 2,560 x 2,048 331, 245, 206 (203), 200 (187);
+// there are more of them to deal out, for the slabs' way through memory at some 5 TB/s and another launch.  us as measured (before a k's operands were read
+// ahead, which takes some 4 % off every form), whole with 128 rows, whole 64, cut 128, cut 64 (the model): 509 x 2,048 x 2,048 259, 224, 117 (103), 131 (125); 509 x 2,560 x 2,048 331, 245, 206 (203), 200 (187);
 // 509 x 2,048 x 16,384 2,063, 1,898, 704 (706), 907 (860); 509 x 32,768 x 2,048 1,387 (1,372), 1,759, 1,448 (1,447), 1,849; 256 x 32,768 x 2,048 792 (784), 999,
 // 729 (723), 939; 128 x 2,048 x 2,048 222, 149, 112 (102), 77 (64); 64 x 2,048 x 16,384 cut 64 145, 1,578 whole.
 static TilePlan tile_plan(int M, int N, int K, long long floats) {
