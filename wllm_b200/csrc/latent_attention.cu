@@ -11,6 +11,9 @@
 //   wllm_latent_prepare   one CTA a token: the cache row (norm in 32-bit from the projection's partial sums, the turn in
 //                         32-bit), the queries' plain parts rounded for the product with Uk, their turned parts placed
 //                         behind the columns that product will fill
+//   wllm_latent_expand    the other way round, for long prompts that nothing is cached of yet: with the latent rows' own products k = Uk c and v = Uv c (one
+//                         matrix product over the step's rows) attention is that of heads with keys and values of their own, a fourth of the arithmetic
+//                         where dim and the value's size are 128 and rank 512.  This lays those rows out in pages of 64 tokens for the attention kernels.
 //   wllm_head_linear_few  the same for bfloat16 steps of few tokens: a warp an output, the matrices read once.
 //   wllm_head_linear      y[n, h, :N] = x[n, h, :K] W_h^T for every head h: the two maps above.  Every output is one
 //                         ascending chain of fused multiply-adds over K in 32-bit, so a token's result does not depend on
@@ -31,7 +34,8 @@ latent_prepare_kernel(const TI* __restrict__ fused, int row_stride, int in_split
                       const int* __restrict__ positions, const int* __restrict__ slots, const float* __restrict__ inv_freq,
                       const void* __restrict__ gain, int gain_dtype, float eps, TO* __restrict__ pages, int page_size,
                       TO* __restrict__ q_plain, TO* __restrict__ q_mapped, int heads, int dim, int rot, int rot_dims,
-                      int interleaved, int rank, int hd, int q_rank, const void* __restrict__ q_gain, TO* __restrict__ cq_out) {
+                      int interleaved, int rank, int hd, int q_rank, const void* __restrict__ q_gain, TO* __restrict__ cq_out,
+                      TO* __restrict__ rows_out) {
     extern __shared__ float sm[];             // [rank] the latent columns, [half] sines, [half] cosines, [q_rank] the queries' latent columns
     __shared__ float scratch[32];
     pdl_launch_dependents();
@@ -97,12 +101,14 @@ latent_prepare_kernel(const TI* __restrict__ fused, int row_stride, int in_split
         for (int e = threadIdx.x; e < hd - rank; e += blockDim.x)
             dst[rank + e] = e < rot ? from_f32<TO>(turned([&](int i) { return in(qw + rank + i); }, e)) : from_f32<TO>(0.f);
     }
+    if (rows_out != nullptr)
+        for (int c = threadIdx.x; c < rank; c += blockDim.x) rows_out[(size_t)t * rank + c] = from_f32<TO>((sm[c] * inv) * value_at(gain, gain_dtype, c));
     if (q_plain != nullptr && q_rank == 0)    // null: the next product reads the plain parts from the fused row itself
         for (int item = threadIdx.x; item < heads * dim; item += blockDim.x) {
             const int h = item / dim, c = item % dim;
             q_plain[(size_t)t * heads * dim + item] = from_f32<TO>(in(h * (dim + rot) + c));
         }
-    const int tail = hd - rank;
+    const int tail = q_mapped ? hd - rank : 0;
     for (int item = threadIdx.x; item < heads * tail; item += blockDim.x) {
         const int h = item / tail, e = item % tail;
         const int base = h * (dim + rot) + dim;
@@ -112,12 +118,13 @@ latent_prepare_kernel(const TI* __restrict__ fused, int row_stride, int in_split
 }
 
 // fused [n, >= heads * (dim + rot) + rank + rot] (or `in_splits` 32-bit slabs), pages [page][1][slot][hd] with hd >= rank + rot,
-// q_plain [n, heads * dim] (or null), q_mapped [n, heads * hd] (columns rank .. hd of every head are written here), gain [rank].
+// q_plain [n, heads * dim] (or null), q_mapped [n, heads * hd] (columns rank .. hd of every head are written here; or null), gain [rank].
+// rows_out (null: not wanted): the latent rows of the step's tokens [n, rank] once more, one behind the other.
 WLLM_API int wllm_latent_prepare(const void* fused, int in_dtype, int row_stride, int in_splits, long long in_split_stride,
                                  const int* positions, const int* slots, const float* inv_freq, const void* gain, int gain_dtype,
                                  float eps, void* pages, int page_size, void* q_plain, void* q_mapped, int out_dtype, int n,
                                  int heads, int dim, int rot, int rot_dims, int interleaved, int rank, int hd, int q_rank,
-                                 const void* q_gain, void* cq_out, cudaStream_t stream) {
+                                 const void* q_gain, void* cq_out, void* rows_out, cudaStream_t stream) {
     if (n <= 0) return WLLM_OK;
     if (heads <= 0 || dim <= 0 || rot < 0 || rot_dims < 0 || rot_dims > rot || (rot_dims & 1) || rank <= 0 || hd < rank + rot ||
         page_size <= 0 || in_splits < 1)
@@ -128,12 +135,46 @@ WLLM_API int wllm_latent_prepare(const void* fused, int in_dtype, int row_stride
     if (smem > 48 * 1024) return WLLM_BAD_SIZE;
 #define GO(TI, TO) wllm_launch(latent_prepare_kernel<TI, TO>, n, 256, smem, stream, (const TI*)fused, row_stride, in_splits, \
         (size_t)in_split_stride, positions, slots, inv_freq, gain, gain_dtype, eps, (TO*)pages, page_size, (TO*)q_plain, \
-        (TO*)q_mapped, heads, dim, rot, rot_dims, interleaved, rank, hd, q_rank, q_gain, (TO*)cq_out)
+        (TO*)q_mapped, heads, dim, rot, rot_dims, interleaved, rank, hd, q_rank, q_gain, (TO*)cq_out, (TO*)rows_out)
     if (in_dtype == WLLM_BF16 && out_dtype == WLLM_BF16) return GO(bf16, bf16);
     if (in_dtype == WLLM_F32 && out_dtype == WLLM_BF16) return GO(float, bf16);
     if (in_dtype == WLLM_F32 && out_dtype == WLLM_F32) return GO(float, float);
 #undef GO
     return WLLM_BAD_DTYPE;
+}
+
+// ---------------------------------------------------------------------------------------------------
+// Keys and values of a step's tokens, kv [n, heads * dim | heads * dim], into pages [page][head][64][dim] of a buffer of their own: request r's begin at page
+// q_start / 64 + r (so that no two share one, whatever the lengths), and row r of `table` [requests, max_pages] names them, zeros behind.
+// grid (tokens), 256 threads: a copy of 4 heads dim bytes each way.
+// ---------------------------------------------------------------------------------------------------
+constexpr int LE_PAGE = 64;
+
+__global__ void __launch_bounds__(256)
+latent_expand_kernel(const bf16* __restrict__ kv, const int* __restrict__ token_req, const int* __restrict__ req_q_start, const int* __restrict__ req_q_len,
+                     bf16* __restrict__ keys, bf16* __restrict__ values, int* __restrict__ table, int max_pages, int heads, int dim) {
+    pdl_begin();
+    const int t = blockIdx.x, r = token_req[t], start = req_q_start[r], local = t - start, base = start / LE_PAGE + r;
+    const int per = dim / 8, each = heads * per;
+    const size_t to = ((size_t)(base + local / LE_PAGE) * heads * LE_PAGE + local % LE_PAGE) * dim;
+    const uint4* src = reinterpret_cast<const uint4*>(kv + (size_t)t * 2 * heads * dim);
+    for (int i = threadIdx.x; i < 2 * each; i += blockDim.x) {
+        const int at = i < each ? i : i - each, h = at / per, c = at % per;
+        reinterpret_cast<uint4*>((i < each ? keys : values) + to + (size_t)h * LE_PAGE * dim)[c] = src[i];
+    }
+    if (local == 0) {
+        const int pages = (req_q_len[r] + LE_PAGE - 1) / LE_PAGE;
+        for (int i = threadIdx.x; i < max_pages; i += blockDim.x) table[(size_t)r * max_pages + i] = i < pages ? base + i : 0;
+    }
+}
+
+WLLM_API int wllm_latent_expand(const void* kv, const int* token_req, const int* req_q_start, const int* req_q_len, void* keys, void* values, int* table,
+                                int max_pages, int n, int heads, int dim, cudaStream_t stream) {
+    if (n <= 0) return WLLM_OK;
+    if (heads <= 0 || dim <= 0 || dim % 8 != 0 || max_pages <= 0) return WLLM_BAD_SIZE;
+    if (((uintptr_t)kv | (uintptr_t)keys | (uintptr_t)values) & 15) return WLLM_BAD_ALIGN;
+    return wllm_launch(latent_expand_kernel, n, 256, 0, stream, (const bf16*)kv, token_req, req_q_start, req_q_len, (bf16*)keys, (bf16*)values, table, max_pages,
+                       heads, dim);
 }
 
 // ---------------------------------------------------------------------------------------------------

@@ -356,13 +356,14 @@ def rope_head_norm_kv_write(qkv: torch.Tensor, q_out: torch.Tensor, positions: t
 def latent_prepare(fused: torch.Tensor, parts: int, positions: torch.Tensor, slots, inv_freq: torch.Tensor, gain: torch.Tensor,
                    eps: float, pages: torch.Tensor, page_size: int, q_plain: torch.Tensor, q_mapped: torch.Tensor, heads: int,
                    dim: int, rot: int, rot_dims: int, rank: int, hd: int, pairing: str = "half", q_rank: int = 0,
-                   q_gain: torch.Tensor | None = None, cq_out: torch.Tensor | None = None) -> None:
+                   q_gain: torch.Tensor | None = None, cq_out: torch.Tensor | None = None, rows_out: torch.Tensor | None = None) -> None:
     """From the fused projection row [heads * (dim + rot) | rank + rot] of every token (csrc/latent_attention.cu): the
     cache row [rms(latent columns) * gain | the rot columns behind them, turned | zeros] into `pages` at `slots`; the
     queries' plain parts into `q_plain` [n, heads * dim] (None: they are read where they are); their turned parts into
     columns rank .. of every head of `q_mapped` [n, heads * hd].  Norm and turn are 32-bit, from the projection's partial sums where it left them.
     With `q_rank` > 0 the row is [q_rank | rank] instead (queries that pass a latent row of their own; nothing turns): those
-    columns, normed with `q_gain` [q_rank], go to `cq_out` [n, q_rank] for the product that makes the queries."""
+    columns, normed with `q_gain` [q_rank], go to `cq_out` [n, q_rank] for the product that makes the queries.
+    `rows_out` [n, rank]: the latent rows once more, one behind the other; `q_mapped` may then be None (nothing is laid out for mapped queries)."""
     if pairing not in ("half", "interleaved"):
         raise KernelError(f"rotary pairing {pairing!r} not supported (half, interleaved)")
     _need_cuda(fused, positions, slots, inv_freq, gain, pages, q_plain, q_mapped)
@@ -371,19 +372,40 @@ def latent_prepare(fused: torch.Tensor, parts: int, positions: torch.Tensor, slo
     _need_cuda(q_gain, cq_out)
     if q_rank:
         assert rot == 0 and q_gain.shape == (q_rank,) and q_gain.is_contiguous() and q_gain.dtype == gain.dtype
-        assert cq_out.shape == (n, q_rank) and cq_out.is_contiguous() and cq_out.dtype == q_mapped.dtype
-    assert q_mapped.shape == (n, heads * hd) and q_mapped.is_contiguous()
-    assert q_plain is None or (q_plain.shape == (n, heads * dim) and q_plain.is_contiguous() and q_plain.dtype == q_mapped.dtype)
-    assert q_mapped.dtype == pages.dtype and pages.is_contiguous() and pages.shape[-1] == hd and pages.shape[-3] == 1
+        assert cq_out.shape == (n, q_rank) and cq_out.is_contiguous() and cq_out.dtype == pages.dtype
+    assert q_mapped is not None or rows_out is not None
+    _need_cuda(rows_out)
+    for t, width in ((q_mapped, heads * hd), (rows_out, rank), (q_plain, heads * dim)):
+        assert t is None or (t.shape == (n, width) and t.is_contiguous() and t.dtype == pages.dtype)
+    assert pages.is_contiguous() and pages.shape[-1] == hd and pages.shape[-3] == 1
     assert gain.shape == (rank,) and gain.is_contiguous()
     assert inv_freq.dtype == torch.float32 and inv_freq.numel() == rot_dims // 2 and inv_freq.is_contiguous()
     lib = load_family("latent_attention")
     _check(lib.wllm_latent_prepare(ptr, dt, row_stride, nparts, part_stride, _ptr(_int32(positions, "positions")),
                                    _ptr(_int32(slots, "slots") if slots is not None else None), _ptr(inv_freq), _ptr(gain),
-                                   _dt(gain), c_float(eps), _ptr(pages), page_size, _ptr(q_plain), _ptr(q_mapped), _dt(q_mapped),
+                                   _dt(gain), c_float(eps), _ptr(pages), page_size, _ptr(q_plain), _ptr(q_mapped), _dt(pages),
                                    n, heads, dim, rot, rot_dims, 1 if pairing == "interleaved" else 0, rank, hd, q_rank,
-                                   _ptr(q_gain if q_rank else None), _ptr(cq_out if q_rank else None), _stream()),
+                                   _ptr(q_gain if q_rank else None), _ptr(cq_out if q_rank else None), _ptr(rows_out), _stream()),
            "latent_prepare")
+
+
+LATENT_PAGE = 64               # tokens of a page that latent_expand lays out
+
+
+def latent_expand(kv: torch.Tensor, token_req: torch.Tensor, req_q_start: torch.Tensor, req_q_len: torch.Tensor, keys: torch.Tensor, values: torch.Tensor,
+                  table: torch.Tensor, heads: int, dim: int) -> None:
+    """The step's keys and values `kv` [n, 2 * heads * dim] (bfloat16; all heads' keys, then their values) into pages `keys`, `values`
+    [n // 64 + requests, heads, 64, dim] with a block table [requests, pages of the longest] of their own (csrc/latent_attention.cu)."""
+    _need_cuda(kv, token_req, req_q_start, req_q_len, keys, values, table)
+    n, R = kv.shape[0], req_q_len.shape[0]
+    assert kv.dtype == torch.bfloat16 and kv.is_contiguous() and kv.shape[1] == 2 * heads * dim and token_req.shape == (n,) and req_q_start.shape == (R,)
+    for t in (keys, values):
+        assert t.dtype == kv.dtype and t.is_contiguous() and t.shape == (n // LATENT_PAGE + R, heads, LATENT_PAGE, dim)
+    assert table.dim() == 2 and table.shape[0] == R
+    lib = load_family("latent_attention")
+    _check(lib.wllm_latent_expand(_ptr(kv), _ptr(_int32(token_req, "token_req")), _ptr(_int32(req_q_start, "req_q_start")),
+                                  _ptr(_int32(req_q_len, "req_q_len")), _ptr(keys), _ptr(values), _ptr(_int32(table, "table")), table.shape[1], n, heads, dim,
+                                  _stream()), "latent_expand")
 
 
 HEAD_LINEAR_BATCHED_ROWS = 32     # bfloat16 steps of this many tokens or more: the heads' maps are one batched matrix product

@@ -22,7 +22,9 @@ kv_rank + rot_dim elements, values the rows' first kv_rank elements (the cache g
 One fused product makes q and the down projection; `ops.latent_prepare` norms, turns and writes the cache row and lays
 the queries out; `ops.head_linear` applies up_k^T head by head, the paged attention kernels run with their window,
 `ops.head_linear` applies up_v, and the output projection follows.  Whole prompts, portions and decoded tokens are one
-case.
+case.  bfloat16 steps of whole prompts alone, without a turning part, make every head's keys and values instead (up_k c and up_v c, one product over the
+step's latent rows) and run the attention of heads with keys and values of their own: fewer operations than over rows of kv_rank elements.  The cache
+holds the same rows.
 """
 from __future__ import annotations
 
@@ -63,7 +65,7 @@ class LatentAttention:
         self.gate_col = self.q_width + self.rank + self.rot
         self.width = self.gate_col + (self.heads * self.vd if self.gate_name is not None else 0)    # columns of the fused product
         self.tag = ""
-        self.w_in = self.w_uk_t = self.w_uv = self.wo = self.gain = self.q_gain = self.w_uq = None
+        self.w_in = self.w_uk_t = self.w_uv = self.w_ukv = self.wo = self.gain = self.q_gain = self.w_uq = None
 
     def cache_need(self):
         return KVNeed(1, self.row, self.window, self.rank, 0, values_in_keys=True)
@@ -92,8 +94,11 @@ class LatentAttention:
             self.q_gain = fetch(self.qlat["norm"]).to(self.gain.dtype).contiguous()
             self.w_uq = fetch(self.qlat["up"]).contiguous()
         # up_k head by head, transposed: [heads, kv_rank, plain_dim], so that the queries' map is x W^T like every product
-        self.w_uk_t = fetch(n["up_k"]).view(self.heads, self.dim, self.rank).transpose(1, 2).contiguous()
-        self.w_uv = fetch(n["up_v"]).view(self.heads, self.vd, self.rank).contiguous()
+        up_k, up_v = fetch(n["up_k"]), fetch(n["up_v"])
+        self.w_uk_t = up_k.view(self.heads, self.dim, self.rank).transpose(1, 2).contiguous()
+        self.w_uv = up_v.view(self.heads, self.vd, self.rank).contiguous()
+        if self.model_dtype == torch.bfloat16 and self._expandable():
+            self.w_ukv = torch.cat([up_k, up_v], dim=0).contiguous()
         self.wo = fetch(n["o_proj"]).contiguous()
         self.position.to(self.wo.device)
 
@@ -108,30 +113,65 @@ class LatentAttention:
         if not cache.writes:
             raise ValueError("a latent attention mixer writes its own cache")
         n, H, R, row = fused.shape[-2], self.heads, self.rank, self.row
+        expand = self._expands(ctx)
         cols = fused if fused.shape[-1] == self.width else fused[..., col0:col0 + self.width]
         group = ctx.cache.groups[cache.group]
         pages = group.keys(cache.layer)
         # a product that left one tensor in the model's type holds the queries' plain parts as the next product reads them
         in_place = parts == 0 and cols.dtype == self.model_dtype
+        if expand and in_place and not self.q_rank and (cols.data_ptr() % 16 or cols.stride(0) % 8):
+            in_place = False              # the attention kernels read query rows in steps of 16 bytes
         q_plain = None if in_place or self.q_rank else ctx.buffer(self.tag + "latent_q_plain", (n, H * self.dim), self.model_dtype)
-        q_mapped = ctx.buffer(self.tag + "latent_q", (n, H * row), self.model_dtype)
+        q_mapped = None if expand else ctx.buffer(self.tag + "latent_q", (n, H * row), self.model_dtype)
+        rows = ctx.buffer(self.tag + "latent_rows", (n, R), self.model_dtype) if expand else None
         cq = ctx.buffer(self.tag + "latent_cq", (n, self.q_rank), self.model_dtype) if self.q_rank else None
         ops.latent_prepare(cols, parts, ctx.positions, ctx.group_slots[cache.group], self.position.inv_freq, self.gain, self.eps,
                            pages, group.page_size, q_plain, q_mapped, H, self.dim, self.rot, self.position.rotary_dim, R, row,
-                           pairing=getattr(self.position, "pairing", "half"), q_rank=self.q_rank, q_gain=self.q_gain, cq_out=cq)
+                           pairing=getattr(self.position, "pairing", "half"), q_rank=self.q_rank, q_gain=self.q_gain, cq_out=cq, rows_out=rows)
         if self.q_rank:
             # the queries from their normed latent row: one more product, then head by head as below
             plain = ops.linear(cq, self.w_uq, ctx.buffer(self.tag + "latent_q_up", (n, H * self.dim), self.model_dtype)).view(n, H, self.dim)
         else:
             plain = cols[:, :self.q_width].unflatten(1, (H, self.dim + self.rot))[:, :, :self.dim] if in_place else q_plain.view(n, H, self.dim)
-        ops.head_linear(plain, self.w_uk_t, q_mapped.view(n, H, row)[:, :, :R])
-        mixed = ctx.buffer(self.tag + "latent_mixed", (n, H * R), self.model_dtype)
-        self.attend(q_mapped, mixed, pages, ctx, cache.group)
         heads_out = ctx.buffer(self.tag + "attn", (n, H * self.vd), self.model_dtype)
-        ops.head_linear(mixed.view(n, H, R), self.w_uv, heads_out.view(n, H, self.vd))
+        if expand:
+            self.attend_expanded(plain.flatten(1) if plain.is_contiguous() else cols[:, :H * self.dim], rows, heads_out, ctx)
+        else:
+            ops.head_linear(plain, self.w_uk_t, q_mapped.view(n, H, row)[:, :, :R])
+            mixed = ctx.buffer(self.tag + "latent_mixed", (n, H * R), self.model_dtype)
+            self.attend(q_mapped, mixed, pages, ctx, cache.group)
+            ops.head_linear(mixed.view(n, H, R), self.w_uv, heads_out.view(n, H, self.vd))
         if self.gate_name is not None:
             ops.sigmoid_gate(heads_out, cols, parts, self.gate_col)
         return as_branch(ops.project(heads_out, self.wo, lambda name, shape, dt: ctx.buffer(self.tag + "branch_" + name, shape, dt)))
+
+    # Tokens of a step of whole prompts from where on keys and values of their own are made.  Steps of a model of four layers with one such mixer (16 heads of
+    # 128, rank 512; us, that way and over the latent rows): 64 tokens 662 and 690, 3 x 33 674 and 751, 128 619 and 692, 512 907 and 945, 1,021 1,006 and
+    # 1,092, 3 x 1,021 1,557 and 1,697, 2 x 2,048 2,316 and 2,739; 4 tokens 660 and 655 to 709, 16 requests of 16 1,171 and 1,175.  The attention costs a fourth
+    # of the operations then, the product that makes keys and values as much as the two maps that fall away.
+    EXPAND_FROM = 64
+
+    def _expandable(self) -> bool:
+        """Heads that the tensor-memory attention takes with keys and values of their own, and a product that the tensor-memory kernel takes."""
+        return self.rot == 0 and self.dim == self.vd and self.dim % 64 == 0 and self.dim <= 256 and self.rank % 8 == 0
+
+    def _expands(self, ctx) -> bool:
+        """Whether this step's attention runs over keys and values made from the step's latent rows: whole prompts alone, nothing cached before them."""
+        if self.w_ukv is None or ctx.num_single or ctx.n_tokens < self.EXPAND_FROM or ctx.host is None:
+            return False
+        if "whole_prompts" not in ctx.memo:
+            ctx.memo["whole_prompts"] = bool((ctx.host["req_q_len"] == ctx.host["req_ctx_len"]).all())
+        return ctx.memo["whole_prompts"]
+
+    def attend_expanded(self, q, rows, out, ctx) -> None:
+        n, H, dim, R = rows.shape[0], self.heads, self.dim, ctx.n_requests
+        kv = ops.linear(rows, self.w_ukv, ctx.buffer(self.tag + "latent_kv", (n, 2 * H * dim), self.model_dtype))
+        shape = (n // ops.LATENT_PAGE + R, H, ops.LATENT_PAGE, dim)
+        keys, values = (ctx.buffer(self.tag + "latent_" + name, shape, self.model_dtype) for name in ("keys", "values"))
+        table = ctx.buffer(self.tag + "latent_table", (R, -(-ctx.max_q_len // ops.LATENT_PAGE)), torch.int32)
+        ops.latent_expand(kv, ctx.token_req, ctx.req_q_start, ctx.req_q_len, keys, values, table, H, dim)
+        ops.attention_mma_prefill(q, out, keys, values, ctx.req_q_start, ctx.req_q_len, ctx.req_ctx_len, table, ctx.max_q_len, H, H, dim, ops.LATENT_PAGE,
+                                  self.window or 0, self.scale, skip_single=False)
 
     def attend(self, q, out, pages, ctx, group: int) -> None:
         """Every token of the step over its request's cached rows: one key/value head for all query heads, the values
