@@ -8,12 +8,12 @@
 // A row of C therefore depends on its own row of A only, bit for bit, which makes the 32-bit path of the
 // engine independent of batching.  (Zero padding past K adds fma(0, 0, acc) = acc.)
 //
-// Three kernels with that same arithmetic:
+// Two kernels with that same arithmetic:
 //   tile kernel    steps of more than 32 rows, bound by the FMA pipes: BM x 128 x 16 tiles (BM = 64 or 128), 256
 //                  threads with 4 x 8 or 8 x 8 outputs each, operands transposed in shared memory and read
 //                  as float4, the next tile fetched into registers while the current one is multiplied.  A tile's CTA walks its segments (the
 //                  sums of finished ones wait in shared memory), or every segment has a CTA of its own and a second kernel adds the sums: see tile_plan.
-//   wide kernel    very many tiles (K and the pitches in steps of 4 floats, 16-byte aligned operands), where it is faster: see gemm_f32_wide_kernel.
+//                  (Neighbouring columns two an instruction, fma.rn.f32x2, and 8 x 16 outputs a thread: 4,096 x 32,768 x 2,048 10,860 us for 10,412.)
 //   skinny kernel  steps of at most 32 rows, bound by streaming W once: a warp owns 32 rows of W and one
 //                  segment (so a matrix of few rows and long K still gives every SM many warps), streams it
 //                  through its own ring of cp.async stages and keeps one chain per row of A in each lane;
@@ -271,117 +271,6 @@ gemm_f32_skinny_kernel(const float* __restrict__ A, int lda, const float* __rest
     }
 }
 
-// ------------------------------------------------------------------------------------------------
-// wide kernel: 128 x 128 tiles, 128 threads with 8 x 16 outputs each, two CTAs an SM.
-//
-// The tile kernel's scheme with two changes.  Neighbouring columns are multiplied two an instruction (fma.rn.f32x2: each half is the fused
-// multiply-add of its own chain, so the bits are the same), so that half the instructions compete for the schedulers, and a thread has twice the columns, 24
-// floats read from shared memory for 128 products instead of 16 for 64.  A tile keeps the running total of its segments in C.  From some fourteen tiles an SM on
-// it is the faster one: 4,096 x 32,768 x 2,048 11,347 -> 11,084 us (49.6 TFLOP/s).  Cut by segments it loses to the tile kernel cut that way: 509 x 2,048 x 16,384
-// 759 and 704 us.  (Rows left as they lie in memory, brought by cp.async and read four k at a time, cannot be paired: 39 TFLOP/s; A that way and W transposed: 51.)
-// ------------------------------------------------------------------------------------------------
-constexpr int WT = 128, WTHREADS = 128;
-
-// grid (row tiles, column tiles)
-__global__ void __launch_bounds__(WTHREADS, 2)
-gemm_f32_wide_kernel(const float* __restrict__ A, int lda, const float* __restrict__ W, int ldw, float* __restrict__ out, int ld_out, int M, int N, int K) {
-    __shared__ __align__(16) float As[2][TBK][WT + 4];
-    __shared__ __align__(16) float Ws[2][TBK][WT + 4];
-    constexpr int CHUNKS = WT * TBK / 4 / WTHREADS;         // groups of four k a thread and operand: rows crow + 32 i, k ck .. ck + 3
-    pdl_launch_dependents();
-    const int tid = threadIdx.x, m0 = blockIdx.x * WT, n0 = blockIdx.y * WT;       // neighbours in the grid share a tile of W
-    const int tiles = (K + TBK - 1) / TBK;
-    const int crow = tid >> 2, ck = (tid & 3) * 4;
-    auto fetch = [&](const float* __restrict__ src, int ld, int rows, int r0, int t, float4 (&reg)[CHUNKS]) {
-        const int gk = t * TBK + ck;
-#pragma unroll
-        for (int i = 0; i < CHUNKS; ++i) {
-            const int row = r0 + crow + 32 * i;
-            reg[i] = row < rows && gk < K ? *reinterpret_cast<const float4*>(src + (size_t)row * ld + gk) : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-    };
-    auto stash = [&](float (*to)[WT + 4], const float4 (&reg)[CHUNKS]) {
-#pragma unroll
-        for (int i = 0; i < CHUNKS; ++i) {
-            const int row = crow + 32 * i;
-            to[ck][row] = reg[i].x; to[ck + 1][row] = reg[i].y; to[ck + 2][row] = reg[i].z; to[ck + 3][row] = reg[i].w;
-        }
-    };
-    const int tx = tid & 7, ty = tid >> 3;      // outputs: rows 4 ty .. and 64 + 4 ty .., columns 4 tx .. + 32 h (h < 4), four each
-    float2 acc[8][8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = make_float2(0.f, 0.f);
-    // what the accumulators hold joins the running total (add) or becomes it
-    const bool vec_out = (ld_out & 3) == 0 && ((uintptr_t)out & 15) == 0;
-    auto leave = [&](bool add) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int gm = m0 + (i < 4 ? 4 * ty + i : WT / 2 + 4 * ty + i - 4);
-            if (gm >= M) continue;
-#pragma unroll
-            for (int h = 0; h < 4; ++h) {
-                const int gn = n0 + 32 * h + 4 * tx;
-                float* to = out + (size_t)gm * ld_out + gn;
-                float4 v = make_float4(acc[i][2 * h].x, acc[i][2 * h].y, acc[i][2 * h + 1].x, acc[i][2 * h + 1].y);
-                if (vec_out && gn + 3 < N) {
-                    if (add) {
-                        const float4 b = *reinterpret_cast<const float4*>(to);
-                        v = make_float4(b.x + v.x, b.y + v.y, b.z + v.z, b.w + v.w);
-                    }
-                    *reinterpret_cast<float4*>(to) = v;
-                } else {
-                    if (gn < N) to[0] = add ? to[0] + v.x : v.x;
-                    if (gn + 1 < N) to[1] = add ? to[1] + v.y : v.y;
-                    if (gn + 2 < N) to[2] = add ? to[2] + v.z : v.z;
-                    if (gn + 3 < N) to[3] = add ? to[3] + v.w : v.w;
-                }
-            }
-        }
-    };
-    float4 ra[CHUNKS], rw[CHUNKS];
-    fetch(W, ldw, N, n0, 0, rw);                // the weights are no kernel's output
-    pdl_wait();
-    fetch(A, lda, M, m0, 0, ra);
-    stash(As[0], ra);
-    stash(Ws[0], rw);
-    __syncthreads();
-    for (int t = 0; t < tiles; ++t) {
-        const int cur = t & 1;
-        if (t + 1 < tiles) {
-            fetch(A, lda, M, m0, t + 1, ra);
-            fetch(W, ldw, N, n0, t + 1, rw);
-        }
-#pragma unroll
-        for (int k = 0; k < TBK; ++k) {
-            float a[8];
-            float2 b[8];
-            *reinterpret_cast<float4*>(a) = *reinterpret_cast<const float4*>(&As[cur][k][4 * ty]);
-            *reinterpret_cast<float4*>(a + 4) = *reinterpret_cast<const float4*>(&As[cur][k][WT / 2 + 4 * ty]);
-#pragma unroll
-            for (int h = 0; h < 4; ++h) *reinterpret_cast<float4*>(&b[2 * h]) = *reinterpret_cast<const float4*>(&Ws[cur][k][32 * h + 4 * tx]);
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-#pragma unroll
-                for (int j = 0; j < 8; ++j) acc[i][j] = fma2(make_float2(a[i], a[i]), b[j], acc[i][j]);
-        }
-        if (t + 1 < tiles) {
-            stash(As[cur ^ 1], ra);
-            stash(Ws[cur ^ 1], rw);
-            if (((t + 1) & (SEG / TBK - 1)) == 0) {        // a segment ends here and another follows
-                leave(t + 1 > SEG / TBK);
-#pragma unroll
-                for (int i = 0; i < 8; ++i)
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) acc[i][j] = make_float2(0.f, 0.f);
-            }
-        }
-        __syncthreads();
-    }
-    leave(tiles > SEG / TBK);
-}
-
 // C[m][n] = the segments' sums added in ascending order, behind (add) those that it holds.
 __global__ void __launch_bounds__(256)
 gemm_f32_fold_kernel(const float* __restrict__ parts, float* __restrict__ C, int ldc, int M, int N, int segs, bool add) {
@@ -462,7 +351,7 @@ static int turn_of(int M, int N, int segs, long long floats) {
     return (int)(room < segs ? (room < 65535 ? room : 65535) : (segs < 65535 ? segs : 65535));
 }
 
-// How a product of more than 32 rows runs: tiles of `rows` (64, 128; 0: the wide kernel) rows, segments with CTAs of their own `turn` at a time (1: a tile's CTA
+// How a product of more than 32 rows runs: tiles of `rows` (64 or 128) rows, segments with CTAs of their own `turn` at a time (1: a tile's CTA
 // walks them all).
 struct TilePlan { int rows, turn; };
 
@@ -487,7 +376,6 @@ static TilePlan tile_plan(int M, int N, int K, long long floats) {
         const double cut = round * rounds + 4.0 * M * N * (2 * segs + 1) / 5e6 + 3.0 * ((segs + turn - 1) / turn);
         if (cut < least) { least = cut; best = {rows, turn}; }
     }
-    if (best.rows == 128 && best.turn == 1 && (M + 127) / 128 * cols >= 14ll * sms) best.rows = 0;
     return best;
 }
 
@@ -532,8 +420,6 @@ WLLM_API int wllm_gemm_f32(const float* A, int lda, const float* W, int ldw, flo
     }
     // without room for two slabs a tile's CTA walks its segments: the same bits
     const TilePlan plan = tile_plan(M, N, K, scratch == nullptr ? 0 : scratch_floats);
-    if (plan.rows == 0)
-        return wllm_launch(gemm_f32_wide_kernel, dim3((M + WT - 1) / WT, (N + WT - 1) / WT), WTHREADS, 0, stream, A, lda, W, ldw, C, ldc, M, N, K);
     if (plan.turn > 1)
         return plan.rows == 64 ? launch_cut<64>(A, lda, W, ldw, C, ldc, M, N, K, scratch, plan.turn, stream)
                                : launch_cut<128>(A, lda, W, ldw, C, ldc, M, N, K, scratch, plan.turn, stream);
