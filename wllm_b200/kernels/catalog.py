@@ -15,6 +15,7 @@ FAMILIES = {
     "activation": [{}],
     "linear_attention": [{}],
     "linear_attention_chunks": [{}],
+    "delta_rule_chunks": [{}],
     "delta_rule": [{}],
     "state_space": [{}],
     "rg_lru": [{}],

@@ -1145,6 +1145,7 @@ def linattn_decay(low: torch.Tensor, parts: int, low_off: int, w2: torch.Tensor,
     return decay
 
 
+CHUNK_SCRATCH = 256 << 20       # bytes that a step's chunks may take: a chunk of each of very many requests takes more, and such steps are walked
 LINATTN_CHUNKS_FROM = 128      # portions of at least this many tokens
 
 
@@ -1369,6 +1370,38 @@ def delta_scan(q, k, v, beta, decay, state, out, req_q_start, req_q_len, req_slo
         return out
     _check(lib.wllm_delta_scan(_ptr(q), _ptr(k), _ptr(v), _ptr(beta), _ptr(decay), 1 if channel else 0, _ptr(state), _ptr(out),
                                *index, R, heads, kv_heads, dim, vdim, 2 ** 31 - 1, 1 if single else 0, _stream()), name)
+    return out
+
+
+DELTA_CHUNK_MIN = 16        # the shortest requests that delta_chunks takes in chunks
+
+
+def delta_chunks_bytes(lens, heads: int) -> int:
+    """Bytes of scratch that delta_chunks asks for; `lens`: the requests' tokens (int32 array on the host)."""
+    lib = load_family("delta_rule_chunks")
+    lib.wllm_delta_chunks_bytes.restype = ctypes.c_longlong
+    return int(lib.wllm_delta_chunks_bytes(c_void_p(lens.ctypes.data), len(lens), heads))
+
+
+def delta_chunks(q, k, v, beta, decay, state, out, req_q_start, req_q_len, req_slot, lens, heads: int, kv_heads: int, channel: bool, scratch: torch.Tensor):
+    """delta_scan for heads of 128 by 128, the requests of DELTA_CHUNK_MIN tokens and more in chunks of 64 tokens on the tensor cores
+    (csrc/delta_rule_chunks.cu), their sums in another order; shorter ones token by token.  `lens`: req_q_len on the host (int32); `scratch` (uint8):
+    delta_chunks_bytes, or less that holds a chunk of every request."""
+    _need_cuda(q, k, v, beta, decay, state, out, req_q_start, req_q_len, req_slot, scratch)
+    n, R, D = q.shape[0], req_q_len.shape[0], 128
+    assert all(t.dtype == torch.float32 and t.is_contiguous() for t in (q, k, v, beta, decay, state, out))
+    assert q.shape == k.shape == (n, kv_heads * D) and v.shape == out.shape == (n, heads * D) and beta.shape == (n, heads)
+    assert decay.shape == (n, heads * D if channel else heads) and state.shape[1:] == (heads, D, D)
+    assert lens.dtype.name == "int32" and len(lens) == R and lens.flags["C_CONTIGUOUS"] and scratch.dtype == torch.uint8 and scratch.is_contiguous()
+    index = (_ptr(_int32(req_q_start, "req_q_start")), _ptr(_int32(req_q_len, "req_q_len")), _ptr(_int32(req_slot, "req_slot")))
+    rows = (_ptr(q), _ptr(k), _ptr(v), _ptr(beta), _ptr(decay), 1 if channel else 0, _ptr(state), _ptr(out))
+    name, launched = f"delta_chunks(heads={heads}/{kv_heads})", ctypes.c_int(0)
+    if ((lens > 0) & (lens < DELTA_CHUNK_MIN)).any():
+        _check(load_family("delta_rule").wllm_delta_scan(*rows, *index, R, heads, kv_heads, D, D, DELTA_CHUNK_MIN, 0, _stream()), name)
+    _check(load_family("delta_rule_chunks").wllm_delta_chunks(*rows, *index, c_void_p(lens.ctypes.data), R, heads, kv_heads, _ptr(scratch),
+                                                              ctypes.c_longlong(scratch.numel()), ctypes.byref(launched), _stream()), name)
+    global launches
+    launches += launched.value - 1
     return out
 
 

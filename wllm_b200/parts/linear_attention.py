@@ -39,7 +39,8 @@ spec options: num_heads, num_kv_heads, key_dim, value_dim, conv_taps, eps, unit_
 o_proj, q_conv/k_conv/v_conv [channels, taps], beta_proj, decay_proj [heads, hidden], decay_log, decay_bias [heads],
 head_norm_weight [value_dim] (checkpoint names).  One product makes q | k | v | g | beta | decay; what enters the
 recurrence is 32-bit (csrc/delta_rule.cu).  A 32-bit model's recurrence walks token by token and gives the same bits however a prompt
-is cut; a bfloat16 model's long portions are walked in blocks of eight tokens, whose sums run in another order.
+is cut; a bfloat16 model's long portions are walked in blocks of eight tokens or go in chunks of 64 on the tensor cores (csrc/delta_rule_chunks.cu), whose
+sums run in another order.
 """
 from __future__ import annotations
 
@@ -138,14 +139,16 @@ class LinearAttention:
         turn = dict(q_scale=self.q_scale, k_scale=self.k_scale, inv_freq=self.position.inv_freq if rot else None, rot_dim=rot)
         o = ctx.buffer(self.tag + "la_o", (n, H * V), f32)
         state = ctx.state(cache.state_names["state"])
+        room = 0
         if ctx.max_q_len >= ops.LINATTN_CHUNKS_FROM and ops.linattn_chunks_ok(fused, parts, offsets, D, V, rot, getattr(self.position, "pairing", "half")):
+            room = ops.linattn_chunks_bytes(ctx.host["req_q_len"], H, D, V)
+        if 0 < room <= ops.CHUNK_SCRATCH:
             # long portions of bfloat16 models: chunks on the tensor cores, from the product's rows as they are
             if low:
                 ops.linattn_decay(fused, parts, col0 + self.off_low, self.w_up, self.b_up, H, D, decay, tau=self.tau)
-            lens = ctx.host["req_q_len"]
-            scratch = ctx.buffer(self.tag + "la_chunks", (ops.linattn_chunks_bytes(lens, H, D, V),), torch.uint8)
+            scratch = ctx.buffer(self.tag + "la_chunks", (room,), torch.uint8)
             ops.linattn_chunks(fused, *offsets, H, D, V, ctx.positions, decay, self.head_decay, state, o, ctx.req_q_start, ctx.req_q_len,
-                               ctx.req_slot, lens, scratch, **turn)
+                               ctx.req_slot, ctx.host["req_q_len"], scratch, **turn)
         else:
             self._walk(fused, parts, offsets, turn, decay, state, o, ctx, col0)
         gated = ctx.buffer(self.tag + "la_gated", (n, H * V), self.model_dtype)
@@ -252,6 +255,11 @@ class DeltaRule:
     # The shortest request that takes part: many short ones fill the device either way (64 of 20 tokens 230 us by the walk, 292 in blocks; 32 of 40 194
     # and 195, per channel 233 and 200; 16 of 64 144 and 136, 176 and 137).
     REQUEST_FROM = 40
+    # Where heads of 128 by 128 go in chunks of 64 tokens instead: the walk in blocks costs some 0.12 us a token of 16 heads, chunks some 6.2 us each, full or
+    # not, and 11 us more to begin with, so that their requests' tokens must be at least 52 a chunk and 90 more.  us in blocks and in chunks: 2,048 tokens 277 and 201,
+    # 512 75 and 62, 384 59 and 57, 256 44 and 51, 128 27 and 37; 3 x 1,021 370 and 319, 1,531 beside 24 single tokens 247 and 191, 4 x 300 150 and 140,
+    # 16 x 512 871 and 866, 16 x 130 251 and 345, 512 beside 100 of 20 593 and 1,127, 256 beside 47 single tokens 107 and 124.
+    CHUNKS_FROM, CHUNK_TOKENS, CHUNK_START = 128, 52, 90
 
     def __init__(self, spec, hidden_size: int, model_dtype: torch.dtype):
         self.heads, self.kv_heads = int(spec.num_heads), int(spec.num_kv_heads)
@@ -346,6 +354,20 @@ class DeltaRule:
                              0 if host is None else int((host["req_q_len"] >= self.REQUEST_FROM).sum()))
         return ctx.memo[key]
 
+    def _chunk_room(self, ctx) -> int:
+        """Bytes of scratch of the step's chunks, 0 where it is walked; worked out once a step."""
+        host = getattr(ctx, "host", None)
+        if self.model_dtype != torch.bfloat16 or self.dim != 128 or self.vdim != 128 or ctx.max_q_len < self.CHUNKS_FROM or host is None:
+            return 0
+        key = ("delta_chunks", self.heads)
+        if key not in ctx.memo:
+            lens = host["req_q_len"]
+            long = lens[lens >= ops.DELTA_CHUNK_MIN]
+            pays = int(long.sum()) >= self.CHUNK_TOKENS * int(((long + 63) // 64).sum()) + self.CHUNK_START
+            room = ops.delta_chunks_bytes(lens, self.heads) if pays else 0
+            ctx.memo[key] = room if room <= ops.CHUNK_SCRATCH else 0
+        return ctx.memo[key]
+
     def mix(self, fused: torch.Tensor, parts: int, col0: int, ctx, cache: CacheRef):
         """The mixer on the columns from col0 of a fused product [n, W] (or partial sums [parts, n, W])."""
         n, H, G, D, V, f32 = fused.shape[-2], self.heads, self.kv_heads, self.dim, self.vdim, torch.float32
@@ -367,14 +389,20 @@ class DeltaRule:
         if channel:
             ops.lowrank_map(fused, parts, off["a_low"], self.decay_up, H, D, decay, self.dt_bias, self.a_log)
         o = ctx.buffer(self.tag + "delta_o", (n, H * V), f32)
+        state = ctx.state(cache.state_names["state"])
         # (a 32-bit model's walk gives the same bits however a prompt is cut)
-        blocks, walked = None, 0
-        if self.model_dtype == torch.bfloat16 and ctx.max_q_len >= self.REQUEST_FROM and \
-                (ctx.max_q_len + n) * self.share >= 2 * (self.CHANNEL_BLOCKS_FROM if channel else self.BLOCKS_FROM):
-            floats, walked = self._in_blocks(ctx, n)
-            blocks = ctx.buffer(self.tag + "delta_blocks", (floats,), f32)
-        ops.delta_scan(q, k, v, beta, decay, ctx.state(cache.state_names["state"]), o, ctx.req_q_start, ctx.req_q_len, ctx.req_slot,
-                       H, G, D, V, channel, blocks, ctx.max_q_len, single, walked, self.REQUEST_FROM)
+        room = self._chunk_room(ctx)
+        if room:
+            scratch = ctx.buffer(self.tag + "delta_chunks", (room,), torch.uint8)
+            ops.delta_chunks(q, k, v, beta, decay, state, o, ctx.req_q_start, ctx.req_q_len, ctx.req_slot, ctx.host["req_q_len"], H, G, channel, scratch)
+        else:
+            blocks, walked = None, 0
+            if self.model_dtype == torch.bfloat16 and ctx.max_q_len >= self.REQUEST_FROM and \
+                    (ctx.max_q_len + n) * self.share >= 2 * (self.CHANNEL_BLOCKS_FROM if channel else self.BLOCKS_FROM):
+                floats, walked = self._in_blocks(ctx, n)
+                blocks = ctx.buffer(self.tag + "delta_blocks", (floats,), f32)
+            ops.delta_scan(q, k, v, beta, decay, state, o, ctx.req_q_start, ctx.req_q_len, ctx.req_slot,
+                           H, G, D, V, channel, blocks, ctx.max_q_len, single, walked, self.REQUEST_FROM)
         gated = ctx.buffer(self.tag + "delta_gated", (n, H * V), self.model_dtype)
         if self.gate_maps is None:
             ops.head_gate_norm(o, fused, parts, off["g"], self.norm_weight, self.eps, gated, H, V)
