@@ -3,18 +3,21 @@
 // A step of few tokens is bound by what the host does for a launch.  The same checks and the same call through Python's tensor attributes and ctypes took 6 to
 // 11 us a launch where the CUDA call takes 3; here they take under one.  Every function checks what it is given at every call, with the errors of the functions
 // in kernels/ops.py that call it, takes the current stream, lets go of the interpreter's lock for the launch, and returns the entry point's status.  Nothing is
-// kept from call to call but the entry points' addresses (bind, bind_attention).
+// kept from call to call but the entry points' addresses.  An entry point is looked for by the first call that needs it and has passed its checks (binder), so that
+// what is refused is refused before anything is compiled or loaded.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <initializer_list>
+#include <sstream>
+#include <string>
 
 namespace {
 
 struct Failed {};                      // a Python error is set
-PyObject* kernel_error = nullptr;
+PyObject *kernel_error = nullptr, *binder = nullptr;
 
 [[noreturn]] void fail(PyObject* type, const char* what) {
     PyErr_SetString(type, what);
@@ -83,6 +86,11 @@ bool shaped(T t, std::initializer_list<int64_t> sizes) {
         if (t->size(i++) != s) return false;
     return true;
 }
+std::string sizes(T t) {
+    std::ostringstream text;
+    text << t->sizes() << " stride " << t->strides();
+    return text.str();
+}
 void* stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
 
 // a fused projection [n, W] (parts 0), or float32 partial sums [parts, n, W]
@@ -141,9 +149,21 @@ RopeRowFn rope_row_fn;
 DecodeFn decode_fn[257];               // by head size
 PrefillFn prefill_fn[257];
 
-template <typename Fn, typename... Args>
-PyObject* launch(Fn fn, Args... args) {
-    if (!fn) fail(PyExc_RuntimeError, "the entry point is not bound");
+// the binder hands the addresses over: of one entry point (its name), or of a head size's two (the size)
+PyObject* asked(const char* name) { return PyUnicode_FromString(name); }
+PyObject* asked(int head_size) { return PyLong_FromLong(head_size); }
+
+// (the arguments, and with them what is left to check in them, are worked out before this is entered)
+template <typename Fn, typename Which, typename... Args>
+PyObject* launch(Fn& fn, Which which, Args... args) {
+    if (!fn) {
+        PyObject* what = asked(which);
+        PyObject* done = what && binder ? PyObject_CallOneArg(binder, what) : nullptr;
+        Py_XDECREF(what);
+        Py_XDECREF(done);
+        if (PyErr_Occurred()) throw Failed{};
+        if (!fn) fail(PyExc_RuntimeError, "the entry point is not bound");
+    }
     int status;
     Py_BEGIN_ALLOW_THREADS
     status = fn(args...);
@@ -172,13 +192,15 @@ PyObject* gemm(Args v, Py_ssize_t n) {
     T a = tensor(v[0]), w = tensor(v[1]), out = tensor(v[2]), status = tensor(v[10]);
     on_device({a, w, out});
     if (!truth(v[11]) && !product_ok(a, w))
-        fail(kernel_error, "gemm_bf16_tc: bfloat16 operands with K and row pitches in steps of 8 elements, 16-byte aligned");
+        fail(kernel_error, ("gemm_bf16_tc: bfloat16 operands with K and row pitches in steps of 8 elements, 16-byte aligned; got a" + sizes(a) + " w" +
+                            sizes(w)).c_str());
     const int epilogue = small(v[3]), splits = small(v[5]);
     const int64_t M = a->size(0), K = a->size(1), N = w->size(0), cols = truth(v[4]) ? N / 2 : N;
     NEED(w->size(1) == K);
     NEED((splits == 1 ? shaped(out, {M, cols}) : shaped(out, {splits, M, cols})) && out->stride(-1) == 1 && (epilogue == 1 ? f32(out) : b16(out)));
     NEED(splits == 1 || (epilogue == 1 && out->is_contiguous()));
-    return launch(gemm_fn, at_(a), (int)a->stride(0), at_(w), (int)w->stride(0), at_(out), (int)out->stride(-2), (int)M, (int)N, (int)K, epilogue, splits,
+    return launch(gemm_fn, "wllm_gemm_bf16_tc_params",
+                  at_(a), (int)a->stride(0), at_(w), (int)w->stride(0), at_(out), (int)out->stride(-2), (int)M, (int)N, (int)K, epilogue, splits,
                   small(v[6]), static_cast<int*>(at_(status)), small(v[7]), real(v[8]), real(v[9]), stream());
 }
 
@@ -199,7 +221,8 @@ PyObject* norm(Args v, Py_ssize_t n) {
             split_stride = resid->numel();
         } else NEED(shaped(delta, {resid->size(0), H}));
     }
-    return launch(norm_fn, static_cast<float*>(at_(resid)), at_(delta), type_or_f32(delta), splits > 1 ? splits : 1, split_stride, at_(weight),
+    return launch(norm_fn, "wllm_norm",
+                  static_cast<float*>(at_(resid)), at_(delta), type_or_f32(delta), splits > 1 ? splits : 1, split_stride, at_(weight),
                   type_or_f32(weight), real(v[3]), real(v[4]), truth(v[8]) ? 1 : 0, at_(out), type_of(out), maybe_ints(rows, "rows"), (int)n_out, (int)H, stream());
 }
 
@@ -214,7 +237,8 @@ PyObject* sandwich(Args v, Py_ssize_t n) {
     for (T g : {post, weight, gain_a, gain_b}) NEED(!g || (shaped(g, {H}) && g->is_contiguous() && g->scalar_type() == post->scalar_type()));
     NEED(!bias || (f32(bias) && shaped(bias, {H}) && bias->is_contiguous()));
     const Branch pa(a, small(v[2]), N, H), pb(b, small(v[14]), N, H);
-    return launch(sandwich_fn, static_cast<float*>(at_(resid)), pa.p, pa.type, pa.parts, pa.stride, at_(gain_a), pb.p, pb.type, pb.parts, pb.stride, at_(gain_b),
+    return launch(sandwich_fn, "wllm_sandwich_norm_offset",
+                  static_cast<float*>(at_(resid)), pa.p, pa.type, pa.parts, pa.stride, at_(gain_a), pb.p, pb.type, pb.parts, pb.stride, at_(gain_b),
                   real(v[16]), real(v[17]), at_(post), real(v[18]), truth(v[5]) ? 1 : 0, real(v[6]), at_(weight), real(v[8]), truth(v[9]) ? 1 : 0, real(v[10]),
                   type_of(post), at_(out), type_of(out), maybe_ints(rows, "rows"), (int)n_out, (int)H, floats(bias), stream());
 }
@@ -239,7 +263,8 @@ PyObject* rope(Args v, Py_ssize_t n) {
     NEED(qkv->size(-1) == (int64_t)(nq + nkv) * hd + (int64_t)nkv * vd);
     rotation(q_out, f.n, nq, hd, inv_freq, rot, slots, kp, vp);
     const bool unit = v[15] != Py_None;
-    return launch(rope_fn, f.p, f.type, f.row_stride, f.parts, f.part_stride, at_(q_out), type_of(q_out), (int)q_out->stride(0), ints(positions, "positions"),
+    return launch(rope_fn, "wllm_rope_kv_write_general",
+                  f.p, f.type, f.row_stride, f.parts, f.part_stride, at_(q_out), type_of(q_out), (int)q_out->stride(0), ints(positions, "positions"),
                   maybe_ints(slots, "slots"), floats(inv_freq), at_(kp), at_(vp), f.n, nq, nkv, hd, rot, small(v[11]), truth(v[13]) ? 1 : 0, vd, unit ? 1 : 0,
                   unit ? real(v[15]) : 0.f, real(v[16]), stream());
 }
@@ -264,7 +289,8 @@ PyObject* rope_row(Args v, Py_ssize_t n) {
         NEED(v_first && f32(v_first) && shaped(v_first, {f.n, (int64_t)nkv * vd}) && v_first->is_contiguous());
         NEED(mix == 1 || (blend && f32(blend) && blend->numel() == 1));
     }
-    return launch(rope_row_fn, f.p, f.type, f.row_stride, f.parts, f.part_stride, at_(q_out), type_of(q_out), (int)q_out->stride(0), ints(positions, "positions"),
+    return launch(rope_row_fn, "wllm_rope_row_norm_kv_write",
+                  f.p, f.type, f.row_stride, f.parts, f.part_stride, at_(q_out), type_of(q_out), (int)q_out->stride(0), ints(positions, "positions"),
                   maybe_ints(slots, "slots"), floats(inv_freq), at_(kp), at_(vp), f.n, nq, nkv, hd, rot, small(v[11]), truth(v[18]) ? 1 : 0, vd, at_(q_gain),
                   at_(k_gain), type_of(q_gain), small(v[15]), small(v[16]), real(v[14]), floats(bias), static_cast<float*>(mix ? at_(v_first) : nullptr),
                   mix == 2 ? floats(blend) : nullptr, mix, real(v[24]), stream());
@@ -288,7 +314,8 @@ PyObject* attention_decode(Args v, Py_ssize_t n) {
     attention_operands(q, out, kp, vp, sinks, slopes, nq);
     NEED(f32(scratch) && scratch->numel() >= (int64_t)R * nq * splits * (hd + 2));
     NEED(hd > 0 && hd <= 256);
-    return launch(decode_fn[hd], at_(q), (int)q->stride(0), at_(out), (int)out->stride(0), at_(kp), at_(vp), (long long)kp->size(0), ints(start, "req_q_start"),
+    return launch(decode_fn[hd], hd,
+                  at_(q), (int)q->stride(0), at_(out), (int)out->stride(0), at_(kp), at_(vp), (long long)kp->size(0), ints(start, "req_q_start"),
                   ints(len, "req_q_len"), ints(ctx, "req_ctx_len"), ints(table, "block_table"), (int)table->size(1), R, nq, small(v[9]), small(v[11]), small(v[12]),
                   real(v[13]), small(v[14]), splits, static_cast<float*>(at_(scratch)), static_cast<int*>(at_(status)), floats(sinks), real(v[19]), small(v[20]),
                   floats(slopes), stream());
@@ -308,7 +335,8 @@ PyObject* attention_prefill(Args v, Py_ssize_t n) {
         NEED(halves->numel() >= whole(v[19]));
     }
     NEED(hd > 0 && hd <= 256);
-    return launch(prefill_fn[hd], at_(q), (int)q->stride(0), at_(out), (int)out->stride(0), at_(kp), at_(vp), (long long)kp->size(0), ints(start, "req_q_start"),
+    return launch(prefill_fn[hd], hd,
+                  at_(q), (int)q->stride(0), at_(out), (int)out->stride(0), at_(kp), at_(vp), (long long)kp->size(0), ints(start, "req_q_start"),
                   ints(len, "req_q_len"), ints(ctx, "req_ctx_len"), ints(table, "block_table"), (int)table->size(1), R, small(v[8]), nq, small(v[10]), small(v[12]),
                   small(v[13]), real(v[14]), truth(v[15]) ? 1 : 0, small(v[16]), split_above, static_cast<float*>(split_above > 0 ? at_(halves) : nullptr),
                   static_cast<int*>(at_(status)), floats(sinks), real(v[22]), small(v[23]), floats(slopes), stream());
@@ -340,11 +368,14 @@ PyObject* bind_attention(Args v, Py_ssize_t n) { // head size, address of decode
     prefill_fn[hd] = reinterpret_cast<PrefillFn>(p);
     Py_RETURN_NONE;
 }
-PyObject* errors(Args v, Py_ssize_t n) {         // the class that ops.KernelError is
-    count(n, 1);
+PyObject* errors(Args v, Py_ssize_t n) {         // the class that ops.KernelError is; what binds an entry point
+    count(n, 2);
     Py_INCREF(v[0]);
+    Py_INCREF(v[1]);
     Py_XDECREF(kernel_error);
+    Py_XDECREF(binder);
     kernel_error = v[0];
+    binder = v[1];
     Py_RETURN_NONE;
 }
 

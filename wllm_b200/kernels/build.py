@@ -196,8 +196,9 @@ def load_family(family: str, defines: dict | None = None) -> ctypes.CDLL:
 _host = None
 
 
-def load_host_calls(kernel_error: type):
-    """The module of native checks and launches (compiled on first use); `kernel_error`: the class of the errors that it raises."""
+def load_host_calls(kernel_error: type, binder):
+    """The module of native checks and launches (compiled on first use); `kernel_error`: the class of the errors that it raises; `binder`: called with the
+    entry point (or head size) whose address it needs."""
     global _host
     if _host is None:
         with _lock:
@@ -211,7 +212,7 @@ def load_host_calls(kernel_error: type):
                     loader.exec_module(host)
                 except ImportError as e:
                     raise KernelBuildError(f"cannot load {path}: {e}") from e
-                host.errors(kernel_error)
+                host.errors(kernel_error, binder)
                 _host = host
     return _host
 

@@ -84,28 +84,23 @@ def _check(status: int, what: str) -> None:
 
 # The functions that a step calls most hand their arguments to csrc/host_calls.cpp, which checks them, calls the entry point and returns its status.
 _host = None
-_bound: set = set()
+_HOST_FAMILIES = {"wllm_gemm_bf16_tc_params": "gemm_bf16_tc", "wllm_norm": "norm", "wllm_sandwich_norm_offset": "norm",
+                  "wllm_rope_kv_write_general": "rope_cache", "wllm_rope_row_norm_kv_write": "rope_cache"}
 
 
-def _host_call(family: str, entry: str):
-    """The module of native calls, with that entry point of that family bound."""
+def _bind(what) -> None:
+    """The module of native calls needs an entry point (its name), or the attention of a head size (the size), for a call that has passed its checks."""
+    if isinstance(what, int):
+        lib = load_family("attention_mma", {"HEAD_DIM": what})
+        _host.bind_attention(what, entry_address(lib, "wllm_attention_mma_decode_biased"), entry_address(lib, "wllm_attention_mma_prefill_biased"))
+    else:
+        _host.bind(what, entry_address(load_family(_HOST_FAMILIES[what]), what))
+
+
+def _host_calls():
     global _host
     if _host is None:
-        _host = load_host_calls(KernelError)
-    if entry not in _bound:
-        _host.bind(entry, entry_address(load_family(family), entry))
-        _bound.add(entry)
-    return _host
-
-
-def _host_attention(hd: int):
-    global _host
-    if _host is None:
-        _host = load_host_calls(KernelError)
-    if hd not in _bound:
-        lib = load_family("attention_mma", {"HEAD_DIM": hd})
-        _host.bind_attention(hd, entry_address(lib, "wllm_attention_mma_decode_biased"), entry_address(lib, "wllm_attention_mma_prefill_biased"))
-        _bound.add(hd)
+        _host = load_host_calls(KernelError, _bind)
     return _host
 
 
@@ -152,7 +147,7 @@ def rmsnorm(resid: torch.Tensor, delta, weight, eps: float, offset: float, out: 
     `delta` is [S, n, H] float32 partial sums that are added in order.  `center`: the row's mean is taken off
     first (a layer norm without a bias).  `weight` None: nothing is normed, `out` is the residual's rows rounded to
     its element type."""
-    status = _host_call("norm", "wllm_norm").norm(resid, delta, weight, eps, offset, out, rows, delta_splits, center)
+    status = _host_calls().norm(resid, delta, weight, eps, offset, out, rows, delta_splits, center)
     if status:
         _check(status, "norm")
     global launches
@@ -198,7 +193,7 @@ def sandwich_norm(resid: torch.Tensor, a, out: torch.Tensor, post_weight: torch.
         out = norm(resid) * (offset + weight), or, with `weight` None, resid as it is (rounded to out's type).
     `a`, `b`: (tensor [n, H] or float32 partial sums [S, n, H], S or 0).  With `rows` the residual is read at those rows
     and left as it is."""
-    status = _host_call("norm", "wllm_sandwich_norm_offset").sandwich(
+    status = _host_calls().sandwich(
         resid, *a, out, post_weight, post_center, post_eps, weight, offset, center, eps, rows, gain_a, *(b if b is not None else (None, 0)), gain_b,
         inner_eps, factor, post_offset, bias)
     if status:
@@ -283,7 +278,7 @@ def rope_kv_write(qkv: torch.Tensor, q_out: torch.Tensor, positions: torch.Tenso
     if pairing not in ("half", "interleaved"):
         raise KernelError(f"rotary pairing {pairing!r} not supported (half, interleaved)")
     # (nkv = 0: a row of query heads alone, nothing goes to the pages)
-    status = _host_call("rope_cache", "wllm_rope_kv_write_general").rope(
+    status = _host_calls().rope(
         qkv, q_out, positions, slots, inv_freq, k_pages, v_pages, nq, nkv, hd, rot_dim, page_size, in_splits, pairing == "interleaved", vd, unit_norm_eps,
         turn_scale)
     if status:
@@ -312,7 +307,7 @@ def rope_row_norm_kv_write(qkv: torch.Tensor, q_out: torch.Tensor, positions: to
         raise KernelError(f"rotary pairing {pairing!r} not supported (half, interleaved)")
     if mix not in (None, "first", "later"):
         raise KernelError(f"value mixing {mix!r}: 'first' or 'later'")
-    status = _host_call("rope_cache", "wllm_rope_row_norm_kv_write").rope_row(
+    status = _host_calls().rope_row(
         qkv, q_out, positions, slots, inv_freq, k_pages, v_pages, nq, nkv, hd, rot_dim, page_size, q_gain, k_gain, eps, q_count, k_count, in_splits,
         pairing == "interleaved", vd, bias, v_first, blend, _MIX[mix], turn_scale)
     if status:
@@ -636,7 +631,11 @@ def _status_word(device) -> torch.Tensor:
 def _device_status(device: torch.device) -> torch.Tensor:
     """_status_word of a tensor's device, whose index is known."""
     status = _tc_status.get(device)
-    return _status_word(device) if status is None else status
+    if status is None:
+        if device.type != "cuda":
+            raise KernelError("the engine's kernels run on a CUDA device only; got a tensor on " + str(device))
+        status = _status_word(device)
+    return status
 
 
 def mma_head_dim_ok(hd: int) -> bool:
@@ -683,7 +682,7 @@ def attention_mma_decode(q, out, k_pages, v_pages, req_q_start, req_q_len, req_c
     `sinks`: float32 [nq], one more term e^sink of every row's softmax denominator.  `cap` > 0: scores become
     cap * tanh(score / cap); `keep` > 0 (with a window): the sequence's first `keep` keys stay visible behind the window.
     `slopes`: float32 [nq]; the score of key j from position p loses slopes[head] * (p - j), after the scale and the cap."""
-    status = _host_attention(hd).attention_decode(
+    status = _host_calls().attention_decode(
         q, out, k_pages, v_pages, req_q_start, req_q_len, req_ctx_len, block_table, nq, nkv, hd, page_size, window, scale, split_keys, max_splits, scratch,
         _device_status(q.device), sinks, cap, keep, slopes)
     if status:
@@ -733,7 +732,7 @@ def attention_mma_prefill(q, out, k_pages, v_pages, req_q_start, req_q_len, req_
     keys is computed by two CTAs, half of the keys each; `halves` (float32) holds their partial results.
     `cap`, `keep`, `slopes`: as for attention_mma_decode; with any of them no tile is shared by two CTAs."""
     floats = attention_prefill_halves_floats(req_q_len.shape[0], max_q_len, nq, nkv, hd) if split_above > 0 else 0
-    status = _host_attention(hd).attention_prefill(
+    status = _host_calls().attention_prefill(
         q, out, k_pages, v_pages, req_q_start, req_q_len, req_ctx_len, block_table, max_q_len, nq, nkv, hd, page_size, window, scale, skip_single, multi,
         split_above, halves, floats, _device_status(q.device), sinks, cap, keep, slopes)
     if status:
@@ -882,7 +881,7 @@ _tc_status: dict = {}
 
 def tc_gemm_ok(a: torch.Tensor, w: torch.Tensor) -> bool:
     """Shapes the tensor-memory GEMM takes: bfloat16, unit inner strides, K and pitches in steps of 8."""
-    return _host_call("gemm_bf16_tc", "wllm_gemm_bf16_tc_params").tc_gemm_ok(a, w)
+    return _host_calls().tc_gemm_ok(a, w)
 
 
 @functools.lru_cache(maxsize=4096)
@@ -970,7 +969,7 @@ def gemm_bf16_tc(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = No
     half_rows: the tile of products of at most 128 rows (see tile_plan, which chooses it when None)."""
     code = _TC_EPILOGUES[epilogue]
     gated = code in _TC_GATED
-    host = _host_call("gemm_bf16_tc", "wllm_gemm_bf16_tc_params")
+    host = _host_calls()
     if out is None or half_rows is None:
         _need_cuda(a, w, out)
         if not checked and not host.tc_gemm_ok(a, w):        # `checked`: the caller has asked tc_gemm_ok already
