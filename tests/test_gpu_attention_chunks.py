@@ -39,3 +39,19 @@ def test_chunks_give_the_tiled_kernels_bits(lens, before, nq, nkv, hd, vd, ps, e
     scratch = torch.full((n * nq * chunks * (vd + 2),), float("nan"), device=DEV)
     ops.paged_attention_simt_chunks(q, got, k.to(DEV), v.to(DEV), positions, *meta, max(lens), nq, nkv, hd, ps, hd ** -0.5, scratch, chunks, vd=vd, **more)
     assert bool(want.isfinite().all()) and torch.equal(want, got)
+
+
+def test_pools_and_tables_that_do_not_fit_are_refused():
+    """What the kernel indexes by: rows of hd and vd elements, a table of two axes, chunks that hold the longest context."""
+    from wllm_b200.kernels import ops
+    n, nq, nkv, hd, vd, ps, ctx = 4, 2, 1, 32, 16, 16, 70
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    z = lambda *shape: torch.zeros(shape, device=DEV)
+    args = dict(q=z(n, nq * hd), out=z(n, nq * vd), k_pages=z(6, nkv, ps, hd), v_pages=z(6, nkv, ps, vd), positions=i32([66, 67, 68, 69]), req_q_start=i32([0]),
+                req_q_len=i32([n]), req_ctx_len=i32([ctx]), block_table=i32([[1, 2, 3, 4, 5]]), max_q_len=n, nq=nq, nkv=nkv, hd=hd, page_size=ps, scale=0.2,
+                scratch=z(n * nq * 2 * (vd + 2)), max_chunks=2, vd=vd, max_ctx=ctx)
+    ops.paged_attention_simt_chunks(**args)
+    for wrong in (dict(k_pages=z(6, nkv, ps, 16)), dict(v_pages=z(6, nkv, ps, 8)), dict(k_pages=args["v_pages"], v_pages=args["k_pages"]),
+                  dict(block_table=i32([1, 2, 3, 4, 5])), dict(max_chunks=1), dict(scratch=args["scratch"][:-1])):
+        with pytest.raises(AssertionError):
+            ops.paged_attention_simt_chunks(**{**args, **wrong})

@@ -559,14 +559,15 @@ def simt_by_chunks(tokens: int, max_ctx: int, nq: int, nkv: int, vd: int) -> int
 def paged_attention_simt_chunks(q: torch.Tensor, out: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, positions: torch.Tensor,
                                 req_q_start: torch.Tensor, req_q_len: torch.Tensor, req_ctx_len: torch.Tensor, block_table: torch.Tensor, max_q_len: int,
                                 nq: int, nkv: int, hd: int, page_size: int, scale: float, scratch: torch.Tensor, max_chunks: int, vd: int | None = None,
-                                sinks: torch.Tensor | None = None, cap: float = 0.0, slopes: torch.Tensor | None = None) -> None:
+                                sinks: torch.Tensor | None = None, cap: float = 0.0, slopes: torch.Tensor | None = None, max_ctx: int = 0) -> None:
     """paged_attention_simt_tiled for float32 steps without a window, chunk by chunk (csrc/attention_simt.cu): the same bits.  `scratch` float32,
-    tokens * nq * max_chunks * (vd + 2); `max_chunks`: chunks of 64 keys of the longest context."""
+    tokens * nq * max_chunks * (vd + 2); `max_chunks`: chunks of 64 keys of the longest context, which has `max_ctx` (0: not said)."""
     _need_cuda(q, out, k_pages, v_pages, positions, req_q_start, req_q_len, req_ctx_len, block_table, scratch, sinks, slopes)
     n, vd = q.shape[0], hd if vd is None else vd
     assert q.dtype == k_pages.dtype == v_pages.dtype == out.dtype == scratch.dtype == torch.float32
     assert q.shape == (n, nq * hd) and q.stride(1) == 1 and out.shape == (n, nq * vd) and out.stride(1) == 1 and positions.shape == (n,)
     assert k_pages.is_contiguous() and v_pages.is_contiguous() and scratch.is_contiguous() and scratch.numel() >= n * nq * max_chunks * (vd + 2)
+    assert k_pages.shape[-1] == hd and v_pages.shape[-1] == vd and block_table.dim() == 2 and max_chunks * SIMT_CHUNK >= max_ctx
     assert sinks is None or (sinks.dtype == torch.float32 and sinks.shape == (nq,) and sinks.is_contiguous())
     assert slopes is None or (slopes.dtype == torch.float32 and slopes.shape == (nq,) and slopes.is_contiguous())
     lib = load_family("attention_simt")

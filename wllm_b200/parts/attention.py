@@ -301,7 +301,7 @@ class PagedAttention:
                     scratch = ctx.buffer(self.tag + "attention_chunks", (q.shape[0] * nq * by_chunks * (self.vd + 2),), torch.float32)
                     extra.pop("keep", None)
                     ops.paged_attention_simt_chunks(q, out, k_pages, v_pages, ctx.positions, ctx.req_q_start, ctx.req_q_len, ctx.req_ctx_len, table,
-                                                    ctx.max_q_len, nq, nkv, hd, ps, scale, scratch, by_chunks, **extra)
+                                                    ctx.max_q_len, nq, nkv, hd, ps, scale, scratch, by_chunks, max_ctx=ctx.max_ctx, **extra)
                     return
                 ops.paged_attention_simt_tiled(q, out, k_pages, v_pages, ctx.req_q_start, ctx.req_q_len, ctx.req_ctx_len,
                                                table, ctx.max_q_len, nq, nkv, hd, ps, window, scale, **extra)
