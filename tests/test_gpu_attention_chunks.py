@@ -55,3 +55,29 @@ def test_pools_and_tables_that_do_not_fit_are_refused():
                   dict(block_table=i32([1, 2, 3, 4, 5])), dict(max_chunks=1), dict(scratch=args["scratch"][:-1])):
         with pytest.raises(AssertionError):
             ops.paged_attention_simt_chunks(**{**args, **wrong})
+
+
+# requests of more than a warp's lanes, some that bring nothing, long contexts behind few rows and the other way round
+@pytest.mark.parametrize("lens,before", [([70, 0, 1, 33], [10, 40, 300, 63]), ([1, 0, 3] * 15 + [150] + [1] * 30, [5 + 29 * i for i in range(76)]), ([17], [1000])])
+@pytest.mark.parametrize("nq,nkv,hd", [(8, 1, 64), (6, 2, 32)])
+def test_every_request_has_ctas_of_its_own_rows_and_keys(lens, before, nq, nkv, hd):
+    import numpy as np
+
+    from wllm_b200.kernels import ops
+    ps, R, n, ctx = 16, len(lens), sum(lens), [m + b for m, b in zip(lens, before)]
+    g = torch.Generator().manual_seed(n)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    width = -(-max(ctx) // ps)
+    table = torch.arange(R * width, dtype=torch.int32, device=DEV).view(R, width)
+    k, v = (torch.randn(R * width, nkv, ps, hd, generator=g).to(DEV) for _ in range(2))
+    q = torch.randn(n, nq * hd, generator=g).to(DEV)
+    meta = (i32([sum(lens[:r]) for r in range(R)]), i32(lens), i32(ctx), table)
+    positions = i32([b + j for m, b in zip(lens, before) for j in range(m)])
+    want, got = (torch.full((n, nq * hd), float("nan"), device=DEV) for _ in range(2))
+    ops.paged_attention_simt_tiled(q, want, k, v, *meta, max(lens), nq, nkv, hd, ps, 0, 0.1)
+    chunks, rep = -(-max(ctx) // 64), nq // nkv
+    pairs = ops.simt_chunk_pairs(np.array(lens, dtype=np.int32), np.array(ctx, dtype=np.int32), rep)
+    assert pairs == sum(-(-m * rep // 32) * -(-c // 64) for m, c in zip(lens, ctx))
+    scratch = torch.full((n * nq * chunks * (hd + 2),), float("nan"), device=DEV)
+    ops.paged_attention_simt_chunks(q, got, k, v, positions, *meta, max(lens), nq, nkv, hd, ps, 0.1, scratch, chunks, max_ctx=max(ctx), pairs=pairs)
+    assert bool(want.isfinite().all()) and torch.equal(want, got)

@@ -554,24 +554,54 @@ paged_attention_simt_tiled_kernel(const T* __restrict__ q, int q_stride, T* __re
 }
 
 // --------------------------------------------------------------------------------------
-// tiled, chunk by chunk: grid (tiles of 32 rows x chunks of 64 keys, kv heads, requests), for steps whose tiles are too few to fill the device one behind the
-// other.  A CTA works out its rows' result over one chunk as the tiled kernel does and leaves m, l, o[vd] in scratch[(row * max_chunks + chunk) * (vd + 2)],
+// tiled, chunk by chunk: grid (pairs of a tile of 32 rows and a chunk of 64 keys, over all requests, kv heads), for steps whose tiles are too few to fill the device
+// one behind the other.  A request has the pairs of its own rows and keys alone (us by the tiled kernel, with the longest request's pairs for each, and so, 8 heads of
+// 256 on one: 250 tokens beside 120 single ones at 60 keys 374, 565 and 50; 509 beside 24 at 1,100 467, 238 and 145; 200 beside 48 at 4,096 1,502, 726 and 317; 509
+// alone 228, 93 and 93).  A CTA works out its rows' result over one chunk as the tiled kernel does and leaves m, l, o[vd] in scratch[(row * max_chunks + chunk) * (vd + 2)],
 // where the walk's merge kernel takes them up in order: the same bits.  Without a running total and with one tile of keys and values in shared memory (a tile's
 // values land while its scores are worked out, the next tile's keys during the weighted sum) two CTAs fit on an SM.  Every key is seen from its position on (no window).
 // --------------------------------------------------------------------------------------
+// The nth of all pairs: its request (-1 past the last), tile and chunk.  A warp together.
+__device__ __forceinline__ int chunk_pair(const int* __restrict__ req_q_len, const int* __restrict__ req_ctx_len, int requests, int rep, int max_chunks, int nth,
+                                          int& tile, int& chunk) {
+    const int lane = threadIdx.x & 31;
+    for (int r0 = 0; r0 < requests; r0 += 32) {
+        const int r = r0 + lane;
+        const int tiles = r < requests ? (req_q_len[r] * rep + TL_ROWS - 1) / TL_ROWS : 0;
+        const int chunks = tiles > 0 ? min((req_ctx_len[r] + CHUNK - 1) / CHUNK, max_chunks) : 0;
+        int sum = tiles * chunks;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int other = __shfl_up_sync(0xffffffffu, sum, o);
+            if (lane >= o) sum += other;
+        }
+        const unsigned behind = __ballot_sync(0xffffffffu, sum > nth);
+        if (behind) {
+            const int at = __ffs(behind) - 1, each = __shfl_sync(0xffffffffu, chunks, at);
+            nth -= __shfl_sync(0xffffffffu, sum - tiles * chunks, at);
+            tile = nth / each;
+            chunk = nth - tile * each;
+            return r0 + at;
+        }
+        nth -= __shfl_sync(0xffffffffu, sum, 31);
+    }
+    return -1;
+}
+
 template <typename T, int NE>
 __global__ void __launch_bounds__(TL_WARPS * 32, 2)
 paged_attention_simt_chunk_kernel(const T* __restrict__ q, int q_stride, const T* __restrict__ k_pages, const T* __restrict__ v_pages,
                                   const int* __restrict__ req_q_start, const int* __restrict__ req_q_len, const int* __restrict__ req_ctx_len,
-                                  const int* __restrict__ block_table, int max_pages, int nq, int nkv, int hd, int page_size, float scale, int vd, float cap,
-                                  const float* __restrict__ slopes, float* __restrict__ scratch, int max_chunks) {
+                                  const int* __restrict__ block_table, int max_pages, int requests, int nq, int nkv, int hd, int page_size, float scale, int vd,
+                                  float cap, const float* __restrict__ slopes, float* __restrict__ scratch, int max_chunks) {
     constexpr int VN = Vec<T>::N;
     extern __shared__ __align__(16) unsigned char tl_smem[];
     __shared__ size_t row_of[CHUNK];               // the chunk's keys in the pools
     pdl_begin();
-    const int g = blockIdx.y, r = blockIdx.z, c = blockIdx.x % max_chunks, m0 = blockIdx.x / max_chunks * TL_ROWS;
-    const int q_len = req_q_len[r], rep = nq / nkv, rows = q_len * rep;
-    if (m0 >= rows) return;
+    int tile_at, c;
+    const int g = blockIdx.y, rep = nq / nkv, r = chunk_pair(req_q_len, req_ctx_len, requests, rep, max_chunks, blockIdx.x, tile_at, c);
+    if (r < 0) return;
+    const int q_len = req_q_len[r], rows = q_len * rep, m0 = tile_at * TL_ROWS;
     const int ctx = req_ctx_len[r], q_start = req_q_start[r], pos0 = ctx - q_len;
     const int key_hi = pos0 + (min(rows, m0 + TL_ROWS) - 1) / rep + 1;         // one past the last row's position
     if (c * CHUNK >= key_hi) return;
@@ -785,20 +815,21 @@ WLLM_API int wllm_paged_attention_simt_tiled(const void* q, int q_stride, void* 
 }
 
 // The tiled kernel's result over steps without a window, chunk by chunk, bit for bit.  scratch: n_tokens * nq * max_chunks * (vd + 2) floats; max_chunks: chunks of
-// 64 keys of the longest context; positions [n_tokens].  32-bit rows of up to 256 elements (the bfloat16 form is not built).
+// 64 keys of the longest context; positions [n_tokens]; pairs: the requests' tiles of 32 rows times their chunks, added up (0: not known, those of the longest for
+// each).  32-bit rows of up to 256 elements (the bfloat16 form is not built).
 WLLM_API int wllm_paged_attention_simt_chunks(const void* q, int q_stride, void* out, int out_stride, const void* k_pages, const void* v_pages,
                                               const int* positions, const int* req_q_start, const int* req_q_len, const int* req_ctx_len,
                                               const int* block_table, int max_pages, int n_tokens, int requests, int max_q_len, int nq, int nkv, int hd,
                                               int page_size, float scale, int vd, const float* sinks, float cap, const float* slopes, float* scratch,
-                                              int max_chunks, cudaStream_t stream) {
+                                              int max_chunks, long long pairs, cudaStream_t stream) {
     if (n_tokens <= 0 || requests <= 0 || max_q_len <= 0) return WLLM_OK;
     if (hd <= 0 || hd > 256 || hd % 8 != 0 || vd <= 0 || vd > 256 || vd % 8 != 0 || nq <= 0 || nkv <= 0 || nq % nkv != 0 || page_size <= 0 || max_pages <= 0 ||
         max_chunks < 1 || scratch == nullptr || cap < 0.f || requests > 65535 || nkv > 65535)
         return WLLM_BAD_SIZE;
     if (((uintptr_t)k_pages | (uintptr_t)v_pages) & 15) return WLLM_BAD_ALIGN;
-    const long long tiles = ((long long)max_q_len * (nq / nkv) + TL_ROWS - 1) / TL_ROWS;
-    if (tiles * max_chunks > 0x7fffffff) return WLLM_BAD_SIZE;
-    const dim3 grid((unsigned)(tiles * max_chunks), nkv, requests);
+    if (pairs <= 0) pairs = ((long long)max_q_len * (nq / nkv) + TL_ROWS - 1) / TL_ROWS * max_chunks * requests;
+    if (pairs > 0x7fffffff) return WLLM_BAD_SIZE;
+    const dim3 grid((unsigned)pairs, nkv);
     constexpr int VN = Vec<float>::N, most = (TL_ROWS * 256 + 32 * (256 + VN) + 32 * 256) * (int)sizeof(float);
     const size_t smem = ((size_t)TL_ROWS * hd + 32 * (hd + VN) + 32 * vd) * sizeof(float);
     const int blocks = (n_tokens * nq + WARPS - 1) / WARPS;
@@ -810,8 +841,8 @@ WLLM_API int wllm_paged_attention_simt_chunks(const void* q, int q_stride, void*
             raised = true; \
         } \
         const int st = wllm_launch(paged_attention_simt_chunk_kernel<float, NE>, grid, TL_WARPS * 32, smem, stream, (const float*)q, q_stride, \
-                                   (const float*)k_pages, (const float*)v_pages, req_q_start, req_q_len, req_ctx_len, block_table, max_pages, nq, nkv, hd, \
-                                   page_size, scale, vd, cap, slopes, scratch, max_chunks); \
+                                   (const float*)k_pages, (const float*)v_pages, req_q_start, req_q_len, req_ctx_len, block_table, max_pages, requests, \
+                                   nq, nkv, hd, page_size, scale, vd, cap, slopes, scratch, max_chunks); \
         if (st != WLLM_OK) return st; \
         return wllm_launch(paged_attention_simt_merge_kernel<float, NE>, blocks, WARPS * 32, 0, stream, (float*)out, out_stride, positions, n_tokens, nq, vd, 0, \
                            (const float*)scratch, max_chunks, sinks, 0); \

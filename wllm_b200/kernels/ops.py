@@ -550,18 +550,25 @@ SIMT_CHUNK_SCRATCH = 32 << 20      # floats
 def simt_by_chunks(tokens: int, max_ctx: int, nq: int, nkv: int, vd: int) -> int:
     """Chunks for paged_attention_simt_chunks, or 0: the tiled kernel, whose tiles of 32 rows walk all their keys, a CTA an SM at a time.  A step of few tiles
     ends with the longest of them, so its chunks are dealt out one by one as long as the tiles are less than two rounds and their results fit in 128 MB
-    (us, tiled and by chunks, 8 heads of 256 on one: 509 tokens 231 and 92; 100 67 and 45; 1,000, 250 tiles, 629 and 337; four prompts of 500 to 60, 234 tiles,
-    229 and 136; 16 tokens behind 4,000 1,705 and 57)."""
+    (us, tiled and by chunks, 8 heads of 256 on one: 509 tokens 228 and 93; 100 65 and 42; 1,000, 250 tiles, 629 and 337; four prompts of 500 to 60, 234 tiles,
+    228 and 137; 16 tokens behind 4,000 1,702 and 58; 509 beside 24 single ones at 1,100 keys 467 and 145; 64 beside 128 at 1,000 394 and 202)."""
     chunks, tiles = -(-max_ctx // SIMT_CHUNK), -(-tokens * (nq // nkv) // 32) * nkv
     return chunks if chunks > 1 and tiles < 2 * sm_count() and tokens * nq * chunks * (vd + 2) <= SIMT_CHUNK_SCRATCH else 0
+
+
+def simt_chunk_pairs(lens, ctx_lens, rep: int) -> int:
+    """Pairs of a tile of 32 rows and a chunk of keys of all requests; `lens`, `ctx_lens`: their tokens and contexts (int32 arrays on the host), `rep` heads a
+    key/value head."""
+    return int(((lens.astype("int64") * rep + 31) // 32 * ((ctx_lens + (SIMT_CHUNK - 1)) // SIMT_CHUNK)).sum())
 
 
 def paged_attention_simt_chunks(q: torch.Tensor, out: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, positions: torch.Tensor,
                                 req_q_start: torch.Tensor, req_q_len: torch.Tensor, req_ctx_len: torch.Tensor, block_table: torch.Tensor, max_q_len: int,
                                 nq: int, nkv: int, hd: int, page_size: int, scale: float, scratch: torch.Tensor, max_chunks: int, vd: int | None = None,
-                                sinks: torch.Tensor | None = None, cap: float = 0.0, slopes: torch.Tensor | None = None, max_ctx: int = 0) -> None:
+                                sinks: torch.Tensor | None = None, cap: float = 0.0, slopes: torch.Tensor | None = None, max_ctx: int = 0, pairs: int = 0) -> None:
     """paged_attention_simt_tiled for float32 steps without a window, chunk by chunk (csrc/attention_simt.cu): the same bits.  `scratch` float32,
-    tokens * nq * max_chunks * (vd + 2); `max_chunks`: chunks of 64 keys of the longest context, which has `max_ctx` (0: not said)."""
+    tokens * nq * max_chunks * (vd + 2); `max_chunks`: chunks of 64 keys of the longest context, which has `max_ctx` (0: not said).
+    `pairs`: simt_chunk_pairs of the step (0: not said; every request then has as many CTAs as the longest)."""
     _need_cuda(q, out, k_pages, v_pages, positions, req_q_start, req_q_len, req_ctx_len, block_table, scratch, sinks, slopes)
     n, vd = q.shape[0], hd if vd is None else vd
     assert q.dtype == k_pages.dtype == v_pages.dtype == out.dtype == scratch.dtype == torch.float32
@@ -575,8 +582,8 @@ def paged_attention_simt_chunks(q: torch.Tensor, out: torch.Tensor, k_pages: tor
                                                 _ptr(_int32(positions, "positions")), _ptr(_int32(req_q_start, "req_q_start")),
                                                 _ptr(_int32(req_q_len, "req_q_len")), _ptr(_int32(req_ctx_len, "req_ctx_len")),
                                                 _ptr(_int32(block_table, "block_table")), block_table.shape[1], n, req_q_len.shape[0], max_q_len, nq, nkv, hd,
-                                                page_size, c_float(scale), vd, _ptr(sinks), c_float(cap), _ptr(slopes), _ptr(scratch), max_chunks, _stream()),
-           f"paged_attention_simt_chunks(head_dim={hd}, heads={nq}/{nkv})")
+                                                page_size, c_float(scale), vd, _ptr(sinks), c_float(cap), _ptr(slopes), _ptr(scratch), max_chunks,
+                                                ctypes.c_longlong(pairs), _stream()), f"paged_attention_simt_chunks(head_dim={hd}, heads={nq}/{nkv})")
     global launches
     launches += 1                # the merge kernel
 

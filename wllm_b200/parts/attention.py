@@ -300,6 +300,11 @@ class PagedAttention:
                 if by_chunks:
                     scratch = ctx.buffer(self.tag + "attention_chunks", (q.shape[0] * nq * by_chunks * (self.vd + 2),), torch.float32)
                     extra.pop("keep", None)
+                    if ctx.host is not None:
+                        key = ("chunk_pairs", nq // nkv)
+                        if key not in ctx.memo:
+                            ctx.memo[key] = ops.simt_chunk_pairs(ctx.host["req_q_len"], ctx.host["req_ctx_len"], nq // nkv)
+                        extra["pairs"] = ctx.memo[key]
                     ops.paged_attention_simt_chunks(q, out, k_pages, v_pages, ctx.positions, ctx.req_q_start, ctx.req_q_len, ctx.req_ctx_len, table,
                                                     ctx.max_q_len, nq, nkv, hd, ps, scale, scratch, by_chunks, max_ctx=ctx.max_ctx, **extra)
                     return
