@@ -690,13 +690,18 @@ static int lc_turn(const int* lens, int requests, int H, int D, int V, long long
     }
 }
 
-// Bytes of scratch that wllm_linattn_chunks asks for: 2.5 MB a chunk of 8 heads of 128 x 256, at most 192 MB (4,800 tokens; longer steps go in turns, the state
-// handed on through its slot: the same bits) but a chunk of every request that goes in chunks.  lens: the requests' tokens, on the host.
+// Bytes of scratch that wllm_linattn_chunks asks for: 2.5 MB a chunk of 8 heads of 128 x 256, at most 192 MB (4,992 tokens; longer steps go in turns, the state
+// handed on through its slot: the same bits) but a chunk of every request that goes in chunks.  lens: the requests' tokens, on the host.  turns: how many with that.
 constexpr long long LC_SCRATCH = 192ll << 20;
-WLLM_API long long wllm_linattn_chunks_bytes(const int* lens, int requests, int H, int D, int V) {
+WLLM_API long long wllm_linattn_chunks_bytes(const int* lens, int requests, int H, int D, int V, int* turns) {
+    *turns = 0;
     if (!lc_sizes(H, D, V) || requests <= 0) return 0;
     long long chunks;
-    lc_turn(lens, requests, H, D, V, LC_SCRATCH, chunks);
+    const int turn = lc_turn(lens, requests, H, D, V, LC_SCRATCH, chunks);
+    for (int r = 0; r < requests; ++r) {
+        const int mine = turn > 0 ? (lc_chunks(lens[r]) + turn - 1) / turn : 0;
+        *turns = mine > *turns ? mine : *turns;
+    }
     return chunks * H * ChunkLayout(D, V).size;
 }
 

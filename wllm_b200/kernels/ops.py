@@ -1163,11 +1163,41 @@ def linattn_chunks_ok(fused, parts: int, offsets, dim: int, vdim: int, rot_dim: 
             and fused.stride(1) == 1 and fused.stride(0) % 8 == 0 and fused.data_ptr() % 16 == 0 and all(o % 8 == 0 for o in offsets))
 
 
-def linattn_chunks_bytes(lens, heads: int, dim: int, vdim: int) -> int:
-    """Bytes of scratch that linattn_chunks asks for; `lens`: the requests' tokens (int32 array on the host)."""
+def linattn_chunks_plan(lens, heads: int, dim: int, vdim: int) -> tuple:
+    """(bytes of scratch that linattn_chunks asks for, turns that it takes with them); `lens`: the requests' tokens (int32 array on the host)."""
     lib = load_family("linear_attention_chunks")
     lib.wllm_linattn_chunks_bytes.restype = ctypes.c_longlong
-    return int(lib.wllm_linattn_chunks_bytes(c_void_p(lens.ctypes.data), len(lens), heads, dim, vdim))
+    turns = ctypes.c_int(0)
+    return int(lib.wllm_linattn_chunks_bytes(c_void_p(lens.ctypes.data), len(lens), heads, dim, vdim, ctypes.byref(turns))), turns.value
+
+
+def linattn_chunks_bytes(lens, heads: int, dim: int, vdim: int) -> int:
+    return linattn_chunks_plan(lens, heads, dim, vdim)[0]
+
+
+LINATTN_CHUNK_MIN = 16         # the shortest requests that linattn_chunks takes in chunks
+
+
+def linattn_chunks_pay(lens, heads: int, dim: int, vdim: int, rank: int) -> int:
+    """Bytes of scratch of linattn_chunks where it is the faster way for a step of these requests (`rank`: of the decay's low-rank map, 0 without one), else 0.
+
+    Both ways' us, fitted to B200 measurements from 130 to 8,192 tokens (in brackets the walk's and the chunks' for 8 heads of 128 x 256 with a decay per channel).
+    A chunk costs by the bytes that its kernels hand on (2.56 MB of those heads), full or not, a request its state's way; a turn some 45 (2,048 tokens [253, 86],
+    512 [86, 41], 16 x 130 [183, 145], 130 beside 20 of 20 [74, 99], beside 40 [86, 179], beside 90 [176, 447], 512 beside 20 of 20 [206, 108], beside 90
+    [286, 678: eight turns], 2,048 beside 90 [837, 1,787: thirty-two]).  The walk is bound by its longest request's chain or by all tokens.  Where segments of the
+    long requests fill the device few requests are there, and chunks were the faster way at every size measured (2 to 32 heads)."""
+    room, turns = linattn_chunks_plan(lens, heads, dim, vdim)
+    if room <= 0 or room > CHUNK_SCRATCH:
+        return 0
+    longest = int(lens.max())
+    if linattn_segment_plan(longest, int((lens > 1).sum()), heads, vdim)[1] > 1:
+        return room
+    chunks = (lens[lens >= LINATTN_CHUNK_MIN] + 63) // 64
+    tokens, size = int(lens.sum()), heads * dim * vdim / 2.0 ** 18
+    unit = heads * (772 * dim + 24576 + 6 * dim * vdim) / 2.56e6
+    in_chunks = 22 + max(1.05 * int(chunks.max()), 2.0 * unit * int(chunks.sum()) + 1.6 * size * len(chunks)) + 45 * (turns - 1)
+    walked = max(8 + 0.3 * longest + 0.025 * size * (tokens - longest), 0.07 * size * tokens) + (5 + 0.02 * heads * dim * rank / 65536 * tokens if rank else 0)
+    return room if in_chunks < walked else 0
 
 
 def linattn_chunks(fused, q_off: int, k_off: int, v_off: int, heads: int, dim: int, vdim: int, positions: torch.Tensor, decay, head_decay,

@@ -141,8 +141,8 @@ class LinearAttention:
         state = ctx.state(cache.state_names["state"])
         room = 0
         if ctx.max_q_len >= ops.LINATTN_CHUNKS_FROM and ops.linattn_chunks_ok(fused, parts, offsets, D, V, rot, getattr(self.position, "pairing", "half")):
-            room = ops.linattn_chunks_bytes(ctx.host["req_q_len"], H, D, V)
-        if 0 < room <= ops.CHUNK_SCRATCH:
+            room = self._chunk_room(ctx)
+        if room:
             # long portions of bfloat16 models: chunks on the tensor cores, from the product's rows as they are
             if low:
                 ops.linattn_decay(fused, parts, col0 + self.off_low, self.w_up, self.b_up, H, D, decay, tau=self.tau)
@@ -154,6 +154,17 @@ class LinearAttention:
         gated = ctx.buffer(self.tag + "la_gated", (n, H * V), self.model_dtype)
         ops.head_gate_norm(o, fused, parts, col0 + self.off_g, self.norm_weight, self.eps, gated, H, V)
         return as_branch(ops.project(gated, self.wo, lambda name, shape, dt: ctx.buffer(self.tag + "la_out_" + name, shape, dt)))
+
+    def _chunk_room(self, ctx) -> int:
+        """Bytes of scratch of the step's chunks, 0 where it is walked; worked out once a step."""
+        host = getattr(ctx, "host", None)
+        if host is None:
+            return 0
+        rank = self.rank if self.decay_kind == "low_rank" else 0
+        key = ("linattn_chunks", self.heads, self.dim, self.vdim, rank)
+        if key not in ctx.memo:
+            ctx.memo[key] = ops.linattn_chunks_pay(host["req_q_len"], self.heads, self.dim, self.vdim, rank)
+        return ctx.memo[key]
 
     def _walk(self, fused, parts: int, offsets, turn: dict, decay, state, o, ctx, col0: int) -> None:
         """The recurrence token by token, from 32-bit inputs."""
