@@ -47,3 +47,17 @@ def test_turns_are_those_that_the_scratch_leaves():
     room, turns = plan([64 * 200])              # 512 MB at once
     assert turns == 4 and room == 50 * 2560000
     assert plan([2048] + [20] * 90) == (91 * 2560000, 32)
+
+
+# (heads, lens, whether chunks were the faster way on the device)
+@pytest.mark.parametrize("heads,lens,chunks", [
+    (16, [2048], True), (16, [512], True), (16, [1021, 680, 340], True), (16, [1531] + [1] * 24, True), (16, [256], False), (16, [130] * 16, False),
+    (16, [512] + [20] * 100, False), (16, [256] + [1] * 47, False), (2, [384], True), (2, [130] * 16, False), (4, [300] * 4, False), (4, [512] * 16, True),
+    (8, [384], True), (8, [256], False), (8, [512] + [20] * 100, False), (32, [2048], True), (32, [512], True), (32, [1021, 680, 340], False),
+    (32, [300] * 4, False), (32, [512] * 16, False), (64, [2048], True), (64, [1021, 680, 340], False), (64, [300] * 4, False)])
+def test_the_delta_rule_goes_in_chunks_where_they_are_faster(heads, lens, chunks):
+    from wllm_b200.kernels import ops
+    from wllm_b200.parts.linear_attention import DeltaRule
+    mixer, ctx = DeltaRule.__new__(DeltaRule), _ctx(lens)
+    mixer.heads, mixer.dim, mixer.vdim, mixer.model_dtype = heads, 128, 128, torch.bfloat16
+    assert mixer._chunk_room(ctx) == (ops.delta_chunks_bytes(ctx.host["req_q_len"], heads) if chunks else 0)

@@ -685,12 +685,17 @@ static int dc_turn(const int* lens, int requests, int H, long long most, long lo
 }
 
 // Bytes of scratch that wllm_delta_chunks asks for: 5.6 MB a chunk of 16 heads, at most 192 MB (longer steps go in turns, the state handed on through its slot:
-// the same bits) but a chunk of every request that goes in chunks.  lens: the requests' tokens, on the host.
+// the same bits) but a chunk of every request that goes in chunks.  lens: the requests' tokens, on the host.  turns: how many with that.
 constexpr long long DC_SCRATCH = 192ll << 20;
-WLLM_API long long wllm_delta_chunks_bytes(const int* lens, int requests, int H) {
+WLLM_API long long wllm_delta_chunks_bytes(const int* lens, int requests, int H, int* turns) {
+    *turns = 0;
     if (H <= 0 || H > 65535 || requests <= 0) return 0;
     long long chunks;
-    dc_turn(lens, requests, H, DC_SCRATCH, chunks);
+    const int turn = dc_turn(lens, requests, H, DC_SCRATCH, chunks);
+    for (int r = 0; r < requests; ++r) {
+        const int mine = turn > 0 ? (lc_chunks(lens[r]) + turn - 1) / turn : 0;
+        *turns = mine > *turns ? mine : *turns;
+    }
     return chunks * H * DC_SIZE;
 }
 

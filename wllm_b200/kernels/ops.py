@@ -1413,11 +1413,39 @@ def delta_scan(q, k, v, beta, decay, state, out, req_q_start, req_q_len, req_slo
 DELTA_CHUNK_MIN = 16        # the shortest requests that delta_chunks takes in chunks
 
 
-def delta_chunks_bytes(lens, heads: int) -> int:
-    """Bytes of scratch that delta_chunks asks for; `lens`: the requests' tokens (int32 array on the host)."""
+def delta_chunks_plan(lens, heads: int) -> tuple:
+    """(bytes of scratch that delta_chunks asks for, turns that it takes with them); `lens`: the requests' tokens (int32 array on the host)."""
     lib = load_family("delta_rule_chunks")
     lib.wllm_delta_chunks_bytes.restype = ctypes.c_longlong
-    return int(lib.wllm_delta_chunks_bytes(c_void_p(lens.ctypes.data), len(lens), heads))
+    turns = ctypes.c_int(0)
+    return int(lib.wllm_delta_chunks_bytes(c_void_p(lens.ctypes.data), len(lens), heads, ctypes.byref(turns))), turns.value
+
+
+def delta_chunks_bytes(lens, heads: int) -> int:
+    return delta_chunks_plan(lens, heads)[0]
+
+
+def delta_chunks_pay(lens, heads: int) -> int:
+    """Bytes of scratch of delta_chunks where it is the faster way for a step of these requests, else 0 (the walk in blocks of eight tokens).
+
+    Both ways' us, fitted to B200 measurements with 2 to 64 heads (in brackets blocks and chunks).  Blocks have eight CTAs a request and head, two an SM, each a chain:
+    0.133 a token where one has an SM to itself, 0.225 where two share it, and so many SMs for all tokens.  Chunks have a chain of their own, 2.85 a chunk, and cost
+    by heads and chunks, full or not; a turn brings every request's states once more, and shorter requests are walked in front
+    of them, not beside.  16 heads: 2,048 tokens [274, 195], 512 [73, 59], 384 [57, 54], 256 [42, 47],
+    1,021 + 680 + 340 [240, 203], 1,531 beside 24 single ones [244, 188], 16 x 512 [865, 850], 4 x 300 [147, 134], 16 x 130 [248, 338], 512 beside 100 of 20
+    [433, 1,122].  4 heads: 256 [39, 39], 4 x 300 [48, 52], 16 x 130 [74, 92].  32 heads: 2,048 [458, 388], 512 [121, 108], 1,021 + 680 + 340 [434, 456],
+    4 x 300 [259, 269], 16 x 512 [1,856, 1,919].  64 heads: 2,048 [922, 792], 1,021 + 680 + 340 [895, 943], 4 x 300 [507, 549]."""
+    room, turns = delta_chunks_plan(lens, heads)
+    if room <= 0 or room > CHUNK_SCRATCH:
+        return 0
+    long = lens[lens >= DELTA_CHUNK_MIN]
+    chunks = (long + 63) // 64
+    longest, tokens, requests = int(long.max()), int(long.sum()), len(long)
+    shared = 8 * heads * requests > sm_count()
+    in_blocks = 8 + max((0.225 * -(-8 * heads // (2 * sm_count())) if shared else 0.133) * longest, 0.0069 * heads * tokens)
+    few = int(((lens > 0) & (lens < DELTA_CHUNK_MIN)).sum())
+    in_chunks = max(23 + min(11, 1.4 * heads) + 2.85 * int(chunks.max()), 20 + 0.36 * heads * int(chunks.sum()) + 0.07 * heads * requests * turns) + 12 * (turns - 1) + 0.015 * heads * few
+    return room if in_chunks < in_blocks else 0
 
 
 def delta_chunks(q, k, v, beta, decay, state, out, req_q_start, req_q_len, req_slot, lens, heads: int, kv_heads: int, channel: bool, scratch: torch.Tensor):

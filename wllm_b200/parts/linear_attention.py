@@ -266,11 +266,7 @@ class DeltaRule:
     # The shortest request that takes part: many short ones fill the device either way (64 of 20 tokens 230 us by the walk, 292 in blocks; 32 of 40 194
     # and 195, per channel 233 and 200; 16 of 64 144 and 136, 176 and 137).
     REQUEST_FROM = 40
-    # Where heads of 128 by 128 go in chunks of 64 tokens instead: the walk in blocks costs some 0.12 us a token of 16 heads, chunks some 6.2 us each, full or
-    # not, and 11 us more to begin with, so that their requests' tokens must be at least 52 a chunk and 90 more.  us in blocks and in chunks: 2,048 tokens 277 and 201,
-    # 512 75 and 62, 384 59 and 57, 256 44 and 51, 128 27 and 37; 3 x 1,021 370 and 319, 1,531 beside 24 single tokens 247 and 191, 4 x 300 150 and 140,
-    # 16 x 512 871 and 866, 16 x 130 251 and 345, 512 beside 100 of 20 593 and 1,127, 256 beside 47 single tokens 107 and 124.
-    CHUNKS_FROM, CHUNK_TOKENS, CHUNK_START = 128, 52, 90
+    CHUNKS_FROM = 128        # the longest request from which on heads of 128 by 128 may go in chunks of 64 tokens instead (ops.delta_chunks_pay says where they do)
 
     def __init__(self, spec, hidden_size: int, model_dtype: torch.dtype):
         self.heads, self.kv_heads = int(spec.num_heads), int(spec.num_kv_heads)
@@ -372,11 +368,7 @@ class DeltaRule:
             return 0
         key = ("delta_chunks", self.heads)
         if key not in ctx.memo:
-            lens = host["req_q_len"]
-            long = lens[lens >= ops.DELTA_CHUNK_MIN]
-            pays = int(long.sum()) >= self.CHUNK_TOKENS * int(((long + 63) // 64).sum()) + self.CHUNK_START
-            room = ops.delta_chunks_bytes(lens, self.heads) if pays else 0
-            ctx.memo[key] = room if room <= ops.CHUNK_SCRATCH else 0
+            ctx.memo[key] = ops.delta_chunks_pay(host["req_q_len"], self.heads)
         return ctx.memo[key]
 
     def mix(self, fused: torch.Tensor, parts: int, col0: int, ctx, cache: CacheRef):
