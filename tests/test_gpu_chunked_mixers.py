@@ -112,7 +112,7 @@ def test_steps_in_chunks_are_no_further_from_64_bits_than_walked_ones(name, monk
 
 # tokens at the edges of the 64 that a CTA takes; ranks that are no steps of 16, channels that are no steps of 128; too few tokens for the tensor cores
 @pytest.mark.parametrize("n", [63, 64, 65, 200])
-@pytest.mark.parametrize("heads,dim,rank,tau", [(2, 64, 8, 4.0), (3, 40, 24, 1.0), (5, 64, 72, 16.0), (8, 128, 64, 16.0)])
+@pytest.mark.parametrize("heads,dim,rank,tau", [(2, 64, 8, 4.0), (3, 40, 24, 1.0), (5, 64, 72, 16.0), (8, 128, 64, 16.0), (8, 128, 256, 16.0)])
 def test_the_decay_of_linear_attention_alone(n, heads, dim, rank, tau):
     from wllm_b200.kernels import ops
     gen = torch.Generator().manual_seed(n + rank)
@@ -128,8 +128,8 @@ def test_the_decay_of_linear_attention_alone(n, heads, dim, rank, tau):
     ops.linattn_prepare(wide, 0, 0, HD, 2 * HD, heads, dim, dim, torch.arange(n, dtype=torch.int32, device=DEV), q, k, v, low_off=3 * HD + off, w2=w2, b2=b2, tau=tau,
                         decay=beside)
     far = lambda a: float((a.double() - want.exp()).norm() / want.exp().norm())
-    # a decay of 32 bits is within some roundings of 2^-24; the map's sum of `rank` products carries as much again
-    assert far(alone) <= max(1.5 * far(beside), 2e-7), (far(alone), far(beside))
+    # a decay of 32 bits is within some roundings of 2^-24; the map's sum of `rank` products, in either order, is no further off
+    assert far(alone) <= 1.03 * far(beside), (far(alone), far(beside))
     forgets = want < -0.01                       # where the logarithm tells more than the rounding of the decay itself
     logs = lambda a: float(((a.double().log() - want)[forgets] / want[forgets]).abs().max())
     assert logs(alone) <= max(1.5 * logs(beside), 2e-5), (logs(alone), logs(beside))

@@ -191,8 +191,9 @@ linattn_prepare_kernel(const void* __restrict__ fused, int in_dtype, int row_str
     }
 }
 
-// The low-rank maps for many tokens, bfloat16 maps, on the tensor cores (mma.sync); form 0 of bfloat16 rows alone, whose high pieces are all there is (2,048
-// tokens of rank 64, 1,024 channels: 14 us, 23 on the FMA pipes).  A CTA takes 64 tokens, whose low-rank rows (form 1: through tanh) it holds in shared memory as a high and a low bfloat16 piece each (together some sixteen bits), and walks tiles of 128
+// The low-rank maps for many tokens, bfloat16 maps, on the tensor cores (mma.sync).  A CTA takes 64 tokens, whose low-rank rows (form 1: through tanh) it holds in
+// shared memory as a high and a low bfloat16 piece each (together some sixteen bits); of form 0, which takes bfloat16 rows alone, the high pieces are all there is
+// (2,048 tokens of rank 64, 1,024 channels: 14 us, 23 on the FMA pipes; distance from 64 bits 3.4e-8 both, rank 256 3.7e-8 and 3.9e-8).  It walks tiles of 128
 // channels; 2 x 4 warps, 32 tokens by 32 channels each.  grid (CTAs that share the channels' tiles, tiles of tokens), 256 threads.
 constexpr int DEC_TM = 64, DEC_TN = 128, DEC_MAX_RANK = 256;
 
@@ -225,7 +226,7 @@ linattn_decay_mma_kernel(const void* __restrict__ low, int in_dtype, int row_str
         if (FORM == 1) v = tanhf(v);
         const bf16 h = __float2bfloat16_rn(v);
         hi[tt * pitch + r] = h;
-        lo[tt * pitch + r] = __float2bfloat16_rn(v - __bfloat162float(h));
+        if (FORM != 0) lo[tt * pitch + r] = __float2bfloat16_rn(v - __bfloat162float(h));
     }
     const int tiles = (HD + DEC_TN - 1) / DEC_TN;
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
@@ -247,7 +248,7 @@ linattn_decay_mma_kernel(const void* __restrict__ low, int in_dtype, int row_str
             for (int mi = 0; mi < 2; ++mi) {
                 const int at = (wm * 32 + mi * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * pitch + k + (lane >> 4) * 8;
                 dec_ldsm4(hi + at, ah[mi]);
-                dec_ldsm4(lo + at, al[mi]);
+                if (FORM != 0) dec_ldsm4(lo + at, al[mi]);
             }
 #pragma unroll
             for (int nj = 0; nj < 2; ++nj)
@@ -256,6 +257,17 @@ linattn_decay_mma_kernel(const void* __restrict__ low, int in_dtype, int row_str
             for (int mi = 0; mi < 2; ++mi)
 #pragma unroll
                 for (int nj = 0; nj < 2; ++nj) {
+                    if (FORM == 0) {                     // sixteen products a sum, and the sums added up with a rounding each
+                        float part[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+                        dec_mma(part[0], ah[mi], bw[nj][0], bw[nj][1]);
+                        dec_mma(part[1], ah[mi], bw[nj][2], bw[nj][3]);
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            acc[mi][2 * nj][e] += part[0][e];
+                            acc[mi][2 * nj + 1][e] += part[1][e];
+                        }
+                        continue;
+                    }
                     dec_mma(acc[mi][2 * nj], al[mi], bw[nj][0], bw[nj][1]);
                     dec_mma(acc[mi][2 * nj + 1], al[mi], bw[nj][2], bw[nj][3]);
                     dec_mma(acc[mi][2 * nj], ah[mi], bw[nj][0], bw[nj][1]);
