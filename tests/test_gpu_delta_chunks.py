@@ -108,3 +108,28 @@ def test_which_steps_go_in_chunks(lens, chunks):
     assert rule._chunk_room(ctx()) == 0
     rule.model_dtype, rule.vdim = torch.bfloat16, 64
     assert rule._chunk_room(ctx()) == 0
+
+
+@pytest.mark.parametrize("channel", [False, True])
+def test_chunks_are_no_further_from_64_bits_than_the_walks(channel):
+    """Decays as such models are initialised and stay: rates A softplus(a + bias), A of 1 to 16, steps of 1e-3 to 1e-1."""
+    lens, H, far = [700, 130], 3, {}
+    for seed in range(3):
+        gen = torch.Generator().manual_seed(seed)
+        q, k, v, beta, _, state, slots = _case(lens, H, H, "long", channel, 20 + seed)
+        width = D if channel else 1
+        A, step = 1 + 15 * torch.rand(H, 1, generator=gen), 1e-3 * 100.0 ** torch.rand(H, width, generator=gen)
+        rate = (A * torch.nn.functional.softplus(0.9 * torch.randn(sum(lens), H, width, generator=gen) + step + torch.log(-torch.expm1(-step)))).double()
+        decay = (torch.expm1(-rate) if channel else torch.exp(-rate)[..., 0]).float()
+        g = (1 + decay.double()) if channel else decay.double()[..., None]
+        want, want_o = state.double().clone(), torch.zeros(sum(lens), H, D, dtype=torch.float64)
+        for m, slot, s0 in zip(lens, slots, (0, lens[0])):
+            part = slice(s0, s0 + m)
+            want_o[part], want[slot] = _plain(q[part].double(), k[part].double(), v[part].double(), beta[part].double(), g[part], state[slot].double())
+        for way in ("walk", "blocks", "chunks"):
+            o, S = _run(way, lens, H, H, channel, q, k, v, beta, decay, state, slots)
+            a, b = far.get(way, (0.0, 0.0))
+            far[way] = a + float((o.double() - want_o).norm() / want_o.norm()) / 3, b + float((S.double() - want)[slots].norm() / want[slots].norm()) / 3
+    # (three drawings; a hundredth or two between them)
+    for i in range(2):
+        assert far["chunks"][i] <= 1.02 * max(far["walk"][i], far["blocks"][i]), far

@@ -13,6 +13,13 @@ __device__ __forceinline__ void lc_mma(float (&c)[4], const uint4& a, uint32_t b
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b0), "r"(b1));
 }
+// A product of its own, added with a rounding: the tensor cores cut off what they add to a sum that is there, and cuts all go one way.
+__device__ __forceinline__ void lc_mma_add(float (&sum)[4], const uint4& a, uint32_t b0, uint32_t b1) {
+    float c[4] = {0.f, 0.f, 0.f, 0.f};
+    lc_mma(c, a, b0, b1);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) sum[i] += c[i];
+}
 __device__ __forceinline__ float2 lc_mul2(float2 a, float2 b) {         // two products an instruction
     unsigned long long d;
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)));

@@ -32,13 +32,6 @@ constexpr int DP_THREADS = 256, DW_THREADS = 512, DO_THREADS = 256;       // of 
 constexpr long long DC_OP = 4ll * 8 * 3 * 512, DC_Q = 0, DC_K = DC_OP, DC_W = 2 * DC_OP, DC_P = 3 * DC_OP, DC_G = DC_P + 4 * 4 * 3 * 512, DC_U = DC_G + DC * 4,
                     DC_S = DC_U + (long long)LC * DCV * 4, DC_R = DC_S + 3ll * DC * DCV * 2, DC_SIZE = DC_R + 3ll * LC * DCV * 2;
 
-__device__ __forceinline__ float2 dc_fma2(float2 a, float2 b, float2 c) {
-    unsigned long long d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)),
-        "l"(*reinterpret_cast<unsigned long long*>(&c)));
-    return *reinterpret_cast<float2*>(&d);
-}
-
 struct DeltaPrepareSmem {
     // (pitches: X is read as pairs along its rows, eight rows a warp; K down its columns too)
     static constexpr int XP = DC + 8, DP = DC + 4, AP = LC + 4, PAIRS = LB * (LB + 1) / 2;
@@ -84,7 +77,7 @@ __device__ __forceinline__ void delta_chunk_prepare(const float* __restrict__ q,
                 else e[u][i].x = e[u][i].y = decay[(size_t)(first + t) * H + h];
             }
         }
-    auto fade = [](float2 x, float2 d) { return CHANNEL ? dc_fma2(x, d, x) : lc_mul2(x, d); };
+    auto fade = [](float2 x, float2 d) { return CHANNEL ? fma2(x, d, x) : lc_mul2(x, d); };
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
 #pragma unroll
@@ -107,10 +100,10 @@ __device__ __forceinline__ void delta_chunk_prepare(const float* __restrict__ q,
             for (int i = j; i < LB; ++i) {
                 if (i > j) w = fade(w, e[u][i]);
                 else if (KEYS) continue;
-                const float2 y = lc_mul2(xx[i], w);
+                const float y = fmaf(xx[i].x, w.x, xx[i].y * w.y);
                 const int at = KEYS ? i * (i - 1) / 2 + j : i * (i + 1) / 2 + j;
-                if (at < 32) x[at & 31] = y.x + y.y;
-                else more[at & 3] = y.x + y.y;
+                if (at < 32) x[at & 31] = y;
+                else more[at & 3] = y;
             }
             *reinterpret_cast<float2*>(&sm.K[B * LB + j][c2]) = w;
         }
@@ -229,7 +222,7 @@ __device__ __forceinline__ void delta_chunk_prepare(const float* __restrict__ q,
                 lc_mma(small[u], a[1], b[1][0], b[1][1]);
                 lc_mma(small[u], a[0], b[1][0], b[1][1]);
                 lc_mma(small[u], a[1], b[0][0], b[0][1]);
-                lc_mma(big[u], a[0], b[0][0], b[0][1]);
+                lc_mma_add(big[u], a[0], b[0][0], b[0][1]);
             }
         }
 #pragma unroll
@@ -271,14 +264,17 @@ __device__ __forceinline__ void delta_chunk_prepare(const float* __restrict__ q,
         const int pitch = values ? Smem::DP : Smem::XP;
         float* to = reinterpret_cast<float*>(mine + DC_U) + column;
         for (int I = 0; I < 4; ++I) {
-            float x[16];
+            // (what the tokens in front take away is summed for itself, small beside what it is taken from, and taken away in one rounding)
+            float x[16], own[16];
 #pragma unroll
-            for (int i = 0; i < 16; ++i)
-                x[i] = sm.beta[16 * I + i] * (values ? ahead[i] : X[(16 * I + i) * pitch] * sm.before[2 * I + (i >> 3)][column]);
+            for (int i = 0; i < 16; ++i) {
+                x[i] = 0.f;
+                own[i] = values ? ahead[i] : X[(16 * I + i) * pitch] * sm.before[2 * I + (i >> 3)][column];
+            }
             if (values && I < 3) look(I + 1);
 #pragma unroll 4
             for (int s = 0; s < 16 * I; ++s) {
-                const float y = -X[s * pitch];
+                const float y = X[s * pitch];
                 const float4* l = reinterpret_cast<const float4*>(&sm.A[s][16 * I]);
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
@@ -290,8 +286,9 @@ __device__ __forceinline__ void delta_chunk_prepare(const float* __restrict__ q,
                 }
             }
 #pragma unroll
-            for (int j = 0; j < 15; ++j) {
-                const float y = -x[j];
+            for (int j = 0; j < 16; ++j) {
+                const float y = x[j] = fmaf(sm.beta[16 * I + j], own[j], -x[j]);
+                if (j == 15) break;
                 const float4* l = reinterpret_cast<const float4*>(&sm.A[16 * I + j][16 * I]);
 #pragma unroll
                 for (int i = (j + 1) / 4; i < 4; ++i) {
@@ -459,7 +456,10 @@ delta_chunk_walk_kernel(float* __restrict__ state, const int* __restrict__ req_q
 #pragma unroll
                 for (int i = 2 - p; i >= 0; --i)
 #pragma unroll
-                    for (int j = 0; j < 2; ++j) lc_mma(p + i == 0 ? big[j] : small[ks][j], a[i], b[2 * j], b[2 * j + 1]);
+                    for (int j = 0; j < 2; ++j) {
+                        if (p + i == 0) lc_mma_add(big[j], a[i], b[2 * j], b[2 * j + 1]);
+                        else lc_mma(small[ks][j], a[i], b[2 * j], b[2 * j + 1]);
+                    }
             }
         }
 #pragma unroll
@@ -597,7 +597,10 @@ delta_chunk_out_kernel(float* __restrict__ out, const int* __restrict__ req_q_st
 #pragma unroll
                 for (int i = 2 - p; i >= 0; --i)
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) lc_mma(p + i == 0 ? big[j] : small[j], now[i], b[j >> 1][2 * (j & 1)], b[j >> 1][2 * (j & 1) + 1]);
+                    for (int j = 0; j < 4; ++j) {
+                        if (p + i == 0) lc_mma_add(big[j], now[i], b[j >> 1][2 * (j & 1)], b[j >> 1][2 * (j & 1) + 1]);
+                        else lc_mma(small[j], now[i], b[j >> 1][2 * (j & 1)], b[j >> 1][2 * (j & 1) + 1]);
+                    }
             }
         }
     }
@@ -631,7 +634,10 @@ delta_chunk_out_kernel(float* __restrict__ out, const int* __restrict__ req_q_st
 #pragma unroll
                 for (int i = 2 - p; i >= 0; --i)
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) lc_mma(p + i == 0 ? own[j] : small[j], now[i], b[j >> 1][2 * (j & 1)], b[j >> 1][2 * (j & 1) + 1]);
+                    for (int j = 0; j < 4; ++j) {
+                        if (p + i == 0) lc_mma_add(own[j], now[i], b[j >> 1][2 * (j & 1)], b[j >> 1][2 * (j & 1) + 1]);
+                        else lc_mma(small[j], now[i], b[j >> 1][2 * (j & 1)], b[j >> 1][2 * (j & 1) + 1]);
+                    }
             }
         }
     } else {
@@ -664,8 +670,8 @@ delta_chunk_out_kernel(float* __restrict__ out, const int* __restrict__ req_q_st
         float* to = out + ((size_t)(first + t) * H + h) * DCV + v0 + wn * 32 + fcol;
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-            *reinterpret_cast<float2*>(to + j * 8) = make_float2(big[j][half * 2] + own[j][half * 2] + small[j][half * 2],
-                                                                 big[j][half * 2 + 1] + own[j][half * 2 + 1] + small[j][half * 2 + 1]);
+            *reinterpret_cast<float2*>(to + j * 8) = make_float2(own[j][half * 2] + (big[j][half * 2] + small[j][half * 2]),
+                                                                 own[j][half * 2 + 1] + (big[j][half * 2 + 1] + small[j][half * 2 + 1]));
     }
 }
 

@@ -181,10 +181,10 @@ linattn_chunk_prepare_kernel(const bf16* __restrict__ fused, int row_stride, int
 #pragma unroll
             for (int i = j; i < LB; ++i) {
                 if (i > j) w = lc_mul2(w, e[u][i]);
-                const float2 y = lc_mul2(qq[i], w);
+                const float y = fmaf(qq[i].x, w.x, qq[i].y * w.y);
                 const int at = i * (i + 1) / 2 + j;
-                if (at < 32) x[at & 31] = y.x + y.y;
-                else more[at & 3] = y.x + y.y;
+                if (at < 32) x[at & 31] = y;
+                else more[at & 3] = y;
             }
             *reinterpret_cast<float2*>(&sm.K[B * LB + j][c2]) = w;
         }
@@ -611,8 +611,8 @@ linattn_chunk_out_kernel(const bf16* __restrict__ v, int row_stride, float* __re
         float* to = out + ((size_t)(first + t) * H + h) * V + v0 + wn * 32 + fcol;
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-            *reinterpret_cast<float2*>(to + j * 8) = make_float2(big[j][half * 2] + own[j][half * 2] + small[j][half * 2],
-                                                                 big[j][half * 2 + 1] + own[j][half * 2 + 1] + small[j][half * 2 + 1]);
+            *reinterpret_cast<float2*>(to + j * 8) = make_float2(own[j][half * 2] + (big[j][half * 2] + small[j][half * 2]),
+                                                                 own[j][half * 2 + 1] + (big[j][half * 2 + 1] + small[j][half * 2 + 1]));
     }
 }
 
