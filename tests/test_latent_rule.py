@@ -42,3 +42,26 @@ def test_only_whole_prompts_do():
 
 def test_keys_behind_a_window_are_no_gain():
     assert _mixer(16, 128, 512, window=64)._expansion_worth(np.array([4096])) < _mixer(16, 128, 512)._expansion_worth(np.array([4096])) / 4
+
+
+@pytest.mark.parametrize("rot", [0, 16])
+def test_the_values_maps_are_held_once(rot):
+    """Where every head's keys and values are made by one matrix, the maps of the values alone are its second half."""
+    import torch
+
+    from wllm_b200.config import resolve_architecture
+    from wllm_b200.engine import ComposedModel
+    layer = {"type": "latent_attention", "mlp": {"kind": "dense", "ff": 32}, "mixer": {"heads": 2, "dim": 64, "vdim": 64, "kv_rank": 24, "q_rank": 16, "scale": 0.1}}
+    raw = {"architecture": "Gudarax", "vocab": 31, "width": 32, "max_positions": 64, "norm": {"eps": 1e-6}, "embedding": {"scale": 1.0}, "token_side": {"dim": 8},
+           "layers": [layer]}
+    arch = resolve_architecture("Gudarax")
+    model = ComposedModel(arch.make_plan(arch.config_class.from_dict(raw, where="test")), torch.bfloat16)
+    weights = {p.name: torch.randn(tuple(p.shape)).bfloat16() for p in model.param_specs()}
+    mixer = model.blocks[0].mixer
+    mixer.rot = rot                       # (with a turned part nothing is expanded)
+    mixer.load(weights.__getitem__)
+    up_k, up_v = weights[mixer.names["up_k"]], weights[mixer.names["up_v"]]
+    assert torch.equal(mixer.w_uv.flatten(0, 1), up_v) and torch.equal(mixer.w_uk_t, up_k.view(2, 64, 24).transpose(1, 2))
+    assert (mixer.w_ukv is None) == (rot > 0)
+    if rot == 0:
+        assert torch.equal(mixer.w_ukv, torch.cat([up_k, up_v])) and mixer.w_uv.untyped_storage().data_ptr() == mixer.w_ukv.untyped_storage().data_ptr()

@@ -96,9 +96,10 @@ class LatentAttention:
         # up_k head by head, transposed: [heads, kv_rank, plain_dim], so that the queries' map is x W^T like every product
         up_k, up_v = fetch(n["up_k"]), fetch(n["up_v"])
         self.w_uk_t = up_k.view(self.heads, self.dim, self.rank).transpose(1, 2).contiguous()
-        self.w_uv = up_v.view(self.heads, self.vd, self.rank).contiguous()
         if self.model_dtype == torch.bfloat16 and self._expandable():
             self.w_ukv = torch.cat([up_k, up_v], dim=0).contiguous()
+            up_v = self.w_ukv[self.heads * self.dim:]                # one copy of the values' maps, in either form
+        self.w_uv = up_v.view(self.heads, self.vd, self.rank).contiguous()
         self.wo = fetch(n["o_proj"]).contiguous()
         self.position.to(self.wo.device)
 
