@@ -92,6 +92,27 @@ def test_a_value_that_is_no_number_stays_with_its_column_and_later_tokens(channe
         assert bool(o[64:70, 1].isfinite().all()) and float((o[64:, 1][:, other] - want[0][64:, 1][:, other]).abs().max()) < 1e-5
 
 
+# a block's first token, inside a tile of sixteen, a chunk's first, the last of a partly filled chunk
+@pytest.mark.parametrize("at", [72, 85, 64, 149])
+@pytest.mark.parametrize("bad", ["v", "k", "q", "beta", "decay"])
+@pytest.mark.parametrize("what", [float("inf"), float("nan")])
+@pytest.mark.parametrize("channel", [False, True])
+def test_what_is_no_number_reaches_no_earlier_token(at, bad, what, channel):
+    lens, H = [150], 2
+    case = dict(zip(("q", "k", "v", "beta", "decay", "state", "slots"), _case(lens, H, 2, "long", channel, 7)))
+    run = lambda way: _run(way, lens, H, 2, channel, *case.values())
+    clean_o, clean_S = run("chunks")
+    case[bad] = case[bad].clone()
+    case[bad][(at, 0, 9) if case[bad].dim() == 3 else (at, 0)] = what
+    (o, S), (walk_o, walk_S) = run("chunks"), run("walk")
+    slot, chunk = case["slots"][0], at - at % 64
+    assert torch.equal(o[:chunk], clean_o[:chunk]) and torch.equal(o[:, 1], clean_o[:, 1]) and torch.equal(S[slot, 1], clean_S[slot, 1])
+    # (the chunk's earlier tokens are added up one by one then: up to 64 sums of numbers of the outputs' size, each rounded at 2^-24)
+    assert float((o[chunk:at] - clean_o[chunk:at]).abs().max() if at > chunk else 0.0) < 1e-5
+    assert bool(o.isfinite()[walk_o.isfinite()].all()) and bool(S.isfinite()[walk_S.isfinite()].all())
+    assert not bool(o[at, 0].isfinite().all())
+
+
 # (lens, whether the chunks pay): full chunks, mostly empty ones, a portion beside single tokens, too short
 @pytest.mark.parametrize("lens,chunks", [([2048], True), ([704, 20], True), ([512] + [20] * 30, False), ([1531] + [1] * 24, True), ([127], False), ([130], False)])
 def test_which_steps_go_in_chunks(lens, chunks):
