@@ -1,4 +1,5 @@
-"""32-bit products of more than 64 rows: tile edges, segments' ends, both ways of adding the segments, beside the same rows in smaller products."""
+"""32-bit products of more than 32 rows: tile edges, segments' ends, tiles of 64 and 128 rows whose CTAs walk their segments or that are cut by them, beside the same
+rows in smaller products."""
 from __future__ import annotations
 
 import math
@@ -11,8 +12,7 @@ pytestmark = pytest.mark.gpu
 
 
 # rows and columns one past, at and one short of a tile; K within a stage, of one segment, one group past it, of several, its last one short;
-# (M, N) of few tiles, whose segments have CTAs of their own (also where they fill more than a round), of very many, whose segments one CTA of the wide kernel
-# walks, and between, where the tile kernel's do
+# (M, N) of few tiles, whose segments have CTAs of their own (tiles of 64 rows; the sixth and eighth of 128), and of more, of 128 rows, whose CTAs walk them
 @pytest.mark.parametrize("M,N,K", [(65, 1, 4), (127, 129, 1024), (128, 128, 1028), (129, 255, 2048), (300, 130, 5000), (1100, 8501, 1060), (1030, 8320, 3076),
                                    (1030, 5300, 2052), (2100, 15801, 1060)])
 def test_every_row_has_the_bits_of_a_smaller_product(M, N, K):
@@ -28,8 +28,8 @@ def test_every_row_has_the_bits_of_a_smaller_product(M, N, K):
         assert torch.equal(ops.gemm_f32(a[rows], w), out[rows, :N])
 
 
-# K of 3 to 5 segments; the last one short; two and more turns, the last of one segment
-@pytest.mark.parametrize("M,N,K", [(65, 130, 2060), (300, 129, 5120), (130, 256, 4100)])
+# K of 3 to 5 segments; the last one short; two and more turns, the last of one segment; tiles of 64 rows, and of 128 (the last)
+@pytest.mark.parametrize("M,N,K", [(65, 130, 2060), (300, 129, 5120), (130, 256, 4100), (1400, 2050, 4100)])
 def test_less_scratch_gives_the_same_bits(M, N, K, monkeypatch):
     """Room for every slab, for four, three and two, for one and for none; memory that runs out on the way; operands that lie across 16 bytes ask for none."""
     import ctypes
