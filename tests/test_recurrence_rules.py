@@ -28,7 +28,7 @@ def _linear(heads, dim, vdim, rank):
     ((8, 128, 256, 0), [2048], True), ((8, 128, 256, 0), [130] + [40] * 16, False), ((8, 128, 256, 0), [512] + [20] * 90, False),
     ((4, 64, 64, 64), [130] + [20] * 90, True), ((4, 64, 64, 64), [2048] + [20] * 200, True),
     ((16, 64, 128, 64), [130] + [20] * 90, False), ((16, 64, 128, 64), [2048] + [20] * 90, True), ((16, 64, 128, 64), [2048] + [20] * 200, False),
-    ((32, 128, 128, 64), [2048], True), ((32, 128, 128, 64), [512] * 4, True), ((32, 128, 128, 64), [130] + [20] * 20, False), ((32, 128, 128, 64), [512] + [20] * 40, False)])
+    ((32, 128, 128, 64), [2048], True), ((32, 128, 128, 64), [130] * 16, False), ((32, 128, 128, 64), [512] * 4, True), ((32, 128, 128, 64), [130] + [20] * 20, False), ((32, 128, 128, 64), [512] + [20] * 40, False)])
 def test_linear_attention_goes_in_chunks_where_they_are_faster(sizes, lens, chunks):
     from wllm_b200.kernels import ops
     mixer, ctx = _linear(*sizes), _ctx(lens)

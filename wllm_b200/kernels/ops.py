@@ -1196,7 +1196,9 @@ def linattn_chunks_pay(lens, heads: int, dim: int, vdim: int, rank: int) -> int:
     tokens, size = int(lens.sum()), heads * dim * vdim / 2.0 ** 18
     unit = heads * (772 * dim + 24576 + 6 * dim * vdim) / 2.56e6
     in_chunks = 22 + max(1.05 * int(chunks.max()), 2.0 * unit * int(chunks.sum()) + 1.6 * size * len(chunks)) + 45 * (turns - 1)
-    walked = max(8 + 0.3 * longest + 0.025 * size * (tokens - longest), 0.07 * size * tokens) + (5 + 0.02 * heads * dim * rank / 65536 * tokens if rank else 0)
+    walked = max(8 + (0.25 + 0.05 * size) * longest + 0.025 * size * (tokens - longest), 0.07 * size * tokens)
+    if rank:
+        walked += 5 + (0.006 + 0.014 * heads * dim * rank / 65536) * tokens
     return room if in_chunks < walked else 0
 
 
