@@ -493,23 +493,28 @@ def pesanex_kernel_table(size: dict, pk: dict, T: int, batch: int, context: int)
         bufs = [torch.empty(n, H * D, device=dev), torch.empty(n, H * D, device=dev), torch.empty(n, H * V, device=dev)]
         decay = torch.empty(n, H * D, device=dev)
         pos = torch.arange(n, dtype=torch.int32, device=dev)
-        row(f"{tag}/recurrence inputs (decay from the low-rank map)",
-            lambda: ops.linattn_prepare(fused, 0, 0, H * D, 2 * H * D, H, D, V, pos, *bufs, q_scale=D ** -0.5,
-                                        low_off=2 * H * D + 2 * H * V, w2=w2, b2=b2, tau=16.0, decay=decay),
-            n * ((2 * H * D + H * V + rank) * 2 + (3 * H * D + H * V) * 4))
         o = torch.empty(n, H * V, device=dev)
-        if R == 1:
-            rs, rl, rslot = one * 0, one * n, one * 0
-            seg_len, max_seg = ops.linattn_segment_plan(n, 1, H, V)
-        else:
-            rs, rl, rslot = starts, lens, starts
-            seg_len, max_seg = 0, 1
-        seg_state = torch.empty(R * max_seg * H * D * V, device=dev)
-        seg_decay = torch.empty(R * max_seg * H * D, device=dev)
+        rs, rl, rslot = (one * 0, one * n, one * 0) if R == 1 else (starts, lens, starts)
         walk_bytes = n * (3 * H * D + 2 * H * V) * 4 + R * 2 * H * D * V * 4
-        row(f"{tag}/recurrence" + (f" ({max_seg} segments of {seg_len})" if max_seg > 1 else ""),
-            lambda: ops.linattn_scan(bufs[0], bufs[1], bufs[2], decay, None, state, o, rs, rl, rslot, H, D, V, seg_len, max_seg,
-                                     seg_state, seg_decay), walk_bytes, 4.0 * n * H * D * V)
+        chunks = _linear_chunks(n, R, H, D, V, rank, dev)
+        if chunks:
+            host, scratch = chunks
+            row(f"{tag}/recurrence: decay from the low-rank map", lambda: ops.linattn_decay(fused, 0, 2 * H * D + 2 * H * V, w2, b2, H, D, decay, tau=16.0),
+                n * (rank * 2 + H * D * 4) + H * D * rank * 2)
+            row(f"{tag}/recurrence in chunks, with its inputs",
+                lambda: ops.linattn_chunks(fused, 0, H * D, 2 * H * D, H, D, V, pos, decay, None, state, o, rs, rl, rslot, host, scratch, q_scale=D ** -0.5),
+                n * ((2 * H * D + H * V) * 2 + (H * D + H * V) * 4) + R * 2 * H * D * V * 4, 4.0 * n * H * D * V)
+        else:
+            row(f"{tag}/recurrence inputs (decay from the low-rank map)",
+                lambda: ops.linattn_prepare(fused, 0, 0, H * D, 2 * H * D, H, D, V, pos, *bufs, q_scale=D ** -0.5,
+                                            low_off=2 * H * D + 2 * H * V, w2=w2, b2=b2, tau=16.0, decay=decay),
+                n * ((2 * H * D + H * V + rank) * 2 + (3 * H * D + H * V) * 4))
+            seg_len, max_seg = ops.linattn_segment_plan(n, 1, H, V) if R == 1 else (0, 1)
+            seg_state = torch.empty(R * max_seg * H * D * V, device=dev)
+            seg_decay = torch.empty(R * max_seg * H * D, device=dev)
+            row(f"{tag}/recurrence" + (f" ({max_seg} segments of {seg_len})" if max_seg > 1 else ""),
+                lambda: ops.linattn_scan(bufs[0], bufs[1], bufs[2], decay, None, state, o, rs, rl, rslot, H, D, V, seg_len, max_seg,
+                                         seg_state, seg_decay), walk_bytes, 4.0 * n * H * D * V)
         gated = torch.empty(n, H * V, dtype=bf, device=dev)
         row(f"{tag}/head norm and gate", lambda: ops.head_gate_norm(o, fused, 0, 2 * H * D + H * V, nw, 1e-6, gated, H, V),
             n * H * V * (4 + 2 + 2))
@@ -962,7 +967,8 @@ GUDARAX_SIZES = {
 
 
 def _delta_rule_options(n: int, lens, heads: int, dim: int, dev) -> tuple:
-    """The options of delta_prepare and delta_scan with which a bfloat16 model's step of one prompt of n tokens, or of n single tokens, runs the delta rule."""
+    """The options of delta_prepare and delta_scan with which a bfloat16 model's step of one prompt of n tokens, or of n single tokens, runs the delta rule
+    where it does not go in chunks (_delta_recurrence)."""
     import torch
 
     from wllm_b200.kernels import ops
@@ -973,6 +979,34 @@ def _delta_rule_options(n: int, lens, heads: int, dim: int, dev) -> tuple:
         return {"shift": None}, {}
     scratch = torch.empty(ops.delta_block_floats(n, 1, heads, dim), device=dev)
     return {"shift": None}, {"blocks": scratch, "max_q_len": n, "walked": 1, "blocks_from": DeltaRule.REQUEST_FROM}
+
+
+def _delta_recurrence(n: int, lens, heads: int, kv_heads: int, dim: int, vdim: int, dev, walk: dict):
+    """The recurrence of such a step: in chunks where the engine takes them, else delta_scan with the options `walk`."""
+    import numpy as np
+    import torch
+
+    from wllm_b200.kernels import ops
+    from wllm_b200.parts.linear_attention import DeltaRule
+    host = np.full(lens.shape[0], n // lens.shape[0], dtype=np.int32)
+    room = ops.delta_chunks_pay(host, heads) if dim == vdim == 128 and int(host.max()) >= DeltaRule.CHUNKS_FROM else 0
+    if not room:
+        return lambda q, k, v, beta, decay, state, out, starts, req_lens, slots, channel=False: ops.delta_scan(
+            q, k, v, beta, decay, state, out, starts, req_lens, slots, heads, kv_heads, dim, vdim, channel, **walk)
+    scratch = torch.empty(room, dtype=torch.uint8, device=dev)
+    return lambda q, k, v, beta, decay, state, out, starts, req_lens, slots, channel=False: ops.delta_chunks(
+        q, k, v, beta, decay, state, out, starts, req_lens, slots, host, heads, kv_heads, channel, scratch)
+
+
+def _linear_chunks(n: int, requests: int, heads: int, dim: int, vdim: int, rank: int, dev):
+    """(lengths on the host, scratch) where a bfloat16 model's step of such requests runs linear attention in chunks, else None."""
+    import numpy as np
+    import torch
+
+    from wllm_b200.kernels import ops
+    host = np.full(requests, n // requests, dtype=np.int32)
+    room = ops.linattn_chunks_pay(host, heads, dim, vdim, rank) if int(host.max()) > ops.LINATTN_CHUNKS_FROM else 0
+    return (host, torch.empty(room, dtype=torch.uint8, device=dev)) if room else None
 
 
 def gudarax_config(size: dict) -> dict:
@@ -1108,21 +1142,29 @@ def gudarax_kernel_table(size: dict, pk: dict, T: int, batch: int, context: int)
         # Pesanex's recurrence with as many query/key heads as value heads (it has no grouped form)
         wide = rnd(n, 2 * dh * dd + 2 * HV, dtype=bf)
         bufs = [torch.empty(n, dh * dd, device=dev), torch.empty(n, dh * dd, device=dev), torch.empty(n, HV, device=dev)]
-        row(f"{tag}/decayed state: inputs (scales, no turn)",
-            lambda: ops.linattn_prepare(wide, 0, 0, dh * dd, 2 * dh * dd, dh, dd, dv, pos, *bufs, q_scale=dd ** -0.5),
-            n * ((2 * dh * dd + HV) * 2 + (2 * dh * dd + HV) * 4))
         state = torch.zeros(batch + 1, dh, dd, dv, device=dev)
         o = torch.empty(n, HV, device=dev)
-        seg_len, max_seg = ops.linattn_segment_plan(n, 1, dh, dv) if R == 1 else (0, 1)
-        seg_state, seg_decay = torch.empty(R * max_seg * dh * dd * dv, device=dev), torch.empty(R * max_seg * dh * dd, device=dev)
-        row(f"{tag}/decayed state: recurrence" + (f" ({max_seg} segments of {seg_len})" if max_seg > 1 else ""),
-            lambda: ops.linattn_scan(bufs[0], bufs[1], bufs[2], None, head_decay, state, o, rs, rl, rslot, dh, dd, dv, seg_len, max_seg, seg_state,
-                                     seg_decay), n * (2 * dh * dd + 2 * HV) * 4 + R * 2 * dh * dd * dv * 4, 4.0 * n * dh * dd * dv)
+        chunks = _linear_chunks(n, R, dh, dd, dv, 0, dev)
+        if chunks:
+            host, scratch = chunks
+            row(f"{tag}/decayed state: recurrence in chunks, with its inputs",
+                lambda: ops.linattn_chunks(wide, 0, dh * dd, 2 * dh * dd, dh, dd, dv, pos, None, head_decay, state, o, rs, rl, rslot, host, scratch, q_scale=dd ** -0.5),
+                n * ((2 * dh * dd + HV) * 2 + HV * 4) + R * 2 * dh * dd * dv * 4, 4.0 * n * dh * dd * dv)
+        else:
+            row(f"{tag}/decayed state: inputs (scales, no turn)",
+                lambda: ops.linattn_prepare(wide, 0, 0, dh * dd, 2 * dh * dd, dh, dd, dv, pos, *bufs, q_scale=dd ** -0.5),
+                n * ((2 * dh * dd + HV) * 2 + (2 * dh * dd + HV) * 4))
+            seg_len, max_seg = ops.linattn_segment_plan(n, 1, dh, dv) if R == 1 else (0, 1)
+            seg_state, seg_decay = torch.empty(R * max_seg * dh * dd * dv, device=dev), torch.empty(R * max_seg * dh * dd, device=dev)
+            row(f"{tag}/decayed state: recurrence" + (f" ({max_seg} segments of {seg_len})" if max_seg > 1 else ""),
+                lambda: ops.linattn_scan(bufs[0], bufs[1], bufs[2], None, head_decay, state, o, rs, rl, rslot, dh, dd, dv, seg_len, max_seg, seg_state,
+                                         seg_decay), n * (2 * dh * dd + 2 * HV) * 4 + R * 2 * dh * dd * dv * 4, 4.0 * n * dh * dd * dv)
         fused = rnd(n, Wd, dtype=bf)
         dq, dk, dvv = torch.empty(n, GD, device=dev), torch.empty(n, GD, device=dev), torch.empty(n, HV, device=dev)
         beta, decay = torch.empty(n, dh, device=dev), torch.empty(n, dh, device=dev)
         conv_state = torch.zeros(batch + 1, taps - 1, 2 * GD + HV, device=dev)
         as_run, walk = _delta_rule_options(n, rl, dh, dd, dev)
+        recur = _delta_recurrence(n, rl, dh, dg, dd, dv, dev, walk)
         row(f"{tag}/delta rule: inputs (convolutions, SiLU, unit norms, step sizes, decays)",
             lambda: ops.delta_prepare(fused, 0, off, dh, dg, dd, dv, taps, *conv, a_log, dt_bias, token_req, rs, rslot, conv_state, 1e-6, dd ** -0.5,
                                       dq, dk, dvv, beta, decay, **as_run), n * ((2 * GD + HV + 2 * dh) * 2 * min(taps, 2) + (2 * GD + HV + 2 * dh) * 4))
@@ -1131,7 +1173,7 @@ def gudarax_kernel_table(size: dict, pk: dict, T: int, batch: int, context: int)
                 lambda: ops.delta_conv_update(fused, 0, off, dh, dg, dd, dv, taps, rs, rl, rslot, conv_state), R * (taps - 1) * (2 * GD + HV) * (2 + 4))
         dstate = torch.zeros(batch + 1, dh, dd, dv, device=dev)
         do = torch.empty(n, HV, device=dev)
-        row(f"{tag}/delta rule: recurrence", lambda: ops.delta_scan(dq, dk, dvv, beta, decay, dstate, do, rs, rl, rslot, dh, dg, dd, dv, **walk),
+        row(f"{tag}/delta rule: recurrence", lambda: recur(dq, dk, dvv, beta, decay, dstate, do, rs, rl, rslot),
             n * (2 * GD + 2 * HV + 2 * dh) * 4 + R * 2 * dh * dd * dv * 4, 6.0 * n * dh * dd * dv)
         gated = torch.empty(n, HV, dtype=bf, device=dev)
         row(f"{tag}/head norm and gate", lambda: ops.head_gate_norm(do, fused, 0, off["g"], nw, 1e-6, gated, dh, dv), n * HV * (4 + 2 + 2))
@@ -1330,12 +1372,12 @@ def fusanex_kernel_table(size: dict, pk: dict, T: int, batch: int, context: int)
         beta, ddecay = torch.empty(n, G, device=dev), torch.empty(n, G, device=dev)
         conv_state = torch.zeros(batch + 1, taps - 1, 3 * HD, device=dev)
         as_run, walk = _delta_rule_options(n, ctx.req_q_len, G, md, dev)
+        recur = _delta_recurrence(n, ctx.req_q_len, G, G, md, md, dev, walk)
         row(f"{tag}/delta rule: inputs (convolutions, SiLU, unit norms, step sizes, decays)",
             lambda: ops.delta_prepare(dfused, 0, off, G, G, md, md, taps, *conv, a_log, dt_bias, ctx.token_req, ctx.req_q_start, ctx.req_slot, conv_state,
                                       1e-6, md ** -0.5, dq, dk, dv, beta, ddecay, **as_run), n * (3 * HD + 2 * G) * (2 + 4))
         dstate, do = torch.zeros(batch + 1, G, md, md, device=dev), torch.empty(n, HD, device=dev)
-        row(f"{tag}/delta rule: recurrence", lambda: ops.delta_scan(dq, dk, dv, beta, ddecay, dstate, do, ctx.req_q_start, ctx.req_q_len, ctx.req_slot, G, G, md, md,
-                                                                                   **walk),
+        row(f"{tag}/delta rule: recurrence", lambda: recur(dq, dk, dv, beta, ddecay, dstate, do, ctx.req_q_start, ctx.req_q_len, ctx.req_slot),
             n * (4 * HD + 2 * G) * 4 + R * 2 * G * md * md * 4, 6.0 * n * G * md * md)
         s = W // blocks
         fused = rnd(n, 2 * W, dtype=bf)
@@ -1396,13 +1438,13 @@ def fusanex_kernel_table(size: dict, pk: dict, T: int, batch: int, context: int)
         ss, sd = torch.empty(R * max_seg * HD * md, device=dev), torch.empty(R * max_seg * HD, device=dev)
         bonus, decay01 = rnd(HD), torch.rand(n, HD, device=dev) * 0.2 + 0.8
         moved = n * 5 * HD * 4 + R * 2 * HD * md * 4
-        row(f"{tag}/decayed state: recurrence (decay per key channel)",
+        row(f"{tag}/decayed state: recurrence, walked (decay per key channel)",
             lambda: ops.linattn_scan(r, k, v, decay01, None, state, o, ctx.req_q_start, ctx.req_q_len, ctx.req_slot, mh, md, md, seg_len, max_seg, ss, sd), moved,
             4.0 * n * HD * md)
         minus = decay01 - 1.0
         row(f"{tag}/time mixing: recurrence with a bonus",
             lambda: ops.linattn_scan(r, k, v, minus, None, state, o, ctx.req_q_start, ctx.req_q_len, ctx.req_slot, mh, md, md, seg_len, max_seg, ss, sd, bonus=bonus),
-            moved, 4.0 * n * HD * md, like=f"{tag}/decayed state: recurrence (decay per key channel)")
+            moved, 4.0 * n * HD * md, like=f"{tag}/decayed state: recurrence, walked (decay per key channel)")
         both = torch.empty(n, nq * hd + HD, dtype=bf, device=dev)
         plain_out = torch.empty(n, HD, dtype=bf, device=dev)
         hw, rw = rnd(md, dtype=bf), rnd(HD, dtype=bf)
@@ -1586,6 +1628,7 @@ def vifirax_kernel_table(size: dict, pk: dict, T: int, batch: int, context: int)
         decay = torch.empty(n, dh, device=dev)
         cstate = torch.zeros(batch + 1, dtaps - 1, 2 * GD + HV, device=dev)
         as_run, walk = _delta_rule_options(n, ctx.req_q_len, dh, dd, dev)
+        recur = _delta_recurrence(n, ctx.req_q_len, dh, dg, dd, dv, dev, walk)
         prep = lambda o_, a_, b_, d_: ops.delta_prepare(fused, 0, o_, dh, dg, dd, dv, dtaps, *conv, a_, b_, ctx.token_req, ctx.req_q_start, ctx.req_slot, cstate, 1e-6,
                                                             dd ** -0.5, dq, dk, dvv, beta, d_, **as_run)
         moved = n * (2 * GD + HV) * (2 + 4)
@@ -1604,8 +1647,8 @@ def vifirax_kernel_table(size: dict, pk: dict, T: int, batch: int, context: int)
         decay.uniform_(0.9, 1.0)
         chan.uniform_(-0.1, 0.0)
         sb, sf = R * 2 * dh * dd * dv * 4, 6.0 * n * dh * dd * dv
-        row(f"{tag}/delta rule: recurrence", lambda: ops.delta_scan(dq, dk, dvv, beta, decay, state, do, *reqs, dh, dg, dd, dv, **walk), n * (2 * GD + 2 * HV + 2 * dh) * 4 + sb, sf)
-        row(f"{tag}/delta rule: recurrence, decays per key channel", lambda: ops.delta_scan(dq, dk, dvv, beta, chan, state, do, *reqs, dh, dg, dd, dv, True, **walk),
+        row(f"{tag}/delta rule: recurrence", lambda: recur(dq, dk, dvv, beta, decay, state, do, *reqs), n * (2 * GD + 2 * HV + 2 * dh) * 4 + sb, sf)
+        row(f"{tag}/delta rule: recurrence, decays per key channel", lambda: recur(dq, dk, dvv, beta, chan, state, do, *reqs, True),
             n * (2 * GD + 2 * HV + dh + dh * dd) * 4 + sb, sf, like=f"{tag}/delta rule: recurrence")
         hw, gated = rnd(dv, dtype=bf), torch.empty(n, HV, dtype=bf, device=dev)
         row(f"{tag}/head norm and SiLU gate", lambda: ops.head_gate_norm(do, gate, 0, 0, hw, 1e-6, gated, dh, dv), n * HV * (4 + 4 + 2))
@@ -1630,20 +1673,20 @@ def vifirax_kernel_table(size: dict, pk: dict, T: int, batch: int, context: int)
         lv = rnd(n, inner)
         seg = (sh, sn, sv, seg_len, max_seg, ss, sd)
         sb, sf = R * 2 * sh * sn * sv * 4, 4.0 * n * sh * sn * sv
-        row(f"{tag}/decayed state: recurrence (decay per key channel)", lambda: ops.linattn_scan(lq, lk, lv, ldec, None, sstate, so, *reqs, *seg),
+        row(f"{tag}/decayed state: recurrence, walked (decay per key channel)", lambda: ops.linattn_scan(lq, lk, lv, ldec, None, sstate, so, *reqs, *seg),
             n * (3 * sh * sn + 2 * inner) * 4 + sb, sf)
         hdec = torch.rand(sh, device=dev) * 0.1 + 0.9
-        row(f"{tag}/decayed state: recurrence (one decay per head)", lambda: ops.linattn_scan(lq, lk, lv, None, hdec, sstate, so, *reqs, *seg),
+        row(f"{tag}/decayed state: recurrence, walked (one decay per head)", lambda: ops.linattn_scan(lq, lk, lv, None, hdec, sstate, so, *reqs, *seg),
             n * (2 * sh * sn + 2 * inner) * 4 + sb, sf)
         xs, bs, cs = xbc[:, :inner], xbc[:, inner:inner + sg * sn], xbc[:, inner + sg * sn:]
         if one:
             xbc16 = xbc.to(bf)
             xs = xbc16[:, :inner]
             row(f"{tag}/state space: recurrence in chunks", lambda: ops.ssd_chunks(xbc16, pairs_, sstate, so, *reqs, sh, sh // sg, sn, sv),
-                n * (C * 2 + inner * 4 + sh * 8) + sb, sf, like=f"{tag}/decayed state: recurrence (one decay per head)")
+                n * (C * 2 + inner * 4 + sh * 8) + sb, sf, like=f"{tag}/decayed state: recurrence, walked (one decay per head)")
         else:
             row(f"{tag}/state space: recurrence", lambda: ops.linattn_scan(cs, bs, xs, None, None, sstate, so, *reqs, *seg, pairs=pairs_, share=sh // sg),
-                n * (C + inner + 2 * sh) * 4 + sb, sf, like=f"{tag}/decayed state: recurrence (one decay per head)")
+                n * (C + inner + 2 * sh) * 4 + sb, sf, like=f"{tag}/decayed state: recurrence, walked (one decay per head)")
         skip, nw, sgated = rnd(sh, dtype=bf), rnd(inner, dtype=bf), torch.empty(n, inner, dtype=bf, device=dev)
         row(f"{tag}/state space: skip, gate, norm in parts", lambda: ops.ssd_gate_norm(so, xs, skip, sfused, 0, 0, nw, 1e-6, sgated, parts),
             n * inner * (4 + (2 if one else 4) + 2 + 2),

@@ -9,6 +9,8 @@ print what it achieved against the roofline.  The same command under `ncu` gives
     python -m wllm_b200.kernels.cases gemm-f32 --m 16 --n 49152 --k 3072
     python -m wllm_b200.kernels.cases attention-f32 --requests 16 --context 6000 --tokens 1 --heads 16 --kv-heads 16
     python -m wllm_b200.kernels.cases recurrence --requests 1 --tokens 2048 --heads 8 --dim 128 --vdim 256
+    python -m wllm_b200.kernels.cases recurrence --chunks --requests 1 --tokens 2048 --heads 8 --dim 128 --vdim 256
+    python -m wllm_b200.kernels.cases recurrence --delta --requests 1 --tokens 2048 --heads 16 --dim 128 --vdim 128
     python -m wllm_b200.kernels.cases experts --tokens 2048 --experts 32 --top 4 --width 2048 --ff 1024
 
 Operands are larger than L2 where the case is bound by memory (several weight copies are cycled), so the
@@ -23,6 +25,7 @@ import math
 import os
 import sys
 
+import numpy as np
 import torch
 
 from . import ops
@@ -210,6 +213,8 @@ def sampling(args) -> None:
 def recurrence(args) -> None:
     """The decayed-state recurrence of linear attention (csrc/linear_attention.cu) over `requests` portions of `tokens`
     tokens each (1: a decode step), decay per key channel or per head."""
+    if args.chunks or args.delta:
+        return recurrence_chunks(args)
     R, T, H, D, V = args.requests, args.tokens, args.heads, args.dim, args.vdim
     n = R * T
     g = torch.Generator(device=DEV).manual_seed(1)
@@ -233,6 +238,34 @@ def recurrence(args) -> None:
     print(f"recurrence requests={R} tokens={T} heads={H} dim={D} vdim={V} segments={max_seg}x{seg_len}: {ms * 1e3:.1f} us, "
           f"{moved / 1e6:.1f} MB that must move ({moved / ms / 1e6:.0f} GB/s, {moved / ms / 1e6 / hbm:.3f} of {src} copy bandwidth), "
           f"{fma / ms / 1e9:.2f} T 32-bit multiply-adds and multiplies a second")
+
+
+def recurrence_chunks(args) -> None:
+    """The same recurrence, or the gated delta rule (`--delta`), in chunks of 64 tokens on the tensor cores (csrc/linear_attention_chunks.cu,
+    csrc/delta_rule_chunks.cu)."""
+    R, T, H, D, V = args.requests, args.tokens, args.heads, args.dim, args.vdim
+    n, g = R * T, torch.Generator(device=DEV).manual_seed(1)
+    rand = lambda *shape: torch.randn(*shape, device=DEV, generator=g)
+    host = np.full(R, T, dtype=np.int32)
+    starts, lens, slots = torch.arange(R, dtype=torch.int32, device=DEV) * T, torch.full((R,), T, dtype=torch.int32, device=DEV), torch.arange(R, dtype=torch.int32, device=DEV)
+    decay = torch.rand(n, H * D, device=DEV, generator=g) * 0.1 + 0.9
+    state, out = torch.zeros(R, H, D, V, device=DEV), torch.empty(n, H * V, device=DEV)
+    if args.delta:
+        unit = lambda x: (x / x.norm(dim=-1, keepdim=True)).view(n, H * D).contiguous()
+        q, k, v, beta = unit(rand(n, H, D)), unit(rand(n, H, D)), rand(n, H * V), torch.rand(n, H, device=DEV, generator=g)
+        per = decay[:, ::D].contiguous() if args.per_head else decay - 1.0
+        room, turns = ops.delta_chunks_plan(host, H)
+        scratch = torch.empty(room, dtype=torch.uint8, device=DEV)
+        ms = timed(lambda: ops.delta_chunks(q, k, v, beta, per, state, out, starts, lens, slots, host, H, H, not args.per_head, scratch), args.iters)
+    else:
+        fused, positions = rand(n, 2 * H * D + H * V).bfloat16(), torch.arange(n, dtype=torch.int32, device=DEV) % T
+        head_decay = torch.full((H,), 0.97, device=DEV)
+        room, turns = ops.linattn_chunks_plan(host, H, D, V)
+        scratch = torch.empty(room, dtype=torch.uint8, device=DEV)
+        ms = timed(lambda: ops.linattn_chunks(fused, 0, H * D, 2 * H * D, H, D, V, positions, None if args.per_head else decay, head_decay, state, out, starts, lens,
+                                              slots, host, scratch, q_scale=D ** -0.5), args.iters)
+    print(f"{'delta rule' if args.delta else 'recurrence'} in chunks requests={R} tokens={T} heads={H} dim={D} vdim={V}: {ms * 1e3:.1f} us, {room / 1e6:.0f} MB of scratch, "
+          f"{turns} turns")
 
 
 def experts(args) -> None:
@@ -313,6 +346,8 @@ def main(argv=None) -> int:
     rc.add_argument("--dim", type=int, default=128)
     rc.add_argument("--vdim", type=int, default=256)
     rc.add_argument("--per-head", action="store_true", help="one decay per head (retention) instead of one per key channel")
+    rc.add_argument("--chunks", action="store_true", help="in chunks of 64 tokens on the tensor cores, as bfloat16 models' long portions go")
+    rc.add_argument("--delta", action="store_true", help="the gated delta rule in such chunks (heads of 128 by 128)")
     rc.add_argument("--no-segments", action="store_true", help="walk every portion in one go")
     ex = sub.add_parser("experts")
     ex.add_argument("--tokens", type=int, default=2048)
