@@ -18,9 +18,11 @@
 // 32-bit numbers are three bfloat16 pieces each (24 bits), and of nine products the six of some weight are taken, large and small ones summed apart.  A chunk's
 // products are summed from zero and join the state in one rounding.
 //
-// Measured, 16 heads, launches back to back, us; behind, the walk in blocks of eight tokens: 2,048 tokens 199 (prepare 86, walk 89, out 36 kernel by kernel) and 277,
-// 8,192 787 and 1,086, 512 62 and 75, 3 x 1,021 318 and 370, 1,531 beside 24 single tokens 192 and 247; a decay per key channel within 2 %.  A chunk costs the same
-// full or not, so that steps of many short requests stay with the blocks: 16 x 130 344 and 251.
+// Measured, 16 heads, captured in a graph, us; behind, the walk in blocks of eight tokens: 2,048 tokens 194 (prepare 87, walk 90, out 38 kernel by kernel under the
+// profiler: profiles/recurrence_chunks_2048.txt) and 274, 8,192 772 and 1,078, 512 59 and 73, 256 47 and 42, 3 x 1,021 310 and 365, 1,531 beside 24 single tokens 187 and 243; a
+// decay per key channel within 2 %.  A chunk costs the same full or not, so that steps of many short requests stay with the blocks: 16 x 130 338 and 248.
+// Distance from 64 bits where models' decays lie (A softplus(a + bias), A of 1 to 16, steps of 1e-3 to 1e-1), a decay per head and per channel: outputs 1.3e-7 and 1.5e-7
+// where the blocks have 1.5e-7 and 1.8e-7, states 0.8e-7 to 1.4e-7 and 1.1e-7 to 1.7e-7; where nearly all is forgotten within two tokens 0.9e-7 for 0.86e-7.
 #include "chunk_common.cuh"
 
 constexpr int DC = 128, DCV = 128;     // key channels and value columns of a head
@@ -342,8 +344,8 @@ __device__ __forceinline__ void delta_chunk_prepare(const float* __restrict__ q,
 }
 
 // grid (2, chunks of the turn, H), 256 threads, two CTAs an SM: one of a (chunk, head)'s queries, one of its keys.  Bound by latency and
-// shared memory (65 % of its throughput): few of a phase's instructions are independent.  86 us for 2,048 tokens of 16 heads (both in one CTA of 512 threads, one an
-// SM: 92).
+// shared memory (64 % of its throughput): few of a phase's instructions are independent.  87 us for 2,048 tokens of 16 heads under the profiler (both in one CTA of 512
+// threads, one an SM: 92).
 template <bool CHANNEL>
 __global__ void __launch_bounds__(DP_THREADS, 2)
 delta_chunk_prepare_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v, const float* __restrict__ beta,
@@ -372,8 +374,8 @@ struct DeltaWalkSmem {
 
 // grid (128 / VT, H, requests), 512 threads.  R: warps w, w + 4, w + 8, w + 12 rows 16 w .., a fourth of the channels each; the state: warps w and w + 8 channels
 // 16 w .., half of the tokens each.  Warps of the same rows hand one another their sums and finish a part of the columns.  Bound by shared memory (72 % of its
-// throughput) and the latency of two products a chunk.  88 us for 2,048 tokens of 16 heads.  (Eight warps the same, 130 with 32 columns a CTA; operands straight to the registers of the one
-// warp that reads them, without the ring, 96.)
+// throughput) and the latency of two products a chunk.  90 us for 2,048 tokens of 16 heads under the profiler.  (In turn: this form 88, eight warps a CTA 89, 32 columns a CTA 130; operands
+// straight to the registers of the one warp that reads them, without the ring, 96.)
 template <bool CHANNEL>
 __global__ void __launch_bounds__(DW_THREADS, 1)
 delta_chunk_walk_kernel(float* __restrict__ state, const int* __restrict__ req_q_len, const int* __restrict__ req_slot, int H, int b0, int turn,
@@ -524,7 +526,7 @@ struct DeltaOutSmem {
 };
 
 // grid (128 / 64, H, chunks of the turn), 256 threads, two CTAs an SM: warp w rows 16 (w & 3) .., columns 32 (w >> 2) ..  Bound by its operands' way from memory:
-// 36 us for 2,048 tokens of 16 heads.  (128 columns and 512 threads, one CTA an SM: 41.)
+// 38 us for 2,048 tokens of 16 heads under the profiler.  (In turn: this form 36, 128 columns and 512 threads, one CTA an SM, 41.)
 __global__ void __launch_bounds__(DO_THREADS, 2)
 delta_chunk_out_kernel(float* __restrict__ out, const int* __restrict__ req_q_start, const int* __restrict__ req_q_len, const int* __restrict__ req_slot,
                        int requests, int H, int b0, int turn, const unsigned char* __restrict__ scratch) {

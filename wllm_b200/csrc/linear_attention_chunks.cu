@@ -56,8 +56,9 @@ struct PrepareSmem {
     float sums[LBLOCKS][D / 64][PAIRS];
 };
 
-// grid (chunks of the turn, H), 256 threads, two CTAs an SM.  Bound by instructions: the sums inside the blocks, A between them, the operands' pieces, a third each.
-// (A between blocks by FMA, a thread a channel inside them: 40 us for 2,048 tokens of 8 heads of 128 x 256 where this form takes 19.)
+// grid (chunks of the turn, H), 256 threads, two CTAs an SM.  Bound by latency: a round of CTAs that issues in 46 % of its cycles and waits for the fused rows,
+// shared memory and the instruction in front by turns (profiles/recurrence_chunks_2048.txt).  (A between blocks by FMA, a thread a channel inside them: 40 us for
+// 2,048 tokens of 8 heads of 128 x 256 where this form takes 21.)
 template <int D, bool PER_CHANNEL>
 __global__ void __launch_bounds__(LC_THREADS, 2)
 linattn_chunk_prepare_kernel(const bf16* __restrict__ fused, int row_stride, int q_off, int k_off, const int* __restrict__ positions,
@@ -690,7 +691,7 @@ static int lc_turn(const int* lens, int requests, int H, int D, int V, long long
     }
 }
 
-// Bytes of scratch that wllm_linattn_chunks asks for: 2.5 MB a chunk of 8 heads of 128 x 256, at most 192 MB (4,992 tokens; longer steps go in turns, the state
+// Bytes of scratch that wllm_linattn_chunks asks for: 2.56 MB a chunk of 8 heads of 128 x 256, at most 192 MB (4,992 tokens; longer steps go in turns, the state
 // handed on through its slot: the same bits) but a chunk of every request that goes in chunks.  lens: the requests' tokens, on the host.  turns: how many with that.
 constexpr long long LC_SCRATCH = 192ll << 20;
 WLLM_API long long wllm_linattn_chunks_bytes(const int* lens, int requests, int H, int D, int V, int* turns) {
@@ -761,9 +762,10 @@ static int launch_chunks(const bf16* fused, int row_stride, int q_off, int k_off
 // turn apart) and scaled.  decay [n, H, D] per key channel, or null with head_decay [H].  D 64 or 128, V in steps of 64.  lens: req_q_len on the host.  Requests
 // of LC_FROM tokens go in chunks, shorter ones token by token.
 // scratch (16-byte aligned): wllm_linattn_chunks_bytes, or less (more turns, the same bits) but a chunk of every request that goes in chunks.  launched: kernels.
-// 8 heads of 128 x 256, launches back to back, us; behind, linattn_prepare and the walk in segments: 2,048 tokens 78 (19 + 29 + 30 kernel by kernel) and 223;
-// 512 33 and 80; 128 32 and 52; 1,531 beside 24 single tokens 87 and 212; 256 beside 47 56 and 145; 16 requests of 130 138 and 151.  Below 128 tokens the host
-// bounds either.
+// 8 heads of 128 x 256, captured in a graph, us; behind, linattn_prepare and the walk in segments.  A decay per head: 2,048 tokens 74 and 205 (21 + 32 + 32 kernel by
+// kernel under the profiler), 512 34 and 70, 130 27 and 36, 1,531 beside 24 single tokens 85 and 204, 16 requests of 130 139 and 143.  A decay per channel and its map
+// (linattn_decay): 2,048 86 and 253, 512 41 and 86, 130 34 and 46, 1,531 beside 24 95 and 244, 16 of 130 145 and 183.  (Products of up to 128 rows leave partial sums,
+// which are not read here.)  Distance from 64 bits, decays near one: outputs 2.3e-7 to 2.6e-7 where the walk has 2.4e-7 to 3.0e-7, states 1.8e-7 to 2.4e-7 and 2.3e-7 to 3.0e-7.
 WLLM_API int wllm_linattn_chunks(const void* fused, int row_stride, int q_off, int k_off, int v_off, const int* positions, const float* inv_freq,
                                  int rot_dim, float q_scale, float k_scale, const float* decay, const float* head_decay, float* state, float* out,
                                  const int* req_q_start, const int* req_q_len, const int* req_slot, const int* lens, int requests, int H, int D, int V,

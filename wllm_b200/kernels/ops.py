@@ -1433,8 +1433,8 @@ def delta_chunks_pay(lens, heads: int) -> int:
     Both ways' us, fitted to B200 measurements with 2 to 64 heads (in brackets blocks and chunks).  Blocks have eight CTAs a request and head, two an SM, each a chain:
     0.133 a token where one has an SM to itself, 0.225 where two share it, and so many SMs for all tokens.  Chunks have a chain of their own, 2.85 a chunk, and cost
     by heads and chunks, full or not; a turn brings every request's states once more, and shorter requests are walked in front
-    of them, not beside.  16 heads: 2,048 tokens [274, 195], 512 [73, 59], 384 [57, 54], 256 [42, 47],
-    1,021 + 680 + 340 [240, 203], 1,531 beside 24 single ones [244, 188], 16 x 512 [865, 850], 4 x 300 [147, 134], 16 x 130 [248, 338], 512 beside 100 of 20
+    of them, not beside.  16 heads: 2,048 tokens [274, 194], 512 [73, 59], 384 [57, 54], 256 [42, 47],
+    1,021 + 680 + 340 [240, 203], 1,531 beside 24 single ones [243, 187], 16 x 512 [864, 846], 4 x 300 [147, 134], 16 x 130 [248, 338], 512 beside 100 of 20
     [433, 1,122].  4 heads: 256 [39, 39], 4 x 300 [48, 52], 16 x 130 [74, 92].  32 heads: 2,048 [458, 388], 512 [121, 108], 1,021 + 680 + 340 [434, 456],
     4 x 300 [259, 269], 16 x 512 [1,856, 1,919].  64 heads: 2,048 [922, 792], 1,021 + 680 + 340 [895, 943], 4 x 300 [507, 549]."""
     room, turns = delta_chunks_plan(lens, heads)
