@@ -41,7 +41,10 @@ def test_only_whole_prompts_do():
 
 
 def test_keys_behind_a_window_are_no_gain():
-    assert _mixer(16, 128, 512, window=64)._expansion_worth(np.array([4096])) < _mixer(16, 128, 512)._expansion_worth(np.array([4096])) / 4
+    from wllm_b200.kernels import ops
+    lens = np.array([4096], dtype=np.int32)
+    worth = lambda window: ops.latent_expand_worth(lens, lens, 16, 128, 512, window)
+    assert worth(64) < worth(0) / 4 and worth(4096) == worth(0) and ops.latent_expand_worth(lens, lens + np.int32(1), 16, 128, 512, 0) == 0
 
 
 @pytest.mark.parametrize("rot", [0, 16])

@@ -707,6 +707,38 @@ WLLM_API long long wllm_delta_chunks_bytes(const int* lens, int requests, int H,
     return chunks * H * DC_SIZE;
 }
 
+// Bytes of scratch where chunks are the faster way for a step of these requests, else 0 (the walk in blocks of eight tokens).  sms: of the device; most: bytes
+// that a step's chunks may take.
+//
+// Both ways' us, fitted to B200 measurements with 2 to 64 heads (in brackets blocks and chunks).  Blocks have eight CTAs a request and head, two an SM, each a chain:
+// 0.133 a token where one has an SM to itself, 0.225 where two share it, and so many SMs for all tokens.  Chunks have a chain of their own, 2.85 a chunk, and cost
+// by heads and chunks, full or not; a turn brings every request's states once more, and shorter requests are walked in front of them, not beside.
+// 16 heads: 2,048 tokens [274, 194], 512 [73, 59], 384 [57, 54], 256 [42, 47], 1,021 + 680 + 340 [240, 203], 1,531 beside 24 single ones [243, 187], 16 x 512
+// [864, 846], 4 x 300 [147, 134], 16 x 130 [248, 338], 512 beside 100 of 20 [433, 1,122].  4 heads: 256 [39, 39], 4 x 300 [48, 52], 16 x 130 [74, 92].  32 heads:
+// 2,048 [458, 388], 512 [121, 108], 1,021 + 680 + 340 [434, 456], 4 x 300 [259, 269], 16 x 512 [1,856, 1,919].  64 heads: 2,048 [922, 792], 1,021 + 680 + 340
+// [895, 943], 4 x 300 [507, 549].
+WLLM_API long long wllm_delta_chunks_pay(const int* lens, int requests, int H, int sms, long long most) {
+    int turns;
+    const long long room = wllm_delta_chunks_bytes(lens, requests, H, &turns);
+    if (room <= 0 || room > most) return 0;
+    int longest = 0;
+    double tokens = 0, chunks = 0, several = 0, few = 0;
+    for (int r = 0; r < requests; ++r) {
+        const int mine = lc_chunks(lens[r]);
+        few += lens[r] > 0 && mine == 0;
+        if (mine == 0) continue;
+        longest = lens[r] > longest ? lens[r] : longest;
+        tokens += lens[r];
+        chunks += mine;
+        several += 1;
+    }
+    const double each = 8.0 * H * several > sms ? 0.225 * ((8 * H + 2 * sms - 1) / (2 * sms)) : 0.133;
+    const double alone = each * longest, all = 0.0069 * H * tokens, in_blocks = 8 + (alone > all ? alone : all);
+    const double chain = 23 + (1.4 * H < 11 ? 1.4 * H : 11) + 2.85 * lc_chunks(longest), work = 20 + 0.36 * H * chunks + 0.07 * H * several * turns;
+    const double in_chunks = (chain > work ? chain : work) + 12.0 * (turns - 1) + 0.015 * H * few;
+    return in_chunks < in_blocks ? room : 0;
+}
+
 // The requests of LC_FROM tokens or more, from and to their state slots; shorter ones are left to wllm_delta_scan.  q, k [n, G, 128], v, out [n, H, 128],
 // beta [n, H], decay [n, H] or (channel) decays less one [n, H, 128], state [slots, H, 128, 128]; lens: req_q_len on the host.
 // scratch (16-byte aligned): wllm_delta_chunks_bytes, or less (more turns, the same bits) but a chunk of every request that goes in chunks.  launched: kernels.

@@ -177,6 +177,32 @@ WLLM_API int wllm_latent_expand(const void* kv, const int* token_req, const int*
                        heads, dim);
 }
 
+// What keys and values of their own save a step of whole prompts of these lengths, over what they cost it, in tokens: 64 where both ways take the same time; 0 where a
+// request has keys in front (ctx_lens: the requests' contexts).  window: keys that a token sees, 0 all of them.
+//
+// Fitted to 300 B200 measurements (4 to 64 heads of 64 to 256, rank 64 to 512, 1 to 17 prompts of 20 to 4,096 tokens).  What falls away goes by the rank: the two maps, the
+// scores and sums over rows of that size, and the longest prompt's chain of key tiles.  What comes goes by the heads' tiles of 128 rows, full or not (256 in heads of
+// steps of 128 and prompts of more rows).  us that way and over the latent rows: 16 heads of 128, rank 512: 1,021 tokens 64 and 152, 64 26 and 33, 16 x 64 54 and 67, 8 x 130
+// 75 and 77, 16 x 20 45 and 41; rank 256: 1,021 62 and 104, 8 x 130 72 and 59, 16 x 130 116 and 87; rank 128: 1,021 61 and 87, 128 31 and 29, 8 x 130 71 and 47; rank 64:
+// 512 50 and 47, 8 x 130 71 and 43; heads of 256, rank 64: 340 + 680 + 1,021 125 and 104; 64 heads, rank 512: 8 x 33 70 and 64, 16 x 200 406 and 603.
+WLLM_API double wllm_latent_expand_worth(const int* lens, const int* ctx_lens, int requests, int heads, int dim, int rank, int window) {
+    int longest = 0;
+    double tokens = 0, seen = 0;
+    for (int r = 0; r < requests; ++r) {
+        if (lens[r] != ctx_lens[r]) return 0;
+        longest = lens[r] > longest ? lens[r] : longest;
+        tokens += lens[r];
+        seen += (double)lens[r] * (window > 0 && window < lens[r] ? window : lens[r]);
+    }
+    const bool large = dim % 128 == 0 && longest > 128;
+    const int rows = large ? 256 : 128;
+    double tiles = 0;
+    for (int r = 0; r < requests; ++r) tiles += (lens[r] + rows - 1) / rows * (rows / 128);
+    const double chain = window > 0 && window < longest ? window : longest;
+    const double saved = rank * (3.4 / 512 + 0.8e-6 * heads * tokens + 7.3e-9 * heads * seen + 11.5e-5 * chain);
+    return 64 * saved / (2.5 + (large ? 7.2 : 0) + (large ? 4.2e-4 : 3.4e-4) * heads * tiles * dim);
+}
+
 // ---------------------------------------------------------------------------------------------------
 // y[t, h, j] = sum_k x[t, h, k] * w[h, j, k]: tiles of 64 tokens by 64 outputs of one head, 16 columns of K a step
 // through shared memory, 4 x 4 outputs a thread, every output one chain over k in ascending order.

@@ -706,6 +706,38 @@ WLLM_API long long wllm_linattn_chunks_bytes(const int* lens, int requests, int 
     return chunks * H * ChunkLayout(D, V).size;
 }
 
+// Bytes of scratch where chunks are the faster way for a step of these requests, else 0.  rank: of the decay's low-rank map, 0 without one; segments: the walk
+// would cut its long requests into segments; most: bytes that a step's chunks may take.
+//
+// Both ways' us, fitted to B200 measurements from 130 to 8,192 tokens (in brackets the walk's and the chunks' for 8 heads of 128 x 256 with a decay per channel).
+// A chunk costs by the bytes that its kernels hand on (2.56 MB of those heads), full or not, a request its state's way; a turn some 45 (2,048 tokens [253, 86],
+// 512 [86, 41], 16 x 130 [183, 145], 130 beside 20 of 20 [74, 99], beside 40 [86, 179], beside 90 [176, 447], 512 beside 20 of 20 [206, 108], beside 90
+// [286, 678: eight turns], 2,048 beside 90 [837, 1,787: thirty-two]).  The walk is bound by its longest request's chain or by all tokens.  Where segments of the
+// long requests fill the device few requests are there, and chunks were the faster way at every size measured (2 to 32 heads).
+WLLM_API long long wllm_linattn_chunks_pay(const int* lens, int requests, int H, int D, int V, int rank, int segments, long long most) {
+    int turns;
+    const long long room = wllm_linattn_chunks_bytes(lens, requests, H, D, V, &turns);
+    if (room <= 0 || room > most) return 0;
+    if (segments) return room;
+    int longest = 0, deepest = 0;
+    double tokens = 0, chunks = 0, several = 0;
+    for (int r = 0; r < requests; ++r) {
+        const int mine = lc_chunks(lens[r]);
+        longest = lens[r] > longest ? lens[r] : longest;
+        deepest = mine > deepest ? mine : deepest;
+        tokens += lens[r];
+        chunks += mine;
+        several += mine > 0;
+    }
+    const double size = (double)H * D * V / (1 << 18), unit = H * (double)ChunkLayout(D, V).size / 2.56e6;
+    const double chain = 1.05 * deepest, work = 2.0 * unit * chunks + 1.6 * size * several;
+    const double in_chunks = 22 + (chain > work ? chain : work) + 45.0 * (turns - 1);
+    const double alone = 8 + (0.25 + 0.05 * size) * longest + 0.025 * size * (tokens - longest), all = 0.07 * size * tokens;
+    double walked = alone > all ? alone : all;
+    if (rank > 0) walked += 5 + (0.006 + 0.014 * H * D * rank / 65536) * tokens;
+    return in_chunks < walked ? room : 0;
+}
+
 template <int D>
 static int launch_chunks(const bf16* fused, int row_stride, int q_off, int k_off, int v_off, const int* positions, const float* inv_freq, int rot_dim,
                          float q_scale, float k_scale, const float* decay, const float* head_decay, float* state, float* out, const int* req_q_start,

@@ -387,6 +387,14 @@ def latent_prepare(fused: torch.Tensor, parts: int, positions: torch.Tensor, slo
 LATENT_PAGE = 64               # tokens of a page that latent_expand lays out
 
 
+def latent_expand_worth(lens, ctx_lens, heads: int, dim: int, rank: int, window: int) -> float:
+    """What every head's own keys and values save a step of whole prompts, over what they cost it, in tokens (csrc/latent_attention.cu); 64 where both ways take the
+    same time, 0 where a request has keys in front.  `lens`, `ctx_lens`: the requests' tokens and contexts (int32 arrays on the host)."""
+    lib = load_family("latent_attention")
+    lib.wllm_latent_expand_worth.restype = ctypes.c_double
+    return lib.wllm_latent_expand_worth(c_void_p(lens.ctypes.data), c_void_p(ctx_lens.ctypes.data), len(lens), heads, dim, rank, window)
+
+
 def latent_expand(kv: torch.Tensor, token_req: torch.Tensor, req_q_start: torch.Tensor, req_q_len: torch.Tensor, keys: torch.Tensor, values: torch.Tensor,
                   table: torch.Tensor, heads: int, dim: int) -> None:
     """The step's keys and values `kv` [n, 2 * heads * dim] (bfloat16; all heads' keys, then their values) into pages `keys`, `values`
@@ -1175,31 +1183,13 @@ def linattn_chunks_bytes(lens, heads: int, dim: int, vdim: int) -> int:
     return linattn_chunks_plan(lens, heads, dim, vdim)[0]
 
 
-LINATTN_CHUNK_MIN = 16         # the shortest requests that linattn_chunks takes in chunks
-
-
-def linattn_chunks_pay(lens, heads: int, dim: int, vdim: int, rank: int) -> int:
-    """Bytes of scratch of linattn_chunks where it is the faster way for a step of these requests (`rank`: of the decay's low-rank map, 0 without one), else 0.
-
-    Both ways' us, fitted to B200 measurements from 130 to 8,192 tokens (in brackets the walk's and the chunks' for 8 heads of 128 x 256 with a decay per channel).
-    A chunk costs by the bytes that its kernels hand on (2.56 MB of those heads), full or not, a request its state's way; a turn some 45 (2,048 tokens [253, 86],
-    512 [86, 41], 16 x 130 [183, 145], 130 beside 20 of 20 [74, 99], beside 40 [86, 179], beside 90 [176, 447], 512 beside 20 of 20 [206, 108], beside 90
-    [286, 678: eight turns], 2,048 beside 90 [837, 1,787: thirty-two]).  The walk is bound by its longest request's chain or by all tokens.  Where segments of the
-    long requests fill the device few requests are there, and chunks were the faster way at every size measured (2 to 32 heads)."""
-    room, turns = linattn_chunks_plan(lens, heads, dim, vdim)
-    if room <= 0 or room > CHUNK_SCRATCH:
-        return 0
-    longest = int(lens.max())
-    if linattn_segment_plan(longest, int((lens > 1).sum()), heads, vdim)[1] > 1:
-        return room
-    chunks = (lens[lens >= LINATTN_CHUNK_MIN] + 63) // 64
-    tokens, size = int(lens.sum()), heads * dim * vdim / 2.0 ** 18
-    unit = heads * (772 * dim + 24576 + 6 * dim * vdim) / 2.56e6
-    in_chunks = 22 + max(1.05 * int(chunks.max()), 2.0 * unit * int(chunks.sum()) + 1.6 * size * len(chunks)) + 45 * (turns - 1)
-    walked = max(8 + (0.25 + 0.05 * size) * longest + 0.025 * size * (tokens - longest), 0.07 * size * tokens)
-    if rank:
-        walked += 5 + (0.006 + 0.014 * heads * dim * rank / 65536) * tokens
-    return room if in_chunks < walked else 0
+def linattn_chunks_pay(lens, heads: int, dim: int, vdim: int, rank: int, longest: int = 0, several: int = -1) -> int:
+    """Bytes of scratch of linattn_chunks where it is the faster way for a step of these requests, else 0 (csrc/linear_attention_chunks.cu has the figures).  `rank`:
+    of the decay's low-rank map, 0 without one; `longest`, `several`: the longest request and how many bring more than one token, where they are known."""
+    segments = linattn_segment_plan(longest or int(lens.max()), several if several >= 0 else int((lens > 1).sum()), heads, vdim)[1] > 1
+    lib = load_family("linear_attention_chunks")
+    lib.wllm_linattn_chunks_pay.restype = ctypes.c_longlong
+    return lib.wllm_linattn_chunks_pay(c_void_p(lens.ctypes.data), len(lens), heads, dim, vdim, rank, segments, ctypes.c_longlong(CHUNK_SCRATCH))
 
 
 def linattn_chunks(fused, q_off: int, k_off: int, v_off: int, heads: int, dim: int, vdim: int, positions: torch.Tensor, decay, head_decay,
@@ -1428,26 +1418,10 @@ def delta_chunks_bytes(lens, heads: int) -> int:
 
 
 def delta_chunks_pay(lens, heads: int) -> int:
-    """Bytes of scratch of delta_chunks where it is the faster way for a step of these requests, else 0 (the walk in blocks of eight tokens).
-
-    Both ways' us, fitted to B200 measurements with 2 to 64 heads (in brackets blocks and chunks).  Blocks have eight CTAs a request and head, two an SM, each a chain:
-    0.133 a token where one has an SM to itself, 0.225 where two share it, and so many SMs for all tokens.  Chunks have a chain of their own, 2.85 a chunk, and cost
-    by heads and chunks, full or not; a turn brings every request's states once more, and shorter requests are walked in front
-    of them, not beside.  16 heads: 2,048 tokens [274, 194], 512 [73, 59], 384 [57, 54], 256 [42, 47],
-    1,021 + 680 + 340 [240, 203], 1,531 beside 24 single ones [243, 187], 16 x 512 [864, 846], 4 x 300 [147, 134], 16 x 130 [248, 338], 512 beside 100 of 20
-    [433, 1,122].  4 heads: 256 [39, 39], 4 x 300 [48, 52], 16 x 130 [74, 92].  32 heads: 2,048 [458, 388], 512 [121, 108], 1,021 + 680 + 340 [434, 456],
-    4 x 300 [259, 269], 16 x 512 [1,856, 1,919].  64 heads: 2,048 [922, 792], 1,021 + 680 + 340 [895, 943], 4 x 300 [507, 549]."""
-    room, turns = delta_chunks_plan(lens, heads)
-    if room <= 0 or room > CHUNK_SCRATCH:
-        return 0
-    long = lens[lens >= DELTA_CHUNK_MIN]
-    chunks = (long + 63) // 64
-    longest, tokens, requests = int(long.max()), int(long.sum()), len(long)
-    shared = 8 * heads * requests > sm_count()
-    in_blocks = 8 + max((0.225 * -(-8 * heads // (2 * sm_count())) if shared else 0.133) * longest, 0.0069 * heads * tokens)
-    few = int(((lens > 0) & (lens < DELTA_CHUNK_MIN)).sum())
-    in_chunks = max(23 + min(11, 1.4 * heads) + 2.85 * int(chunks.max()), 20 + 0.36 * heads * int(chunks.sum()) + 0.07 * heads * requests * turns) + 12 * (turns - 1) + 0.015 * heads * few
-    return room if in_chunks < in_blocks else 0
+    """Bytes of scratch of delta_chunks where it is the faster way for a step of these requests, else 0 (csrc/delta_rule_chunks.cu has the figures)."""
+    lib = load_family("delta_rule_chunks")
+    lib.wllm_delta_chunks_pay.restype = ctypes.c_longlong
+    return lib.wllm_delta_chunks_pay(c_void_p(lens.ctypes.data), len(lens), heads, sm_count(), ctypes.c_longlong(CHUNK_SCRATCH))
 
 
 def delta_chunks(q, k, v, beta, decay, state, out, req_q_start, req_q_len, req_slot, lens, heads: int, kv_heads: int, channel: bool, scratch: torch.Tensor):

@@ -146,7 +146,7 @@ class LatentAttention:
             ops.sigmoid_gate(heads_out, cols, parts, self.gate_col)
         return as_branch(ops.project(heads_out, self.wo, lambda name, shape, dt: ctx.buffer(self.tag + "branch_" + name, shape, dt)))
 
-    # Tokens that a step of whole prompts has, and is worth (_expansion_worth), from where on keys and values of their own are made.  Steps of a model of four layers with one such mixer (16 heads of
+    # Tokens that a step of whole prompts has, and is worth (ops.latent_expand_worth), from where on keys and values of their own are made.  Steps of a model of four layers with one such mixer (16 heads of
     # 128, rank 512; us, that way and over the latent rows): 64 tokens 662 and 690, 128 619 and 692, 512 907 and 945, 1,021 1,006 and 1,092, 2 x 2,048 2,316 and
     # 2,739; 4 tokens 660 and 655 to 709.
     EXPAND_FROM = 64
@@ -162,24 +162,9 @@ class LatentAttention:
             return False
         key = ("latent_expand", self.heads, self.dim, self.rank, self.window)
         if key not in ctx.memo:
-            lens = ctx.host["req_q_len"]
-            ctx.memo[key] = bool((lens == ctx.host["req_ctx_len"]).all()) and self._expansion_worth(lens) >= self.EXPAND_FROM
+            worth = ops.latent_expand_worth(ctx.host["req_q_len"], ctx.host["req_ctx_len"], self.heads, self.dim, self.rank, self.window or 0)
+            ctx.memo[key] = worth >= self.EXPAND_FROM
         return ctx.memo[key]
-
-    def _expansion_worth(self, lens) -> float:
-        """What keys and values of their own save a step of whole prompts of these lengths, over what they cost it, in tokens: 64 where both ways take the same time.
-        Fitted to 300 B200 measurements (4 to 64 heads of 64 to 256, rank 64 to 512, 1 to 17 prompts of 20 to 4,096 tokens).  What falls away goes by the rank: the two maps, the scores and sums over rows of that size, and
-        the longest prompt's chain of key tiles.  What comes goes by the heads' tiles of 128 rows, full or not (256 in heads of steps of 128 and prompts of more
-        rows).  us that way and over the latent rows: 16 heads of 128, rank 512: 1,021 tokens 64 and 152, 64 26 and 33, 16 x 64 54 and 67, 8 x 130 75 and 77, 16 x 20
-        45 and 41; rank 256: 1,021 62 and 104, 8 x 130 72 and 59, 16 x 130 116 and 87; rank 128: 1,021 61 and 87, 128 31 and 29, 8 x 130 71 and 47; rank 64: 512 50
-        and 47, 8 x 130 71 and 43; heads of 256, rank 64: 340 + 680 + 1,021 125 and 104; 64 heads, rank 512: 8 x 33 70 and 64, 16 x 200 406 and 603."""
-        longest = int(lens.max())
-        large = self.dim % 128 == 0 and longest > 128
-        rows = 256 if large else 128
-        tiles = int(((lens + (rows - 1)) // rows).sum()) * (rows // 128)
-        seen = float((lens.astype("float64") * lens.clip(max=self.window or longest)).sum())
-        saved = self.rank * (3.4 / 512 + 0.8e-6 * self.heads * int(lens.sum()) + 7.3e-9 * self.heads * seen + 11.5e-5 * min(longest, self.window or longest))
-        return 64.0 * saved / (2.5 + (7.2 if large else 0.0) + (4.2e-4 if large else 3.4e-4) * self.heads * tiles * self.dim)
 
     def attend_expanded(self, q, rows, out, ctx) -> None:
         n, H, dim, R = rows.shape[0], self.heads, self.dim, ctx.n_requests

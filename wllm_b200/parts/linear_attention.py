@@ -163,7 +163,7 @@ class LinearAttention:
         rank = self.rank if self.decay_kind == "low_rank" else 0
         key = ("linattn_chunks", self.heads, self.dim, self.vdim, rank)
         if key not in ctx.memo:
-            ctx.memo[key] = ops.linattn_chunks_pay(host["req_q_len"], self.heads, self.dim, self.vdim, rank)
+            ctx.memo[key] = ops.linattn_chunks_pay(host["req_q_len"], self.heads, self.dim, self.vdim, rank, ctx.max_q_len, getattr(ctx, "num_multi", -1))
         return ctx.memo[key]
 
     def _walk(self, fused, parts: int, offsets, turn: dict, decay, state, o, ctx, col0: int) -> None:
