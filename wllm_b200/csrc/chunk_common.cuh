@@ -95,3 +95,40 @@ __device__ __forceinline__ float lc_sums(float (&x)[N], int lane) {
     }
     return x[0];
 }
+
+// The chunks that one turn takes of every request, `most` bytes of scratch at hand and `each` a chunk of all heads; in `chunks` how many that are of all requests.
+// lens: the requests' tokens, on the host.
+inline int lc_turn(const int* lens, int requests, long long each, long long most, long long& chunks) {
+    int longest = 0;
+    for (int r = 0; r < requests; ++r) longest = lens[r] > longest ? lens[r] : longest;
+    int turn = lc_chunks(longest);
+    for (;; turn = (turn + 1) / 2) {
+        chunks = 0;
+        for (int r = 0; r < requests; ++r) {
+            const int mine = lc_chunks(lens[r]);
+            chunks += mine < turn ? mine : turn;
+        }
+        if (turn <= 1 || (chunks * each <= most && chunks <= 65535)) return turn;
+    }
+}
+// Bytes that a step's chunks ask for, at most LC_SCRATCH but a chunk of every request that goes in chunks, and the turns with them.
+constexpr long long LC_SCRATCH = 192ll << 20;
+inline long long lc_bytes(const int* lens, int requests, long long each, int& turns) {
+    long long chunks;
+    const int turn = lc_turn(lens, requests, each, LC_SCRATCH, chunks);
+    turns = 0;
+    for (int r = 0; r < requests; ++r) {
+        const int mine = turn > 0 ? (lc_chunks(lens[r]) + turn - 1) / turn : 0;
+        turns = mine > turns ? mine : turns;
+    }
+    return chunks * each;
+}
+// Chunks of a turn from chunk b0 on.
+inline int lc_count(const int* lens, int requests, int b0, int turn) {
+    int count = 0;
+    for (int r = 0; r < requests; ++r) {
+        const int mine = lc_chunks(lens[r]) - b0;
+        count += mine < 0 ? 0 : (mine < turn ? mine : turn);
+    }
+    return count;
+}

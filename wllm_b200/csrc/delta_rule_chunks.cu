@@ -677,34 +677,12 @@ delta_chunk_out_kernel(float* __restrict__ out, const int* __restrict__ req_q_st
     }
 }
 
-// The chunks that one turn takes of every request, `most` bytes of scratch at hand, and in `chunks` how many that are of all requests.
-static int dc_turn(const int* lens, int requests, int H, long long most, long long& chunks) {
-    int longest = 0;
-    for (int r = 0; r < requests; ++r) longest = lens[r] > longest ? lens[r] : longest;
-    int turn = lc_chunks(longest);
-    for (;; turn = (turn + 1) / 2) {
-        chunks = 0;
-        for (int r = 0; r < requests; ++r) {
-            const int mine = lc_chunks(lens[r]);
-            chunks += mine < turn ? mine : turn;
-        }
-        if (turn <= 1 || (chunks * H * DC_SIZE <= most && chunks <= 65535)) return turn;
-    }
-}
-
 // Bytes of scratch that wllm_delta_chunks asks for: 5.6 MB a chunk of 16 heads, at most 192 MB (longer steps go in turns, the state handed on through its slot:
 // the same bits) but a chunk of every request that goes in chunks.  lens: the requests' tokens, on the host.  turns: how many with that.
-constexpr long long DC_SCRATCH = 192ll << 20;
 WLLM_API long long wllm_delta_chunks_bytes(const int* lens, int requests, int H, int* turns) {
     *turns = 0;
     if (H <= 0 || H > 65535 || requests <= 0) return 0;
-    long long chunks;
-    const int turn = dc_turn(lens, requests, H, DC_SCRATCH, chunks);
-    for (int r = 0; r < requests; ++r) {
-        const int mine = turn > 0 ? (lc_chunks(lens[r]) + turn - 1) / turn : 0;
-        *turns = mine > *turns ? mine : *turns;
-    }
-    return chunks * H * DC_SIZE;
+    return lc_bytes(lens, requests, H * DC_SIZE, *turns);
 }
 
 // Bytes of scratch where chunks are the faster way for a step of these requests, else 0 (the walk in blocks of eight tokens).  sms: of the device; most: bytes
@@ -750,7 +728,7 @@ WLLM_API int wllm_delta_chunks(const float* q, const float* k, const float* v, c
     if (H <= 0 || H > 65535 || G <= 0 || H % G != 0 || requests > 65535) return WLLM_BAD_SIZE;
     if ((((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)scratch) & 15) || (((uintptr_t)decay | (uintptr_t)state | (uintptr_t)out) & 7)) return WLLM_BAD_ALIGN;
     long long all;
-    const int turn = dc_turn(lens, requests, H, scratch_bytes, all);
+    const int turn = lc_turn(lens, requests, H * DC_SIZE, scratch_bytes, all);
     if (all > 65535 || all * H * DC_SIZE > scratch_bytes) return WLLM_BAD_SIZE;
     static bool raised = false;
     if (!raised) {
@@ -769,11 +747,7 @@ WLLM_API int wllm_delta_chunks(const float* q, const float* k, const float* v, c
     for (int r = 0; r < requests; ++r) longest = lens[r] > longest ? lens[r] : longest;
     unsigned char* room = (unsigned char*)scratch;
     for (int b0 = 0; b0 < lc_chunks(longest); b0 += turn) {
-        int count = 0;
-        for (int r = 0; r < requests; ++r) {
-            const int mine = lc_chunks(lens[r]) - b0;
-            count += mine < 0 ? 0 : (mine < turn ? mine : turn);
-        }
+        const int count = lc_count(lens, requests, b0, turn);
 #define PREPARE(C) wllm_launch(delta_chunk_prepare_kernel<C>, dim3(2, count, H), DP_THREADS, sizeof(DeltaPrepareSmem), stream, q, k, v, beta, decay, req_q_start, \
         req_q_len, req_slot, requests, H, G, b0, turn, room)
 #define WALK(C) wllm_launch(delta_chunk_walk_kernel<C>, dim3(DCV / VT, H, requests), DW_THREADS, sizeof(DeltaWalkSmem), stream, state, req_q_len, req_slot, \

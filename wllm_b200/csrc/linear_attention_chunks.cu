@@ -675,35 +675,12 @@ linattn_short_kernel(const bf16* __restrict__ fused, int row_stride, int q_off, 
 // Sizes that the chunked form is built for.
 static bool lc_sizes(int H, int D, int V) { return H > 0 && H <= 65535 && (D == 64 || D == 128) && V > 0 && V % 64 == 0; }
 
-// The chunks that one turn takes of every request, `most` bytes of scratch at hand, and in `chunks` how many that are of all requests.
-static int lc_turn(const int* lens, int requests, int H, int D, int V, long long most, long long& chunks) {
-    const long long each = (long long)H * ChunkLayout(D, V).size;
-    int longest = 0;
-    for (int r = 0; r < requests; ++r) longest = lens[r] > longest ? lens[r] : longest;
-    int turn = lc_chunks(longest);
-    for (;; turn = (turn + 1) / 2) {
-        chunks = 0;
-        for (int r = 0; r < requests; ++r) {
-            const int mine = lc_chunks(lens[r]);
-            chunks += mine < turn ? mine : turn;
-        }
-        if (turn <= 1 || (chunks * each <= most && chunks <= 65535)) return turn;
-    }
-}
-
 // Bytes of scratch that wllm_linattn_chunks asks for: 2.56 MB a chunk of 8 heads of 128 x 256, at most 192 MB (4,992 tokens; longer steps go in turns, the state
 // handed on through its slot: the same bits) but a chunk of every request that goes in chunks.  lens: the requests' tokens, on the host.  turns: how many with that.
-constexpr long long LC_SCRATCH = 192ll << 20;
 WLLM_API long long wllm_linattn_chunks_bytes(const int* lens, int requests, int H, int D, int V, int* turns) {
     *turns = 0;
     if (!lc_sizes(H, D, V) || requests <= 0) return 0;
-    long long chunks;
-    const int turn = lc_turn(lens, requests, H, D, V, LC_SCRATCH, chunks);
-    for (int r = 0; r < requests; ++r) {
-        const int mine = turn > 0 ? (lc_chunks(lens[r]) + turn - 1) / turn : 0;
-        *turns = mine > *turns ? mine : *turns;
-    }
-    return chunks * H * ChunkLayout(D, V).size;
+    return lc_bytes(lens, requests, H * ChunkLayout(D, V).size, *turns);
 }
 
 // Bytes of scratch where chunks are the faster way for a step of these requests, else 0.  rank: of the decay's low-rank map, 0 without one; segments: the walk
@@ -768,11 +745,7 @@ static int launch_chunks(const bf16* fused, int row_stride, int q_off, int k_off
         *launched += 1;
     }
     for (int b0 = 0; b0 < lc_chunks(longest); b0 += turn) {
-        int count = 0;
-        for (int r = 0; r < requests; ++r) {
-            const int mine = lc_chunks(lens[r]) - b0;
-            count += mine < 0 ? 0 : (mine < turn ? mine : turn);
-        }
+        const int count = lc_count(lens, requests, b0, turn);
 #define PREPARE(C) wllm_launch(linattn_chunk_prepare_kernel<D, C>, dim3(count, H), LC_THREADS, sizeof(PrepareSmem<D>), stream, fused, row_stride, q_off, k_off, \
         positions, inv_freq, rot_dim, q_scale, k_scale, decay, head_decay, req_q_start, req_q_len, req_slot, requests, H, V, b0, turn, scratch)
         int st = decay ? PREPARE(true) : PREPARE(false);
@@ -807,7 +780,7 @@ WLLM_API int wllm_linattn_chunks(const void* fused, int row_stride, int q_off, i
     if (!lc_sizes(H, D, V) || requests > 65535 || rot_dim < 0 || rot_dim > D || rot_dim % 16 != 0 || (!decay && !head_decay)) return WLLM_BAD_SIZE;
     if (((row_stride | q_off | k_off | v_off) & 7) || (((uintptr_t)fused | (uintptr_t)scratch) & 15) || (((uintptr_t)state | (uintptr_t)out) & 7)) return WLLM_BAD_ALIGN;
     long long chunks;
-    const int turn = lc_turn(lens, requests, H, D, V, scratch_bytes, chunks);
+    const int turn = lc_turn(lens, requests, H * ChunkLayout(D, V).size, scratch_bytes, chunks);
     if (chunks > 65535 || chunks * H * ChunkLayout(D, V).size > scratch_bytes) return WLLM_BAD_SIZE;
 #define CHUNKS(DD) launch_chunks<DD>((const bf16*)fused, row_stride, q_off, k_off, v_off, positions, inv_freq, rot_dim, q_scale, k_scale, decay, head_decay, \
         state, out, req_q_start, req_q_len, req_slot, lens, requests, H, V, (unsigned char*)scratch, turn, launched, stream)
